@@ -23,6 +23,9 @@ extern "C" int yalm_gemm_glu_f16(void *h, int ldh, const void *a, const void *w1
 namespace yalm {
 namespace prefill {
 
+// prefill_gemm.cu: the three projections as one launch
+int gemm_qkv_f16(float *c, int ldc, const void *a, const void *wq, const void *wk, const void *wv, int M, int q_dim, int kv_dim, int K, cudaStream_t st);
+
 // x[i, :] = float(E[tokens[i], :])   (src/infer.cu:632-640, for a batch of rows)
 __global__ void embed_rows_kernel(float *__restrict__ x, const __half *__restrict__ table, const int *__restrict__ tokens, int dim) {
 	const __half *row = table + (size_t)tokens[blockIdx.x] * dim;
@@ -317,11 +320,9 @@ int Model::forward_batch(InferenceState &s, const int *tokens, int n, int pos0, 
 	for (auto &bp : blocks) {
 		const Block &b = *bp;
 		rmsnorm_rows_kernel<<<n, 256, 0, st>>>(P.xb, P.x, b._rms_att_weight, dim, c.norm_eps);
-		// q | k | v of the chunk: three GEMMs into one (n, q_dim + 2 kv_dim) fp32 buffer
+		// q | k | v of the chunk into one (n, q_dim + 2 kv_dim) fp32 buffer
 		const int ld = q_dim + 2 * kv_dim;
-		if ((rc = yalm_gemm_f16(P.qkv, ld, P.xb, b._wq, n, q_dim, dim, 0, st))) return rc;
-		if ((rc = yalm_gemm_f16(P.qkv + q_dim, ld, P.xb, b._wk, n, kv_dim, dim, 0, st))) return rc;
-		if ((rc = yalm_gemm_f16(P.qkv + q_dim + kv_dim, ld, P.xb, b._wv, n, kv_dim, dim, 0, st))) return rc;
+		if ((rc = gemm_qkv_f16(P.qkv, ld, P.xb, b._wq, b._wk, b._wv, n, q_dim, kv_dim, dim, st))) return rc;
 		rope_append_rows_kernel<<<n, 256, 0, st>>>(P.q16, reinterpret_cast<__half *>(b._key_cache), reinterpret_cast<__half *>(b._value_cache),
 		                                          P.qkv, q_dim, kv_dim, c.head_dim, c.rotary_dim, c.max_seq_len, pos0, c.rope_theta, c.qkv_clip);
 		if ((rc = yalm_attn_prefill(P.att, P.q16, b._key_cache, b._value_cache, n, pos0, c.n_heads, c.n_kv_heads, c.head_dim, c.max_seq_len, st)))

@@ -1,35 +1,47 @@
-// Dense fp16 GEMM on the 5th-generation tensor cores for the batched prefill / perplexity path.
+// Dense fp16 / bf16 GEMM on the 5th-generation tensor cores for the batched prefill / perplexity path.
 //
 // The reference has no batched pass at all: it hydrates the KV cache and scores a text one token at a time, every token a
-// full sweep over the weights (src/main.cpp:91-97, 174-184).  With M >= 128 positions in flight the projections ARE
-// GEMMs, C[M, N] = A[M, K] * W[N, K]^T — W exactly as the .yalm file stores it ((out, in) row-major = K-major "B") — and
+// full sweep over the weights (src/main.cpp:91-97, 174-184).  With many positions in flight the projections ARE
+// GEMMs, C[M, N] = A[M, K] * W[N, K]^T - W exactly as the .yalm file stores it ((out, in) row-major = K-major "B") - and
 // this is the one place in the project where tensor cores are the right tool.
 //
-// One CTA per 128 x 128 output tile (128 x 256 accumulator columns for the fused w1 | w3 tile), 192 threads:
-//   warp 0      TMA producer: cp.async.bulk.tensor.2d of a 128-row x 64-column fp16 box of A and of W per pipeline stage
-//               (SWIZZLE_128B tensor maps; rows / columns past the edge are zero-filled by the TMA unit), mbarrier
-//               complete_tx completion
-//   warp 1      one elected thread issues tcgen05.mma.cta_group::1.kind::f16 (M 128, N 128 | 256, K 16) straight out of
-//               shared memory (K-major SWIZZLE_128B descriptors), fp32 accumulator in TMEM; tcgen05.commit hands each
-//               stage back to the producer and finally the accumulator to the epilogue.  Also owns the TMEM allocation.
-//   warps 2-5   epilogue: tcgen05.ld (32 lanes x 32 columns per instruction) -> registers -> fused tail -> global:
-//               plain fp32 store (q | k | v, logits), fp32 residual add in place (wo, w2: x += ...), or
-//               act(w1 x) * (w3 x) -> fp16 (the A operand of the w2 GEMM).
+// Two kernels, 192 threads a CTA and the same roles: warp 0 brings 64-column (128-byte, SWIZZLE_128B) boxes of both operands
+// with cp.async.bulk.tensor.2d into a ring of pipeline stages (mbarrier complete_tx; rows / columns past the edge are
+// zero-filled), one thread of warp 1 issues tcgen05.mma.kind::f16 out of shared memory into a fp32 accumulator in TMEM,
+// warps 2-5 read it back (tcgen05.ld) and run the fused tail: plain fp32 store (q | k | v, logits), fp32 residual add in place
+// (wo, w2: x += ...), or act(w1 x) * (w3 x) -> fp16 (the A operand of the w2 GEMM).
+//
+//  * gemm_pair_kernel (many rows): a pair of CTAs (cta_group::2) owns a tile of 256 rows x n columns, each CTA staging 128 rows of A
+//    and half of the columns of W: twice the products per staged byte of one CTA per 128 x 128 tile.  Persistent over tiles, the
+//    accumulator double-buffered so that a tile's tail runs under the next tile's products.  n and the number of K parts are
+//    picked per shape (plan_pair).  Bound by the tensor pipe at the clock that the power limit leaves.
+//    512 rows, cold L2, against one CTA per 128 x 128 tile: 4096 x 14336 88 -> 65 us (919 TFLOP/s), w1 | w3 14336 x 4096 158 -> 109 us
+//    (1108), 32000 x 4096 242 -> 117 us (1150), q | k | v 74 -> 41 us, 4096 x 4096 41 -> 35 us.
+//  * gemm_few_kernel (few rows): bound by the bytes of W.  W is the 128-row operand, the positions are the N of the
+//    instruction (16 .. 128), so a stage is W bytes and little else; K is split over a cluster of CTAs until the GPU is full.
+//    17 rows, cold L2, against the 128 x 128 tiles: 4096 x 4096 35 -> 18 us, 4096 x 14336 80 -> 36 us, w1 | w3 82 -> 59 us, 32000 x 4096 84 -> 63 us.
+//
+// K parts of a tile are summed through distributed shared memory in a fixed order: each CTA of the cluster finishes its share
+// of the columns, so results do not depend on timing and no workspace is needed.
 // Activations enter as fp16 (rmsnorm / attention / GLU outputs are rounded once, like the KV cache); sums are fp32.
 #include "common.cuh"
 
 #include <cuda.h> // CUtensorMap + enums only: cuTensorMapEncodeTiled is resolved at run time (cudaGetDriverEntryPoint)
 
+#include <algorithm>
 #include <mutex>
 
 #include "gemv.cuh"
+#include "launch.h"
+#include "tcgen.cuh"
 
 namespace yalm {
 namespace prefill {
 
-constexpr int BM = 128, BN = 128, BK = 64; // BK fp16 = 128 bytes = one SWIZZLE_128B row
+constexpr int BK = 64;            // 64 16-bit elements = 128 bytes = one SWIZZLE_128B row
+constexpr int kRowBytes = 2 * BK; // of an operand row in a stage
 constexpr int kGemmThreads = 192;
-constexpr int kTileBytes = BM * BK * 2;    // 16 KB: one 128-row operand box
+constexpr int kSegments = 8;
 
 enum Tail { kStoreF32 = 0, kAddF32 = 1, kGluF16 = 2 };
 
@@ -41,116 +53,327 @@ struct GemmArgs {
 	int ldc;
 	float alpha; // kStoreF32 / kAddF32: the product is scaled before it is stored / added
 	int bf16;    // operands are bf16 instead of fp16 (same instruction kind, other format bits and tensor-map type)
-	int nseg;    // > 0: output columns [seg_end[s - 1], seg_end[s]) multiply rows s M .. s M + M - 1 of A (one input per segment)
-	int seg_end[8];
+	int nseg;    // output columns [seg_end[s - 1], seg_end[s]) are segment s; tiles never straddle two segments
+	int seg_end[kSegments];
+	int a_step;  // segment s multiplies rows s a_step .. s a_step + M - 1 of the A operand (0: the same rows for all)
+	int n_tile;  // columns of a tile (per matrix)
+	int m_tiles, items, splits, kb_per; // 256-row tiles, tiles in all, K parts of a tile and their length in 64-wide blocks
+	int stages;
 };
 
-// ---- PTX ---------------------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t s32(const void *p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-	asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-	asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity) {
-	uint32_t ok = 0;
-	const long long t0 = clock64();
-	while (!ok) {
-		asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-		             : "=r"(ok)
-		             : "r"(bar), "r"(parity)
-		             : "memory");
-		if (!ok && clock64() - t0 > 4000000000ll) __trap(); // ~2 s: a bug, never a hang
-	}
-}
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int c0, int c1, uint32_t bar) {
-	asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-	             "l"(map), "r"(c0), "r"(c1), "r"(bar)
-	             : "memory");
-}
-__device__ __forceinline__ void tmem_alloc(uint32_t slot, uint32_t cols) {
-	asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(cols) : "memory");
-	asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc(uint32_t addr, uint32_t cols) {
-	asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(cols) : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-// D[tmem] (+)= A[smem] * B[smem]^T, one 128 x N x 16 fp16 step
-__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-	asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-	             "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-	             : "memory");
-}
-// arrive on `bar` once every tcgen05.mma issued so far by this thread has completed (implies fence::before_thread_sync)
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-	asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-// 32 lanes x 32 consecutive fp32 columns of the accumulator -> 32 registers per thread (thread = TMEM lane = tile row)
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
-	uint32_t r[32];
-	asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-	             "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-	             "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-	             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-	               "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
-	               "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
-	               "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-	             : "r"(taddr)
-	             : "memory");
-	asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+// One tensor map per weight matrix: the segments' own matrices (wq, wk, wv), or w1 and w3, or one W.
+struct WeightMaps {
+	CUtensorMap m[3];
+};
+
+// ---- tails ------------------------------------------------------------------------------------------------------------
+constexpr int kPatch = 32 * 36 * 4; // bytes of one warp's staging patch: 32 rows of 32 fp32, padded to 36
+
+// A warp's 32 rows x 32 columns: lane = row holds v.  Through the warp's patch of shared memory, so that 8 lanes store (and for the
+// residual read) 128 consecutive bytes of a row: straight from the lanes every 16-byte piece would be half a sector of its own.
+__device__ __forceinline__ void store_patch_f32(const GemmArgs &g, uint32_t patch, const float (&v)[32], int row0, int col, int col_end) {
+	const int lane = threadIdx.x & 31, r0 = lane >> 3, cc = (lane & 7) * 4;
+	__syncwarp();
 #pragma unroll
-	for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-}
-
-// Shared-memory matrix descriptor of a K-major operand tile in the canonical SWIZZLE_128B layout the TMA box lands in:
-// rows of 128 bytes, 8-row groups 1024 bytes apart (stride byte offset), version 1 (sm_100), layout type 2 (128B swizzle).
-// Fields (cute/arch/mma_sm100_desc.hpp: SmemDescriptor): [0,14) address >> 4, [16,30) leading byte offset >> 4 (1: unused
-// for swizzled K-major), [32,46) stride byte offset >> 4, [46,48) version, [61,64) layout type.
-__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr) {
-	return (uint64_t)((addr & 0x3FFFF) >> 4) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
-}
-// Instruction descriptor (InstrDescriptor): fp32 accumulator [4,6) = 1, A / B format fp16 = 0, both K-major, N >> 3 at
-// [17,23), M >> 4 at [24,29).
-__host__ __device__ constexpr uint32_t instr_desc_f16(int M, int N) {
-	return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
-}
-// A format at [7,10) and B format at [10,13): 0 = fp16, 1 = bf16 (both operands the same type here)
-constexpr uint32_t kInstrDescBf16 = (1u << 7) | (1u << 10);
-
-// NB = 1: one W matrix, accumulator 128 x 128.  NB = 2: w1 | w3 tiles side by side, accumulator 128 x 256, GLU tail.
-template <int NB>
-__global__ void __launch_bounds__(kGemmThreads, 1)
-gemm_f16_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, const __grid_constant__ CUtensorMap tb2, const GemmArgs g) {
-	constexpr int kStage = kTileBytes * (1 + NB);
-	constexpr int kStages = NB == 1 ? 6 : 4;
-	constexpr int NACC = BN * NB; // accumulator columns (fp32) = UMMA N
-	extern __shared__ uint8_t smem_raw[];
-	const uint32_t base = (s32(smem_raw) + 1023u) & ~1023u; // the swizzle pattern repeats every 1024 bytes
-	const uint32_t bars = base + kStages * kStage;           // full[kStages] | empty[kStages] | accumulator ready | TMEM address
-	const uint32_t full0 = bars, empty0 = bars + 8 * kStages, acc_bar = bars + 16 * kStages, tslot = acc_bar + 8;
-	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-	const int m0 = blockIdx.x * BM;
-	int n0 = blockIdx.y * BN, a0 = m0, n_end = g.N;
-	if (g.nseg > 0) { // tiles never straddle two segments
-		int t = blockIdx.y, start = 0, s = 0;
-		for (; s < g.nseg - 1; ++s) {
-			const int tiles = (g.seg_end[s] - start + BN - 1) / BN;
-			if (t < tiles) break;
-			t -= tiles, start = g.seg_end[s];
+	for (int i = 0; i < 32; i += 4) st_shared4(patch + (lane * 36 + i) * 4, make_float4(g.alpha * v[i], g.alpha * v[i + 1], g.alpha * v[i + 2], g.alpha * v[i + 3]));
+	__syncwarp();
+	const int c0 = col + cc;
+	float *base = g.c + (size_t)(row0 + r0) * g.ldc + c0;
+	if (c0 + 4 <= col_end) {
+		float4 x[8];
+		if (g.tail == kAddF32) { // x += W v (src/infer.cpp:335-337), residual stream stays fp32
+#pragma unroll
+			for (int t = 0; t < 8; ++t)
+				if (row0 + r0 + 4 * t < g.M) x[t] = *reinterpret_cast<const float4 *>(base + (size_t)(4 * t) * g.ldc);
 		}
-		n0 = start + t * BN, n_end = g.seg_end[s], a0 = s * g.M + m0;
+#pragma unroll
+		for (int t = 0; t < 8; ++t) {
+			if (row0 + r0 + 4 * t >= g.M) continue;
+			float4 o = ld_shared4(patch + ((r0 + 4 * t) * 36 + cc) * 4);
+			if (g.tail == kAddF32) o.x += x[t].x, o.y += x[t].y, o.z += x[t].z, o.w += x[t].w;
+			*reinterpret_cast<float4 *>(base + (size_t)(4 * t) * g.ldc) = o;
+		}
+	} else if (c0 < col_end) {
+		for (int t = 0; t < 8; ++t) {
+			if (row0 + r0 + 4 * t >= g.M) continue;
+			const float4 o = ld_shared4(patch + ((r0 + 4 * t) * 36 + cc) * 4);
+			const float oo[4] = {o.x, o.y, o.z, o.w};
+			float *dst = base + (size_t)(4 * t) * g.ldc;
+			for (int j = 0; j < 4 && c0 + j < col_end; ++j) dst[j] = g.tail == kAddF32 ? dst[j] + oo[j] : oo[j];
+		}
 	}
-	const int nkb = (g.K + BK - 1) / BK;
+}
+__device__ __forceinline__ uint32_t pack_half2(float a, float b) {
+	const __half2 h = __floats2half2_rn(a, b);
+	return *reinterpret_cast<const uint32_t *>(&h);
+}
+// The same for fp16 results: 4 lanes store the 64 bytes of a row.
+__device__ __forceinline__ void store_patch_f16(const GemmArgs &g, uint32_t patch, const float (&v)[32], int row0, int col, int col_end) {
+	const int lane = threadIdx.x & 31, r0 = lane >> 2, cc = (lane & 3) * 8;
+	__syncwarp();
+#pragma unroll
+	for (int i = 0; i < 32; i += 8)
+		st_shared4(patch + (lane * 20 + i / 2) * 4, make_float4(__uint_as_float(pack_half2(v[i], v[i + 1])), __uint_as_float(pack_half2(v[i + 2], v[i + 3])),
+		                                                        __uint_as_float(pack_half2(v[i + 4], v[i + 5])), __uint_as_float(pack_half2(v[i + 6], v[i + 7]))));
+	__syncwarp();
+	const int c0 = col + cc;
+	for (int t = 0; t < 4; ++t) {
+		const int row = row0 + r0 + 8 * t;
+		if (row >= g.M || c0 >= col_end) continue;
+		const float4 o = ld_shared4(patch + ((r0 + 8 * t) * 20 + cc / 2) * 4);
+		__half *dst = g.h + (size_t)row * g.ldc + c0;
+		if (c0 + 8 <= col_end) {
+			*reinterpret_cast<float4 *>(dst) = o;
+		} else {
+			const uint32_t w[4] = {__float_as_uint(o.x), __float_as_uint(o.y), __float_as_uint(o.z), __float_as_uint(o.w)};
+			for (int j = 0; j < 8 && c0 + j < col_end; ++j) {
+				const __half2 p = *reinterpret_cast<const __half2 *>(&w[j >> 1]);
+				dst[j] = (j & 1) ? __high2half(p) : __low2half(p);
+			}
+		}
+	}
+}
+// act(a) u, rounded to fp16 by the caller.  Both activations as a / (1 + exp(-b)) (0.5 (1 + tanh(y)) = 1 / (1 + exp(-2 y))), the
+// quotient by __fdividef: its 2 ulp vanish in the fp16 rounding, and the branch-free form lets a thread's values overlap, where
+// the IEEE quotient's and tanhf's branches ran one after another (13 us for a 128 x 128 tile's tail, as long as 8 K blocks).
+__device__ __forceinline__ float glu(const GemmArgs &g, float a, float u) {
+	const float b = g.act == YALM_ACT_GELU ? 2.0f * 0.797885f * (a + 0.044715f * (a * a * a)) : a;
+	return __fdividef(a, 1.0f + expf(-b)) * u;
+}
+constexpr float kNaN = __builtin_nanf("");
+
+// Column tile t of the output: its segment, first column and the segment's end.
+__device__ __forceinline__ void tile_columns(const GemmArgs &g, int t, int &seg, int &seg0, int &n0, int &n_end) {
+	seg = 0, seg0 = 0;
+	for (; seg < g.nseg - 1; ++seg) {
+		const int tiles = (g.seg_end[seg] - seg0 + g.n_tile - 1) / g.n_tile;
+		if (t < tiles) break;
+		t -= tiles, seg0 = g.seg_end[seg];
+	}
+	n0 = seg0 + t * g.n_tile, n_end = min(g.seg_end[seg], n0 + g.n_tile);
+}
+
+// Shared memory, from a 1024-byte boundary (the swizzle pattern repeats every 1024 bytes): the stages, the tail warps' patches
+// (pair kernel), the barriers.
+constexpr int kTailBytes = 4 * kPatch + 512;
+
+// GLU: w1 | w3 tiles side by side, the pair's first CTA staging w1's rows and the second w3's; accumulator columns n .. 2 n - 1 are w3's.
+// B_SEG: every segment has a weight matrix of its own.
+template <bool GLU, bool B_SEG>
+__global__ void __launch_bounds__(kGemmThreads, 1)
+gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ WeightMaps tb, const __grid_constant__ GemmArgs g) {
+	extern __shared__ uint8_t smem_raw[];
+	const int nacc = GLU ? 2 * g.n_tile : g.n_tile; // accumulator columns = N of the instruction; each CTA stages half of them
+	const uint32_t a_bytes = 128 * kRowBytes, b_bytes = (uint32_t)(nacc / 2) * kRowBytes, stage_bytes = a_bytes + b_bytes;
+	const uint32_t base = (s32(smem_raw) + 1023u) & ~1023u, patch0 = base + g.stages * stage_bytes, bars = patch0 + 4 * kPatch;
+	const uint32_t full0 = bars, empty0 = bars + 8 * g.stages, acc_full0 = empty0 + 8 * g.stages, acc_empty0 = acc_full0 + 16, tslot = acc_empty0 + 16;
+	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+	const int rank = (int)cluster_rank(), half = rank & 1, part = rank >> 1; // CTA of its pair; the pair's part of K
+	const int csize = 2 * g.splits, cluster = blockIdx.x / csize, nclusters = gridDim.x / csize;
+	const int nkb = (g.K + BK - 1) / BK, kb0 = part * g.kb_per, kb1 = min(nkb, kb0 + g.kb_per);
+	bool dead = false;
 
 	if (threadIdx.x == 0) {
-		for (int i = 0; i < kStages; ++i) mbar_init(full0 + 8 * i, 1), mbar_init(empty0 + 8 * i, 1);
+		for (int i = 0; i < g.stages; ++i) mbar_init(full0 + 8 * i, 1), mbar_init(empty0 + 8 * i, 1);
+		for (int i = 0; i < 2; ++i) mbar_init(acc_full0 + 8 * i, 1), mbar_init(acc_empty0 + 8 * i, 8);
+		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+	}
+	if (warp == 1) tmem_alloc<2>(tslot, 512);
+	tc_fence_before();
+	cluster_sync();
+	tc_fence_after();
+	uint32_t tmem;
+	asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(tslot));
+
+	if (warp == 0) {
+		if (lane == 0) { // ---- TMA producer: this CTA's rows of both operands, counted on the first CTA's barrier ----
+			const uint32_t lead_full0 = map_rank(full0, rank & ~1);
+			Ring ring;
+			ring.phase = 1; // the first round of every stage is free
+			for (int item = cluster; item < g.items; item += nclusters) {
+				int seg, seg0, n0, n_end;
+				tile_columns(g, item / g.m_tiles, seg, seg0, n0, n_end);
+				const int a0 = seg * g.a_step + (item % g.m_tiles) * 256 + half * 128;
+				const CUtensorMap *w = B_SEG ? &tb.m[seg] : GLU ? &tb.m[half] : &tb.m[0];
+				const int b0 = GLU ? n0 : (B_SEG ? n0 - seg0 : n0) + half * (nacc / 2);
+				for (int kb = kb0; kb < kb1; ++kb, ring.next(g.stages)) {
+					mbar_wait(empty0 + 8 * ring.s, ring.phase, dead);
+					if (dead) break;
+					const uint32_t dst = base + ring.s * stage_bytes, bar = lead_full0 + 8 * ring.s;
+					if (half == 0) mbar_expect_tx(full0 + 8 * ring.s, 2 * stage_bytes);
+					tma_load_2d<2>(dst, &ta, kb * BK, a0, bar);
+					tma_load_2d<2>(dst + a_bytes, w, kb * BK, b0, bar);
+				}
+			}
+		}
+		__syncwarp();
+	} else if (warp == 1) {
+		if (lane == 0 && half == 0) { // ---- MMA issuer, for both CTAs ----
+			const uint32_t idesc = instr_desc_f16(256, nacc) | (g.bf16 ? kInstrDescBf16 : 0u);
+			const uint16_t pair_mask = (uint16_t)(3u << (rank & ~1));
+			const uint64_t adesc0 = smem_desc_sw128(base), bdesc0 = smem_desc_sw128(base + a_bytes);
+			Ring ring;
+			int done = 0;
+			for (int item = cluster; item < g.items; item += nclusters, ++done) {
+				const int b = done & 1;
+				if (done >= 2) mbar_wait(acc_empty0 + 8 * b, (uint32_t)(done / 2 - 1) & 1u, dead);
+				tc_fence_after();
+				uint32_t more = 0;
+				for (int kb = kb0; kb < kb1; ++kb, ring.next(g.stages)) {
+					mbar_wait(full0 + 8 * ring.s, ring.phase, dead);
+					if (dead) break;
+					tc_fence_after();
+					const uint64_t at = (uint64_t)((ring.s * stage_bytes) >> 4);
+#pragma unroll
+					for (int k = 0; k < BK / 16; ++k, more = 1) // 16 elements = 32 bytes further along K, inside the 128-byte swizzle row
+						umma_f16<2>(tmem + 256 * b, adesc0 + at + 2 * k, bdesc0 + at + 2 * k, idesc, more);
+					umma_commit_pair(empty0 + 8 * ring.s, pair_mask); // the stage is free in both CTAs once these MMAs have read it
+				}
+				umma_commit_pair(acc_full0 + 8 * b, pair_mask); // the accumulator is complete
+			}
+		}
+		__syncwarp();
+	} else if (g.splits == 1) { // ---- tail: warp w reads TMEM lanes 32 (w % 4) .. + 31 (the hardware's lane quarter of a warp) ----
+		const int q = warp & 3;
+		const uint32_t patch = patch0 + q * kPatch, lead_empty0 = map_rank(acc_empty0, rank & ~1);
+		int done = 0;
+		for (int item = cluster; item < g.items; item += nclusters, ++done) {
+			int seg, seg0, n0, n_end;
+			tile_columns(g, item / g.m_tiles, seg, seg0, n0, n_end);
+			const int b = done & 1, row0 = (item % g.m_tiles) * 256 + half * 128 + q * 32;
+			mbar_wait(acc_full0 + 8 * b, (uint32_t)(done / 2) & 1u, dead);
+			__syncwarp();
+			tc_fence_after();
+			const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16) + 256 * b;
+			if (row0 < g.M) {
+#pragma unroll 1
+				for (int c0 = 0; n0 + c0 < n_end; c0 += 32) {
+					float v[32];
+					tmem_ld32(trow + c0, v);
+					if (GLU) {
+						float u[32];
+						tmem_ld32(trow + g.n_tile + c0, u);
+#pragma unroll
+						for (int i = 0; i < 32; ++i) v[i] = glu(g, v[i], u[i]);
+					}
+					if (dead)
+						for (int i = 0; i < 32; ++i) v[i] = kNaN;
+					if (GLU) store_patch_f16(g, patch, v, row0, n0 + c0, n_end);
+					else store_patch_f32(g, patch, v, row0, n0 + c0, n_end);
+				}
+			}
+			tc_fence_before();
+			__syncwarp();
+			if (lane == 0) mbar_arrive_cluster(lead_empty0 + 8 * b);
+		}
+	}
+
+	if (g.splits > 1) { // one tile per cluster: the pairs' sums meet in shared memory, pair p finishes columns p n / splits ..
+		int seg, seg0, n0, n_end;
+		tile_columns(g, cluster / g.m_tiles, seg, seg0, n0, n_end);
+		const int q = warp & 3, row = q * 32 + lane, row0 = (cluster % g.m_tiles) * 256 + half * 128 + q * 32;
+		const int share = g.n_tile / g.splits;                    // columns (per matrix) that a pair finishes: a multiple of 32
+		const int mats = GLU ? 2 : 1, words = share * mats * 128; // floats that one pair sends another (per CTA)
+		const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16);
+		if (warp >= 2) {
+			mbar_wait(acc_full0, 0, dead);
+			__syncwarp();
+			tc_fence_after();
+		}
+		__syncwarp();
+		cluster_sync(); // every pair's products are complete: the stages may be overwritten
+		if (warp >= 2) {
+			for (int p = 0; p < g.splits; ++p) {
+				if (p == part) continue;
+				// slot of this pair in p's buffer: pairs in order, p itself left out; a float4 of columns per thread, rows side by side
+				const uint32_t dst = map_rank(base, (uint32_t)(2 * p + half)) + (uint32_t)((part < p ? part : part - 1) * words) * 4;
+				for (int m = 0; m < mats; ++m)
+#pragma unroll 1
+					for (int c0 = 0; c0 < share; c0 += 32) {
+						float v[32];
+						tmem_ld32(trow + m * g.n_tile + p * share + c0, v);
+#pragma unroll
+						for (int i = 0; i < 32; i += 4)
+							st_cluster4(dst + (uint32_t)((((m * share + c0 + i) >> 2) * 128 + row) * 16), make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]));
+					}
+			}
+		}
+		__syncwarp();
+		cluster_sync(); // the other pairs' sums of this pair's columns are here
+		if (warp >= 2 && row0 < g.M) {
+			const uint32_t patch = patch0 + q * kPatch;
+#pragma unroll 1
+			for (int c0 = part * share; c0 < (part + 1) * share; c0 += 32) {
+				float v[32], u[GLU ? 32 : 1];
+				auto total = [&](float (&out)[32], int m) { // the parts of K in order
+					float own[32];
+					tmem_ld32(trow + m * g.n_tile + c0, own);
+#pragma unroll
+					for (int i = 0; i < 32; ++i) out[i] = 0.f;
+#pragma unroll 1
+					for (int p = 0; p < g.splits; ++p) {
+						if (p == part) {
+#pragma unroll
+							for (int i = 0; i < 32; ++i) out[i] += own[i];
+							continue;
+						}
+						const uint32_t src = base + (uint32_t)((p < part ? p : p - 1) * words) * 4;
+#pragma unroll
+						for (int i = 0; i < 32; i += 4) {
+							const float4 o = ld_shared4(src + (uint32_t)((((m * share + c0 - part * share + i) >> 2) * 128 + row) * 16));
+							out[i] += o.x, out[i + 1] += o.y, out[i + 2] += o.z, out[i + 3] += o.w;
+						}
+					}
+				};
+				total(v, 0);
+				if constexpr (GLU) {
+					total(u, 1);
+#pragma unroll
+					for (int i = 0; i < 32; ++i) v[i] = glu(g, v[i], u[i]);
+				}
+				if (dead)
+					for (int i = 0; i < 32; ++i) v[i] = kNaN;
+				if (n0 + c0 < n_end) {
+					if (GLU) store_patch_f16(g, patch, v, row0, n0 + c0, n_end);
+					else store_patch_f32(g, patch, v, row0, n0 + c0, n_end);
+				}
+			}
+		}
+	}
+	tc_fence_before();
+	__syncwarp();
+	cluster_sync(); // no CTA leaves while another may still signal its barriers or work on its TMEM
+	if (warp == 1) {
+		tc_fence_after();
+		tmem_dealloc<2>(tmem, 512);
+	}
+}
+
+// Few rows: 128 rows of W (of w1 and w3 each for GLU) against all M <= 128 positions.  A cluster of `splits` CTAs shares a tile's K;
+// CTA r finishes the groups of 8 positions g with g % splits == r.  TMEM lane = row of W, column = position.
+template <bool GLU, bool B_SEG>
+__global__ void __launch_bounds__(kGemmThreads)
+gemm_few_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ WeightMaps tb, const __grid_constant__ GemmArgs g) {
+	extern __shared__ uint8_t smem_raw[];
+	constexpr int MATS = GLU ? 2 : 1;
+	const int np = (g.M + 15) / 16 * 16; // positions, padded to the instruction's N
+	const uint32_t w_bytes = 128 * kRowBytes, a_bytes = (uint32_t)np * kRowBytes, stage_bytes = MATS * w_bytes + a_bytes;
+	const uint32_t base = (s32(smem_raw) + 1023u) & ~1023u, bars = base + g.stages * stage_bytes;
+	const uint32_t full0 = bars, empty0 = bars + 8 * g.stages, acc_bar = empty0 + 8 * g.stages, tslot = acc_bar + 8;
+	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+	const int part = g.splits > 1 ? (int)cluster_rank() : 0, tile = blockIdx.x / g.splits;
+	const int nkb = (g.K + BK - 1) / BK, kb0 = part * g.kb_per, kb1 = min(nkb, kb0 + g.kb_per);
+	const uint32_t cols = MATS * np <= 32 ? 32 : MATS * np <= 64 ? 64 : MATS * np <= 128 ? 128 : 256; // TMEM columns
+	int seg, seg0, n0, n_end;
+	tile_columns(g, tile, seg, seg0, n0, n_end);
+	bool dead = false;
+
+	if (threadIdx.x == 0) {
+		for (int i = 0; i < g.stages; ++i) mbar_init(full0 + 8 * i, 1), mbar_init(empty0 + 8 * i, 1);
 		mbar_init(acc_bar, 1);
 		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 	}
-	if (warp == 1) tmem_alloc(tslot, NACC);
+	if (warp == 1) tmem_alloc<1>(tslot, cols);
 	tc_fence_before();
 	__syncthreads();
 	tc_fence_after();
@@ -159,78 +382,110 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ 
 
 	if (warp == 0) {
 		if (lane == 0) { // ---- TMA producer ----
-			for (int kb = 0; kb < nkb; ++kb) {
-				const int s = kb % kStages, r = kb / kStages;
-				if (r > 0) mbar_wait(empty0 + 8 * s, (uint32_t)(r - 1) & 1u);
-				const uint32_t dst = base + s * kStage, bar = full0 + 8 * s;
-				mbar_expect_tx(bar, kStage);
-				tma_load_2d(dst, &ta, kb * BK, a0, bar);
-				tma_load_2d(dst + kTileBytes, &tb, kb * BK, n0, bar);
-				if (NB == 2) tma_load_2d(dst + 2 * kTileBytes, &tb2, kb * BK, n0, bar);
+			const CUtensorMap *w = &tb.m[B_SEG ? seg : 0];
+			const int w0 = B_SEG ? n0 - seg0 : n0;
+			Ring ring;
+			ring.phase = 1; // the first round of every stage is free
+			for (int kb = kb0; kb < kb1; ++kb, ring.next(g.stages)) {
+				mbar_wait(empty0 + 8 * ring.s, ring.phase, dead);
+				if (dead) break;
+				const uint32_t dst = base + ring.s * stage_bytes, bar = full0 + 8 * ring.s;
+				mbar_expect_tx(bar, stage_bytes);
+				tma_load_2d<1>(dst, w, kb * BK, w0, bar);
+				if (GLU) tma_load_2d<1>(dst + w_bytes, &tb.m[1], kb * BK, w0, bar);
+				tma_load_2d<1>(dst + MATS * w_bytes, &ta, kb * BK, seg * g.a_step, bar);
 			}
 		}
+		__syncwarp();
 	} else if (warp == 1) {
 		if (lane == 0) { // ---- MMA issuer ----
-			const uint32_t idesc = instr_desc_f16(BM, NACC) | (g.bf16 ? kInstrDescBf16 : 0u);
-			for (int kb = 0; kb < nkb; ++kb) {
-				const int s = kb % kStages, r = kb / kStages;
-				mbar_wait(full0 + 8 * s, (uint32_t)r & 1u);
+			const uint32_t idesc = instr_desc_f16(128, np) | (g.bf16 ? kInstrDescBf16 : 0u);
+			const uint64_t wdesc0 = smem_desc_sw128(base), vdesc0 = smem_desc_sw128(base + w_bytes), adesc0 = smem_desc_sw128(base + MATS * w_bytes);
+			Ring ring;
+			uint32_t more = 0;
+			for (int kb = kb0; kb < kb1; ++kb, ring.next(g.stages)) {
+				mbar_wait(full0 + 8 * ring.s, ring.phase, dead);
+				if (dead) break;
 				tc_fence_after();
-				const uint32_t a = base + s * kStage, b = a + kTileBytes;
+				const uint64_t at = (uint64_t)((ring.s * stage_bytes) >> 4);
 #pragma unroll
-				for (int k = 0; k < BK / 16; ++k) // 16 fp16 = 32 bytes further along K, inside the 128-byte swizzle row
-					umma_f16(tmem, smem_desc_sw128(a + 32 * k), smem_desc_sw128(b + 32 * k), idesc, (kb | k) != 0);
-				umma_commit(empty0 + 8 * s); // the stage is free once these MMAs have read it
+				for (int k = 0; k < BK / 16; ++k, more = 1) {
+					umma_f16<1>(tmem, wdesc0 + at + 2 * k, adesc0 + at + 2 * k, idesc, more);
+					if (GLU) umma_f16<1>(tmem + np, vdesc0 + at + 2 * k, adesc0 + at + 2 * k, idesc, more);
+				}
+				umma_commit(empty0 + 8 * ring.s);
 			}
-			umma_commit(acc_bar); // the accumulator is complete
+			umma_commit(acc_bar);
 		}
-	} else { // ---- epilogue: warp w reads TMEM lanes 32 * (w % 4) .. + 31 (the hardware's lane quarter of a warp) ----
-		mbar_wait(acc_bar, 0);
+		__syncwarp();
+	}
+	// ---- tail ----
+	const int q = warp & 3, row = q * 32 + lane, groups = (g.M + 7) / 8, mine = (groups + g.splits - 1) / g.splits;
+	const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16);
+	// words of a group of 8 positions: [matrix][4-position half][row][4]
+	auto slot = [&](uint32_t buf, int src, int group, int m, int j) { return buf + (uint32_t)((((src * mine + group / g.splits) * MATS + m) * 2 + j) * 128 + row) * 16; };
+	if (warp >= 2) {
+		mbar_wait(acc_bar, 0, dead);
+		__syncwarp();
 		tc_fence_after();
-		const int q = warp & 3, row = m0 + q * 32 + lane;
-		const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16);
-#pragma unroll 1
-		for (int c0 = 0; c0 < BN; c0 += 32) {
-			float v[32];
-			tmem_ld32(trow + c0, v);
-			if (NB == 2) {
-				float u[32];
-				tmem_ld32(trow + BN + c0, u);
+	}
+	__syncwarp();
+	if (g.splits > 1) {
+		cluster_sync(); // every CTA's products are complete: the stages may be overwritten
+		if (warp >= 2)
+			for (int gr = 0; gr < groups; ++gr) {
+				const int p = gr % g.splits;
+				if (p == part) continue;
+				const uint32_t buf = map_rank(base, (uint32_t)p);
 #pragma unroll
-				for (int i = 0; i < 32; ++i) v[i] = (g.act == YALM_ACT_GELU ? act_gelu(v[i]) : act_silu(v[i])) * u[i];
+				for (int m = 0; m < MATS; ++m) {
+					float v[8];
+					tmem_ld8(trow + m * np + gr * 8, v);
+					st_cluster4(slot(buf, part < p ? part : part - 1, gr, m, 0), make_float4(v[0], v[1], v[2], v[3]));
+					st_cluster4(slot(buf, part < p ? part : part - 1, gr, m, 1), make_float4(v[4], v[5], v[6], v[7]));
+				}
 			}
-			if (row < g.M) {
-				const int col = n0 + c0;
-				if (g.tail == kGluF16) {
-					__half *dst = g.h + (size_t)row * g.ldc + col;
+		__syncwarp();
+		cluster_sync(); // the other CTAs' sums of this CTA's positions are here
+	}
+	if (warp >= 2) {
+		const int col = n0 + row; // lanes are neighbouring output columns
+		for (int gr = part; gr < groups; gr += g.splits) {
+			__syncwarp();
+			float v[MATS][8];
 #pragma unroll
-					for (int i = 0; i < 32; i += 8) {
-						if (col + i + 8 <= n_end) {
-							uint4 pk;
-							__half2 h0 = __floats2half2_rn(v[i], v[i + 1]), h1 = __floats2half2_rn(v[i + 2], v[i + 3]);
-							__half2 h2 = __floats2half2_rn(v[i + 4], v[i + 5]), h3 = __floats2half2_rn(v[i + 6], v[i + 7]);
-							pk.x = *reinterpret_cast<uint32_t *>(&h0), pk.y = *reinterpret_cast<uint32_t *>(&h1);
-							pk.z = *reinterpret_cast<uint32_t *>(&h2), pk.w = *reinterpret_cast<uint32_t *>(&h3);
-							*reinterpret_cast<uint4 *>(dst + i) = pk;
-						} else {
-							for (int j = i; j < i + 8 && col + j < n_end; ++j) dst[j] = __float2half_rn(v[j]);
-						}
+			for (int m = 0; m < MATS; ++m) {
+				float own[8];
+				tmem_ld8(trow + m * np + gr * 8, own);
+#pragma unroll
+				for (int i = 0; i < 8; ++i) v[m][i] = 0.f;
+				for (int p = 0; p < g.splits; ++p) { // the parts of K in order
+					if (p == part) {
+#pragma unroll
+						for (int i = 0; i < 8; ++i) v[m][i] += own[i];
+						continue;
 					}
+					const float4 lo = ld_shared4(slot(base, p < part ? p : p - 1, gr, m, 0)), hi = ld_shared4(slot(base, p < part ? p : p - 1, gr, m, 1));
+					v[m][0] += lo.x, v[m][1] += lo.y, v[m][2] += lo.z, v[m][3] += lo.w, v[m][4] += hi.x, v[m][5] += hi.y, v[m][6] += hi.z, v[m][7] += hi.w;
+				}
+			}
+			if (col < n_end) {
+				const int rows = min(8, g.M - gr * 8);
+				if (GLU) {
+					__half *dst = g.h + (size_t)(gr * 8) * g.ldc + col;
+#pragma unroll
+					for (int i = 0; i < 8; ++i) v[0][i] = dead ? kNaN : glu(g, v[0][i], v[MATS - 1][i]);
+#pragma unroll
+					for (int i = 0; i < 8; ++i)
+						if (i < rows) dst[(size_t)i * g.ldc] = __float2half_rn(v[0][i]);
 				} else {
-					float *dst = g.c + (size_t)row * g.ldc + col;
+					float *dst = g.c + (size_t)(gr * 8) * g.ldc + col;
+					float x[8];
 #pragma unroll
-					for (int i = 0; i < 32; i += 4) {
-						if (col + i + 4 <= n_end) {
-							float4 o = make_float4(g.alpha * v[i], g.alpha * v[i + 1], g.alpha * v[i + 2], g.alpha * v[i + 3]);
-							if (g.tail == kAddF32) { // x += W v (src/infer.cpp:335-337), residual stream stays fp32
-								const float4 x = *reinterpret_cast<const float4 *>(dst + i);
-								o.x += x.x, o.y += x.y, o.z += x.z, o.w += x.w;
-							}
-							*reinterpret_cast<float4 *>(dst + i) = o;
-						} else {
-							for (int j = i; j < i + 4 && col + j < n_end; ++j) dst[j] = g.tail == kAddF32 ? dst[j] + g.alpha * v[j] : g.alpha * v[j];
-						}
-					}
+					for (int i = 0; i < 8; ++i) x[i] = (g.tail == kAddF32 && i < rows) ? dst[(size_t)i * g.ldc] : 0.f;
+#pragma unroll
+					for (int i = 0; i < 8; ++i)
+						if (i < rows) dst[(size_t)i * g.ldc] = dead ? kNaN : x[i] + g.alpha * v[0][i];
 				}
 			}
 		}
@@ -239,7 +494,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ 
 	__syncthreads();
 	if (warp == 1) {
 		tc_fence_after();
-		tmem_dealloc(tmem, NACC);
+		tmem_dealloc<1>(tmem, cols);
 	}
 }
 
@@ -260,36 +515,160 @@ static EncodeTiledFn encode_fn() {
 	return fn;
 }
 
-// (rows, cols) row-major fp16 matrix -> tensor map with a 128-row x 64-column box, 128-byte swizzle, zero fill past the edges
-static int make_map(CUtensorMap *map, const void *ptr, int rows, int cols, bool bf16 = false) {
+// (rows, cols) row-major 16-bit matrix -> tensor map with a box_rows x 64-column box, 128-byte swizzle, zero fill past the edges
+static int make_map(CUtensorMap *map, const void *ptr, int rows, int cols, int box_rows, bool bf16) {
 	EncodeTiledFn fn = encode_fn();
 	if (!fn) return YALM_EINVAL;
 	const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
 	const cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
-	const cuuint32_t box[2] = {BK, BM}, estr[2] = {1, 1};
+	const cuuint32_t box[2] = {BK, (cuuint32_t)box_rows}, estr[2] = {1, 1};
 	const CUresult r = fn(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(ptr), dims, strides, box, estr,
 	                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
 	                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
 	return r == CUDA_SUCCESS ? 0 : YALM_EINVAL;
 }
 
-template <int NB>
-static int launch(const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &tb2, const GemmArgs &g, cudaStream_t st) {
-	constexpr int kStage = kTileBytes * (1 + NB), kStages = NB == 1 ? 6 : 4;
-	const size_t smem = (size_t)kStages * kStage + 1024 + 256;
-	static bool configured = false;
-	if (!configured) {
-		YALM_TRY(cudaFuncSetAttribute(gemm_f16_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-		configured = true;
+constexpr int kMaxDevices = 64;
+
+static int column_tiles(const GemmArgs &g, int n) {
+	int tiles = 0;
+	for (int i = 0, at = 0; i < g.nseg; ++i) tiles += (g.seg_end[i] - at + n - 1) / n, at = g.seg_end[i];
+	return tiles;
+}
+
+static int launch_clusters(void (*kernel)(const CUtensorMap, const WeightMaps, const GemmArgs), int ctas, int cluster, size_t smem, const CUtensorMap &ta,
+                           const WeightMaps &tb, const GemmArgs &g, cudaStream_t st) {
+	cudaLaunchConfig_t cfg = {};
+	cfg.gridDim = dim3(ctas), cfg.blockDim = dim3(kGemmThreads), cfg.dynamicSmemBytes = smem, cfg.stream = st;
+	cudaLaunchAttribute at[1];
+	at[0].id = cudaLaunchAttributeClusterDimension;
+	at[0].val.clusterDim.x = cluster, at[0].val.clusterDim.y = 1, at[0].val.clusterDim.z = 1;
+	cfg.attrs = at, cfg.numAttrs = 1;
+	YALM_TRY(cudaLaunchKernelEx(&cfg, kernel, ta, tb, g));
+	return 0;
+}
+
+static size_t pair_stage_bytes(bool glu, int n) { return (size_t)(128 + (glu ? n : n / 2)) * kRowBytes; }
+static int pair_stages(bool glu, int n) { return (int)std::min<size_t>(10, 196608 / pair_stage_bytes(glu, n)); }
+static size_t pair_smem(bool glu, int n) { return pair_stages(glu, n) * pair_stage_bytes(glu, n) + kTailBytes + 1024; }
+
+// Tile width and K parts of the pair kernel, by estimated cycles: waves of tiles x K blocks x the larger of the MMA's cycles (2 per
+// column and block) and the staging's (an SM receives about 48 bytes a cycle), plus pipeline fill, the last tail and, with K parts, the
+// exchange.  slots: clusters of 2, 4, 8 CTAs that run at once.  Parts of K only where all tiles run at once.
+static void plan_pair(GemmArgs &g, bool glu, const int (&slots)[3]) {
+	const int nkb = (g.K + BK - 1) / BK;
+	double best = 1e30;
+	g.m_tiles = (g.M + 255) / 256;
+	const int widest = glu ? 128 : 256, step = glu ? 16 : 32;
+	for (int si = 0; si < 3; ++si) {
+		const int S = 1 << si, per = (nkb + S - 1) / S;
+		if (S > 1 && (nkb < 8 * S || (nkb + per - 1) / per != S)) break; // (the last part must not be empty)
+		for (int n = widest; n >= 2 * step; n -= step) {
+			if (S > 1 && n % (32 * S)) continue;
+			const int items = g.m_tiles * column_tiles(g, n);
+			if (slots[si] < 1 || (S > 1 && items > slots[si])) continue;
+			const int waves = (items + slots[si] - 1) / slots[si], nacc = glu ? 2 * n : n;
+			const double block = std::max(2.0 * nacc, (128 + nacc / 2) * (double)kRowBytes / 48.0);
+			const double cost = waves * per * block + 2500 + 16.0 * nacc / S + (S > 1 ? 3000 + 8.0 * nacc : 0);
+			if (cost < best * 0.999) best = cost, g.n_tile = n, g.splits = S, g.items = items, g.kb_per = per;
+		}
 	}
-	int ntiles = (g.N + BN - 1) / BN;
-	if (g.nseg > 0) {
-		ntiles = 0;
-		for (int i = 0, at = 0; i < g.nseg; ++i) ntiles += (g.seg_end[i] - at + BN - 1) / BN, at = g.seg_end[i];
+	g.stages = pair_stages(glu, g.n_tile);
+}
+
+template <bool GLU, bool B_SEG>
+static int launch_pair(GemmArgs &g, const void *a, int a_rows, const void *const (&w)[3], const int (&w_rows)[3], int nw, cudaStream_t st) {
+	static int slots[kMaxDevices][3]; // 0: not asked yet
+	static std::mutex mu;
+	auto kernel = gemm_pair_kernel<GLU, B_SEG>;
+	const int dev = device_info().device;
+	if (dev < 0 || dev >= kMaxDevices) return YALM_EINVAL;
+	int here[3];
+	{
+		std::lock_guard<std::mutex> lock(mu);
+		if (!slots[dev][0]) {
+			const size_t most = pair_smem(GLU, GLU ? 128 : 256);
+			YALM_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(most + 4096)));
+			for (int i = 2; i >= 0; --i) {
+				cudaLaunchConfig_t cfg = {};
+				cfg.gridDim = dim3(2 << i), cfg.blockDim = dim3(kGemmThreads), cfg.dynamicSmemBytes = most;
+				cudaLaunchAttribute at[1];
+				at[0].id = cudaLaunchAttributeClusterDimension;
+				at[0].val.clusterDim.x = 2 << i, at[0].val.clusterDim.y = 1, at[0].val.clusterDim.z = 1;
+				cfg.attrs = at, cfg.numAttrs = 1;
+				YALM_TRY(cudaOccupancyMaxActiveClusters(&slots[dev][i], kernel, &cfg));
+			}
+		}
+		for (int i = 0; i < 3; ++i) here[i] = slots[dev][i];
 	}
-	const dim3 grid((g.M + BM - 1) / BM, ntiles);
-	gemm_f16_kernel<NB><<<grid, kGemmThreads, smem, st>>>(ta, tb, tb2, g);
-	return (int)cudaGetLastError();
+	if (here[0] < 1) return (int)cudaErrorLaunchOutOfResources;
+	plan_pair(g, GLU, here);
+	CUtensorMap ta;
+	WeightMaps tb;
+	int rc = make_map(&ta, a, a_rows, g.K, 128, g.bf16);
+	for (int i = 0; i < 3 && !rc; ++i) {
+		if (i < nw) rc = make_map(&tb.m[i], w[i], w_rows[i], g.K, GLU ? g.n_tile : g.n_tile / 2, g.bf16);
+		else tb.m[i] = tb.m[0];
+	}
+	if (rc) return rc;
+	const int clusters = g.splits > 1 ? g.items : std::min(g.items, here[0]);
+	return launch_clusters(kernel, clusters * 2 * g.splits, 2 * g.splits, pair_smem(GLU, g.n_tile), ta, tb, g, st);
+}
+
+// Few rows: an SM's shared memory for stages, or half of it (two CTAs at once) where there are more tiles than SMs.  K parts
+// while every CTA still has an SM to itself: more CTAs than SMs would halve the stages of each.
+template <bool GLU, bool B_SEG>
+static int launch_few(GemmArgs &g, const void *a, int a_rows, const void *const (&w)[3], const int (&w_rows)[3], int nw, cudaStream_t st) {
+	static bool configured[kMaxDevices];
+	static std::mutex mu;
+	auto kernel = gemm_few_kernel<GLU, B_SEG>;
+	const DeviceInfo &d = device_info();
+	if (d.device < 0 || d.device >= kMaxDevices) return YALM_EINVAL;
+	const int np = (g.M + 15) / 16 * 16, mats = GLU ? 2 : 1, nkb = (g.K + BK - 1) / BK;
+	const size_t stage = (size_t)(mats * 128 + np) * kRowBytes;
+	g.n_tile = 128, g.m_tiles = 1, g.items = column_tiles(g, 128);
+	g.splits = 1, g.kb_per = nkb;
+	for (int S = 2; S <= 8 && nkb >= 4 * S && g.items * S <= d.sms; S *= 2) {
+		const int per = (nkb + S - 1) / S;
+		if ((nkb + per - 1) / per == S) g.splits = S, g.kb_per = per; // (the last part must not be empty)
+	}
+	const size_t room = g.items * g.splits <= d.sms ? 212992 : 106496;
+	g.stages = std::max(2, std::min(std::min(16, g.kb_per), (int)(room / stage)));
+	// the exchange reuses the stages: (parts - 1) x groups of 8 positions per CTA x 4 KB x matrices
+	const size_t groups = ((g.M + 7) / 8 + g.splits - 1) / g.splits, exchange = (size_t)(g.splits - 1) * groups * mats * 4096;
+	while (g.stages * stage < exchange) ++g.stages;
+	const size_t smem = g.stages * stage + 512 + 1024;
+	if ((int)smem > d.max_smem_optin) return YALM_EINVAL;
+	{
+		std::lock_guard<std::mutex> lock(mu);
+		if (!configured[d.device]) {
+			YALM_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, d.max_smem_optin));
+			configured[d.device] = true;
+		}
+	}
+	CUtensorMap ta;
+	WeightMaps tb;
+	int rc = make_map(&ta, a, a_rows, g.K, np, g.bf16);
+	for (int i = 0; i < 3 && !rc; ++i) {
+		if (i < nw) rc = make_map(&tb.m[i], w[i], w_rows[i], g.K, 128, g.bf16);
+		else tb.m[i] = tb.m[0];
+	}
+	if (rc) return rc;
+	return launch_clusters(kernel, g.items * g.splits, g.splits, smem, ta, tb, g, st);
+}
+
+// Where the few-rows kernel ends: 128 positions are one operand of it, and up to there it is ahead of the pairs (4096 x 14336: 43 us
+// against 53 at 128 rows, 35 against 53 at 1 row).  With two matrices its two 128-row products read as much shared memory a cycle as
+// there is from about 80 positions on (14336 x 4096: 65.6 us against 67.6 at 64 rows, 73.8 against 68.3 at 128).
+template <bool GLU, bool B_SEG>
+static int launch(GemmArgs &g, const void *a, int a_rows, const void *const (&w)[3], const int (&w_rows)[3], int nw, cudaStream_t st) {
+	return g.M <= (GLU ? 64 : 128) ? launch_few<GLU, B_SEG>(g, a, a_rows, w, w_rows, nw, st) : launch_pair<GLU, B_SEG>(g, a, a_rows, w, w_rows, nw, st);
+}
+
+// c (M, ldc) fp32 = a (M, K) fp16 times the rows of wq, wk and wv, side by side: the three projections of a layer as one launch.
+int gemm_qkv_f16(float *c, int ldc, const void *a, const void *wq, const void *wk, const void *wv, int M, int q_dim, int kv_dim, int K, cudaStream_t st) {
+	GemmArgs g{M, q_dim + 2 * kv_dim, K, kStoreF32, 0, c, nullptr, ldc, 1.0f, 0, 3, {q_dim, q_dim + kv_dim, q_dim + 2 * kv_dim}, 0};
+	return launch<false, true>(g, a, M, {wq, wk, wv}, {q_dim, kv_dim, kv_dim}, 3, st);
 }
 
 } // namespace prefill
@@ -302,30 +681,22 @@ using namespace yalm::prefill;
 extern "C" int yalm_gemm_16(float *c, int ldc, const void *a, const void *w, int M, int N, int K, int accumulate, int bf16, float alpha, yalm_stream_t s) {
 	if (!c || !a || !w || M < 1 || N < 1 || K < 8 || K % 8 || ldc < N || ldc % 4 || ((uintptr_t)a & 15) || ((uintptr_t)w & 15) || ((uintptr_t)c & 15))
 		return YALM_EINVAL;
-	CUtensorMap ta, tb;
-	int rc = make_map(&ta, a, M, K, bf16 != 0);
-	if (!rc) rc = make_map(&tb, w, N, K, bf16 != 0);
-	if (rc) return rc;
-	GemmArgs g{M, N, K, accumulate ? kAddF32 : kStoreF32, 0, c, nullptr, ldc, alpha, bf16 != 0, 0, {}};
-	return launch<1>(ta, tb, tb, g, (cudaStream_t)s);
+	GemmArgs g{M, N, K, accumulate ? kAddF32 : kStoreF32, 0, c, nullptr, ldc, alpha, bf16 != 0, 1, {N}, 0};
+	return launch<false, false>(g, a, M, {w, nullptr, nullptr}, {N, 0, 0}, 1, (cudaStream_t)s);
 }
 // The same with one input per segment of output columns: columns [segment_end[i - 1], segment_end[i]) of c = a_i w^T, a_i = rows
 // i M .. i M + M - 1 of a (n_segments M, K).  Segment bounds are multiples of 4 (the last one is N).
 extern "C" int yalm_gemm_16_segments(float *c, int ldc, const void *a, const void *w, int M, int N, int K, int n_segments, const int *segment_end, int bf16,
                                      yalm_stream_t s) {
 	if (!c || !a || !w || M < 1 || N < 1 || K < 8 || K % 8 || ldc < N || ldc % 4 || ((uintptr_t)a & 15) || ((uintptr_t)w & 15) || ((uintptr_t)c & 15) || n_segments < 1 ||
-	    n_segments > 8 || !segment_end || segment_end[n_segments - 1] != N)
+	    n_segments > kSegments || !segment_end || segment_end[n_segments - 1] != N)
 		return YALM_EINVAL;
-	GemmArgs g{M, N, K, kStoreF32, 0, c, nullptr, ldc, 1.0f, bf16 != 0, n_segments, {}};
+	GemmArgs g{M, N, K, kStoreF32, 0, c, nullptr, ldc, 1.0f, bf16 != 0, n_segments, {}, M};
 	for (int i = 0, at = 0; i < n_segments; ++i) {
 		if (segment_end[i] <= at || (i + 1 < n_segments && segment_end[i] % 4)) return YALM_EINVAL;
 		g.seg_end[i] = at = segment_end[i];
 	}
-	CUtensorMap ta, tb;
-	int rc = make_map(&ta, a, n_segments * M, K, bf16 != 0);
-	if (!rc) rc = make_map(&tb, w, N, K, bf16 != 0);
-	if (rc) return rc;
-	return launch<1>(ta, tb, tb, g, (cudaStream_t)s);
+	return launch<false, false>(g, a, n_segments * M, {w, nullptr, nullptr}, {N, 0, 0}, 1, (cudaStream_t)s);
 }
 extern "C" int yalm_gemm_f16(float *c, int ldc, const void *a, const void *w, int M, int N, int K, int accumulate, yalm_stream_t s) {
 	return yalm_gemm_16(c, ldc, a, w, M, N, K, accumulate, 0, 1.0f, s);
@@ -335,13 +706,8 @@ extern "C" int yalm_gemm_f16(float *c, int ldc, const void *a, const void *w, in
 extern "C" int yalm_gemm_glu_f16(void *h, int ldh, const void *a, const void *w1, const void *w3, int M, int N, int K, int act,
                                  yalm_stream_t s) {
 	if (!h || !a || !w1 || !w3 || M < 1 || N < 1 || K < 8 || K % 8 || ldh < N || ldh % 8) return YALM_EINVAL;
-	CUtensorMap ta, tb, tb2;
-	int rc = make_map(&ta, a, M, K);
-	if (!rc) rc = make_map(&tb, w1, N, K);
-	if (!rc) rc = make_map(&tb2, w3, N, K);
-	if (rc) return rc;
-	GemmArgs g{M, N, K, kGluF16, act, nullptr, static_cast<__half *>(h), ldh, 1.0f, 0, 0, {}};
-	return launch<2>(ta, tb, tb2, g, (cudaStream_t)s);
+	GemmArgs g{M, N, K, kGluF16, act, nullptr, static_cast<__half *>(h), ldh, 1.0f, 0, 1, {N}, 0};
+	return launch<true, false>(g, a, M, {w1, w3, nullptr}, {N, N, 0}, 2, (cudaStream_t)s);
 }
 
 // Host-pointer test entry: c (M, N) fp32 = a (M, K) fp16 * w (N, K)^T fp16 [+ c]; w3 != NULL: h (M, N) fp16 = GLU.
