@@ -1,7 +1,7 @@
 // Batched prefill / perplexity: n consecutive positions through the whole model in one pass.
 // The reference walks a prompt token by token (src/main.cpp:91-97, 174-184); here the projections of a chunk are dense
 // GEMMs on the tcgen05 tensor cores (prefill_gemm.cu), attention is a causal flash-attention over the head-major KV ring
-// (tensor-core mma.sync m16n8k16, online softmax in fp32), and the KV rows of the whole chunk are appended at once.
+// (prompt_attn.cu, online softmax in fp32), and the KV rows of the whole chunk are appended at once.
 // Arithmetic definitions are the decode path's (rmsnorm association order, interleaved-pair RoPE with accurate
 // powf/cosf/sinf, clip, gelu/silu, fp16 KV rows); what differs is the summation order inside the GEMMs and that the GEMM
 // inputs (normalised x, q, attention output, GLU output) are rounded to fp16 once.  Oracle: the token loop.
@@ -21,6 +21,11 @@ extern "C" int yalm_gemm_glu_f16(void *h, int ldh, const void *a, const void *w1
                                  yalm_stream_t s);
 
 namespace yalm {
+namespace prompt { // prompt_attn.cu
+int causal_f16(void *out, const void *q, const void *keys, const void *values, int n, int pos0, int n_heads, int n_kv, int head_dim, int max_seq_len,
+               cudaStream_t st);
+}
+
 namespace prefill {
 
 // prefill_gemm.cu: the three projections as one launch
@@ -79,158 +84,6 @@ __global__ void __launch_bounds__(256) rope_append_rows_kernel(__half *__restric
 	}
 }
 
-// ---- causal flash attention over the KV ring (no wrap: pos0 + n <= max_seq_len) ----------------------------------------
-// grid (ceil(n / 64), n_heads), 4 warps x 16 query rows; K / V tiles of 64 positions in shared memory;
-// S = Q K^T and O += P V on mma.sync.m16n8k16 (fp16 in, fp32 accumulate); scores / softmax as src/infer.cpp:216-248:
-// s = (q . k) / sqrt(head_dim), p = exp(s - max) / sum.
-__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr) {
-	asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-__device__ __forceinline__ void ldsm4t(uint32_t (&r)[4], uint32_t addr) {
-	asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
-	             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-	             : "r"(addr));
-}
-__device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-	asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-	             : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-	             : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ uint32_t pack_h2(float a, float b) {
-	const __half2 h = __floats2half2_rn(a, b);
-	return *reinterpret_cast<const uint32_t *>(&h);
-}
-
-template <int HD>
-__global__ void __launch_bounds__(128) attn_prefill_kernel(__half *__restrict__ out, const __half *__restrict__ q16, const __half *__restrict__ kc,
-                                                           const __half *__restrict__ vc, int n, int pos0, int n_heads, int n_kv_heads,
-                                                           int max_seq_len) {
-	constexpr int LD = HD + 8;  // padded row (halves): 16 bytes of skew keep ldmatrix conflict-free
-	constexpr int KS = HD / 16; // k-steps of Q K^T
-	constexpr int DT = HD / 8;  // 8-wide output tiles of P V
-	extern __shared__ __align__(16) __half smem[];
-	__half *Qs = smem, *Ks = Qs + 64 * LD, *Vs = Ks + 64 * LD;
-	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-	const int h = blockIdx.y, kvh = h / (n_heads / n_kv_heads), i0 = blockIdx.x * 64;
-	const int q_dim = n_heads * HD;
-	const __half *kbase = kc + (size_t)kvh * max_seq_len * HD, *vbase = vc + (size_t)kvh * max_seq_len * HD;
-	// Q tile (rows past n: zeros)
-	for (int c = threadIdx.x; c < 64 * (HD / 8); c += 128) {
-		const int r = c / (HD / 8), d = (c % (HD / 8)) * 8;
-		uint4 v = make_uint4(0, 0, 0, 0);
-		if (i0 + r < n) v = *reinterpret_cast<const uint4 *>(q16 + (size_t)(i0 + r) * q_dim + h * HD + d);
-		*reinterpret_cast<uint4 *>(Qs + r * LD + d) = v;
-	}
-	__syncthreads();
-	uint32_t qf[KS][4];
-	{
-		const int r = warp * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, cofs = (lane >> 4) * 8;
-#pragma unroll
-		for (int ks = 0; ks < KS; ++ks) ldsm4(qf[ks], (uint32_t)__cvta_generic_to_shared(Qs + r * LD + ks * 16 + cofs));
-	}
-	float o[DT][4];
-#pragma unroll
-	for (int t = 0; t < DT; ++t) o[t][0] = o[t][1] = o[t][2] = o[t][3] = 0.f;
-	float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f; // rows lane/4 and lane/4 + 8 of the warp's 16
-	const int rA = i0 + warp * 16 + (lane >> 2), rB = rA + 8;
-	// causal limits (rows past n reuse the last valid row's limit: finite garbage, never stored)
-	const int limA = pos0 + min(rA, n - 1), limB = pos0 + min(rB, n - 1);
-	const int last_key = pos0 + min(i0 + 63, n - 1);
-	const float div = sqrtf((float)HD);
-	for (int j0 = 0; j0 <= last_key; j0 += 64) {
-		__syncthreads(); // the previous tile's reads are done
-		for (int c = threadIdx.x; c < 64 * (HD / 8); c += 128) {
-			const int r = c / (HD / 8), d = (c % (HD / 8)) * 8;
-			uint4 kv = make_uint4(0, 0, 0, 0), vv = kv;
-			if (j0 + r < max_seq_len && j0 + r <= last_key) {
-				kv = *reinterpret_cast<const uint4 *>(kbase + (size_t)(j0 + r) * HD + d);
-				vv = *reinterpret_cast<const uint4 *>(vbase + (size_t)(j0 + r) * HD + d);
-			}
-			*reinterpret_cast<uint4 *>(Ks + r * LD + d) = kv;
-			*reinterpret_cast<uint4 *>(Vs + r * LD + d) = vv;
-		}
-		__syncthreads();
-		// ---- S = Q K^T: 8 key tiles of 8 ----
-		float s[8][4];
-#pragma unroll
-		for (int t = 0; t < 8; ++t) s[t][0] = s[t][1] = s[t][2] = s[t][3] = 0.f;
-		{
-			const int kr = (lane & 7) + (lane >> 4) * 8, kcofs = ((lane >> 3) & 1) * 8;
-#pragma unroll
-			for (int ks = 0; ks < KS; ++ks)
-#pragma unroll
-				for (int t = 0; t < 8; t += 2) {
-					uint32_t b[4];
-					ldsm4(b, (uint32_t)__cvta_generic_to_shared(Ks + (t * 8 + kr) * LD + ks * 16 + kcofs));
-					mma16816(s[t], qf[ks], b[0], b[1]);
-					mma16816(s[t + 1], qf[ks], b[2], b[3]);
-				}
-		}
-		// ---- scale, causal mask, online softmax (fp32) ----
-		float mxA = -INFINITY, mxB = -INFINITY;
-#pragma unroll
-		for (int t = 0; t < 8; ++t) {
-			const int key = j0 + t * 8 + (lane & 3) * 2;
-			s[t][0] = key <= limA ? s[t][0] / div : -INFINITY;
-			s[t][1] = key + 1 <= limA ? s[t][1] / div : -INFINITY;
-			s[t][2] = key <= limB ? s[t][2] / div : -INFINITY;
-			s[t][3] = key + 1 <= limB ? s[t][3] / div : -INFINITY;
-			mxA = fmaxf(mxA, fmaxf(s[t][0], s[t][1]));
-			mxB = fmaxf(mxB, fmaxf(s[t][2], s[t][3]));
-		}
-		mxA = fmaxf(mxA, __shfl_xor_sync(kFull, mxA, 1)), mxA = fmaxf(mxA, __shfl_xor_sync(kFull, mxA, 2));
-		mxB = fmaxf(mxB, __shfl_xor_sync(kFull, mxB, 1)), mxB = fmaxf(mxB, __shfl_xor_sync(kFull, mxB, 2));
-		const float nA = fmaxf(m0, mxA), nB = fmaxf(m1, mxB); // finite from the first tile on (key 0 is visible to every row)
-		const float cA = m0 == -INFINITY ? 0.f : __expf(m0 - nA), cB = m1 == -INFINITY ? 0.f : __expf(m1 - nB);
-		m0 = nA, m1 = nB;
-		l0 *= cA, l1 *= cB;
-#pragma unroll
-		for (int t = 0; t < DT; ++t) o[t][0] *= cA, o[t][1] *= cA, o[t][2] *= cB, o[t][3] *= cB;
-		uint32_t pf[4][4]; // P as A fragments: key steps of 16
-#pragma unroll
-		for (int t = 0; t < 8; ++t) {
-			const float p0 = __expf(s[t][0] - nA), p1 = __expf(s[t][1] - nA), p2 = __expf(s[t][2] - nB), p3 = __expf(s[t][3] - nB);
-			l0 += p0 + p1, l1 += p2 + p3;
-			pf[t >> 1][(t & 1) * 2] = pack_h2(p0, p1);
-			pf[t >> 1][(t & 1) * 2 + 1] = pack_h2(p2, p3);
-		}
-		// ---- O += P V ----
-		{
-			const int vr = (lane & 7) + ((lane >> 3) & 1) * 8, vcofs = (lane >> 4) * 8;
-#pragma unroll
-			for (int kk = 0; kk < 4; ++kk)
-#pragma unroll
-				for (int t = 0; t < DT; t += 2) {
-					uint32_t b[4];
-					ldsm4t(b, (uint32_t)__cvta_generic_to_shared(Vs + (kk * 16 + vr) * LD + t * 8 + vcofs));
-					mma16816(o[t], pf[kk], b[0], b[1]);
-					mma16816(o[t + 1], pf[kk], b[2], b[3]);
-				}
-		}
-	}
-	l0 += __shfl_xor_sync(kFull, l0, 1), l0 += __shfl_xor_sync(kFull, l0, 2);
-	l1 += __shfl_xor_sync(kFull, l1, 1), l1 += __shfl_xor_sync(kFull, l1, 2);
-#pragma unroll
-	for (int t = 0; t < DT; ++t) {
-		const int d = h * HD + t * 8 + (lane & 3) * 2;
-		if (rA < n) *reinterpret_cast<__half2 *>(out + (size_t)rA * q_dim + d) = __floats2half2_rn(o[t][0] / l0, o[t][1] / l0);
-		if (rB < n) *reinterpret_cast<__half2 *>(out + (size_t)rB * q_dim + d) = __floats2half2_rn(o[t][2] / l1, o[t][3] / l1);
-	}
-}
-
-template <int HD>
-static int launch_attn(__half *out, const __half *q16, const __half *kc, const __half *vc, int n, int pos0, int n_heads, int n_kv_heads,
-                       int max_seq_len, cudaStream_t st) {
-	const size_t smem = (size_t)3 * 64 * (HD + 8) * sizeof(__half);
-	static bool configured = false;
-	if (!configured && smem > 48 * 1024) {
-		YALM_TRY(cudaFuncSetAttribute(attn_prefill_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-		configured = true;
-	}
-	attn_prefill_kernel<HD><<<dim3((n + 63) / 64, n_heads), 128, smem, st>>>(out, q16, kc, vc, n, pos0, n_heads, n_kv_heads, max_seq_len);
-	return (int)cudaGetLastError();
-}
-
 } // namespace prefill
 } // namespace yalm
 
@@ -242,16 +95,7 @@ extern "C" int yalm_attn_prefill(void *out16, const void *q16, const uint16_t *k
                                  int n_heads, int n_kv_heads, int head_dim, int max_seq_len, yalm_stream_t s) {
 	if (!out16 || !q16 || !key_cache || !value_cache || n < 1 || pos0 < 0 || pos0 + n > max_seq_len || n_kv_heads < 1 || n_heads % n_kv_heads)
 		return YALM_EINVAL;
-	auto o = static_cast<__half *>(out16);
-	auto q = static_cast<const __half *>(q16);
-	auto k = reinterpret_cast<const __half *>(key_cache), v = reinterpret_cast<const __half *>(value_cache);
-	cudaStream_t st = (cudaStream_t)s;
-	switch (head_dim) {
-	case 128: return launch_attn<128>(o, q, k, v, n, pos0, n_heads, n_kv_heads, max_seq_len, st);
-	case 64: return launch_attn<64>(o, q, k, v, n, pos0, n_heads, n_kv_heads, max_seq_len, st);
-	case 32: return launch_attn<32>(o, q, k, v, n, pos0, n_heads, n_kv_heads, max_seq_len, st);
-	}
-	return YALM_EINVAL;
+	return prompt::causal_f16(out16, q16, key_cache, value_cache, n, pos0, n_heads, n_kv_heads, head_dim, max_seq_len, (cudaStream_t)s);
 }
 
 // ---- Model::forward_batch ------------------------------------------------------------------------------------------

@@ -1,0 +1,619 @@
+// Attention of a prompt portion on the 5th-generation tensor cores: many query rows over a head-major ring of fp16 or bf16 keys and
+// values, one softmax per row (src/infer.cpp:216-248 per row; the layered models' windows, pooled blocks and sinks beside it).
+//
+// Rows.  The G query heads that share a kv head are stacked, row r = (position r / G, head r % G), so a tile of 128 rows covers
+// 128 / G positions: a few positions already fill it, a causal edge wastes little, and every key tile is read once for all G heads.
+// A CTA owns two such tiles (A, B) of one kv head; a cluster of CTAs shares their keys where that fills the GPU, and joins
+// (sum, maximum, accumulator) through distributed shared memory in a fixed order.
+//
+// 12 warps.  Warp 0 streams key and value tiles of 128 positions with cp.async.bulk.tensor.3d into a ring of stages.  One thread of
+// warp 1 issues the products: S = Q K^T into TMEM, O += P V with P out of TMEM (its fp16 / bf16 words take the place of the scores).
+// Warps 4-7 and 8-11 are the softmax of tiles A and B, a thread per row: scores from TMEM, online maximum and sum in fp32, P back to
+// TMEM.  The two tiles alternate: while one's scores go through the softmax the tensor pipe works for the other.  O stays in TMEM; it is
+// rescaled only when a row's maximum has grown by more than 2^8 since its last rescaling (the weights of the meantime are up to 256
+// times larger, in fp32 sums and 16-bit operands alike, and the final division takes it out again).  Warps 2 and 3 serve the layered
+// models: they round pooled fp32 means into stages, and clear the value rows of a ring tile that hold no position (a weight of zero
+// times whatever lies there must be zero).
+//
+// Bound by the exponentials (16 a cycle and SM, as many cycles as the products of a tile pair) and, for short contexts, by the chain
+// copy - product - softmax - product and the launch.
+#include "common.cuh"
+#include "launch.h"
+#include "stack_rows.cuh"
+#include "tcgen.cuh"
+
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+
+#include <algorithm>
+#include <mutex>
+
+namespace yalm {
+namespace prompt {
+
+constexpr int kThreads = 384, kTile = 128, kMaxDevices = 64;
+
+struct Args {
+	void *out;          // fp16 rows (n, heads DV), or fp32 rows of stride ldo
+	const void *q;      // fp16 rows (n, heads DK), or fp32 rows of stride ldq
+	int ldo, ldq;
+	const float *key_pool, *value_pool; // (kv head, block, channel) fp32 means
+	const float *sink;                  // per query head, or null
+	int n, G, n_kv, v_heads, ring, max_blocks, window, pool, pos0;
+	const int *ctl;
+	float q_sign, c; // score (in powers of two) = c (q q_sign) . k
+	int parts;
+	int wide; // fp16 output rows are 16-byte aligned
+};
+
+// Key tiles of a CTA's rows: pooled blocks in tiles of 128 first, then the positions lo .. last in runs of slots that end at the ring's end.
+struct Tiles {
+	int ring, blocks, pooled, lo, last, s0, first_run, per_wrap, total;
+	__device__ Tiles(const Args &a, int i_first, int i_last) : ring(a.ring), last(i_last) {
+		lo = lo_of(a, i_first), blocks = blocks_of(a, i_last);
+		pooled = (blocks + kTile - 1) / kTile;
+		s0 = lo % ring, per_wrap = (ring + kTile - 1) / kTile;
+		const int len = last - lo + 1, head = min(len, ring - s0), rest = len - head;
+		first_run = (head + kTile - 1) / kTile;
+		total = pooled + first_run + rest / ring * per_wrap + (rest % ring + kTile - 1) / kTile;
+	}
+	static __device__ __forceinline__ int lo_of(const Args &a, int i) { return a.window > 0 ? max(0, i - a.window + 1) : 0; }
+	static __device__ __forceinline__ int blocks_of(const Args &a, int i) {
+		return (a.window > 0 && a.pool > 0 && i - a.window + 1 >= a.pool) ? min((i - a.window + 1) / a.pool, a.max_blocks) : 0;
+	}
+	// tile k: first block, or first slot and its position; how many of its 128 rows are blocks / positions.  Returns whether it is a pooled one.
+	__device__ __forceinline__ bool at(int k, int &slot, int &pos, int &valid) const {
+		if (k < pooled) {
+			slot = pos = k * kTile, valid = min(kTile, blocks - slot);
+			return true;
+		}
+		k -= pooled;
+		if (k < first_run) {
+			slot = s0 + k * kTile, pos = lo + k * kTile;
+		} else {
+			k -= first_run;
+			const int wrap = k / per_wrap;
+			slot = (k - wrap * per_wrap) * kTile, pos = lo + (ring - s0) + wrap * ring + slot;
+		}
+		valid = min(min(kTile, ring - slot), last - pos + 1);
+		return false;
+	}
+};
+
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, int c0, int c1, int c2, uint32_t bar) {
+	asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst), "l"(map),
+	             "r"(c0), "r"(c1), "r"(c2), "r"(bar)
+	             : "memory");
+}
+// D[tmem] (+)= A[tmem] * B[smem]^T
+__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+	asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d), "r"(tmem_a),
+	             "l"(bdesc), "r"(idesc), "r"(accumulate)
+	             : "memory");
+}
+__device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+__device__ __forceinline__ float ex2(float x) {
+	float y;
+	asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+	return y;
+}
+#define YALM_R32(r, o)                                                                                                                               \
+	"=r"(r[o]), "=r"(r[o + 1]), "=r"(r[o + 2]), "=r"(r[o + 3]), "=r"(r[o + 4]), "=r"(r[o + 5]), "=r"(r[o + 6]), "=r"(r[o + 7]), "=r"(r[o + 8]),      \
+	    "=r"(r[o + 9]), "=r"(r[o + 10]), "=r"(r[o + 11]), "=r"(r[o + 12]), "=r"(r[o + 13]), "=r"(r[o + 14]), "=r"(r[o + 15]), "=r"(r[o + 16]),       \
+	    "=r"(r[o + 17]), "=r"(r[o + 18]), "=r"(r[o + 19]), "=r"(r[o + 20]), "=r"(r[o + 21]), "=r"(r[o + 22]), "=r"(r[o + 23]), "=r"(r[o + 24]),     \
+	    "=r"(r[o + 25]), "=r"(r[o + 26]), "=r"(r[o + 27]), "=r"(r[o + 28]), "=r"(r[o + 29]), "=r"(r[o + 30]), "=r"(r[o + 31])
+#define YALM_V32(r, o)                                                                                                                               \
+	"r"(r[o]), "r"(r[o + 1]), "r"(r[o + 2]), "r"(r[o + 3]), "r"(r[o + 4]), "r"(r[o + 5]), "r"(r[o + 6]), "r"(r[o + 7]), "r"(r[o + 8]), "r"(r[o + 9]), \
+	    "r"(r[o + 10]), "r"(r[o + 11]), "r"(r[o + 12]), "r"(r[o + 13]), "r"(r[o + 14]), "r"(r[o + 15]), "r"(r[o + 16]), "r"(r[o + 17]),             \
+	    "r"(r[o + 18]), "r"(r[o + 19]), "r"(r[o + 20]), "r"(r[o + 21]), "r"(r[o + 22]), "r"(r[o + 23]), "r"(r[o + 24]), "r"(r[o + 25]),             \
+	    "r"(r[o + 26]), "r"(r[o + 27]), "r"(r[o + 28]), "r"(r[o + 29]), "r"(r[o + 30]), "r"(r[o + 31])
+// 32 columns without waiting for them (tmem_wait_ld, then pin() the registers, before they are used)
+template <int O, int N>
+__device__ __forceinline__ void tmem_ld32_async(uint32_t taddr, uint32_t (&r)[N]) {
+	asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+	             "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+	             "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+	             : YALM_R32(r, O)
+	             : "r"(taddr)
+	             : "memory");
+}
+template <int N>
+__device__ __forceinline__ void pin(uint32_t (&r)[N]) {
+#pragma unroll
+	for (int i = 0; i < N; ++i) asm volatile("" : "+r"(r[i]));
+}
+template <int O, int N>
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[N]) {
+	asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], "
+	             "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+	             "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31};" ::YALM_V32(r, O),
+	             "r"(taddr)
+	             : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+template <typename T>
+__device__ __forceinline__ uint32_t pack2(float a, float b) {
+	if constexpr (__is_same(T, __half)) {
+		const __half2 h = __floats2half2_rn(a, b);
+		return *reinterpret_cast<const uint32_t *>(&h);
+	} else {
+		const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+		return *reinterpret_cast<const uint32_t *>(&h);
+	}
+}
+// Byte offset of 16-byte piece c of row r in an operand tile of 128 rows: sub-tiles of 64 elements a row, SWIZZLE_128B
+__device__ __forceinline__ uint32_t tile_at(int r, int c) { return (uint32_t)((c >> 3) * (kTile * 128) + r * 128 + (((c & 7) ^ (r & 7)) << 4)); }
+// Descriptor of a value tile as the B operand of P V: N (channels) is the contiguous direction.  Groups of 8 positions 1024 bytes
+// apart, blocks of 64 channels one sub-tile apart.
+__device__ __forceinline__ uint64_t desc_mn(uint32_t addr) {
+	return (uint64_t)((addr & 0x3FFFF) >> 4) | ((uint64_t)((kTile * 128) >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
+}
+constexpr uint32_t kBMajorMn = 1u << 16; // instruction descriptor: B is N-major
+
+template <int DK, int DV>
+struct Shape {
+	static constexpr int DKP = DK < 64 ? 64 : DK, DVP = DV < 64 ? 64 : DV; // channels a row takes in shared memory
+	static constexpr int Q_BYTES = kTile * DKP * 2, K_BYTES = Q_BYTES, V_BYTES = kTile * DVP * 2, STAGE = K_BYTES > V_BYTES ? K_BYTES : V_BYTES;
+	static constexpr int STAGES = STAGE == 32768 ? 4 : 8;
+	static constexpr int SMEM = 2 * Q_BYTES + STAGES * STAGE + 512 + 1024;
+};
+
+// T: operand type.  LAYERED: fp32 rows in and out, pooled blocks, ring tiles with rows that hold no position, sinks.
+template <typename T, int DK, int DV, bool LAYERED>
+__global__ void __launch_bounds__(kThreads, 1)
+prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv, const __grid_constant__ Args a) {
+	using SH = Shape<DK, DV>;
+	constexpr int NST = SH::STAGES;
+	extern __shared__ uint8_t smem_raw[];
+	const uint32_t base = (s32(smem_raw) + 1023u) & ~1023u, q0 = base, kv0 = q0 + 2 * SH::Q_BYTES, bars = kv0 + NST * SH::STAGE;
+	const uint32_t full0 = bars, empty0 = full0 + 8 * NST, s_full0 = empty0 + 8 * NST, p_full0 = s_full0 + 16, o_full = p_full0 + 16, v_clean0 = o_full + 8,
+	               tslot = v_clean0 + 8 * NST;
+	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+	const int parts = a.parts, part = parts > 1 ? (int)cluster_rank() : 0;
+	const int rows = a.n * a.G, pairs = (rows + 2 * kTile - 1) / (2 * kTile);
+	const int pair = pairs - 1 - (int)(blockIdx.x / parts); // the longest rows first
+	const int g = blockIdx.y, r0 = pair * 2 * kTile, nt = r0 + kTile < rows ? 2 : 1;
+	const int p0 = a.ctl ? a.ctl[CTL_POS] : a.pos0;
+	const Tiles tiles(a, p0 + r0 / a.G, p0 + min((r0 + 2 * kTile - 1) / a.G, a.n - 1));
+	const int per = (tiles.total + parts - 1) / parts, k_begin = min(part * per, tiles.total), k_end = min(k_begin + per, tiles.total), nk = k_end - k_begin;
+	const bool first_pooled = LAYERED && nk > 0 && k_begin < tiles.pooled;
+	bool dead = false;
+
+	// Key / value tile i of this part (0, 1, ..) takes ring entries 2 i (keys) and 2 i + 1 (values).  Every round of a stage is waited
+	// for, also where the entry is not a copy: a parity tells neighbouring rounds apart and no more.
+	auto load = [&](int i, int is_v) {
+		const int e = 2 * i + is_v, s = e % NST;
+		if (e >= NST) mbar_wait(empty0 + 8 * s, (uint32_t)(e / NST - 1) & 1u, dead);
+		int slot, pos, valid;
+		if (tiles.at(k_begin + i, slot, pos, valid) || dead) return; // pooled tiles are filled by other warps
+		const uint32_t dst = kv0 + s * SH::STAGE, bar = full0 + 8 * s;
+		mbar_expect_tx(bar, is_v ? SH::V_BYTES : SH::K_BYTES);
+		const int d = is_v ? SH::DVP : SH::DKP, head = is_v ? g % a.v_heads : g;
+		for (int c = 0; c < d; c += 64) tma_load_3d(dst + (c / 64) * (kTile * 128), is_v ? &tv : &tk, c, slot, head, bar);
+	};
+	// a pooled tile's means into its two stages, rounded; rows past the last block are zero
+	auto fill_pooled = [&](int i, int tid, int nthreads) {
+		int slot, pos, valid;
+		tiles.at(k_begin + i, slot, pos, valid);
+#pragma unroll
+		for (int is_v = 0; is_v < 2; ++is_v) {
+			const int D = is_v ? DV : DK, pieces = (is_v ? SH::DVP : SH::DKP) / 8, head = is_v ? g % a.v_heads : g;
+			const float *src = (is_v ? a.value_pool : a.key_pool) + ((size_t)head * a.max_blocks + slot) * D;
+			const uint32_t dst = kv0 + ((2 * i + is_v) % NST) * SH::STAGE;
+#pragma unroll 4
+			for (int x = tid; x < kTile * pieces; x += nthreads) {
+				const int r = x / pieces, c = x % pieces;
+				float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
+				if (r < valid && c * 8 < D) {
+					lo = *reinterpret_cast<const float4 *>(src + (size_t)r * D + c * 8);
+					hi = *reinterpret_cast<const float4 *>(src + (size_t)r * D + c * 8 + 4);
+				}
+				st_shared4(dst + tile_at(r, c), make_float4(__uint_as_float(pack2<T>(lo.x, lo.y)), __uint_as_float(pack2<T>(lo.z, lo.w)),
+				                                            __uint_as_float(pack2<T>(hi.x, hi.y)), __uint_as_float(pack2<T>(hi.z, hi.w))));
+			}
+		}
+		proxy_fence();
+	};
+
+	if (threadIdx.x == 0) {
+		// a value stage (odd) is free again once its products are done and, in a layered model, warps 2 and 3 have passed it
+		for (int i = 0; i < NST; ++i) mbar_init(full0 + 8 * i, 1), mbar_init(empty0 + 8 * i, LAYERED && (i & 1) ? 3 : 1);
+		for (int i = 0; i < 2; ++i) mbar_init(s_full0 + 8 * i, 1), mbar_init(p_full0 + 8 * i, 4);
+		mbar_init(o_full, 1);
+		if (LAYERED)
+			for (int i = 0; i < NST; ++i) mbar_init(v_clean0 + 8 * i, 1);
+		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+		for (int e = 0; e < NST && e < 2 * nk; ++e) load(e >> 1, e & 1); // the stages are free: the first tiles travel while the queries are staged
+	}
+	if (warp == 1) tmem_alloc<1>(tslot, 512);
+	if (warp > 0) { // the queries' rows (rows past the last: zero), and the first tile where it is a pooled one
+		constexpr int PIECES = DK / 8;
+		for (int x = threadIdx.x - 32; x < 2 * kTile * PIECES; x += kThreads - 32) {
+			const int r = x / PIECES, c = x % PIECES, row = r0 + r;
+			float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+			if (row < rows) {
+				const int i = row / a.G, h = g * a.G + row % a.G;
+				if constexpr (LAYERED) {
+					const float *src = static_cast<const float *>(a.q) + (size_t)i * a.ldq + (size_t)h * DK + c * 8;
+					const float4 lo = *reinterpret_cast<const float4 *>(src), hi = *reinterpret_cast<const float4 *>(src + 4);
+					const float f = a.q_sign;
+					v = make_float4(__uint_as_float(pack2<T>(lo.x * f, lo.y * f)), __uint_as_float(pack2<T>(lo.z * f, lo.w * f)),
+					                __uint_as_float(pack2<T>(hi.x * f, hi.y * f)), __uint_as_float(pack2<T>(hi.z * f, hi.w * f)));
+				} else
+					v = *reinterpret_cast<const float4 *>(static_cast<const T *>(a.q) + ((size_t)i * a.n_kv * a.G + h) * DK + c * 8);
+			}
+			st_shared4(q0 + (r / kTile) * SH::Q_BYTES + tile_at(r % kTile, c), v);
+		}
+		if constexpr (LAYERED)
+			if (first_pooled) fill_pooled(0, threadIdx.x - 32, kThreads - 32);
+		proxy_fence();
+	}
+	tc_fence_before();
+	__syncthreads();
+	tc_fence_after();
+	uint32_t tmem;
+	asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(tslot));
+
+	float mref = -INFINITY, l = 0.f; // of this thread's row: reference of the weights (in powers of two), their sum
+
+	if (warp == 0) {
+		if (lane == 0) {
+			if (first_pooled) mbar_arrive(full0), mbar_arrive(full0 + 8);
+			for (int e = NST; e < 2 * nk; ++e) load(e >> 1, e & 1);
+		}
+		__syncwarp();
+	} else if (warp == 1) {
+		if (lane == 0 && nk > 0) { // ---- products ----
+			constexpr uint32_t fmt = __is_same(T, __half) ? 0u : kInstrDescBf16;
+			const uint32_t qk_desc = instr_desc_f16(128, kTile) | fmt, pv_desc = instr_desc_f16(128, SH::DVP) | fmt | kBMajorMn;
+			auto wait_full = [&](int e) {
+				mbar_wait(full0 + 8 * (e % NST), (uint32_t)(e / NST) & 1u, dead);
+				tc_fence_after();
+			};
+			auto scores = [&](int t, int e) {
+				const uint32_t qa = q0 + t * SH::Q_BYTES, ka = kv0 + (e % NST) * SH::STAGE;
+#pragma unroll
+				for (int k = 0; k < DK / 16; ++k) {
+					const uint32_t off = (k >> 2) * (kTile * 128) + (k & 3) * 32;
+					umma_f16<1>(tmem + t * kTile, smem_desc_sw128(qa + off), smem_desc_sw128(ka + off), qk_desc, k);
+				}
+				umma_commit(s_full0 + 8 * t);
+			};
+			uint32_t cleaned = 0; // a bit per stage: parity of its rounds of clearing
+			wait_full(0);
+			for (int t = 0; t < nt; ++t) scores(t, 0);
+			umma_commit(empty0);
+			for (int i = 0; i < nk && !dead; ++i) {
+				const int ev = 2 * i + 1, ek = 2 * i + 2;
+				wait_full(ev);
+				if constexpr (LAYERED) {
+					int slot, pos, valid;
+					if (!tiles.at(k_begin + i, slot, pos, valid) && valid < kTile) {
+						const int sv = ev % NST;
+						mbar_wait(v_clean0 + 8 * sv, (cleaned >> sv) & 1u, dead);
+						cleaned ^= 1u << sv;
+						tc_fence_after();
+					}
+				}
+				const uint64_t vdesc = desc_mn(kv0 + (ev % NST) * SH::STAGE);
+				for (int t = 0; t < nt; ++t) {
+					mbar_wait(p_full0 + 8 * t, (uint32_t)i & 1u, dead);
+					tc_fence_after();
+#pragma unroll
+					for (int k = 0; k < kTile / 16; ++k) // 16 positions = 2048 bytes further in every sub-tile, 8 columns of P
+						umma_ts(tmem + 256 + t * SH::DVP, tmem + t * kTile + 8 * k, vdesc + (2048 >> 4) * k, pv_desc, (i | k) != 0);
+					if (t == nt - 1) umma_commit(empty0 + 8 * (ev % NST));
+					if (i + 1 < nk) {
+						if (t == 0) wait_full(ek);
+						scores(t, ek);
+						if (t == nt - 1) umma_commit(empty0 + 8 * (ek % NST));
+					}
+				}
+			}
+			umma_commit(o_full);
+		}
+		__syncwarp();
+	} else if (warp < 4) {
+		if constexpr (LAYERED) {
+			const int tid = threadIdx.x - 64;
+			for (int i = 0; i < nk; ++i) {
+				int slot, pos, valid;
+				const bool pooled = tiles.at(k_begin + i, slot, pos, valid);
+				const int ek = 2 * i, ev = 2 * i + 1;
+				if (pooled && i > 0) {
+					if (ek >= NST) mbar_wait(empty0 + 8 * (ek % NST), (uint32_t)(ek / NST - 1) & 1u, dead);
+					if (ev >= NST) mbar_wait(empty0 + 8 * (ev % NST), (uint32_t)(ev / NST - 1) & 1u, dead);
+					fill_pooled(i, tid, 64);
+					asm volatile("bar.sync 1, 64;" ::: "memory");
+					if (tid == 0) mbar_arrive(full0 + 8 * (ek % NST)), mbar_arrive(full0 + 8 * (ev % NST));
+				}
+				mbar_wait(full0 + 8 * (ev % NST), (uint32_t)(ev / NST) & 1u, dead); // of every tile, to stay with the rounds
+				if (!pooled && valid < kTile) {
+					const uint32_t dst = kv0 + (ev % NST) * SH::STAGE;
+					constexpr int PIECES = SH::DVP / 8;
+					for (int x = valid * PIECES + tid; x < kTile * PIECES; x += 64) st_shared4(dst + tile_at(x / PIECES, x % PIECES), make_float4(0.f, 0.f, 0.f, 0.f));
+					proxy_fence();
+					asm volatile("bar.sync 1, 64;" ::: "memory");
+					if (tid == 0) mbar_arrive(v_clean0 + 8 * (ev % NST));
+				}
+				__syncwarp();
+				if (lane == 0) mbar_arrive(empty0 + 8 * (ev % NST));
+			}
+		}
+		__syncwarp();
+	} else {
+		const int t = (warp - 4) >> 2, q = warp & 3, r = r0 + t * kTile + q * 32 + lane;
+		if (t < nt && nk > 0) { // ---- softmax: one row per thread ----
+			const int i = p0 + min(r, rows - 1) / a.G; // rows past the last repeat it: finite values that are never stored
+			const int lo = Tiles::lo_of(a, i), nb = LAYERED ? Tiles::blocks_of(a, i) : 0;
+			const uint32_t lanes = (uint32_t)(q * 32) << 16, sp = tmem + lanes + t * kTile, op = tmem + lanes + 256 + t * SH::DVP;
+			const float c = a.c;
+			for (int k = 0; k < nk; ++k) {
+				int slot, pos, valid;
+				const bool pooled = tiles.at(k_begin + k, slot, pos, valid);
+				const int from = pooled ? 0 : lo - pos, to = pooled ? nb - slot - 1 : min(i - pos, valid - 1); // visible: from .. to of the tile
+				mbar_wait(s_full0 + 8 * t, (uint32_t)k & 1u, dead);
+				__syncwarp();
+				tc_fence_after();
+				uint32_t s[kTile];
+				tmem_ld32_async<0>(sp, s);
+				tmem_ld32_async<32>(sp + 32, s);
+				tmem_ld32_async<64>(sp + 64, s);
+				tmem_ld32_async<96>(sp + 96, s);
+				tmem_wait_ld();
+				pin(s);
+				if (__any_sync(kFull, from > 0 || to < kTile - 1)) {
+#pragma unroll
+					for (int x = 0; x < kTile; ++x)
+						if (x < from || x > to) s[x] = 0xff800000u; // -inf
+				}
+				float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+				for (int x = 0; x < kTile; ++x) mx4[x & 3] = fmaxf(mx4[x & 3], __uint_as_float(s[x]));
+				const float top = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * c;
+				const bool grow = top > mref + 8.0f;
+				if (__any_sync(kFull, grow)) {
+					const float f = grow ? ex2(mref - top) : 1.0f; // mref -inf: 0
+					if (grow) mref = top;
+					l *= f;
+					if (k > 0) { // the products into O so far are complete: they were issued before these scores
+#pragma unroll 1
+						for (int x = 0; x < DV; x += 32) {
+							uint32_t o[32];
+							tmem_ld32_async<0>(op + x, o);
+							tmem_wait_ld();
+							pin(o);
+#pragma unroll
+							for (int y = 0; y < 32; ++y) o[y] = __float_as_uint(__uint_as_float(o[y]) * f);
+							tmem_st32<0>(op + x, o);
+						}
+					}
+				}
+				const float ref = mref == -INFINITY ? 0.f : mref; // a row may see nothing yet: all its weights are then 0
+				float l4[4] = {0.f, 0.f, 0.f, 0.f};
+				uint32_t p[kTile / 2];
+#pragma unroll
+				for (int x = 0; x < kTile; x += 2) {
+					const float w0 = ex2(fmaf(__uint_as_float(s[x]), c, -ref)), w1 = ex2(fmaf(__uint_as_float(s[x + 1]), c, -ref));
+					l4[x & 2] += w0, l4[(x & 2) + 1] += w1;
+					p[x / 2] = pack2<T>(w0, w1);
+				}
+				tmem_st32<0>(sp, p);
+				tmem_st32<32>(sp + 32, p);
+				l += (l4[0] + l4[1]) + (l4[2] + l4[3]);
+				tmem_wait_st();
+				tc_fence_before();
+				__syncwarp();
+				if (lane == 0) mbar_arrive(p_full0 + 8 * t);
+			}
+			mbar_wait(o_full, 0, dead);
+			__syncwarp();
+			tc_fence_after();
+		}
+	}
+
+	// ---- the rows' results: this part finishes columns part DV / parts .. of both tiles ----
+	const bool softmax_warp = warp >= 4;
+	const int t = (warp - 4) >> 2, q = warp & 3, tr = q * 32 + lane, row = r0 + t * kTile + tr, share = DV / parts;
+	const uint32_t op = tmem + ((uint32_t)(q * 32) << 16) + 256 + t * SH::DVP;
+	// from the start of shared memory (queries and stages are done with): [other part][tile][4 columns][row][4], then (reference, sum) [part][row of 256]
+	const uint32_t ml0 = base + (uint32_t)((parts - 1) * 2 * share * kTile * 4);
+	__syncwarp();
+	if (parts > 1) {
+		cluster_sync(); // every part is done with its shared memory
+		if (softmax_warp && t < nt) {
+			for (int p = 0; p < parts; ++p) {
+				const uint32_t there = map_rank(base, (uint32_t)p);
+				asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(there + (ml0 - base) + (uint32_t)((part * 2 * kTile + t * kTile + tr) * 8)), "f"(mref), "f"(l)
+				             : "memory");
+				if (p == part || nk == 0) continue;
+				const uint32_t dst = there + (uint32_t)(((part < p ? part : part - 1) * 2 + t) * share * kTile * 4);
+				for (int x = 0; x < share; x += 8) {
+					float v[8];
+					tmem_ld8(op + p * share + x, v);
+					st_cluster4(dst + (uint32_t)(((x >> 2) * kTile + tr) * 16), make_float4(v[0], v[1], v[2], v[3]));
+					st_cluster4(dst + (uint32_t)((((x >> 2) + 1) * kTile + tr) * 16), make_float4(v[4], v[5], v[6], v[7]));
+				}
+			}
+		}
+		__syncwarp();
+		cluster_sync(); // the other parts' share of these columns is here
+	}
+	if (softmax_warp && t < nt) {
+		float M = mref, Lsum = l;
+		auto of_part = [&](int p, float &pm, float &pl) {
+			asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(pm), "=f"(pl) : "r"(ml0 + (uint32_t)((p * 2 * kTile + t * kTile + tr) * 8)) : "memory");
+		};
+		if (parts > 1) {
+			M = -INFINITY, Lsum = 0.f;
+			for (int p = 0; p < parts; ++p) {
+				float pm, pl;
+				of_part(p, pm, pl);
+				M = fmaxf(M, pm);
+			}
+			for (int p = 0; p < parts; ++p) {
+				float pm, pl;
+				of_part(p, pm, pl);
+				if (pl > 0.f) Lsum += pl * ex2(pm - M);
+			}
+		}
+		const int i = min(row, rows - 1) / a.G, h = g * a.G + min(row, rows - 1) % a.G;
+		float f = LAYERED ? stack::softmax_finish(M * 0.69314718055994531f, Lsum, a.sink, h) : 1.0f / Lsum;
+		if (dead) f = __int_as_float(0x7fc00000);
+		for (int x = 0; x < share; x += 8) {
+			float v[8];
+#pragma unroll
+			for (int y = 0; y < 8; ++y) v[y] = 0.f;
+			for (int p = 0; p < parts; ++p) { // the parts of the keys in order
+				float w = 1.0f;
+				if (parts > 1) {
+					float pm, pl;
+					of_part(p, pm, pl);
+					w = pl > 0.f ? ex2(pm - M) : 0.f;
+				}
+				if (p == part) {
+					float own[8];
+					__syncwarp();
+					tmem_ld8(op + part * share + x, own);
+					if (nk > 0 && w > 0.f)
+#pragma unroll
+						for (int y = 0; y < 8; ++y) v[y] += w * own[y];
+				} else if (w > 0.f) {
+					const uint32_t src = base + (uint32_t)(((p < part ? p : p - 1) * 2 + t) * share * kTile * 4);
+					const float4 lo = ld_shared4(src + (uint32_t)(((x >> 2) * kTile + tr) * 16)), hi = ld_shared4(src + (uint32_t)((((x >> 2) + 1) * kTile + tr) * 16));
+					v[0] += w * lo.x, v[1] += w * lo.y, v[2] += w * lo.z, v[3] += w * lo.w, v[4] += w * hi.x, v[5] += w * hi.y, v[6] += w * hi.z, v[7] += w * hi.w;
+				}
+			}
+			if (row < rows) {
+				const int col = h * DV + part * share + x;
+				if constexpr (LAYERED) {
+					float *dst = static_cast<float *>(a.out) + (size_t)i * a.ldo + col;
+#pragma unroll
+					for (int y = 0; y < 8; y += 2) *reinterpret_cast<float2 *>(dst + y) = make_float2(v[y] * f, v[y + 1] * f);
+				} else {
+					uint4 pk;
+					pk.x = pack2<T>(v[0] * f, v[1] * f), pk.y = pack2<T>(v[2] * f, v[3] * f), pk.z = pack2<T>(v[4] * f, v[5] * f), pk.w = pack2<T>(v[6] * f, v[7] * f);
+					T *dst = static_cast<T *>(a.out) + (size_t)i * a.n_kv * a.G * DV + col;
+					if (a.wide) {
+						*reinterpret_cast<uint4 *>(dst) = pk;
+					} else {
+						uint32_t *d32 = reinterpret_cast<uint32_t *>(dst);
+						d32[0] = pk.x, d32[1] = pk.y, d32[2] = pk.z, d32[3] = pk.w;
+					}
+				}
+			}
+		}
+	}
+	tc_fence_before();
+	__syncthreads();
+	if (warp == 1) {
+		tc_fence_after();
+		tmem_dealloc<1>(tmem, 512);
+	}
+}
+
+// ---- host side ------------------------------------------------------------------------------------------------------
+typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
+                                  const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+static EncodeTiledFn encode_fn() {
+	static EncodeTiledFn fn = nullptr;
+	static std::once_flag once;
+	std::call_once(once, [] {
+		void *p = nullptr;
+		cudaDriverEntryPointQueryResult q;
+		if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
+			fn = reinterpret_cast<EncodeTiledFn>(p);
+	});
+	return fn;
+}
+// (heads, ring, d) ring of which `rows` slots count -> boxes of 64 channels x 128 slots of one head; channels and slots past the end are zero
+static int make_map(CUtensorMap *map, const void *ptr, int d, int rows, int ring, int heads, bool bf16) {
+	EncodeTiledFn fn = encode_fn();
+	if (!fn) return YALM_EINVAL;
+	const cuuint64_t dims[3] = {(cuuint64_t)d, (cuuint64_t)rows, (cuuint64_t)heads};
+	const cuuint64_t strides[2] = {(cuuint64_t)d * 2, (cuuint64_t)ring * d * 2};
+	const cuuint32_t box[3] = {64, kTile, 1}, estr[3] = {1, 1, 1};
+	const CUresult r = fn(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void *>(ptr), dims, strides, box, estr,
+	                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+	                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+	return r == CUDA_SUCCESS ? 0 : YALM_EINVAL;
+}
+
+// Parts of the keys: as many as still give every CTA an SM and at least 3 key tiles (the exchange costs about two).  est_tiles: key
+// tiles of the longest rows.
+template <typename T, int DK, int DV, bool LAYERED>
+static int launch(Args &a, const void *keys, const void *values, int map_rows, int est_tiles, cudaStream_t st) {
+	using SH = Shape<DK, DV>;
+	static bool configured[kMaxDevices];
+	static std::mutex mu;
+	auto kernel = prompt_attn_kernel<T, DK, DV, LAYERED>;
+	const DeviceInfo &dev = device_info();
+	if (dev.device < 0 || dev.device >= kMaxDevices) return YALM_EINVAL;
+	{
+		std::lock_guard<std::mutex> lock(mu);
+		if (!configured[dev.device]) {
+			YALM_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SH::SMEM));
+			configured[dev.device] = true;
+		}
+	}
+	CUtensorMap tk, tv;
+	int rc = make_map(&tk, keys, DK, map_rows, a.ring, a.n_kv, LAYERED);
+	if (!rc) rc = make_map(&tv, values, DV, map_rows, a.ring, a.v_heads, LAYERED);
+	if (rc) return rc;
+	const int pairs = (a.n * a.G + 2 * kTile - 1) / (2 * kTile), units = pairs * a.n_kv;
+	a.parts = 1;
+	while (a.parts * 2 <= std::min(8, DV / 8) && units * a.parts * 2 <= (a.parts == 1 ? dev.sms : 128) && est_tiles >= 6 * a.parts) a.parts *= 2;
+	cudaLaunchConfig_t cfg = {};
+	cfg.gridDim = dim3(pairs * a.parts, a.n_kv), cfg.blockDim = dim3(kThreads), cfg.dynamicSmemBytes = SH::SMEM, cfg.stream = st;
+	cudaLaunchAttribute at[1];
+	at[0].id = cudaLaunchAttributeClusterDimension;
+	at[0].val.clusterDim.x = a.parts, at[0].val.clusterDim.y = 1, at[0].val.clusterDim.z = 1;
+	cfg.attrs = at, cfg.numAttrs = 1;
+	YALM_TRY(cudaLaunchKernelEx(&cfg, kernel, tk, tv, a));
+	return 0;
+}
+
+constexpr float kLog2e = 1.4426950408889634f;
+
+// Causal attention over an fp16 ring without wrap (slot = position): rows past the portion's last position are zero-filled by the copies.
+int causal_f16(void *out, const void *q, const void *keys, const void *values, int n, int pos0, int n_heads, int n_kv, int head_dim, int max_seq_len,
+               cudaStream_t st) {
+	Args a{};
+	a.out = out, a.q = q, a.n = n, a.G = n_heads / n_kv, a.n_kv = n_kv, a.v_heads = n_kv, a.ring = max_seq_len, a.pos0 = pos0;
+	a.q_sign = 1.f, a.c = kLog2e / sqrtf((float)head_dim), a.wide = ((uintptr_t)out & 15) == 0;
+	const int rows = pos0 + n, est = (rows + kTile - 1) / kTile;
+	switch (head_dim) {
+	case 128: return launch<__half, 128, 128, false>(a, keys, values, rows, est, st);
+	case 64: return launch<__half, 64, 64, false>(a, keys, values, rows, est, st);
+	case 32: return launch<__half, 32, 32, false>(a, keys, values, rows, est, st);
+	}
+	return YALM_EINVAL;
+}
+
+int window_bf16(float *out, int ldo, const float *q, int ldq, const void *keys, const void *values, const float *key_pool, const float *value_pool, int n,
+                int n_heads, int n_kv, int dk, int dv, int ring, int max_blocks, int window, int pool, float scale, int pos0, const int *ctl, const float *sink,
+                int v_heads, cudaStream_t st) {
+	Args a{};
+	a.out = out, a.ldo = ldo, a.q = q, a.ldq = ldq, a.key_pool = key_pool, a.value_pool = value_pool, a.sink = sink;
+	a.n = n, a.G = n_heads / n_kv, a.n_kv = n_kv, a.v_heads = v_heads, a.ring = ring, a.max_blocks = max_blocks, a.window = window;
+	a.pool = key_pool ? pool : 0, a.pos0 = pos0, a.ctl = ctl;
+	a.q_sign = scale > 0.f ? 1.f : scale < 0.f ? -1.f : 0.f, a.c = scale == 0.f ? 1.f : fabsf(scale) * kLog2e; // the maximum is taken before the scale
+	int seen = ctl ? ring : pos0 + n; // positions that the longest row can see (the position of a control block is known on the device only)
+	if (window > 0) seen = std::min(seen, window + 2 * kTile / a.G);
+	const int est = (std::min(seen, ring) + kTile - 1) / kTile;
+#define YALM_WINDOW_CASE(K_, V_) \
+	if (dk == K_ && dv == V_) return launch<__nv_bfloat16, K_, V_, true>(a, keys, values, ring, est, st)
+	YALM_WINDOW_CASE(64, 32);
+	YALM_WINDOW_CASE(64, 64);
+	YALM_WINDOW_CASE(64, 128);
+	YALM_WINDOW_CASE(128, 32);
+	YALM_WINDOW_CASE(128, 64);
+	YALM_WINDOW_CASE(128, 128);
+#undef YALM_WINDOW_CASE
+	return YALM_EINVAL;
+}
+
+} // namespace prompt
+} // namespace yalm
