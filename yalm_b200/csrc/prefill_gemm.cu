@@ -167,7 +167,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
 	const uint32_t a_bytes = 128 * kRowBytes, b_bytes = (uint32_t)(nacc / 2) * kRowBytes, stage_bytes = a_bytes + b_bytes;
 	const uint32_t base = (s32(smem_raw) + 1023u) & ~1023u, patch0 = base + g.stages * stage_bytes, bars = patch0 + 4 * kPatch;
 	const uint32_t full0 = bars, empty0 = bars + 8 * g.stages, acc_full0 = empty0 + 8 * g.stages, acc_empty0 = acc_full0 + 16, tslot = acc_empty0 + 16;
-	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+	const int warp = uniform_warp(), lane = threadIdx.x & 31;
 	const int rank = (int)cluster_rank(), half = rank & 1, part = rank >> 1; // CTA of its pair; the pair's part of K
 	const int csize = 2 * g.splits, cluster = blockIdx.x / csize, nclusters = gridDim.x / csize;
 	const int nkb = (g.K + BK - 1) / BK, kb0 = part * g.kb_per, kb1 = min(nkb, kb0 + g.kb_per);
@@ -186,7 +186,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
 	asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(tslot));
 
 	if (warp == 0) {
-		if (lane == 0) { // ---- TMA producer: this CTA's rows of both operands, counted on the first CTA's barrier ----
+		{ // ---- TMA producer: this CTA's rows of both operands, counted on the first CTA's barrier ----
 			const uint32_t lead_full0 = map_rank(full0, rank & ~1);
 			Ring ring;
 			ring.phase = 1; // the first round of every stage is free
@@ -197,18 +197,20 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
 				const CUtensorMap *w = B_SEG ? &tb.m[seg] : GLU ? &tb.m[half] : &tb.m[0];
 				const int b0 = GLU ? n0 : (B_SEG ? n0 - seg0 : n0) + half * (nacc / 2);
 				for (int kb = kb0; kb < kb1; ++kb, ring.next(g.stages)) {
-					mbar_wait(empty0 + 8 * ring.s, ring.phase, dead);
+					mbar_wait_warp(empty0 + 8 * ring.s, ring.phase, dead);
 					if (dead) break;
 					const uint32_t dst = base + ring.s * stage_bytes, bar = lead_full0 + 8 * ring.s;
-					if (half == 0) mbar_expect_tx(full0 + 8 * ring.s, 2 * stage_bytes);
-					tma_load_2d<2>(dst, &ta, kb * BK, a0, bar);
-					tma_load_2d<2>(dst + a_bytes, w, kb * BK, b0, bar);
+					if (elect_one()) {
+						if (half == 0) mbar_expect_tx(full0 + 8 * ring.s, 2 * stage_bytes);
+						tma_load_2d<2>(dst, &ta, kb * BK, a0, bar);
+						tma_load_2d<2>(dst + a_bytes, w, kb * BK, b0, bar);
+					}
 				}
 			}
 		}
 		__syncwarp();
 	} else if (warp == 1) {
-		if (lane == 0 && half == 0) { // ---- MMA issuer, for both CTAs ----
+		if (half == 0) { // ---- MMA issuer, for both CTAs ----
 			const uint32_t idesc = instr_desc_f16(256, nacc) | (g.bf16 ? kInstrDescBf16 : 0u);
 			const uint16_t pair_mask = (uint16_t)(3u << (rank & ~1));
 			const uint64_t adesc0 = smem_desc_sw128(base), bdesc0 = smem_desc_sw128(base + a_bytes);
@@ -216,20 +218,23 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
 			int done = 0;
 			for (int item = cluster; item < g.items; item += nclusters, ++done) {
 				const int b = done & 1;
-				if (done >= 2) mbar_wait(acc_empty0 + 8 * b, (uint32_t)(done / 2 - 1) & 1u, dead);
+				if (done >= 2) mbar_wait_warp(acc_empty0 + 8 * b, (uint32_t)(done / 2 - 1) & 1u, dead);
 				tc_fence_after();
 				uint32_t more = 0;
 				for (int kb = kb0; kb < kb1; ++kb, ring.next(g.stages)) {
-					mbar_wait(full0 + 8 * ring.s, ring.phase, dead);
+					mbar_wait_warp(full0 + 8 * ring.s, ring.phase, dead);
 					if (dead) break;
 					tc_fence_after();
 					const uint64_t at = (uint64_t)((ring.s * stage_bytes) >> 4);
+					if (elect_one()) {
 #pragma unroll
-					for (int k = 0; k < BK / 16; ++k, more = 1) // 16 elements = 32 bytes further along K, inside the 128-byte swizzle row
-						umma_f16<2>(tmem + 256 * b, adesc0 + at + 2 * k, bdesc0 + at + 2 * k, idesc, more);
-					umma_commit_pair(empty0 + 8 * ring.s, pair_mask); // the stage is free in both CTAs once these MMAs have read it
+						for (int k = 0; k < BK / 16; ++k) // 16 elements = 32 bytes further along K, inside the 128-byte swizzle row
+							umma_f16<2>(tmem + 256 * b, adesc0 + at + 2 * k, bdesc0 + at + 2 * k, idesc, more | k);
+						umma_commit_pair(empty0 + 8 * ring.s, pair_mask); // the stage is free in both CTAs once these MMAs have read it
+					}
+					more = 1;
 				}
-				umma_commit_pair(acc_full0 + 8 * b, pair_mask); // the accumulator is complete
+				if (elect_one()) umma_commit_pair(acc_full0 + 8 * b, pair_mask); // the accumulator is complete
 			}
 		}
 		__syncwarp();
@@ -241,7 +246,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
 			int seg, seg0, n0, n_end;
 			tile_columns(g, item / g.m_tiles, seg, seg0, n0, n_end);
 			const int b = done & 1, row0 = (item % g.m_tiles) * 256 + half * 128 + q * 32;
-			mbar_wait(acc_full0 + 8 * b, (uint32_t)(done / 2) & 1u, dead);
+			mbar_wait_warp(acc_full0 + 8 * b, (uint32_t)(done / 2) & 1u, dead);
 			__syncwarp();
 			tc_fence_after();
 			const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16) + 256 * b;
@@ -276,7 +281,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
 		const int mats = GLU ? 2 : 1, words = share * mats * 128; // floats that one pair sends another (per CTA)
 		const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16);
 		if (warp >= 2) {
-			mbar_wait(acc_full0, 0, dead);
+			mbar_wait_warp(acc_full0, 0, dead);
 			__syncwarp();
 			tc_fence_after();
 		}
@@ -360,7 +365,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ 
 	const uint32_t w_bytes = 128 * kRowBytes, a_bytes = (uint32_t)np * kRowBytes, stage_bytes = MATS * w_bytes + a_bytes;
 	const uint32_t base = (s32(smem_raw) + 1023u) & ~1023u, bars = base + g.stages * stage_bytes;
 	const uint32_t full0 = bars, empty0 = bars + 8 * g.stages, acc_bar = empty0 + 8 * g.stages, tslot = acc_bar + 8;
-	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+	const int warp = uniform_warp(), lane = threadIdx.x & 31;
 	const int part = g.splits > 1 ? (int)cluster_rank() : 0, tile = blockIdx.x / g.splits;
 	const int nkb = (g.K + BK - 1) / BK, kb0 = part * g.kb_per, kb1 = min(nkb, kb0 + g.kb_per);
 	const uint32_t cols = MATS * np <= 32 ? 32 : MATS * np <= 64 ? 64 : MATS * np <= 128 ? 128 : 256; // TMEM columns
@@ -381,41 +386,46 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ 
 	asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(tslot));
 
 	if (warp == 0) {
-		if (lane == 0) { // ---- TMA producer ----
+		{ // ---- TMA producer ----
 			const CUtensorMap *w = &tb.m[B_SEG ? seg : 0];
 			const int w0 = B_SEG ? n0 - seg0 : n0;
 			Ring ring;
 			ring.phase = 1; // the first round of every stage is free
 			for (int kb = kb0; kb < kb1; ++kb, ring.next(g.stages)) {
-				mbar_wait(empty0 + 8 * ring.s, ring.phase, dead);
+				mbar_wait_warp(empty0 + 8 * ring.s, ring.phase, dead);
 				if (dead) break;
 				const uint32_t dst = base + ring.s * stage_bytes, bar = full0 + 8 * ring.s;
-				mbar_expect_tx(bar, stage_bytes);
-				tma_load_2d<1>(dst, w, kb * BK, w0, bar);
-				if (GLU) tma_load_2d<1>(dst + w_bytes, &tb.m[1], kb * BK, w0, bar);
-				tma_load_2d<1>(dst + MATS * w_bytes, &ta, kb * BK, seg * g.a_step, bar);
+				if (elect_one()) {
+					mbar_expect_tx(bar, stage_bytes);
+					tma_load_2d<1>(dst, w, kb * BK, w0, bar);
+					if (GLU) tma_load_2d<1>(dst + w_bytes, &tb.m[1], kb * BK, w0, bar);
+					tma_load_2d<1>(dst + MATS * w_bytes, &ta, kb * BK, seg * g.a_step, bar);
+				}
 			}
 		}
 		__syncwarp();
 	} else if (warp == 1) {
-		if (lane == 0) { // ---- MMA issuer ----
+		{ // ---- MMA issuer ----
 			const uint32_t idesc = instr_desc_f16(128, np) | (g.bf16 ? kInstrDescBf16 : 0u);
 			const uint64_t wdesc0 = smem_desc_sw128(base), vdesc0 = smem_desc_sw128(base + w_bytes), adesc0 = smem_desc_sw128(base + MATS * w_bytes);
 			Ring ring;
 			uint32_t more = 0;
 			for (int kb = kb0; kb < kb1; ++kb, ring.next(g.stages)) {
-				mbar_wait(full0 + 8 * ring.s, ring.phase, dead);
+				mbar_wait_warp(full0 + 8 * ring.s, ring.phase, dead);
 				if (dead) break;
 				tc_fence_after();
 				const uint64_t at = (uint64_t)((ring.s * stage_bytes) >> 4);
+				if (elect_one()) {
 #pragma unroll
-				for (int k = 0; k < BK / 16; ++k, more = 1) {
-					umma_f16<1>(tmem, wdesc0 + at + 2 * k, adesc0 + at + 2 * k, idesc, more);
-					if (GLU) umma_f16<1>(tmem + np, vdesc0 + at + 2 * k, adesc0 + at + 2 * k, idesc, more);
+					for (int k = 0; k < BK / 16; ++k) {
+						umma_f16<1>(tmem, wdesc0 + at + 2 * k, adesc0 + at + 2 * k, idesc, more | k);
+						if (GLU) umma_f16<1>(tmem + np, vdesc0 + at + 2 * k, adesc0 + at + 2 * k, idesc, more | k);
+					}
+					umma_commit(empty0 + 8 * ring.s);
 				}
-				umma_commit(empty0 + 8 * ring.s);
+				more = 1;
 			}
-			umma_commit(acc_bar);
+			if (elect_one()) umma_commit(acc_bar);
 		}
 		__syncwarp();
 	}
@@ -425,7 +435,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ 
 	// words of a group of 8 positions: [matrix][4-position half][row][4]
 	auto slot = [&](uint32_t buf, int src, int group, int m, int j) { return buf + (uint32_t)((((src * mine + group / g.splits) * MATS + m) * 2 + j) * 128 + row) * 16; };
 	if (warp >= 2) {
-		mbar_wait(acc_bar, 0, dead);
+		mbar_wait_warp(acc_bar, 0, dead);
 		__syncwarp();
 		tc_fence_after();
 	}

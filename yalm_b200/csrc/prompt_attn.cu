@@ -43,7 +43,7 @@ struct Args {
 	const int *ctl;
 	float q_sign, c; // score (in powers of two) = c (q q_sign) . k
 	int parts;
-	int wide; // fp16 output rows are 16-byte aligned
+	int wide; // output rows are 16-byte aligned
 };
 
 // Key tiles of a CTA's rows: pooled blocks in tiles of 128 first, then the positions lo .. last in runs of slots that end at the ring's end.
@@ -96,6 +96,28 @@ __device__ __forceinline__ float ex2(float x) {
 	float y;
 	asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
 	return y;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+	float y;
+	asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+	return y;
+}
+// two fp32 values in one 64-bit register: the packed FMA and add of sm_100 (same rounding, half the issue slots)
+__device__ __forceinline__ uint64_t pack64(uint32_t lo, uint32_t hi) {
+	uint64_t r;
+	asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
+	return r;
+}
+__device__ __forceinline__ void unpack64(uint64_t v, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+	uint64_t r;
+	asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+	return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+	uint64_t r;
+	asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+	return r;
 }
 #define YALM_R32(r, o)                                                                                                                               \
 	"=r"(r[o]), "=r"(r[o + 1]), "=r"(r[o + 2]), "=r"(r[o + 3]), "=r"(r[o + 4]), "=r"(r[o + 5]), "=r"(r[o + 6]), "=r"(r[o + 7]), "=r"(r[o + 8]),      \
@@ -167,9 +189,9 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 	constexpr int NST = SH::STAGES;
 	extern __shared__ uint8_t smem_raw[];
 	const uint32_t base = (s32(smem_raw) + 1023u) & ~1023u, q0 = base, kv0 = q0 + 2 * SH::Q_BYTES, bars = kv0 + NST * SH::STAGE;
-	const uint32_t full0 = bars, empty0 = full0 + 8 * NST, s_full0 = empty0 + 8 * NST, p_full0 = s_full0 + 16, o_full = p_full0 + 16, v_clean0 = o_full + 8,
+	const uint32_t full0 = bars, empty0 = full0 + 8 * NST, s_full0 = empty0 + 8 * NST, p_full0 = s_full0 + 16, o_full = p_full0 + 32, v_clean0 = o_full + 8,
 	               tslot = v_clean0 + 8 * NST;
-	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+	const int warp = uniform_warp(), lane = threadIdx.x & 31;
 	const int parts = a.parts, part = parts > 1 ? (int)cluster_rank() : 0;
 	const int rows = a.n * a.G, pairs = (rows + 2 * kTile - 1) / (2 * kTile);
 	const int pair = pairs - 1 - (int)(blockIdx.x / parts); // the longest rows first
@@ -184,13 +206,15 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 	// for, also where the entry is not a copy: a parity tells neighbouring rounds apart and no more.
 	auto load = [&](int i, int is_v) {
 		const int e = 2 * i + is_v, s = e % NST;
-		if (e >= NST) mbar_wait(empty0 + 8 * s, (uint32_t)(e / NST - 1) & 1u, dead);
+		if (e >= NST) mbar_wait_warp(empty0 + 8 * s, (uint32_t)(e / NST - 1) & 1u, dead);
 		int slot, pos, valid;
 		if (tiles.at(k_begin + i, slot, pos, valid) || dead) return; // pooled tiles are filled by other warps
 		const uint32_t dst = kv0 + s * SH::STAGE, bar = full0 + 8 * s;
-		mbar_expect_tx(bar, is_v ? SH::V_BYTES : SH::K_BYTES);
 		const int d = is_v ? SH::DVP : SH::DKP, head = is_v ? g % a.v_heads : g;
-		for (int c = 0; c < d; c += 64) tma_load_3d(dst + (c / 64) * (kTile * 128), is_v ? &tv : &tk, c, slot, head, bar);
+		if (elect_one()) {
+			mbar_expect_tx(bar, is_v ? SH::V_BYTES : SH::K_BYTES);
+			for (int c = 0; c < d; c += 64) tma_load_3d(dst + (c / 64) * (kTile * 128), is_v ? &tv : &tk, c, slot, head, bar);
+		}
 	};
 	// a pooled tile's means into its two stages, rounded; rows past the last block are zero
 	auto fill_pooled = [&](int i, int tid, int nthreads) {
@@ -219,31 +243,48 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 	if (threadIdx.x == 0) {
 		// a value stage (odd) is free again once its products are done and, in a layered model, warps 2 and 3 have passed it
 		for (int i = 0; i < NST; ++i) mbar_init(full0 + 8 * i, 1), mbar_init(empty0 + 8 * i, LAYERED && (i & 1) ? 3 : 1);
-		for (int i = 0; i < 2; ++i) mbar_init(s_full0 + 8 * i, 1), mbar_init(p_full0 + 8 * i, 4);
+		for (int i = 0; i < 2; ++i) mbar_init(s_full0 + 8 * i, 1);
+		for (int i = 0; i < 4; ++i) mbar_init(p_full0 + 8 * i, 4); // [tile][half of the keys]
 		mbar_init(o_full, 1);
 		if (LAYERED)
 			for (int i = 0; i < NST; ++i) mbar_init(v_clean0 + 8 * i, 1);
 		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+	}
+	if (warp == 0) {
+		__syncwarp();
 		for (int e = 0; e < NST && e < 2 * nk; ++e) load(e >> 1, e & 1); // the stages are free: the first tiles travel while the queries are staged
 	}
 	if (warp == 1) tmem_alloc<1>(tslot, 512);
 	if (warp > 0) { // the queries' rows (rows past the last: zero), and the first tile where it is a pooled one
-		constexpr int PIECES = DK / 8;
-		for (int x = threadIdx.x - 32; x < 2 * kTile * PIECES; x += kThreads - 32) {
-			const int r = x / PIECES, c = x % PIECES, row = r0 + r;
-			float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-			if (row < rows) {
-				const int i = row / a.G, h = g * a.G + row % a.G;
-				if constexpr (LAYERED) {
-					const float *src = static_cast<const float *>(a.q) + (size_t)i * a.ldq + (size_t)h * DK + c * 8;
-					const float4 lo = *reinterpret_cast<const float4 *>(src), hi = *reinterpret_cast<const float4 *>(src + 4);
-					const float f = a.q_sign;
-					v = make_float4(__uint_as_float(pack2<T>(lo.x * f, lo.y * f)), __uint_as_float(pack2<T>(lo.z * f, lo.w * f)),
-					                __uint_as_float(pack2<T>(hi.x * f, hi.y * f)), __uint_as_float(pack2<T>(hi.z * f, hi.w * f)));
-				} else
-					v = *reinterpret_cast<const float4 *>(static_cast<const T *>(a.q) + ((size_t)i * a.n_kv * a.G + h) * DK + c * 8);
+		constexpr int PIECES = DK / 8, ALL = 2 * kTile * PIECES, STEP = kThreads - 32, BATCH = LAYERED ? 6 : 12;
+		for (int x0 = threadIdx.x - 32; x0 < ALL; x0 += BATCH * STEP) { // several loads in flight: one at a time this took as long as four key tiles
+			float4 lo[BATCH], hi[LAYERED ? BATCH : 1];
+#pragma unroll
+			for (int b = 0; b < BATCH; ++b) {
+				const int x = x0 + b * STEP, r = x / PIECES, c = x % PIECES, row = r0 + r;
+				lo[b] = make_float4(0.f, 0.f, 0.f, 0.f);
+				if constexpr (LAYERED) hi[b] = lo[b];
+				if (x < ALL && row < rows) {
+					const int i = row / a.G, h = g * a.G + row % a.G;
+					if constexpr (LAYERED) {
+						const float *src = static_cast<const float *>(a.q) + (size_t)i * a.ldq + (size_t)h * DK + c * 8;
+						lo[b] = *reinterpret_cast<const float4 *>(src), hi[b] = *reinterpret_cast<const float4 *>(src + 4);
+					} else
+						lo[b] = *reinterpret_cast<const float4 *>(static_cast<const T *>(a.q) + ((size_t)i * a.n_kv * a.G + h) * DK + c * 8);
+				}
 			}
-			st_shared4(q0 + (r / kTile) * SH::Q_BYTES + tile_at(r % kTile, c), v);
+#pragma unroll
+			for (int b = 0; b < BATCH; ++b) {
+				const int x = x0 + b * STEP, r = x / PIECES, c = x % PIECES;
+				if (x >= ALL) break;
+				float4 v = lo[b];
+				if constexpr (LAYERED) {
+					const float f = a.q_sign;
+					v = make_float4(__uint_as_float(pack2<T>(lo[b].x * f, lo[b].y * f)), __uint_as_float(pack2<T>(lo[b].z * f, lo[b].w * f)),
+					                __uint_as_float(pack2<T>(hi[b].x * f, hi[b].y * f)), __uint_as_float(pack2<T>(hi[b].z * f, hi[b].w * f)));
+				}
+				st_shared4(q0 + (r / kTile) * SH::Q_BYTES + tile_at(r % kTile, c), v);
+			}
 		}
 		if constexpr (LAYERED)
 			if (first_pooled) fill_pooled(0, threadIdx.x - 32, kThreads - 32);
@@ -258,32 +299,32 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 	float mref = -INFINITY, l = 0.f; // of this thread's row: reference of the weights (in powers of two), their sum
 
 	if (warp == 0) {
-		if (lane == 0) {
-			if (first_pooled) mbar_arrive(full0), mbar_arrive(full0 + 8);
-			for (int e = NST; e < 2 * nk; ++e) load(e >> 1, e & 1);
-		}
+		if (first_pooled && elect_one()) mbar_arrive(full0), mbar_arrive(full0 + 8);
+		for (int e = NST; e < 2 * nk; ++e) load(e >> 1, e & 1);
 		__syncwarp();
 	} else if (warp == 1) {
-		if (lane == 0 && nk > 0) { // ---- products ----
+		if (nk > 0) { // ---- products ----
 			constexpr uint32_t fmt = __is_same(T, __half) ? 0u : kInstrDescBf16;
 			const uint32_t qk_desc = instr_desc_f16(128, kTile) | fmt, pv_desc = instr_desc_f16(128, SH::DVP) | fmt | kBMajorMn;
 			auto wait_full = [&](int e) {
-				mbar_wait(full0 + 8 * (e % NST), (uint32_t)(e / NST) & 1u, dead);
+				mbar_wait_warp(full0 + 8 * (e % NST), (uint32_t)(e / NST) & 1u, dead);
 				tc_fence_after();
 			};
 			auto scores = [&](int t, int e) {
-				const uint32_t qa = q0 + t * SH::Q_BYTES, ka = kv0 + (e % NST) * SH::STAGE;
+				const uint64_t qa = smem_desc_sw128(q0 + t * SH::Q_BYTES), ka = smem_desc_sw128(kv0 + (e % NST) * SH::STAGE);
+				if (elect_one()) {
 #pragma unroll
-				for (int k = 0; k < DK / 16; ++k) {
-					const uint32_t off = (k >> 2) * (kTile * 128) + (k & 3) * 32;
-					umma_f16<1>(tmem + t * kTile, smem_desc_sw128(qa + off), smem_desc_sw128(ka + off), qk_desc, k);
+					for (int k = 0; k < DK / 16; ++k) {
+						const uint32_t off = ((k >> 2) * (kTile * 128) + (k & 3) * 32) >> 4;
+						umma_f16<1>(tmem + t * kTile, qa + off, ka + off, qk_desc, k);
+					}
+					umma_commit(s_full0 + 8 * t);
 				}
-				umma_commit(s_full0 + 8 * t);
 			};
 			uint32_t cleaned = 0; // a bit per stage: parity of its rounds of clearing
 			wait_full(0);
 			for (int t = 0; t < nt; ++t) scores(t, 0);
-			umma_commit(empty0);
+			if (elect_one()) umma_commit(empty0);
 			for (int i = 0; i < nk && !dead; ++i) {
 				const int ev = 2 * i + 1, ek = 2 * i + 2;
 				wait_full(ev);
@@ -291,27 +332,32 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 					int slot, pos, valid;
 					if (!tiles.at(k_begin + i, slot, pos, valid) && valid < kTile) {
 						const int sv = ev % NST;
-						mbar_wait(v_clean0 + 8 * sv, (cleaned >> sv) & 1u, dead);
+						mbar_wait_warp(v_clean0 + 8 * sv, (cleaned >> sv) & 1u, dead);
 						cleaned ^= 1u << sv;
 						tc_fence_after();
 					}
 				}
 				const uint64_t vdesc = desc_mn(kv0 + (ev % NST) * SH::STAGE);
 				for (int t = 0; t < nt; ++t) {
-					mbar_wait(p_full0 + 8 * t, (uint32_t)i & 1u, dead);
-					tc_fence_after();
 #pragma unroll
-					for (int k = 0; k < kTile / 16; ++k) // 16 positions = 2048 bytes further in every sub-tile, 8 columns of P
-						umma_ts(tmem + 256 + t * SH::DVP, tmem + t * kTile + 8 * k, vdesc + (2048 >> 4) * k, pv_desc, (i | k) != 0);
-					if (t == nt - 1) umma_commit(empty0 + 8 * (ev % NST));
+					for (int half = 0; half < 2; ++half) {
+						mbar_wait_warp(p_full0 + 16 * t + 8 * half, (uint32_t)i & 1u, dead);
+						tc_fence_after();
+						if (elect_one()) {
+#pragma unroll
+							for (int k = 4 * half; k < 4 * half + 4; ++k) // 16 positions = 2048 bytes further in every sub-tile, 8 columns of P
+								umma_ts(tmem + 256 + t * SH::DVP, tmem + t * kTile + 8 * k, vdesc + (2048 >> 4) * k, pv_desc, (i | k) != 0);
+							if (half && t == nt - 1) umma_commit(empty0 + 8 * (ev % NST));
+						}
+					}
 					if (i + 1 < nk) {
 						if (t == 0) wait_full(ek);
 						scores(t, ek);
-						if (t == nt - 1) umma_commit(empty0 + 8 * (ek % NST));
+						if (t == nt - 1 && elect_one()) umma_commit(empty0 + 8 * (ek % NST));
 					}
 				}
 			}
-			umma_commit(o_full);
+			if (elect_one()) umma_commit(o_full);
 		}
 		__syncwarp();
 	} else if (warp < 4) {
@@ -322,13 +368,13 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 				const bool pooled = tiles.at(k_begin + i, slot, pos, valid);
 				const int ek = 2 * i, ev = 2 * i + 1;
 				if (pooled && i > 0) {
-					if (ek >= NST) mbar_wait(empty0 + 8 * (ek % NST), (uint32_t)(ek / NST - 1) & 1u, dead);
-					if (ev >= NST) mbar_wait(empty0 + 8 * (ev % NST), (uint32_t)(ev / NST - 1) & 1u, dead);
+					if (ek >= NST) mbar_wait_warp(empty0 + 8 * (ek % NST), (uint32_t)(ek / NST - 1) & 1u, dead);
+					if (ev >= NST) mbar_wait_warp(empty0 + 8 * (ev % NST), (uint32_t)(ev / NST - 1) & 1u, dead);
 					fill_pooled(i, tid, 64);
 					asm volatile("bar.sync 1, 64;" ::: "memory");
 					if (tid == 0) mbar_arrive(full0 + 8 * (ek % NST)), mbar_arrive(full0 + 8 * (ev % NST));
 				}
-				mbar_wait(full0 + 8 * (ev % NST), (uint32_t)(ev / NST) & 1u, dead); // of every tile, to stay with the rounds
+				mbar_wait_warp(full0 + 8 * (ev % NST), (uint32_t)(ev / NST) & 1u, dead); // of every tile, to stay with the rounds
 				if (!pooled && valid < kTile) {
 					const uint32_t dst = kv0 + (ev % NST) * SH::STAGE;
 					constexpr int PIECES = SH::DVP / 8;
@@ -353,7 +399,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 				int slot, pos, valid;
 				const bool pooled = tiles.at(k_begin + k, slot, pos, valid);
 				const int from = pooled ? 0 : lo - pos, to = pooled ? nb - slot - 1 : min(i - pos, valid - 1); // visible: from .. to of the tile
-				mbar_wait(s_full0 + 8 * t, (uint32_t)k & 1u, dead);
+				mbar_wait_warp(s_full0 + 8 * t, (uint32_t)k & 1u, dead);
 				__syncwarp();
 				tc_fence_after();
 				uint32_t s[kTile];
@@ -370,7 +416,9 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 				}
 				float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-				for (int x = 0; x < kTile; ++x) mx4[x & 3] = fmaxf(mx4[x & 3], __uint_as_float(s[x]));
+				for (int x = 0; x < kTile; x += 8)
+#pragma unroll
+					for (int y = 0; y < 4; ++y) mx4[y] = max3(mx4[y], __uint_as_float(s[x + 2 * y]), __uint_as_float(s[x + 2 * y + 1]));
 				const float top = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * c;
 				const bool grow = top > mref + 8.0f;
 				if (__any_sync(kFull, grow)) {
@@ -391,23 +439,30 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 					}
 				}
 				const float ref = mref == -INFINITY ? 0.f : mref; // a row may see nothing yet: all its weights are then 0
-				float l4[4] = {0.f, 0.f, 0.f, 0.f};
-				uint32_t p[kTile / 2];
+				const uint64_t c2 = pack64(__float_as_uint(c), __float_as_uint(c)), ref2 = pack64(__float_as_uint(-ref), __float_as_uint(-ref));
+				uint64_t l2[4] = {0, 0, 0, 0};
 #pragma unroll
-				for (int x = 0; x < kTile; x += 2) {
-					const float w0 = ex2(fmaf(__uint_as_float(s[x]), c, -ref)), w1 = ex2(fmaf(__uint_as_float(s[x + 1]), c, -ref));
-					l4[x & 2] += w0, l4[(x & 2) + 1] += w1;
-					p[x / 2] = pack2<T>(w0, w1);
+				for (int half = 0; half < 2; ++half) { // the first half's products start while the second half's weights are formed
+					uint32_t p[32];
+#pragma unroll
+					for (int x = 0; x < 32; ++x) {
+						float e0, e1;
+						unpack64(fma2(pack64(s[64 * half + 2 * x], s[64 * half + 2 * x + 1]), c2, ref2), e0, e1);
+						e0 = ex2(e0), e1 = ex2(e1);
+						l2[x & 3] = add2(l2[x & 3], pack64(__float_as_uint(e0), __float_as_uint(e1)));
+						p[x] = pack2<T>(e0, e1);
+					}
+					tmem_st32<0>(sp + 32 * half, p);
+					tmem_wait_st();
+					tc_fence_before();
+					__syncwarp();
+					if (lane == 0) mbar_arrive(p_full0 + 16 * t + 8 * half);
 				}
-				tmem_st32<0>(sp, p);
-				tmem_st32<32>(sp + 32, p);
-				l += (l4[0] + l4[1]) + (l4[2] + l4[3]);
-				tmem_wait_st();
-				tc_fence_before();
-				__syncwarp();
-				if (lane == 0) mbar_arrive(p_full0 + 8 * t);
+				float la, lb;
+				unpack64(add2(add2(l2[0], l2[1]), add2(l2[2], l2[3])), la, lb);
+				l += la + lb;
 			}
-			mbar_wait(o_full, 0, dead);
+			mbar_wait_warp(o_full, 0, dead);
 			__syncwarp();
 			tc_fence_after();
 		}
@@ -458,49 +513,65 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 				if (pl > 0.f) Lsum += pl * ex2(pm - M);
 			}
 		}
-		const int i = min(row, rows - 1) / a.G, h = g * a.G + min(row, rows - 1) % a.G;
+		const int h = g * a.G + min(row, rows - 1) % a.G;
 		float f = LAYERED ? stack::softmax_finish(M * 0.69314718055994531f, Lsum, a.sink, h) : 1.0f / Lsum;
 		if (dead) f = __int_as_float(0x7fc00000);
-		for (int x = 0; x < share; x += 8) {
-			float v[8];
+		// through a patch of shared memory per warp (after what the parts exchanged), so that neighbouring lanes store neighbouring
+		// bytes: a row per lane, every 16-byte piece went to a line of its own (5 us for 256 rows of 128)
+		const uint32_t ld = (uint32_t)share * 4 + 16, patch = ml0 + (parts > 1 ? parts * 2 * kTile * 8 : 0) + (warp - 4) * 32 * ld;
+		auto put = [&](int x, float4 v) { st_shared4(patch + lane * ld + x * 4, make_float4(v.x * f, v.y * f, v.z * f, v.w * f)); };
+		if (parts == 1) {
 #pragma unroll
-			for (int y = 0; y < 8; ++y) v[y] = 0.f;
-			for (int p = 0; p < parts; ++p) { // the parts of the keys in order
-				float w = 1.0f;
-				if (parts > 1) {
+			for (int x = 0; x < DV; x += 32) {
+				float v[32];
+				tmem_ld32(op + x, v);
+#pragma unroll
+				for (int y = 0; y < 32; y += 4) put(x + y, make_float4(v[y], v[y + 1], v[y + 2], v[y + 3]));
+			}
+		} else {
+			for (int x = 0; x < share; x += 8) {
+				float v[8], own[8];
+				__syncwarp();
+				tmem_ld8(op + part * share + x, own);
+#pragma unroll
+				for (int y = 0; y < 8; ++y) v[y] = 0.f;
+				for (int p = 0; p < parts; ++p) { // the parts of the keys in order
 					float pm, pl;
 					of_part(p, pm, pl);
-					w = pl > 0.f ? ex2(pm - M) : 0.f;
-				}
-				if (p == part) {
-					float own[8];
-					__syncwarp();
-					tmem_ld8(op + part * share + x, own);
-					if (nk > 0 && w > 0.f)
+					if (!(pl > 0.f)) continue;
+					const float w = ex2(pm - M);
+					if (p == part) {
 #pragma unroll
 						for (int y = 0; y < 8; ++y) v[y] += w * own[y];
-				} else if (w > 0.f) {
-					const uint32_t src = base + (uint32_t)(((p < part ? p : p - 1) * 2 + t) * share * kTile * 4);
-					const float4 lo = ld_shared4(src + (uint32_t)(((x >> 2) * kTile + tr) * 16)), hi = ld_shared4(src + (uint32_t)((((x >> 2) + 1) * kTile + tr) * 16));
-					v[0] += w * lo.x, v[1] += w * lo.y, v[2] += w * lo.z, v[3] += w * lo.w, v[4] += w * hi.x, v[5] += w * hi.y, v[6] += w * hi.z, v[7] += w * hi.w;
-				}
-			}
-			if (row < rows) {
-				const int col = h * DV + part * share + x;
-				if constexpr (LAYERED) {
-					float *dst = static_cast<float *>(a.out) + (size_t)i * a.ldo + col;
-#pragma unroll
-					for (int y = 0; y < 8; y += 2) *reinterpret_cast<float2 *>(dst + y) = make_float2(v[y] * f, v[y + 1] * f);
-				} else {
-					uint4 pk;
-					pk.x = pack2<T>(v[0] * f, v[1] * f), pk.y = pack2<T>(v[2] * f, v[3] * f), pk.z = pack2<T>(v[4] * f, v[5] * f), pk.w = pack2<T>(v[6] * f, v[7] * f);
-					T *dst = static_cast<T *>(a.out) + (size_t)i * a.n_kv * a.G * DV + col;
-					if (a.wide) {
-						*reinterpret_cast<uint4 *>(dst) = pk;
 					} else {
-						uint32_t *d32 = reinterpret_cast<uint32_t *>(dst);
-						d32[0] = pk.x, d32[1] = pk.y, d32[2] = pk.z, d32[3] = pk.w;
+						const uint32_t src = base + (uint32_t)(((p < part ? p : p - 1) * 2 + t) * share * kTile * 4);
+						const float4 lo = ld_shared4(src + (uint32_t)(((x >> 2) * kTile + tr) * 16)), hi = ld_shared4(src + (uint32_t)((((x >> 2) + 1) * kTile + tr) * 16));
+						v[0] += w * lo.x, v[1] += w * lo.y, v[2] += w * lo.z, v[3] += w * lo.w, v[4] += w * hi.x, v[5] += w * hi.y, v[6] += w * hi.z, v[7] += w * hi.w;
 					}
+				}
+				put(x, make_float4(v[0], v[1], v[2], v[3])), put(x + 4, make_float4(v[4], v[5], v[6], v[7]));
+			}
+		}
+		__syncwarp();
+		const int per_row = LAYERED ? share / 4 : share / 8; // 16-byte pieces of a row's share
+		for (int x = lane; x < 32 * per_row; x += 32) {
+			const int rr = x / per_row, cc = x % per_row, to = r0 + t * kTile + q * 32 + rr;
+			if (to >= rows) continue;
+			const int i = to / a.G, col = (g * a.G + to % a.G) * DV + part * share;
+			if constexpr (LAYERED) {
+				const float4 v = ld_shared4(patch + rr * ld + cc * 16);
+				float *dst = static_cast<float *>(a.out) + (size_t)i * a.ldo + col + cc * 4;
+				if (a.wide) *reinterpret_cast<float4 *>(dst) = v;
+				else *reinterpret_cast<float2 *>(dst) = make_float2(v.x, v.y), *reinterpret_cast<float2 *>(dst + 2) = make_float2(v.z, v.w);
+			} else {
+				const float4 lo = ld_shared4(patch + rr * ld + cc * 32), hi = ld_shared4(patch + rr * ld + cc * 32 + 16);
+				const uint4 pk = make_uint4(pack2<T>(lo.x, lo.y), pack2<T>(lo.z, lo.w), pack2<T>(hi.x, hi.y), pack2<T>(hi.z, hi.w));
+				T *dst = static_cast<T *>(a.out) + (size_t)i * a.n_kv * a.G * DV + col + cc * 8;
+				if (a.wide) {
+					*reinterpret_cast<uint4 *>(dst) = pk;
+				} else {
+					uint32_t *d32 = reinterpret_cast<uint32_t *>(dst);
+					d32[0] = pk.x, d32[1] = pk.y, d32[2] = pk.z, d32[3] = pk.w;
 				}
 			}
 		}
@@ -598,7 +669,7 @@ int window_bf16(float *out, int ldo, const float *q, int ldq, const void *keys, 
 	Args a{};
 	a.out = out, a.ldo = ldo, a.q = q, a.ldq = ldq, a.key_pool = key_pool, a.value_pool = value_pool, a.sink = sink;
 	a.n = n, a.G = n_heads / n_kv, a.n_kv = n_kv, a.v_heads = v_heads, a.ring = ring, a.max_blocks = max_blocks, a.window = window;
-	a.pool = key_pool ? pool : 0, a.pos0 = pos0, a.ctl = ctl;
+	a.pool = key_pool ? pool : 0, a.pos0 = pos0, a.ctl = ctl, a.wide = ldo % 4 == 0 && ((uintptr_t)out & 15) == 0;
 	a.q_sign = scale > 0.f ? 1.f : scale < 0.f ? -1.f : 0.f, a.c = scale == 0.f ? 1.f : fabsf(scale) * kLog2e; // the maximum is taken before the scale
 	int seen = ctl ? ring : pos0 + n; // positions that the longest row can see (the position of a control block is known on the device only)
 	if (window > 0) seen = std::min(seen, window + 2 * kTile / a.G);

@@ -36,6 +36,26 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, bool &d
 	if (mbar_try(bar, parity)) return;
 	if (!dead) dead = !mbar_wait_long(bar, parity);
 }
+// The same for a whole warp that goes on together: all lanes give up, or none.
+static __device__ __noinline__ bool mbar_wait_warp_long(uint32_t bar, uint32_t parity) {
+	const long long t0 = clock64();
+	while (!__all_sync(0xffffffffu, mbar_try(bar, parity)))
+		if (__any_sync(0xffffffffu, clock64() - t0 > 4000000000ll)) return false; // ~2 s
+	return true;
+}
+__device__ __forceinline__ void mbar_wait_warp(uint32_t bar, uint32_t parity, bool &dead) {
+	if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return;
+	if (!dead) dead = !mbar_wait_warp_long(bar, parity);
+}
+// One lane of a converged warp.  The warps that issue copies and products run their loops whole and elect inside: addresses and
+// descriptors then stay in uniform registers.  From inside a one-lane branch every tcgen05.mma took some 60 cycles more to issue (a
+// 128 x 128 x 16 product 125 cycles instead of 64).
+__device__ __forceinline__ bool elect_one() {
+	uint32_t r;
+	asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+	return r;
+}
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
 // Position in a ring of stages and the parity of its current round, stepped without the divisions of a running count.
 struct Ring {
 	uint32_t s = 0, phase = 0;
