@@ -79,3 +79,82 @@ def test_gemm_segments(M, K, ends):
     for s, end in enumerate(ends):
         assert rel(c[:, at:end], a[s * M:(s + 1) * M].double() @ w[at:end].double().T) < 3e-5
         at = end
+
+
+def attend(q, k, v, seen, scale, sink=None):
+    """q (n, H, dk), k (G, T, dk), v (Gv, T, dv), seen (n, T); 64 bits, head by head."""
+    H, G = q.shape[1], k.shape[0]
+    out = []
+    for h in range(H):
+        g = h // (H // G)
+        s = (q[:, h].double() @ k[g].double().T * scale).masked_fill(~seen, float("-inf"))
+        if sink is not None:
+            s = torch.cat([s, sink[h].double().expand(len(s), 1)], dim=1)
+        p = torch.softmax(s, dim=-1)[:, :k.shape[1]]
+        out.append(p @ v[g % v.shape[0]].double())
+    return torch.stack(out, dim=1)
+
+
+@pytest.mark.parametrize("hd", [128, 64, 32])
+@pytest.mark.parametrize("n,pos0,H,G", [(1, 0, 4, 1), (2, 127, 8, 8), (7, 397, 32, 8), (129, 0, 8, 8), (33, 5000, 8, 8), (300, 77, 64, 8), (512, 511, 12, 2), (512, 0, 32, 8),
+                                        (260, 3000, 3, 1)])
+def test_causal_attention_tiles(n, pos0, H, G, hd):
+    """Rows that fill a tile in part, both tiles, several CTAs; one key tile to many, in one part and in several; 3 query heads per
+    kv head.  Slots past the portion hold NaN.  P is rounded to fp16 (2^-11) and so is the result: 5e-4 of the norm."""
+    ring = pos0 + n + 3
+    q = normal(n, (n, H, hd), dtype=torch.float16)
+    k, v = (normal(s + pos0, (G, ring, hd), dtype=torch.float16) for s in (1, 2))
+    k[:, pos0 + n:], v[:, pos0 + n:] = float("nan"), float("nan")
+    store = torch.full((n * H * hd + 8,), 7.0, device="cuda", dtype=torch.float16)
+    for shift in (0, 2):                                           # 16-byte aligned rows, and rows that are not
+        out = store[shift: shift + n * H * hd]
+        assert L().yalm_attn_prefill(ptr(out), ptr(q), ptr(k), ptr(v), *i32(n, pos0, H, G, hd, ring), None) == 0
+        i = torch.arange(n, device="cuda")[:, None] + pos0
+        seen = torch.arange(pos0 + n, device="cuda")[None] <= i
+        assert rel(out.view(n, H, hd), attend(q, k[:, :pos0 + n], v[:, :pos0 + n], seen, hd ** -0.5)) < 5e-4
+        assert (store[shift + n * H * hd:] == 7.0).all()
+
+
+def test_causal_attention_far_maxima():
+    """A row's largest score in its last tiles, 2^40 above the first: the accumulator is rescaled, in every part."""
+    n, pos0, H, G, hd = 40, 1500, 8, 2, 128
+    q, k, v = normal(1, (n, H, hd), dtype=torch.float16), normal(2, (G, pos0 + n, hd), dtype=torch.float16), normal(3, (G, pos0 + n, hd), dtype=torch.float16)
+    for at, size in ((100, 1.0), (700, 2.0), (1400, 3.0), (1500, 4.0)):
+        k[:, at] = q[0].view(G, H // G, hd)[:, 0] * size
+    out = torch.empty((n, H, hd), device="cuda", dtype=torch.float16)
+    assert L().yalm_attn_prefill(ptr(out), ptr(q), ptr(k), ptr(v), *i32(n, pos0, H, G, hd, pos0 + n), None) == 0
+    seen = torch.arange(pos0 + n, device="cuda")[None] <= torch.arange(n, device="cuda")[:, None] + pos0
+    assert rel(out, attend(q, k, v, seen, hd ** -0.5)) < 5e-4
+
+
+@pytest.mark.parametrize("dk,dv", [(128, 128), (64, 64), (64, 128), (128, 64), (64, 32), (128, 32)])
+@pytest.mark.parametrize("n,pos0,H,G,Gv,window,pool,ring", [
+    (32, 0, 8, 2, 2, 128, 64, 640), (512, 3584, 16, 4, 4, 1024, 64, 1536), (100, 777, 8, 2, 1, 500, 64, 1012), (257, 5000, 8, 8, 4, 300, 1, 557),
+    (300, 4000, 8, 2, 2, 128, 8, 700), (40, 9000, 16, 4, 4, 130, 16, 170), (64, 300, 6, 2, 2, 0, 0, 400), (90, 1000, 4, 4, 4, 200, 0, 289)])
+def test_window_attention_tiles(n, pos0, H, G, Gv, window, pool, ring, dk, dv):
+    """Windows that wrap in the ring, rings that are no multiple of a tile, pooled blocks in one tile and in many (as blocks of one
+    position too), value heads that several key heads share, sinks, a scale of either sign, positions from a control block.  Slots that
+    hold no position are NaN.  Queries, pooled means and weights are rounded to bf16 (2^-9): 4e-3 of the norm."""
+    q = normal(n, (n, H, dk))
+    first = max(0, pos0 - window + 1) if window else 0
+    j = torch.arange(first, pos0 + n, device="cuda")
+    k, v = torch.full((G, ring, dk), float("nan"), device="cuda").bfloat16(), torch.full((Gv, ring, dv), float("nan"), device="cuda").bfloat16()
+    k[:, j % ring], v[:, j % ring] = normal(3, (G, len(j), dk), dtype=torch.bfloat16), normal(4, (Gv, len(j), dv), dtype=torch.bfloat16)
+    blocks = max(1, (pos0 + n) // pool) if pool else 0
+    kp, vp = (normal(5, (G, blocks, dk), pool ** -0.5), normal(6, (Gv, blocks, dv), pool ** -0.5)) if pool else (None, None)
+    sink = normal(7, (H,)) if pos0 % 2 == 0 else None
+    i = torch.arange(n, device="cuda")[:, None] + pos0
+    seen = (j[None] <= i) & ((i - j[None] < window) if window else True)
+    keys, values = k[:, j % ring].float(), v[:, j % ring].float()
+    if pool:
+        keys, values = torch.cat([keys, kp], dim=1), torch.cat([values, vp], dim=1)
+        seen = torch.cat([seen, torch.arange(blocks, device="cuda")[None] * pool + pool - 1 <= i - window], dim=1)
+    ctl = torch.tensor([0, pos0, 0, 0, 0, 0, 0, 0], device="cuda", dtype=torch.int32)
+    for scale, use_ctl, pad in ((dk ** -0.5, False, 0), (-0.05, True, 2)):
+        ldo = H * dv + pad
+        out = torch.full((n, ldo), 7.0, device="cuda")
+        assert L().yalm_attn_window_pool_mma_sink(ptr(out), C.c_int(ldo), ptr(q), C.c_int(H * dk), ptr(k), ptr(v), ptr(kp), ptr(vp),
+                                                  *i32(n, H, G, dk, dv, ring, blocks, window, pool), C.c_float(scale), C.c_int(-1 if use_ctl else pos0),
+                                                  ptr(ctl if use_ctl else None), ptr(sink), C.c_int(Gv), None) == 0
+        assert rel(out[:, :H * dv].reshape(n, H, dv), attend(q, keys, values, seen, scale, sink)) < 4e-3
+        assert (out[:, H * dv:] == 7.0).all()

@@ -15,8 +15,11 @@
 // models: they round pooled fp32 means into stages, and clear the value rows of a ring tile that hold no position (a weight of zero
 // times whatever lies there must be zero).
 //
-// Bound by the exponentials (16 a cycle and SM, as many cycles as the products of a tile pair) and, for short contexts, by the chain
-// copy - product - softmax - product and the launch.
+// Bound by the chain softmax - products of a tile pair (3000 cycles per 128 keys: 1800 from scores to weights, of which the exponentials
+// alone take 1024 at 16 a cycle and SM for each of the two tiles, and 1100 for P V and the next scores) and, for short contexts, by launch,
+// query staging and the store.  Cold L2, against 64-row tiles on mma.sync: 507 rows at 7680 positions, 32 / 8 heads of 128: 672 -> 72 us
+// (919 TFLOP/s); 512 rows at 0: 42 -> 20 us; 20 rows at 7000, 8 / 8 heads: 790 -> 25 us; bf16 window 2048 and pooled blocks, 512 rows, 32 / 8
+// heads: 136 -> 38 us.
 #include "common.cuh"
 #include "launch.h"
 #include "stack_rows.cuh"
@@ -173,6 +176,11 @@ __device__ __forceinline__ uint64_t desc_mn(uint32_t addr) {
 }
 constexpr uint32_t kBMajorMn = 1u << 16; // instruction descriptor: B is N-major
 
+template <int N>
+struct Width {
+	static constexpr int value = N;
+};
+
 template <int DK, int DV>
 struct Shape {
 	static constexpr int DKP = DK < 64 ? 64 : DK, DVP = DV < 64 ? 64 : DV; // channels a row takes in shared memory
@@ -216,7 +224,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 			for (int c = 0; c < d; c += 64) tma_load_3d(dst + (c / 64) * (kTile * 128), is_v ? &tv : &tk, c, slot, head, bar);
 		}
 	};
-	// a pooled tile's means into its two stages, rounded; rows past the last block are zero
+	// a pooled tile's means into its two stages, rounded; value rows past the last block are zero (the scores of such keys are masked)
 	auto fill_pooled = [&](int i, int tid, int nthreads) {
 		int slot, pos, valid;
 		tiles.at(k_begin + i, slot, pos, valid);
@@ -226,7 +234,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 			const float *src = (is_v ? a.value_pool : a.key_pool) + ((size_t)head * a.max_blocks + slot) * D;
 			const uint32_t dst = kv0 + ((2 * i + is_v) % NST) * SH::STAGE;
 #pragma unroll 4
-			for (int x = tid; x < kTile * pieces; x += nthreads) {
+			for (int x = tid; x < (is_v ? kTile : valid) * pieces; x += nthreads) {
 				const int r = x / pieces, c = x % pieces;
 				float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
 				if (r < valid && c * 8 < D) {
@@ -256,34 +264,39 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 	}
 	if (warp == 1) tmem_alloc<1>(tslot, 512);
 	if (warp > 0) { // the queries' rows (rows past the last: zero), and the first tile where it is a pooled one
-		constexpr int PIECES = DK / 8, ALL = 2 * kTile * PIECES, STEP = kThreads - 32, BATCH = LAYERED ? 6 : 12;
-		for (int x0 = threadIdx.x - 32; x0 < ALL; x0 += BATCH * STEP) { // several loads in flight: one at a time this took as long as four key tiles
+		// a thread keeps its 16-byte column and steps down the rows (the position and head of a row follow without a division); all loads of
+		// a batch are in flight together: one at a time this took as long as four key tiles
+		constexpr int PIECES = DK / 8, DOWN = (kThreads - 32) / PIECES, STEPS = (2 * kTile + DOWN - 1) / DOWN, BATCH = LAYERED ? (STEPS + 1) / 2 : STEPS;
+		const int c = (threadIdx.x - 32) % PIECES, di = DOWN / a.G, dh = DOWN % a.G;
+		int r = (threadIdx.x - 32) / PIECES, i = (r0 + r) / a.G, hh = (r0 + r) % a.G;
+		for (int s0 = 0; s0 < STEPS; s0 += BATCH) {
 			float4 lo[BATCH], hi[LAYERED ? BATCH : 1];
+			const int first = r;
 #pragma unroll
 			for (int b = 0; b < BATCH; ++b) {
-				const int x = x0 + b * STEP, r = x / PIECES, c = x % PIECES, row = r0 + r;
 				lo[b] = make_float4(0.f, 0.f, 0.f, 0.f);
 				if constexpr (LAYERED) hi[b] = lo[b];
-				if (x < ALL && row < rows) {
-					const int i = row / a.G, h = g * a.G + row % a.G;
+				if (r < 2 * kTile && r0 + r < rows) {
 					if constexpr (LAYERED) {
-						const float *src = static_cast<const float *>(a.q) + (size_t)i * a.ldq + (size_t)h * DK + c * 8;
+						const float *src = static_cast<const float *>(a.q) + (size_t)i * a.ldq + (size_t)(g * a.G + hh) * DK + c * 8;
 						lo[b] = *reinterpret_cast<const float4 *>(src), hi[b] = *reinterpret_cast<const float4 *>(src + 4);
 					} else
-						lo[b] = *reinterpret_cast<const float4 *>(static_cast<const T *>(a.q) + ((size_t)i * a.n_kv * a.G + h) * DK + c * 8);
+						lo[b] = *reinterpret_cast<const float4 *>(static_cast<const T *>(a.q) + ((size_t)(i * a.n_kv + g) * a.G + hh) * DK + c * 8);
 				}
+				r += DOWN, i += di, hh += dh;
+				if (hh >= a.G) hh -= a.G, ++i;
 			}
 #pragma unroll
 			for (int b = 0; b < BATCH; ++b) {
-				const int x = x0 + b * STEP, r = x / PIECES, c = x % PIECES;
-				if (x >= ALL) break;
+				const int rr = first + b * DOWN;
+				if (rr >= 2 * kTile) break;
 				float4 v = lo[b];
 				if constexpr (LAYERED) {
 					const float f = a.q_sign;
 					v = make_float4(__uint_as_float(pack2<T>(lo[b].x * f, lo[b].y * f)), __uint_as_float(pack2<T>(lo[b].z * f, lo[b].w * f)),
 					                __uint_as_float(pack2<T>(hi[b].x * f, hi[b].y * f)), __uint_as_float(pack2<T>(hi[b].z * f, hi[b].w * f)));
 				}
-				st_shared4(q0 + (r / kTile) * SH::Q_BYTES + tile_at(r % kTile, c), v);
+				st_shared4(q0 + (rr / kTile) * SH::Q_BYTES + tile_at(rr % kTile, c), v);
 			}
 		}
 		if constexpr (LAYERED)
@@ -411,8 +424,13 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 				pin(s);
 				if (__any_sync(kFull, from > 0 || to < kTile - 1)) {
 #pragma unroll
-					for (int x = 0; x < kTile; ++x)
-						if (x < from || x > to) s[x] = 0xff800000u; // -inf
+					for (int x0 = 0; x0 < kTile; x0 += 32) {
+						const int first = from - x0, end = to - x0;
+						const uint32_t seen = (end < 0 ? 0u : end >= 31 ? ~0u : (2u << end) - 1u) & (first <= 0 ? ~0u : first > 31 ? 0u : ~0u << first);
+#pragma unroll
+						for (int x = 0; x < 32; ++x)
+							if (!(seen & (1u << x))) s[x0 + x] = 0xff800000u; // -inf
+					}
 				}
 				float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
@@ -484,11 +502,20 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 				             : "memory");
 				if (p == part || nk == 0) continue;
 				const uint32_t dst = there + (uint32_t)(((part < p ? part : part - 1) * 2 + t) * share * kTile * 4);
-				for (int x = 0; x < share; x += 8) {
-					float v[8];
-					tmem_ld8(op + p * share + x, v);
-					st_cluster4(dst + (uint32_t)(((x >> 2) * kTile + tr) * 16), make_float4(v[0], v[1], v[2], v[3]));
-					st_cluster4(dst + (uint32_t)((((x >> 2) + 1) * kTile + tr) * 16), make_float4(v[4], v[5], v[6], v[7]));
+				if (share % 32 == 0) {
+					for (int x = 0; x < share; x += 32) {
+						float v[32];
+						tmem_ld32(op + p * share + x, v);
+#pragma unroll
+						for (int y = 0; y < 32; y += 4) st_cluster4(dst + (uint32_t)((((x + y) >> 2) * kTile + tr) * 16), make_float4(v[y], v[y + 1], v[y + 2], v[y + 3]));
+					}
+				} else {
+					for (int x = 0; x < share; x += 8) {
+						float v[8];
+						tmem_ld8(op + p * share + x, v);
+						st_cluster4(dst + (uint32_t)(((x >> 2) * kTile + tr) * 16), make_float4(v[0], v[1], v[2], v[3]));
+						st_cluster4(dst + (uint32_t)((((x >> 2) + 1) * kTile + tr) * 16), make_float4(v[4], v[5], v[6], v[7]));
+					}
 				}
 			}
 		}
@@ -529,51 +556,66 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 				for (int y = 0; y < 32; y += 4) put(x + y, make_float4(v[y], v[y + 1], v[y + 2], v[y + 3]));
 			}
 		} else {
-			for (int x = 0; x < share; x += 8) {
-				float v[8], own[8];
+			auto join = [&](auto width, int x) { // columns x .. x + width - 1 of the share, the parts of the keys in order
+				constexpr int W = decltype(width)::value;
+				float v[W], own[W];
 				__syncwarp();
-				tmem_ld8(op + part * share + x, own);
+				if constexpr (W == 32) tmem_ld32(op + part * share + x, own);
+				else tmem_ld8(op + part * share + x, own);
 #pragma unroll
-				for (int y = 0; y < 8; ++y) v[y] = 0.f;
-				for (int p = 0; p < parts; ++p) { // the parts of the keys in order
+				for (int y = 0; y < W; ++y) v[y] = 0.f;
+				for (int p = 0; p < parts; ++p) {
 					float pm, pl;
 					of_part(p, pm, pl);
 					if (!(pl > 0.f)) continue;
 					const float w = ex2(pm - M);
 					if (p == part) {
 #pragma unroll
-						for (int y = 0; y < 8; ++y) v[y] += w * own[y];
+						for (int y = 0; y < W; ++y) v[y] += w * own[y];
 					} else {
 						const uint32_t src = base + (uint32_t)(((p < part ? p : p - 1) * 2 + t) * share * kTile * 4);
-						const float4 lo = ld_shared4(src + (uint32_t)(((x >> 2) * kTile + tr) * 16)), hi = ld_shared4(src + (uint32_t)((((x >> 2) + 1) * kTile + tr) * 16));
-						v[0] += w * lo.x, v[1] += w * lo.y, v[2] += w * lo.z, v[3] += w * lo.w, v[4] += w * hi.x, v[5] += w * hi.y, v[6] += w * hi.z, v[7] += w * hi.w;
+#pragma unroll
+						for (int y = 0; y < W; y += 4) {
+							const float4 o = ld_shared4(src + (uint32_t)((((x + y) >> 2) * kTile + tr) * 16));
+							v[y] += w * o.x, v[y + 1] += w * o.y, v[y + 2] += w * o.z, v[y + 3] += w * o.w;
+						}
 					}
 				}
-				put(x, make_float4(v[0], v[1], v[2], v[3])), put(x + 4, make_float4(v[4], v[5], v[6], v[7]));
-			}
+#pragma unroll
+				for (int y = 0; y < W; y += 4) put(x + y, make_float4(v[y], v[y + 1], v[y + 2], v[y + 3]));
+			};
+			if (share % 32 == 0)
+				for (int x = 0; x < share; x += 32) join(Width<32>(), x);
+			else
+				for (int x = 0; x < share; x += 8) join(Width<8>(), x);
 		}
 		__syncwarp();
-		const int per_row = LAYERED ? share / 4 : share / 8; // 16-byte pieces of a row's share
-		for (int x = lane; x < 32 * per_row; x += 32) {
-			const int rr = x / per_row, cc = x % per_row, to = r0 + t * kTile + q * 32 + rr;
-			if (to >= rows) continue;
-			const int i = to / a.G, col = (g * a.G + to % a.G) * DV + part * share;
-			if constexpr (LAYERED) {
-				const float4 v = ld_shared4(patch + rr * ld + cc * 16);
-				float *dst = static_cast<float *>(a.out) + (size_t)i * a.ldo + col + cc * 4;
-				if (a.wide) *reinterpret_cast<float4 *>(dst) = v;
-				else *reinterpret_cast<float2 *>(dst) = make_float2(v.x, v.y), *reinterpret_cast<float2 *>(dst + 2) = make_float2(v.z, v.w);
-			} else {
-				const float4 lo = ld_shared4(patch + rr * ld + cc * 32), hi = ld_shared4(patch + rr * ld + cc * 32 + 16);
-				const uint4 pk = make_uint4(pack2<T>(lo.x, lo.y), pack2<T>(lo.z, lo.w), pack2<T>(hi.x, hi.y), pack2<T>(hi.z, hi.w));
-				T *dst = static_cast<T *>(a.out) + (size_t)i * a.n_kv * a.G * DV + col + cc * 8;
-				if (a.wide) {
-					*reinterpret_cast<uint4 *>(dst) = pk;
+		const int pieces = LAYERED ? share / 4 : share / 8, lg = 31 - __clz(pieces); // 16-byte pieces of a row's share: a power of two up to 32
+		const int down = 32 >> lg, cc = lane & (pieces - 1), di = down / a.G, dh = down % a.G;
+		int rr = lane >> lg, to = r0 + t * kTile + q * 32 + rr, i = to / a.G, hh = to % a.G;
+#pragma unroll 4
+		for (; rr < 32; rr += down) {
+			const int col = (g * a.G + hh) * DV + part * share;
+			if (to < rows) {
+				if constexpr (LAYERED) {
+					const float4 v = ld_shared4(patch + rr * ld + cc * 16);
+					float *dst = static_cast<float *>(a.out) + (size_t)i * a.ldo + col + cc * 4;
+					if (a.wide) *reinterpret_cast<float4 *>(dst) = v;
+					else *reinterpret_cast<float2 *>(dst) = make_float2(v.x, v.y), *reinterpret_cast<float2 *>(dst + 2) = make_float2(v.z, v.w);
 				} else {
-					uint32_t *d32 = reinterpret_cast<uint32_t *>(dst);
-					d32[0] = pk.x, d32[1] = pk.y, d32[2] = pk.z, d32[3] = pk.w;
+					const float4 lo = ld_shared4(patch + rr * ld + cc * 32), hi = ld_shared4(patch + rr * ld + cc * 32 + 16);
+					const uint4 pk = make_uint4(pack2<T>(lo.x, lo.y), pack2<T>(lo.z, lo.w), pack2<T>(hi.x, hi.y), pack2<T>(hi.z, hi.w));
+					T *dst = static_cast<T *>(a.out) + (size_t)i * a.n_kv * a.G * DV + col + cc * 8;
+					if (a.wide) {
+						*reinterpret_cast<uint4 *>(dst) = pk;
+					} else {
+						uint32_t *d32 = reinterpret_cast<uint32_t *>(dst);
+						d32[0] = pk.x, d32[1] = pk.y, d32[2] = pk.z, d32[3] = pk.w;
+					}
 				}
 			}
+			to += down, i += di, hh += dh;
+			if (hh >= a.G) hh -= a.G, ++i;
 		}
 	}
 	tc_fence_before();
@@ -612,22 +654,32 @@ static int make_map(CUtensorMap *map, const void *ptr, int d, int rows, int ring
 	return r == CUDA_SUCCESS ? 0 : YALM_EINVAL;
 }
 
-// Parts of the keys: as many as still give every CTA an SM and at least 3 key tiles (the exchange costs about two).  est_tiles: key
-// tiles of the longest rows.
+// Parts of the keys: as many as still run all at once and leave every part at least 2 key tiles (the exchange costs about one and a
+// half: 512 rows at position 0, 32 heads, 4 tiles: 18.7 us in one part, 16.7 in two).  est_tiles: key tiles of the longest rows.
 template <typename T, int DK, int DV, bool LAYERED>
 static int launch(Args &a, const void *keys, const void *values, int map_rows, int est_tiles, cudaStream_t st) {
 	using SH = Shape<DK, DV>;
-	static bool configured[kMaxDevices];
+	static int at_once[kMaxDevices][4]; // clusters of 1, 2, 4, 8 CTAs; 0: not asked yet
 	static std::mutex mu;
 	auto kernel = prompt_attn_kernel<T, DK, DV, LAYERED>;
 	const DeviceInfo &dev = device_info();
 	if (dev.device < 0 || dev.device >= kMaxDevices) return YALM_EINVAL;
+	cudaLaunchConfig_t cfg = {};
+	cudaLaunchAttribute at[1];
+	at[0].id = cudaLaunchAttributeClusterDimension;
+	at[0].val.clusterDim.x = 1, at[0].val.clusterDim.y = 1, at[0].val.clusterDim.z = 1;
+	cfg.blockDim = dim3(kThreads), cfg.dynamicSmemBytes = SH::SMEM, cfg.attrs = at, cfg.numAttrs = 1;
+	int room[4];
 	{
 		std::lock_guard<std::mutex> lock(mu);
-		if (!configured[dev.device]) {
+		if (!at_once[dev.device][0]) {
 			YALM_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SH::SMEM));
-			configured[dev.device] = true;
+			for (int i = 3; i >= 0; --i) {
+				at[0].val.clusterDim.x = 1 << i, cfg.gridDim = dim3(1 << i);
+				YALM_TRY(cudaOccupancyMaxActiveClusters(&at_once[dev.device][i], kernel, &cfg));
+			}
 		}
+		for (int i = 0; i < 4; ++i) room[i] = at_once[dev.device][i];
 	}
 	CUtensorMap tk, tv;
 	int rc = make_map(&tk, keys, DK, map_rows, a.ring, a.n_kv, LAYERED);
@@ -635,13 +687,9 @@ static int launch(Args &a, const void *keys, const void *values, int map_rows, i
 	if (rc) return rc;
 	const int pairs = (a.n * a.G + 2 * kTile - 1) / (2 * kTile), units = pairs * a.n_kv;
 	a.parts = 1;
-	while (a.parts * 2 <= std::min(8, DV / 8) && units * a.parts * 2 <= (a.parts == 1 ? dev.sms : 128) && est_tiles >= 6 * a.parts) a.parts *= 2;
-	cudaLaunchConfig_t cfg = {};
-	cfg.gridDim = dim3(pairs * a.parts, a.n_kv), cfg.blockDim = dim3(kThreads), cfg.dynamicSmemBytes = SH::SMEM, cfg.stream = st;
-	cudaLaunchAttribute at[1];
-	at[0].id = cudaLaunchAttributeClusterDimension;
-	at[0].val.clusterDim.x = a.parts, at[0].val.clusterDim.y = 1, at[0].val.clusterDim.z = 1;
-	cfg.attrs = at, cfg.numAttrs = 1;
+	for (int i = 1; i < 4 && (1 << i) <= DV / 8 && units <= room[i] && est_tiles >= (2 << i); ++i) a.parts = 1 << i;
+	at[0].val.clusterDim.x = a.parts;
+	cfg.gridDim = dim3(pairs * a.parts, a.n_kv), cfg.stream = st;
 	YALM_TRY(cudaLaunchKernelEx(&cfg, kernel, tk, tv, a));
 	return 0;
 }
