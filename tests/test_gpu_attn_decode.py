@@ -1,0 +1,34 @@
+"""-m gpu: yalm_attn_decode over every head size and group it has a kernel for, at the edges of its splits (one row, one short of and one
+past a batch of rows for every warp, several splits, the last with few rows), against the softmax in 64 bits.
+
+Bound: fp32 sums of a few thousand terms, the exponential's 2 units: 1e-6 of the norm (measured 3e-7)."""
+import ctypes as C
+
+import pytest
+import torch
+
+from yalm_b200 import api
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("hd", [128, 64, 32, 16])
+@pytest.mark.parametrize("G", [1, 2, 4, 8])
+@pytest.mark.parametrize("n_kv", [1, 3, 8])
+def test_attn_decode_splits(hd, G, n_kv):
+    L, H, ring = api.lib(), G * n_kv, 5000
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(hd + G)
+    k, v = (torch.randn((n_kv, ring, hd), generator=gen, device="cuda").half() for _ in range(2))
+    q = torch.randn((H, hd), generator=gen, device="cuda")
+    work = torch.zeros(L.yalm_attn_workspace_bytes(H, n_kv, hd), device="cuda", dtype=torch.uint8)
+    out = torch.empty((H, hd), device="cuda")
+    p = lambda t: C.c_void_p(t.data_ptr())
+    for rows in (1, 2, 63, 64, 65, 127, 129, 511, 513, 1000, 2049, ring):
+        kk, vv = k.clone(), v.clone()
+        kk[:, rows:], vv[:, rows:] = float("nan"), float("nan")
+        ctl = torch.tensor([0, rows - 1, 0, rows - 1, rows, 0, 0, 0], device="cuda", dtype=torch.int32)
+        assert L.yalm_attn_decode(p(out), p(kk), p(vv), p(q), p(work), H, n_kv, hd, ring, p(ctl), None) == 0   # the same workspace throughout
+        w = torch.softmax(torch.einsum("ghd,gtd->ght", q.view(n_kv, G, hd).double(), k[:, :rows].double()) * hd ** -0.5, dim=-1)
+        want = torch.einsum("ght,gtd->ghd", w, v[:, :rows].double()).reshape(H, hd)
+        assert ((out.double() - want).norm() / want.norm()).item() < 1e-6, rows

@@ -5,7 +5,7 @@
 //    times, and each row is read as 16-byte lane-contiguous pieces (the reference walks one 256-byte
 //    key row per thread);
 //  * the sequence is split over gridDim.x CTAs per KV head (the reference's att_mix runs 32 CTAs on a
-//    148-SM part) with an online softmax per split; the last CTA of each KV head to finish merges the
+//    148-SM part) with an online softmax per group of lanes; the last CTA of each KV head to finish merges the
 //    split partials (arrival counter in the workspace) — no second launch;
 //  * no (n_heads, max_seq_len) score matrix round-trips through memory.
 // Softmax order is irrelevant to the ring buffer, so sliding-window positions and the two attention
@@ -24,7 +24,7 @@ namespace yalm {
 
 constexpr int kAttnThreads = 256;
 constexpr int kAttnWarps = kAttnThreads / 32;
-constexpr int kTile = 512; // rows per online-softmax tile
+constexpr int kTile = 512; // most splits
 
 struct AttnArgs {
 	float *out;            // (n_heads*head_dim)
@@ -34,6 +34,7 @@ struct AttnArgs {
 	float *ws_ml;          // (n_kv_heads, S, G, 2)  running max, running sum
 	unsigned *counters;    // (n_kv_heads) arrival counters, zero between launches
 	int n_kv_heads, max_seq_len;
+	int max_splits; // of which a context uses as many as have a batch of rows for every warp
 	const int *ctl;
 };
 
@@ -45,181 +46,232 @@ __device__ __forceinline__ void unpack8(uint4 v, float (&f)[8]) {
 	f[0] = a.x, f[1] = a.y, f[2] = b.x, f[3] = b.y, f[4] = c.x, f[5] = c.y, f[6] = d.x, f[7] = d.y;
 }
 
-template <int HD, int G>
-__global__ void __launch_bounds__(kAttnThreads) attn_decode_kernel(AttnArgs a) {
-	constexpr int L = HD / 8;    // lanes per K/V row (16 bytes each)
-	constexpr int RPW = 32 / L;  // rows per warp step
-	constexpr int RPC = RPW * kAttnWarps; // rows per CTA step
-	constexpr int UN = 4;        // row-steps in flight per thread
+__device__ __forceinline__ float exp2_approx(float x) { // 2 ulp, results below 2^-126 are 0
+	float y;
+	asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+	return y;
+}
 
+// How a row's HD / 8 lanes share the scores of UN rows x G heads (value index u G + g): after the halving exchanges a lane holds N1
+// complete values, index (sub / DUP) N1 + j.
+template <int HD, int G>
+struct Split {
+	static constexpr int L = HD / 8;                   // lanes per K / V row (16 bytes each)
+	static constexpr int RPW = 32 / L;                 // rows per warp step
+	static constexpr int RPC = RPW * kAttnWarps;       // rows per CTA step
+	static constexpr int UN = G >= 8 ? 2 : G >= 4 ? 4 : 8; // steps in flight per thread, keys and values
+	static constexpr int CTAS = G >= 8 ? 1 : 2;         // resident per SM (8 heads' queries and sums take 128 registers of a lane)
+	static constexpr int NV = UN * G, N1 = NV > L ? NV / L : 1, DUP = NV < L ? L / NV : 1;
+	static constexpr int NG = N1 < G ? N1 : G;         // heads that a lane's values belong to
+	static constexpr int U0 = DUP * (N1 < G ? G / N1 : 1); // lanes sub and sub ^ U0, sub ^ 2 U0, .. hold the same heads of other rows
+};
+
+// Every group of HD / 8 lanes walks rows of its own with an online softmax in registers: no barrier until the CTA's end.  The scores of UN
+// rows are reduced together by halving exchanges (UN G - 1 + .. shuffles for all of them, not log2 of them for each), which leaves about
+// one exponential per lane and row batch.  Latency is what counts at a few thousand positions: a CTA's chain is control block, one batch
+// of keys and values, one exchange of partials; short contexts use fewer splits (at least one batch per warp each), one split writes the
+// result itself.  32 / 8 heads of 128, back to back, against a block-wide softmax per 512 rows: 37 positions 16 -> 6.5 us, 4096 20 -> 12 us, 32768
+// 68 -> 33 us.
+template <int HD, int G>
+__global__ void __launch_bounds__(kAttnThreads, Split<HD, G>::CTAS) attn_decode_kernel(AttnArgs a) {
+	using SP = Split<HD, G>;
+	constexpr int L = SP::L, RPC = SP::RPC, UN = SP::UN, NV = SP::NV, N1 = SP::N1, DUP = SP::DUP, NG = SP::NG;
 	extern __shared__ __align__(16) float smem[];
-	float *red = smem;                       // 36
-	float *p_s = smem + 36;                  // [kTile][G]
-	float *o_s = p_s + kTile * G;            // [kAttnWarps][G][HD]
-	__shared__ float m_run[G], l_run[G], corr_s[G];
+	float *o_s = smem;                         // [kAttnWarps][G][HD]
+	float *w_s = o_s + kAttnWarps * G * HD;    // [splits][G] merge weights (splits <= kTile)
+	__shared__ float m_s[kAttnWarps][G], l_s[kAttnWarps][G], l_all[G];
 	__shared__ unsigned is_last;
 
-	const int kvh = blockIdx.y, S = gridDim.x, split = blockIdx.x;
+	const int kvh = blockIdx.y, split = blockIdx.x;
 	const int kv_len = a.ctl[CTL_KVLEN];
-	constexpr int kv_dim = HD; // row stride inside one head's slab
-	const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-	const int sub = lane % L, rgrp = lane / L;
-
-	// this CTA's row range
+	const int S = min(a.max_splits, max(1, (kv_len + RPC * UN - 1) / (RPC * UN))); // splits that have rows
+	if (split >= S) return;
+	const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, sub = lane % L, rgrp = lane / L;
 	int per = (kv_len + S - 1) / S;
 	per = (per + RPC - 1) / RPC * RPC;
 	const int t_begin = min(split * per, kv_len), t_end = min(t_begin + per, kv_len);
 
-	// q slice of this lane for each of the G heads: dims [sub*8, sub*8+8)
-	float qr[G][8];
+	// q slice of this lane for each of the G heads: dims [sub*8, sub*8+8), times log2(e) / sqrt(HD)
+	const float c = 1.4426950408889634f / sqrtf((float)HD);
+	float qr[G][8], acc[G][8];
 #pragma unroll
 	for (int g = 0; g < G; ++g) {
 		const float *qp = a.q + (size_t)(kvh * G + g) * HD + sub * 8;
-		float4 lo = *reinterpret_cast<const float4 *>(qp), hi = *reinterpret_cast<const float4 *>(qp + 4);
+		const float4 lo = *reinterpret_cast<const float4 *>(qp), hi = *reinterpret_cast<const float4 *>(qp + 4);
 		qr[g][0] = lo.x, qr[g][1] = lo.y, qr[g][2] = lo.z, qr[g][3] = lo.w;
 		qr[g][4] = hi.x, qr[g][5] = hi.y, qr[g][6] = hi.z, qr[g][7] = hi.w;
-	}
-	if (threadIdx.x < G) m_run[threadIdx.x] = -INFINITY, l_run[threadIdx.x] = 0.f;
-	float acc[G][8];
-#pragma unroll
-	for (int g = 0; g < G; ++g)
 #pragma unroll
 		for (int j = 0; j < 8; ++j) acc[g][j] = 0.f;
-	const float inv_div = sqrtf((float)HD);
+	}
+	float m[NG], l[NG]; // of this lane's heads, over its group's rows
+#pragma unroll
+	for (int j = 0; j < NG; ++j) m[j] = -INFINITY, l[j] = 0.f;
 	const __half *kbase = a.kb + (size_t)kvh * a.max_seq_len * HD + sub * 8;
 	const __half *vbase = a.vb + (size_t)kvh * a.max_seq_len * HD + sub * 8;
-	__syncthreads();
 
-	for (int tile0 = t_begin; tile0 < t_end; tile0 += kTile) {
-		const int tile_n = min(kTile, t_end - tile0);
-		// ---- phase 1: scores s[t][g] = q_g . K[t] / sqrt(HD) --------------------------------------
-		// loop bounds are warp-uniform (the shuffles below need the whole warp); rows are guarded
-		for (int rb = wid * RPW; rb < tile_n; rb += RPC * UN) {
-			const int r0 = rb + rgrp;
-			uint4 kv[UN];
+	for (int r0 = t_begin + wid * SP::RPW + rgrp; r0 - rgrp < t_end; r0 += RPC * UN) { // (warp-uniform bound: the shuffles need the whole warp)
+		uint4 kv[UN], vv[UN];
 #pragma unroll
-			for (int u = 0; u < UN; ++u) {
-				const int r = r0 + u * RPC;
-				kv[u] = r < tile_n ? *reinterpret_cast<const uint4 *>(kbase + (size_t)(tile0 + r) * kv_dim)
-				                   : make_uint4(0, 0, 0, 0);
-			}
+		for (int u = 0; u < UN; ++u) kv[u] = r0 + u * RPC < t_end ? ldg_stream(kbase + (size_t)(r0 + u * RPC) * HD) : make_uint4(0, 0, 0, 0);
 #pragma unroll
-			for (int u = 0; u < UN; ++u) {
-				const int r = r0 + u * RPC;
-				float kf[8];
-				unpack8(kv[u], kf);
-				float s[G];
+		for (int u = 0; u < UN; ++u) vv[u] = r0 + u * RPC < t_end ? ldg_stream(vbase + (size_t)(r0 + u * RPC) * HD) : make_uint4(0, 0, 0, 0);
+		float s[NV];
 #pragma unroll
-				for (int g = 0; g < G; ++g) {
-					float d = 0.f;
+		for (int u = 0; u < UN; ++u) {
+			float kf[8];
+			unpack8(kv[u], kf);
 #pragma unroll
-					for (int j = 0; j < 8; ++j) d = fmaf(qr[g][j], kf[j], d);
-					s[g] = d;
-				}
+			for (int g = 0; g < G; ++g) {
+				float d = 0.f;
 #pragma unroll
-				for (int o = L / 2; o > 0; o >>= 1)
-#pragma unroll
-					for (int g = 0; g < G; ++g) s[g] += __shfl_xor_sync(kFull, s[g], o);
-				if (sub == 0 && r < tile_n) {
-#pragma unroll
-					for (int g = 0; g < G; ++g) p_s[r * G + g] = s[g] / inv_div;
-				}
+				for (int j = 0; j < 8; ++j) d = fmaf(qr[g][j], kf[j], d);
+				s[u * G + g] = d;
 			}
 		}
-		__syncthreads();
-		// ---- online softmax bookkeeping for this tile ----------------------------------------------
-		for (int g = 0; g < G; ++g) {
-			float mx = -INFINITY;
-			for (int r = threadIdx.x; r < tile_n; r += kAttnThreads) mx = fmaxf(mx, p_s[r * G + g]);
-			mx = block_max(mx, red);
-			const float m_old = m_run[g];
-			const float m_new = fmaxf(m_old, mx);
-			float sum = 0.f;
-			for (int r = threadIdx.x; r < tile_n; r += kAttnThreads) {
-				float e = expf(p_s[r * G + g] - m_new);
-				p_s[r * G + g] = e;
-				sum += e;
-			}
-			sum = block_sum(sum, red);
-			if (threadIdx.x == 0) {
-				const float c = m_old == -INFINITY ? 0.f : expf(m_old - m_new);
-				corr_s[g] = c;
-				l_run[g] = l_run[g] * c + sum;
-				m_run[g] = m_new;
+		{
+			int n = NV;
+#pragma unroll
+			for (int o = L / 2; o > 0; o >>= 1) {
+				if (n > 1) { // lanes with bit o keep the upper half of the values
+					n >>= 1;
+#pragma unroll
+					for (int i = 0; i < NV / 2; ++i)
+						if (i < n) {
+							const float give = (sub & o) ? s[i] : s[i + n], keep = (sub & o) ? s[i + n] : s[i];
+							s[i] = keep + __shfl_xor_sync(kFull, give, o);
+						}
+				} else
+					s[0] += __shfl_xor_sync(kFull, s[0], o);
 			}
 		}
-		__syncthreads();
+		// this lane's values: index q = (sub / DUP) N1 + j, row q / G, head q % G
+		float mx[NG];
 #pragma unroll
-		for (int g = 0; g < G; ++g) {
-			const float c = corr_s[g];
+		for (int j = 0; j < NG; ++j) mx[j] = -INFINITY;
 #pragma unroll
-			for (int j = 0; j < 8; ++j) acc[g][j] *= c;
+		for (int j = 0; j < N1; ++j) {
+			const int u = ((sub / DUP) * N1 + j) / G;
+			s[j] = r0 + u * RPC < t_end ? s[j] * c : -INFINITY;
+			mx[j % NG] = fmaxf(mx[j % NG], s[j]);
 		}
-		// ---- phase 2: acc[g] += p[t][g] * V[t] ------------------------------------------------------
-		for (int rb = wid * RPW; rb < tile_n; rb += RPC * UN) {
-			const int r0 = rb + rgrp;
-			uint4 vv[UN];
 #pragma unroll
-			for (int u = 0; u < UN; ++u) {
-				const int r = r0 + u * RPC;
-				vv[u] = r < tile_n ? *reinterpret_cast<const uint4 *>(vbase + (size_t)(tile0 + r) * kv_dim)
-				                   : make_uint4(0, 0, 0, 0);
+		for (int o = SP::U0; o < L; o <<= 1)
+#pragma unroll
+			for (int j = 0; j < NG; ++j) mx[j] = fmaxf(mx[j], __shfl_xor_sync(kFull, mx[j], o));
+		bool grow = false;
+#pragma unroll
+		for (int j = 0; j < NG; ++j) grow |= mx[j] > m[j];
+		if (__any_sync(kFull, grow)) {
+			float f[NG];
+#pragma unroll
+			for (int j = 0; j < NG; ++j) {
+				const float top = fmaxf(m[j], mx[j]);
+				f[j] = m[j] == -INFINITY ? 0.f : exp2_approx(m[j] - top);
+				m[j] = top, l[j] *= f[j];
 			}
 #pragma unroll
-			for (int u = 0; u < UN; ++u) {
-				const int r = r0 + u * RPC;
-				if (r < tile_n) {
-					float vf[8];
-					unpack8(vv[u], vf);
+			for (int g = 0; g < G; ++g) {
+				const float fg = __shfl_sync(kFull, f[g % NG], (g / N1) * DUP, L);
 #pragma unroll
-					for (int g = 0; g < G; ++g) {
-						const float p = p_s[r * G + g];
-#pragma unroll
-						for (int j = 0; j < 8; ++j) acc[g][j] = fmaf(p, vf[j], acc[g][j]);
-					}
-				}
+				for (int j = 0; j < 8; ++j) acc[g][j] *= fg;
 			}
 		}
-		__syncthreads(); // p_s is rewritten by the next tile
+#pragma unroll
+		for (int j = 0; j < N1; ++j) {
+			s[j] = s[j] == -INFINITY ? 0.f : exp2_approx(s[j] - m[j % NG]);
+			l[j % NG] += s[j];
+		}
+#pragma unroll
+		for (int u = 0; u < UN; ++u) {
+			float vf[8];
+			unpack8(vv[u], vf);
+#pragma unroll
+			for (int g = 0; g < G; ++g) {
+				const int q = u * G + g;
+				const float p = __shfl_sync(kFull, s[q % N1], (q / N1) * DUP, L);
+#pragma unroll
+				for (int j = 0; j < 8; ++j) acc[g][j] = fmaf(p, vf[j], acc[g][j]);
+			}
+		}
 	}
 
-	// ---- reduce the CTA's accumulators: row groups inside a warp, then warps -----------------------
+	// ---- the warp's row groups, then the CTA's warps ----
 #pragma unroll
-	for (int o = 16; o >= L; o >>= 1)
+	for (int o = SP::U0; o < L; o <<= 1)
 #pragma unroll
-		for (int g = 0; g < G; ++g)
+		for (int j = 0; j < NG; ++j) l[j] += __shfl_xor_sync(kFull, l[j], o);
+	float f[NG];
 #pragma unroll
-			for (int j = 0; j < 8; ++j) acc[g][j] += __shfl_xor_sync(kFull, acc[g][j], o);
-	if (rgrp == 0) {
+	for (int j = 0; j < NG; ++j) {
+		float top = m[j];
 #pragma unroll
-		for (int g = 0; g < G; ++g)
+		for (int o = L; o < 32; o <<= 1) top = fmaxf(top, __shfl_xor_sync(kFull, top, o));
+		f[j] = m[j] == -INFINITY ? 0.f : exp2_approx(m[j] - top);
+		l[j] *= f[j], m[j] = top;
 #pragma unroll
-			for (int j = 0; j < 8; ++j) o_s[(wid * G + g) * HD + sub * 8 + j] = acc[g][j];
+		for (int o = L; o < 32; o <<= 1) l[j] += __shfl_xor_sync(kFull, l[j], o);
+	}
+#pragma unroll
+	for (int g = 0; g < G; ++g) {
+		const float fg = __shfl_sync(kFull, f[g % NG], (g / N1) * DUP, L), mg = __shfl_sync(kFull, m[g % NG], (g / N1) * DUP, L),
+		            lg = __shfl_sync(kFull, l[g % NG], (g / N1) * DUP, L);
+#pragma unroll
+		for (int j = 0; j < 8; ++j) {
+			acc[g][j] *= fg;
+#pragma unroll
+			for (int o = L; o < 32; o <<= 1) acc[g][j] += __shfl_xor_sync(kFull, acc[g][j], o);
+		}
+		if (rgrp == 0) {
+			float *dst = o_s + (wid * G + g) * HD + sub * 8;
+			*reinterpret_cast<float4 *>(dst) = make_float4(acc[g][0], acc[g][1], acc[g][2], acc[g][3]);
+			*reinterpret_cast<float4 *>(dst + 4) = make_float4(acc[g][4], acc[g][5], acc[g][6], acc[g][7]);
+		}
+		if (lane == 0) m_s[wid][g] = mg, l_s[wid][g] = lg;
 	}
 	__syncthreads();
 	float *my_acc = a.ws_acc + ((size_t)kvh * S + split) * G * HD;
 	for (int i = threadIdx.x; i < G * HD; i += kAttnThreads) {
-		float v = 0.f;
+		const int g = i / HD;
+		float M = -INFINITY, sum = 0.f, v = 0.f;
 #pragma unroll
-		for (int w = 0; w < kAttnWarps; ++w) v += o_s[w * G * HD + i];
-		my_acc[i] = v;
+		for (int w = 0; w < kAttnWarps; ++w) M = fmaxf(M, m_s[w][g]);
+#pragma unroll
+		for (int w = 0; w < kAttnWarps; ++w) {
+			const float fw = m_s[w][g] == -INFINITY ? 0.f : exp2_approx(m_s[w][g] - M);
+			sum = fmaf(fw, l_s[w][g], sum);
+			v = fmaf(fw, o_s[w * G * HD + i], v);
+		}
+		if (S == 1) {
+			a.out[(size_t)kvh * G * HD + i] = v / sum;
+		} else {
+			my_acc[i] = v;
+			if (i % HD == 0) {
+				float *ml = a.ws_ml + (((size_t)kvh * S + split) * G + g) * 2;
+				ml[0] = M, ml[1] = sum;
+			}
+		}
 	}
-	if (threadIdx.x < G) {
-		float *ml = a.ws_ml + (((size_t)kvh * S + split) * G + threadIdx.x) * 2;
-		ml[0] = m_run[threadIdx.x];
-		ml[1] = l_run[threadIdx.x];
-	}
+	if (S == 1) return;
 	// ---- last CTA of this KV head merges the splits -------------------------------------------------
-	__threadfence();
 	__syncthreads();
-	if (threadIdx.x == 0) {
-		unsigned prev = atomicAdd(&a.counters[kvh], 1u);
-		is_last = prev == (unsigned)(S - 1);
+	if (threadIdx.x == 0) { // one fence for the CTA: it orders what the barrier before it (and the one after) made visible
+		__threadfence();
+		is_last = atomicAdd(&a.counters[kvh], 1u) == (unsigned)(S - 1);
+		__threadfence();
 	}
 	__syncthreads();
 	if (!is_last) return;
-	__threadfence();
-	float *w_s = p_s; // [S][G] merge weights (S <= kTile)
+	// a thread takes 4 columns of every GROUPS-th split: the partials of a batch are on their way before their weights are known
+	constexpr int C4 = G * HD / 4, GROUPS = kAttnThreads / C4 > kAttnWarps ? kAttnWarps : kAttnThreads / C4, BATCH = 10;
+	const int col = threadIdx.x % C4, grp = threadIdx.x / C4;
+	const float4 *pa = reinterpret_cast<const float4 *>(a.ws_acc + (size_t)kvh * S * G * HD) + col;
+	float4 in[BATCH], sum = make_float4(0.f, 0.f, 0.f, 0.f);
+	auto fetch = [&](int s0) {
+#pragma unroll
+		for (int b = 0; b < BATCH; ++b)
+			if (grp < GROUPS && s0 + b * GROUPS < S) in[b] = __ldcg(pa + (size_t)(s0 + b * GROUPS) * C4);
+	};
+	fetch(grp);
 	for (int g = wid; g < G; g += kAttnWarps) {
 		const float *ml = a.ws_ml + ((size_t)kvh * S * G + g) * 2;
 		float M = -INFINITY;
@@ -227,21 +279,31 @@ __global__ void __launch_bounds__(kAttnThreads) attn_decode_kernel(AttnArgs a) {
 		M = warp_max(M);
 		float Lsum = 0.f;
 		for (int s = lane; s < S; s += 32) {
-			const float m = __ldcg(ml + (size_t)s * G * 2), l = __ldcg(ml + (size_t)s * G * 2 + 1);
-			const float w = m == -INFINITY ? 0.f : expf(m - M);
+			const float ms = __ldcg(ml + (size_t)s * G * 2), ls = __ldcg(ml + (size_t)s * G * 2 + 1);
+			const float w = ms == -INFINITY ? 0.f : exp2_approx(ms - M);
 			w_s[s * G + g] = w;
-			Lsum += w * l;
+			Lsum += w * ls;
 		}
 		Lsum = warp_sum(Lsum);
-		if (lane == 0) l_run[g] = Lsum;
+		if (lane == 0) l_all[g] = Lsum;
 	}
 	__syncthreads();
+	for (int s0 = grp; s0 < S; s0 += BATCH * GROUPS) {
+		if (s0 != grp) fetch(s0);
+#pragma unroll
+		for (int b = 0; b < BATCH; ++b)
+			if (grp < GROUPS && s0 + b * GROUPS < S) {
+				const float w = w_s[(s0 + b * GROUPS) * G + col / (HD / 4)];
+				sum.x = fmaf(w, in[b].x, sum.x), sum.y = fmaf(w, in[b].y, sum.y), sum.z = fmaf(w, in[b].z, sum.z), sum.w = fmaf(w, in[b].w, sum.w);
+			}
+	}
+	if (grp < GROUPS) reinterpret_cast<float4 *>(o_s)[grp * C4 + col] = sum;
+	__syncthreads();
 	for (int i = threadIdx.x; i < G * HD; i += kAttnThreads) {
-		const int g = i / HD;
-		const float *pa = a.ws_acc + (size_t)kvh * S * G * HD + i;
 		float v = 0.f;
-		for (int s = 0; s < S; ++s) v = fmaf(w_s[s * G + g], __ldcg(pa + (size_t)s * G * HD), v);
-		a.out[(size_t)kvh * G * HD + i] = v / l_run[g];
+#pragma unroll
+		for (int k = 0; k < GROUPS; ++k) v += o_s[k * G * HD + i];
+		a.out[(size_t)kvh * G * HD + i] = v / l_all[i / HD];
 	}
 	if (threadIdx.x == 0) a.counters[kvh] = 0; // ready for the next launch
 }
@@ -295,14 +357,15 @@ static bool attn_fast_shape(int head_dim, int g) {
 }
 
 template <int HD, int G>
-static int launch_attn(const AttnArgs &a, int S, cudaStream_t st) {
-	const size_t smem = (36 + (size_t)kTile * G + (size_t)kAttnWarps * G * HD) * sizeof(float);
+static int launch_attn(AttnArgs &a, int S, cudaStream_t st) {
+	a.max_splits = std::max(1, std::min(S, Split<HD, G>::CTAS * device_info().sms / a.n_kv_heads)); // all at once
+	const size_t smem = ((size_t)S * G + (size_t)kAttnWarps * G * HD) * sizeof(float);
 	static bool configured = false;
 	if (!configured && smem > 48 * 1024) {
 		YALM_TRY(cudaFuncSetAttribute(attn_decode_kernel<HD, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
 		configured = true;
 	}
-	attn_decode_kernel<HD, G><<<dim3(S, a.n_kv_heads), kAttnThreads, smem, st>>>(a);
+	attn_decode_kernel<HD, G><<<dim3(a.max_splits, a.n_kv_heads), kAttnThreads, smem, st>>>(a);
 	return (int)cudaGetLastError();
 }
 
