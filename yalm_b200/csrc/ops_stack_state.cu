@@ -332,6 +332,12 @@ __global__ void __launch_bounds__(kScanCols * 8) state_scan_kernel(ScanArgs a) {
 		}
 }
 
+} // namespace stack
+} // namespace yalm
+#include "chunk_scan.cuh"
+namespace yalm {
+namespace stack {
+
 // dt[m, h] = softplus(dt + bias[h]) in place; decay[m, h] = exp(-exp(a_log[h]) * dt)
 __global__ void ssm_prep_rows_kernel(float *__restrict__ dt, int lddt, float *__restrict__ decay, int ldd, const float *__restrict__ bias,
                                      const float *__restrict__ a_log, int H) {
@@ -721,6 +727,25 @@ static int launch_scan(const ScanArgs &a, dim3 grid, cudaStream_t st) {
 	return (int)cudaGetLastError();
 }
 
+// Chunks of 8 positions from kChunkRows on (below, the chunks' preparation is not worth its chain; both sides at 16 heads of 128 x 128).
+constexpr int kChunkRows = 16;
+template <int D, bool DELTA, bool PER_CHANNEL>
+static int launch_chunks_of(const ScanArgs &a, cudaStream_t st) {
+	constexpr int smem = kChunkSlots * ChunkSlot<D>::SIZE * (int)sizeof(float);
+	static bool configured = false;
+	if (!configured) {
+		YALM_TRY(cudaFuncSetAttribute(chunk_scan_kernel<D, DELTA, PER_CHANNEL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+		configured = true;
+	}
+	chunk_scan_kernel<D, DELTA, PER_CHANNEL><<<dim3((a.P + kChunkCols - 1) / kChunkCols, a.H), kChunkThreads, smem, st>>>(a);
+	return (int)cudaGetLastError();
+}
+template <bool DELTA, bool PER_CHANNEL>
+static int launch_chunks(const ScanArgs &a, cudaStream_t st) {
+	return a.D == 64 ? launch_chunks_of<64, DELTA, PER_CHANNEL>(a, st) : launch_chunks_of<128, DELTA, PER_CHANNEL>(a, st);
+}
+
+
 // See ScanArgs.  k, q: (n, kv heads * D) with head h reading kv head h / rep; v, out: (n, H * P); decay: (n, H) or, with
 // decay_per_channel, (n, H * D); vscale, beta: (n, H) or null; skip: (H) or null; state: (H, P, D) fp32.  D <= 256.
 extern "C" int yalm_state_scan_rows(float *out, int ldo, const float *k, int ldk, const float *q, int ldq, const float *v, int ldv, const float *decay,
@@ -732,6 +757,10 @@ extern "C" int yalm_state_scan_rows(float *out, int ldo, const float *k, int ldk
 	ScanArgs a{out, ldo, k, q, v, decay, vscale, beta, skip, ldk, ldq, ldv, ldd, ldvs, ldb, state, n, heads, rep, D, P, pos0, ctl, vec};
 	const dim3 grid((P + kScanCols - 1) / kScanCols, heads);
 	cudaStream_t st = (cudaStream_t)s;
+	if (n >= kChunkRows && (D == 64 || D == 128) && P % 4 == 0 && vec && ((uintptr_t)state & 15) == 0) { // the rows of D floats are copied in 16-byte pieces
+		if (beta) return decay_per_channel ? launch_chunks<true, true>(a, st) : launch_chunks<true, false>(a, st);
+		return decay_per_channel ? launch_chunks<false, true>(a, st) : launch_chunks<false, false>(a, st);
+	}
 	if (beta) return decay_per_channel ? launch_scan<kScanDelta | kScanPerChannel>(a, grid, st) : launch_scan<kScanDelta>(a, grid, st);
 	return decay_per_channel ? launch_scan<kScanPerChannel>(a, grid, st) : launch_scan<0>(a, grid, st);
 }
