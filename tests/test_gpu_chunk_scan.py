@@ -1,4 +1,4 @@
-"""-m gpu: the matrix-state recurrence in chunks of 8 positions (yalm_state_scan_rows from 16 rows on) against the recurrence one position at
+"""-m gpu: the matrix-state recurrence in chunks of 8 positions (yalm_state_scan_rows from 8 rows on) against the recurrence one position at
 a time in 64 bits: last chunks of 1 .. 8 positions, portions that carry the state, fewer columns than a CTA has, heads that share keys,
 decays of 0 and 1, both scalings, a skip.
 
@@ -31,7 +31,7 @@ def step_by_step(k, q, v, decay, beta, vscale, skip, S, rep):
 
 @pytest.mark.parametrize("D,P", [(128, 128), (64, 64), (128, 4), (64, 20), (64, 36)])
 @pytest.mark.parametrize("form", ["delta_channel", "delta_head", "linear_channel", "scaled_head"])
-@pytest.mark.parametrize("portions", [(16,), (17, 24), (31, 5, 33), (100, 64)])
+@pytest.mark.parametrize("portions", [(8,), (9, 24), (31, 5, 33), (100, 64)])
 def test_chunks_match_steps(D, P, form, portions):
     L, H, rep, n = api.lib(), 4, 2, sum(portions)
     g = torch.Generator(device="cuda")

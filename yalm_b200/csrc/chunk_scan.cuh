@@ -13,8 +13,9 @@
 // vector of a chunk is read once for 4 columns (at one column per thread the shared-memory reads were the limit), the 64 partial
 // products meet over the 32 lanes by halving exchanges, which leave lane (t, c) with the sums of position t and column c.
 // The packed fp32 instructions carry two rows each.
-// Bound by the issue slots of the column warps (one per scheduler: about 700 instructions a chunk beside the preparing warps').
-// 512 rows, 16 heads of 128 x 128, decay per channel, delta rule: 125 -> 63 us; without the correction 80 -> 49 us; 64 x 64: 101 -> 49 us.
+// Bound by the column warps, one per scheduler: of about 1550 cycles a chunk 600 go to the products with M_0 (shared-memory reads of four
+// wavefronts each), 620 to the exchanges and T, 320 to the update.  (2 columns x 8 rows a lane: fewer exchanges, more reads, the same time.)
+// 512 rows, 16 heads of 128 x 128, decay per channel, delta rule: 125 -> 60 us; without the correction 80 -> 46 us; 64 x 64: 101 -> 45 us.
 #pragma once
 
 #include "tcgen.cuh"
@@ -73,6 +74,23 @@ __device__ __forceinline__ void exchange_sum(float (&v)[N]) {
 #pragma unroll
 		for (int i = 0; i < n; ++i) {
 			const float give = (lane & o) ? v[i] : v[i + n], keep = (lane & o) ? v[i + n] : v[i];
+			v[i] = keep + __shfl_xor_sync(kFull, give, o);
+		}
+}
+
+// 32 values [position][4] of which slot i holds position (i / 4) ^ (lane / 4): the lanes agree on who keeps what without a select (a lane always
+// keeps the lower slots), but for the last two exchanges, over the columns.  Afterwards v[0] is the sum of (position lane / 4, column lane % 4).
+__device__ __forceinline__ void exchange_chunk(float (&v)[32]) {
+	const int lane = threadIdx.x & 31;
+#pragma unroll
+	for (int o = 16, n = 16; o >= 4; o >>= 1, n >>= 1)
+#pragma unroll
+		for (int i = 0; i < n; ++i) v[i] += __shfl_xor_sync(kFull, v[i + n], o);
+#pragma unroll
+	for (int o = 2; o > 0; o >>= 1)
+#pragma unroll
+		for (int i = 0; i < o; ++i) {
+			const float give = (lane & o) ? v[i] : v[i + o], keep = (lane & o) ? v[i + o] : v[i];
 			v[i] = keep + __shfl_xor_sync(kFull, give, o);
 		}
 }
@@ -164,7 +182,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1) chunk_scan_kernel(const Scan
 				for (int p = 0; p < NP; ++p) w[p] = k[i][p];
 #pragma unroll
 				for (int t = i; t < kChunk; ++t) {
-					f32x2 sb, sa;
+					f32x2 sb = 0, sa = 0;
 #pragma unroll
 					for (int p = 0; p < NP; ++p) {
 						if (t > i) w[p] = mul2(w[p], g[t][p]);
@@ -228,7 +246,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1) chunk_scan_kernel(const Scan
 			for (int tt = 0; tt < kChunk; ++tt) {
 				f32x2 x[NP];
 				if constexpr (DELTA) {
-					load_pairs<NP>(x, sm + SL::K + tt * D + e0);
+					load_pairs<NP>(x, sm + SL::K + (tt ^ t) * D + e0);
 #pragma unroll
 					for (int j = 0; j < 4; ++j) {
 						f32x2 d = mul2(x[0], s[j][0]);
@@ -236,7 +254,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1) chunk_scan_kernel(const Scan
 						W[tt * 4 + j] = sum2(d);
 					}
 				}
-				load_pairs<NP>(x, sm + SL::Q + tt * D + e0);
+				load_pairs<NP>(x, sm + SL::Q + (tt ^ t) * D + e0);
 #pragma unroll
 				for (int j = 0; j < 4; ++j) {
 					f32x2 d = mul2(x[0], s[j][0]);
@@ -247,10 +265,10 @@ __global__ void __launch_bounds__(kChunkThreads, 1) chunk_scan_kernel(const Scan
 			const float v = sm[SL::V + t * kChunkCols + warp * 4 + c];
 			float r = v;
 			if constexpr (DELTA) {
-				exchange_sum(W);
+				exchange_chunk(W);
 				r = v - W[0];
 			}
-			exchange_sum(O);
+			exchange_chunk(O);
 			float u = 0.f, y = O[0];
 			float Tr[8], Br[8];
 			*reinterpret_cast<float4 *>(Tr) = *reinterpret_cast<const float4 *>(sm + SL::T + t * 8), *reinterpret_cast<float4 *>(Tr + 4) = *reinterpret_cast<const float4 *>(sm + SL::T + t * 8 + 4);

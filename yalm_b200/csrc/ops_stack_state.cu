@@ -727,8 +727,9 @@ static int launch_scan(const ScanArgs &a, dim3 grid, cudaStream_t st) {
 	return (int)cudaGetLastError();
 }
 
-// Chunks of 8 positions from kChunkRows on (below, the chunks' preparation is not worth its chain; both sides at 16 heads of 128 x 128).
-constexpr int kChunkRows = 16;
+// From a full chunk of 8 positions on (16 heads of 128 x 128, delta rule: 16 rows 8.4 -> 7.0 us, 64 rows 21 -> 12 us; 64 x 64 the same as step by
+// step at 16 rows, 16 -> 10 us at 64; below 8 rows most of a chunk would be padding).
+constexpr int kChunkRows = 8;
 template <int D, bool DELTA, bool PER_CHANNEL>
 static int launch_chunks_of(const ScanArgs &a, cudaStream_t st) {
 	constexpr int smem = kChunkSlots * ChunkSlot<D>::SIZE * (int)sizeof(float);
