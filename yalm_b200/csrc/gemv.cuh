@@ -106,14 +106,19 @@ __device__ __forceinline__ float clipf(float x, float v) { // src/infer.cpp:195-
 // Interleaved-pair RoPE of one pair whose even element sits at index j_head inside its head
 // (src/infer.cpp:200-213, src/infer.cu:541-556).  Accurate powf/cosf/sinf on purpose: pos*freq
 // reaches 3e4 rad at 32k context and the fast intrinsics lose the parity tolerance there.
+__device__ __forceinline__ void rope_angle(float &fcr, float &fci, int j_head, int pos, float theta, int rotary_dim) {
+	const float freq = j_head >= rotary_dim ? 0.f : 1.0f / powf(theta, (float)j_head / (float)rotary_dim);
+	const float val = pos * freq;
+	fcr = cosf(val), fci = sinf(val);
+}
+__device__ __forceinline__ void rope_turn(float &v0, float &v1, float fcr, float fci) {
+	const float a = v0 * fcr - v1 * fci, b = v0 * fci + v1 * fcr;
+	v0 = a, v1 = b;
+}
 __device__ __forceinline__ void rope_pair(float &v0, float &v1, int j_head, int pos, float theta, int rotary_dim) {
-	float freq = j_head >= rotary_dim ? 0.f : 1.0f / powf(theta, (float)j_head / (float)rotary_dim);
-	float val = pos * freq;
-	float fcr = cosf(val), fci = sinf(val);
-	float a = v0 * fcr - v1 * fci;
-	float b = v0 * fci + v1 * fcr;
-	v0 = a;
-	v1 = b;
+	float fcr, fci;
+	rope_angle(fcr, fci, j_head, pos, theta, rotary_dim);
+	rope_turn(v0, v1, fcr, fci);
 }
 
 } // namespace yalm

@@ -91,20 +91,42 @@ __global__ void __launch_bounds__(kSampleThreads) sample_kernel(const float *__r
 	}
 }
 
-// probs[row] = softmax(logits[row, :])[targets[row]]; one CTA per row.
-__global__ void __launch_bounds__(256) token_probs_kernel(const float *__restrict__ logits, int vocab, const int *__restrict__ targets,
-                                                          float *__restrict__ probs) {
+// probs[row] = softmax(logits[row, :])[targets[row]]; one CTA per row, every logit read once: a thread keeps 32 of them, takes their
+// maximum and sum, and joins (maximum, sum) with what it has so far and with the other threads' at the end.  Bound by the bytes of the
+// logits; two passes of one load at a time by 256 threads took 84 us for 512 rows of 32000, this XX.
+// VEC: rows are 16-byte aligned.
+template <bool VEC>
+__global__ void __launch_bounds__(1024) token_probs_kernel(const float *__restrict__ logits, int vocab, const int *__restrict__ targets,
+                                                           float *__restrict__ probs) {
 	__shared__ float red[33];
 	const float *row = logits + (size_t)blockIdx.x * vocab;
-	float m = -FLT_MAX;
-	for (int i = threadIdx.x; i < vocab; i += blockDim.x) m = fmaxf(m, row[i]);
-	m = block_max(m, red);
-	float s = 0.f;
-	for (int i = threadIdx.x; i < vocab; i += blockDim.x) s += expf(row[i] - m);
-	s = block_sum(s, red);
+	float m = -FLT_MAX, s = 0.f;
+	for (int base = 0; base < vocab; base += 1024 * 32) {
+		float v[32];
+#pragma unroll
+		for (int j = 0; j < 8; ++j) {
+			const int i = base + (j * 1024 + (int)threadIdx.x) * 4;
+			if (VEC && i < vocab) { // (vocab is a multiple of 4)
+				const float4 x = *reinterpret_cast<const float4 *>(row + i);
+				v[4 * j] = x.x, v[4 * j + 1] = x.y, v[4 * j + 2] = x.z, v[4 * j + 3] = x.w;
+			} else {
+#pragma unroll
+				for (int e = 0; e < 4; ++e) v[4 * j + e] = !VEC && i + e < vocab ? row[i + e] : -INFINITY;
+			}
+		}
+		float top = m;
+#pragma unroll
+		for (int j = 0; j < 32; ++j) top = fmaxf(top, v[j]);
+		s *= expf(m - top);
+		m = top;
+#pragma unroll
+		for (int j = 0; j < 32; ++j) s += expf(v[j] - m);
+	}
+	const float M = block_max(m, red);
+	s = block_sum(s * expf(m - M), red);
 	if (threadIdx.x == 0) {
 		const int t = targets[blockIdx.x];
-		probs[blockIdx.x] = (t >= 0 && t < vocab) ? expf(row[t] - m) / s : 0.f;
+		probs[blockIdx.x] = (t >= 0 && t < vocab) ? expf(row[t] - M) / s : 0.f;
 	}
 }
 
@@ -123,7 +145,8 @@ extern "C" int yalm_sample_advance(const float *logits, int vocab, int *ctl, int
 
 extern "C" int yalm_token_probs(const float *logits, int vocab, int n_rows, const int *targets, float *probs, yalm_stream_t s) {
 	if (!logits || !targets || !probs || vocab <= 0 || n_rows < 1) return YALM_EINVAL;
-	token_probs_kernel<<<n_rows, 256, 0, (cudaStream_t)s>>>(logits, vocab, targets, probs);
+	if (vocab % 4 == 0 && ((uintptr_t)logits & 15) == 0) token_probs_kernel<true><<<n_rows, 1024, 0, (cudaStream_t)s>>>(logits, vocab, targets, probs);
+	else token_probs_kernel<false><<<n_rows, 1024, 0, (cudaStream_t)s>>>(logits, vocab, targets, probs);
 	return (int)cudaGetLastError();
 }
 

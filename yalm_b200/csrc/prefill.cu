@@ -42,45 +42,68 @@ __global__ void embed_rows_kernel(float *__restrict__ x, const __half *__restric
 }
 
 // out16[i, :] = half(x[i, :] * (1 / sqrt(mean(x^2) + eps)) * w)   (src/infer.cpp:134-144, one CTA per row)
-__global__ void __launch_bounds__(256) rmsnorm_rows_kernel(__half *__restrict__ out, const float *__restrict__ x, const float *__restrict__ w,
-                                                           int dim, float eps) {
+// Rows of up to 8192 stay in registers between the sum and the scaling, all their loads in flight at once (512 rows of 4096: 6.7 -> XX us).
+constexpr int kNormThreads = 256, kNormKept = 8;
+__global__ void __launch_bounds__(kNormThreads) rmsnorm_rows_kernel(__half *__restrict__ out, const float *__restrict__ x, const float *__restrict__ w,
+                                                                    int dim, float eps) {
 	__shared__ float red[33];
 	const float *row = x + (size_t)blockIdx.x * dim;
+	const bool kept = dim <= kNormThreads * 4 * kNormKept;
+	float4 v[kNormKept];
 	float ss = 0.f;
-	for (int e = threadIdx.x * 4; e < dim; e += blockDim.x * 4) {
-		const float4 v = *reinterpret_cast<const float4 *>(row + e);
-		ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-	}
+	if (kept) {
+#pragma unroll
+		for (int j = 0; j < kNormKept; ++j) {
+			const int e = (threadIdx.x + j * kNormThreads) * 4;
+			v[j] = e < dim ? *reinterpret_cast<const float4 *>(row + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+		}
+#pragma unroll
+		for (int j = 0; j < kNormKept; ++j) ss += v[j].x * v[j].x + v[j].y * v[j].y + v[j].z * v[j].z + v[j].w * v[j].w;
+	} else
+		for (int e = threadIdx.x * 4; e < dim; e += kNormThreads * 4) {
+			const float4 t = *reinterpret_cast<const float4 *>(row + e);
+			ss += t.x * t.x + t.y * t.y + t.z * t.z + t.w * t.w;
+		}
 	ss = block_sum(ss, red);
 	const float scale = 1.0f / sqrtf(ss / dim + eps);
 	__half *dst = out + (size_t)blockIdx.x * dim;
-	for (int e = threadIdx.x * 4; e < dim; e += blockDim.x * 4) {
-		const float4 v = *reinterpret_cast<const float4 *>(row + e), g = *reinterpret_cast<const float4 *>(w + e);
-		*reinterpret_cast<__half2 *>(dst + e) = __floats2half2_rn(v.x * scale * g.x, v.y * scale * g.y);
-		*reinterpret_cast<__half2 *>(dst + e + 2) = __floats2half2_rn(v.z * scale * g.z, v.w * scale * g.w);
-	}
+	auto put = [&](int e, float4 t) {
+		const float4 g = *reinterpret_cast<const float4 *>(w + e);
+		*reinterpret_cast<__half2 *>(dst + e) = __floats2half2_rn(t.x * scale * g.x, t.y * scale * g.y);
+		*reinterpret_cast<__half2 *>(dst + e + 2) = __floats2half2_rn(t.z * scale * g.z, t.w * scale * g.w);
+	};
+	if (kept) {
+#pragma unroll
+		for (int j = 0; j < kNormKept; ++j) {
+			const int e = (threadIdx.x + j * kNormThreads) * 4;
+			if (e < dim) put(e, v[j]);
+		}
+	} else
+		for (int e = threadIdx.x * 4; e < dim; e += kNormThreads * 4) put(e, *reinterpret_cast<const float4 *>(row + e));
 }
 
 // Row i of qkv (fp32: q | k | v) = position pos0 + i: clip, interleaved-pair RoPE on q and k (src/infer.cpp:200-213,
 // 282-292), q -> fp16 (attention operand), k / v -> fp16 rows pos0 + i of the head-major KV ring (src/infer.cpp:294-301).
-__global__ void __launch_bounds__(256) rope_append_rows_kernel(__half *__restrict__ q16, __half *__restrict__ kc, __half *__restrict__ vc,
-                                                               const float *__restrict__ qkv, int q_dim, int kv_dim, int head_dim,
+// A thread takes one pair of a head's channels through every blockDim / half-th head: the angle's power, sine and cosine, most of the work, are
+// formed once per thread instead of once per pair (512 rows of 32 + 8 heads of 128: 18 -> XX us).
+__global__ void __launch_bounds__(512) rope_append_rows_kernel(__half *__restrict__ q16, __half *__restrict__ kc, __half *__restrict__ vc,
+                                                               const float *__restrict__ qkv, int n_heads, int n_kv, int head_dim,
                                                                int rotary_dim, int max_seq_len, int pos0, float theta, float clip) {
-	const int i = blockIdx.x, pos = pos0 + i;
-	const float *row = qkv + (size_t)i * (q_dim + 2 * kv_dim);
-	for (int p = threadIdx.x; p < (q_dim + 2 * kv_dim) / 2; p += blockDim.x) {
-		const int e = 2 * p;
-		float v0 = clipf(row[e], clip), v1 = clipf(row[e + 1], clip);
-		if (e < q_dim) {
-			rope_pair(v0, v1, e % head_dim, pos, theta, rotary_dim);
-			*reinterpret_cast<__half2 *>(q16 + (size_t)i * q_dim + e) = __floats2half2_rn(v0, v1);
-		} else {
-			const bool is_k = e < q_dim + kv_dim;
-			const int c = e - q_dim - (is_k ? 0 : kv_dim), h = c / head_dim, j = c % head_dim;
-			if (is_k) rope_pair(v0, v1, j, pos, theta, rotary_dim);
-			__half *dst = (is_k ? kc : vc) + ((size_t)h * max_seq_len + pos) * head_dim + j;
-			*reinterpret_cast<__half2 *>(dst) = __floats2half2_rn(v0, v1);
-		}
+	const int i = blockIdx.x, pos = pos0 + i, half = head_dim / 2, at_once = blockDim.x / half, q_dim = n_heads * head_dim;
+	const int j = (threadIdx.x % half) * 2, first = threadIdx.x / half;
+	if (first >= at_once) return;
+	const float *row = qkv + (size_t)i * (q_dim + 2 * n_kv * head_dim);
+	float fcr, fci;
+	rope_angle(fcr, fci, j, pos, theta, rotary_dim);
+#pragma unroll 4
+	for (int h = first; h < n_heads + 2 * n_kv; h += at_once) { // q heads, k heads, v heads
+		const float2 v = *reinterpret_cast<const float2 *>(row + (size_t)h * head_dim + j);
+		float v0 = clipf(v.x, clip), v1 = clipf(v.y, clip);
+		if (h < n_heads + n_kv) rope_turn(v0, v1, fcr, fci);
+		__half *dst = h < n_heads ? q16 + (size_t)i * q_dim + h * head_dim
+		                          : (h < n_heads + n_kv ? kc + ((size_t)(h - n_heads) * max_seq_len + pos) * head_dim
+		                                                : vc + ((size_t)(h - n_heads - n_kv) * max_seq_len + pos) * head_dim);
+		*reinterpret_cast<__half2 *>(dst + j) = __floats2half2_rn(v0, v1);
 	}
 }
 
@@ -163,21 +186,21 @@ int Model::forward_batch(InferenceState &s, const int *tokens, int n, int pos0, 
 	int rc;
 	for (auto &bp : blocks) {
 		const Block &b = *bp;
-		rmsnorm_rows_kernel<<<n, 256, 0, st>>>(P.xb, P.x, b._rms_att_weight, dim, c.norm_eps);
+		rmsnorm_rows_kernel<<<n, kNormThreads, 0, st>>>(P.xb, P.x, b._rms_att_weight, dim, c.norm_eps);
 		// q | k | v of the chunk into one (n, q_dim + 2 kv_dim) fp32 buffer
 		const int ld = q_dim + 2 * kv_dim;
 		if ((rc = gemm_qkv_f16(P.qkv, ld, P.xb, b._wq, b._wk, b._wv, n, q_dim, kv_dim, dim, st))) return rc;
-		rope_append_rows_kernel<<<n, 256, 0, st>>>(P.q16, reinterpret_cast<__half *>(b._key_cache), reinterpret_cast<__half *>(b._value_cache),
-		                                          P.qkv, q_dim, kv_dim, c.head_dim, c.rotary_dim, c.max_seq_len, pos0, c.rope_theta, c.qkv_clip);
+		rope_append_rows_kernel<<<n, 512, 0, st>>>(P.q16, reinterpret_cast<__half *>(b._key_cache), reinterpret_cast<__half *>(b._value_cache), P.qkv, c.n_heads,
+		                                          c.n_kv_heads, c.head_dim, c.rotary_dim, c.max_seq_len, pos0, c.rope_theta, c.qkv_clip);
 		if ((rc = yalm_attn_prefill(P.att, P.q16, b._key_cache, b._value_cache, n, pos0, c.n_heads, c.n_kv_heads, c.head_dim, c.max_seq_len, st)))
 			return rc;
 		if ((rc = yalm_gemm_f16(P.x, dim, P.att, b._wo, n, dim, q_dim, 1, st))) return rc; // x += Wo att
-		rmsnorm_rows_kernel<<<n, 256, 0, st>>>(P.xb, P.x, b._rms_ffn_weight, dim, c.norm_eps);
+		rmsnorm_rows_kernel<<<n, kNormThreads, 0, st>>>(P.xb, P.x, b._rms_ffn_weight, dim, c.norm_eps);
 		if ((rc = yalm_gemm_glu_f16(P.hb, hid, P.xb, b._w1, b._w3, n, hid, dim, act, st))) return rc;
 		if ((rc = yalm_gemm_f16(P.x, dim, P.hb, b._w2, n, dim, hid, 1, st))) return rc; // x += W2 hb
 	}
 	if (targets) { // per-position logits -> probability of the given next token (Sampler::sample_prob per row)
-		rmsnorm_rows_kernel<<<n, 256, 0, st>>>(P.xb, P.x, rms_final_weight, dim, c.norm_eps);
+		rmsnorm_rows_kernel<<<n, kNormThreads, 0, st>>>(P.xb, P.x, rms_final_weight, dim, c.norm_eps);
 		if ((rc = yalm_gemm_f16(P.logits, V, P.xb, wcls, n, V, dim, 0, st))) return rc;
 		if ((rc = yalm_token_probs(P.logits, V, n, P.targets, P.probs, st))) return rc;
 		YALM_TRY(cudaMemcpyAsync(probs_out, P.probs, sizeof(float) * n, cudaMemcpyDeviceToHost, st));

@@ -553,7 +553,7 @@ static int launch_clusters(void (*kernel)(const CUtensorMap, const WeightMaps, c
 	cudaLaunchAttribute at[1];
 	at[0].id = cudaLaunchAttributeClusterDimension;
 	at[0].val.clusterDim.x = cluster, at[0].val.clusterDim.y = 1, at[0].val.clusterDim.z = 1;
-	cfg.attrs = at, cfg.numAttrs = 1;
+	cfg.attrs = at, cfg.numAttrs = cluster > 1;
 	YALM_TRY(cudaLaunchKernelEx(&cfg, kernel, ta, tb, g));
 	return 0;
 }

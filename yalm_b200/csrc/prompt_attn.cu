@@ -688,7 +688,7 @@ static int launch(Args &a, const void *keys, const void *values, int map_rows, i
 	const int pairs = (a.n * a.G + 2 * kTile - 1) / (2 * kTile), units = pairs * a.n_kv;
 	a.parts = 1;
 	for (int i = 1; i < 4 && (1 << i) <= DV / 8 && units <= room[i] && est_tiles >= (2 << i); ++i) a.parts = 1 << i;
-	at[0].val.clusterDim.x = a.parts;
+	at[0].val.clusterDim.x = a.parts, cfg.numAttrs = a.parts > 1;
 	cfg.gridDim = dim3(pairs * a.parts, a.n_kv), cfg.stream = st;
 	YALM_TRY(cudaLaunchKernelEx(&cfg, kernel, tk, tv, a));
 	return 0;
