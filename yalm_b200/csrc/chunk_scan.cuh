@@ -109,6 +109,8 @@ __global__ void __launch_bounds__(kChunkThreads, 1) chunk_scan_kernel(const Scan
 	if (threadIdx.x == 0)
 		for (int i = 0; i < kChunkSlots; ++i) mbar_init(full0 + 8 * i, 1), mbar_init(empty0 + 8 * i, col_warps);
 	__syncthreads();
+	chain_wait();
+	chain_next();
 
 	if (warp >= 4) { // ---- prepare chunks warp - 4, warp - 4 + kPrepWarps, .. ; a lane holds rows lane D / 32 .. of every vector ----
 		const int e0 = lane * 2 * NP;

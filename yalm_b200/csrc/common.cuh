@@ -47,6 +47,12 @@ __device__ __forceinline__ uint4 ldg_stream(const void *p) {
 	return r;
 }
 
+// Kernels that are launched with launch_chained (launch.h) may begin while the kernel before them in the stream still runs: what they
+// do before chain_wait() must not touch global memory, and returns from it with everything before them complete and visible.
+// chain_next() lets the next such kernel begin (it waits in turn).
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
 	for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);

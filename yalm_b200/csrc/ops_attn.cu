@@ -83,6 +83,8 @@ __global__ void __launch_bounds__(kAttnThreads, Split<HD, G>::CTAS) attn_decode_
 	__shared__ unsigned is_last;
 
 	const int kvh = blockIdx.y, split = blockIdx.x;
+	chain_wait();
+	chain_next();
 	const int kv_len = a.ctl[CTL_KVLEN];
 	const int S = min(a.max_splits, max(1, (kv_len + RPC * UN - 1) / (RPC * UN))); // splits that have rows
 	if (split >= S) return;
@@ -365,8 +367,7 @@ static int launch_attn(AttnArgs &a, int S, cudaStream_t st) {
 		YALM_TRY(cudaFuncSetAttribute(attn_decode_kernel<HD, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
 		configured = true;
 	}
-	attn_decode_kernel<HD, G><<<dim3(a.max_splits, a.n_kv_heads), kAttnThreads, smem, st>>>(a);
-	return (int)cudaGetLastError();
+	return launch_chained(attn_decode_kernel<HD, G>, dim3(a.max_splits, a.n_kv_heads), dim3(kAttnThreads), smem, st, 1, a);
 }
 
 } // namespace yalm

@@ -8,6 +8,7 @@
 //                       needs per position (src/main.cpp:174-184), one float back per row instead of a vocab row.
 // temperature == 0 is the greedy path (yalm_argmax_advance).
 #include "common.cuh"
+#include "launch.h"
 
 #include <cfloat>
 
@@ -99,6 +100,8 @@ template <bool VEC>
 __global__ void __launch_bounds__(1024) token_probs_kernel(const float *__restrict__ logits, int vocab, const int *__restrict__ targets,
                                                            float *__restrict__ probs) {
 	__shared__ float red[33];
+	chain_wait();
+	chain_next();
 	const float *row = logits + (size_t)blockIdx.x * vocab;
 	float m = -FLT_MAX, s = 0.f;
 	for (int base = 0; base < vocab; base += 1024 * 32) {
@@ -145,9 +148,8 @@ extern "C" int yalm_sample_advance(const float *logits, int vocab, int *ctl, int
 
 extern "C" int yalm_token_probs(const float *logits, int vocab, int n_rows, const int *targets, float *probs, yalm_stream_t s) {
 	if (!logits || !targets || !probs || vocab <= 0 || n_rows < 1) return YALM_EINVAL;
-	if (vocab % 4 == 0 && ((uintptr_t)logits & 15) == 0) token_probs_kernel<true><<<n_rows, 1024, 0, (cudaStream_t)s>>>(logits, vocab, targets, probs);
-	else token_probs_kernel<false><<<n_rows, 1024, 0, (cudaStream_t)s>>>(logits, vocab, targets, probs);
-	return (int)cudaGetLastError();
+	const bool vec = vocab % 4 == 0 && ((uintptr_t)logits & 15) == 0;
+	return launch_chained(vec ? token_probs_kernel<true> : token_probs_kernel<false>, dim3(n_rows), dim3(1024), 0, (cudaStream_t)s, 1, logits, vocab, targets, probs);
 }
 
 // first-max arg-max of a device row into a device int (Sampler::sample_device at temperature 0)

@@ -738,8 +738,7 @@ static int launch_chunks_of(const ScanArgs &a, cudaStream_t st) {
 		YALM_TRY(cudaFuncSetAttribute(chunk_scan_kernel<D, DELTA, PER_CHANNEL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
 		configured = true;
 	}
-	chunk_scan_kernel<D, DELTA, PER_CHANNEL><<<dim3((a.P + kChunkCols - 1) / kChunkCols, a.H), kChunkThreads, smem, st>>>(a);
-	return (int)cudaGetLastError();
+	return launch_chained(chunk_scan_kernel<D, DELTA, PER_CHANNEL>, dim3((a.P + kChunkCols - 1) / kChunkCols, a.H), dim3(kChunkThreads), smem, st, 1, a);
 }
 template <bool DELTA, bool PER_CHANNEL>
 static int launch_chunks(const ScanArgs &a, cudaStream_t st) {

@@ -8,6 +8,7 @@
 #include "yalm_api.h"
 
 #include "gemv.cuh"
+#include "launch.h"
 
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -47,6 +48,8 @@ constexpr int kNormThreads = 256, kNormKept = 8;
 __global__ void __launch_bounds__(kNormThreads) rmsnorm_rows_kernel(__half *__restrict__ out, const float *__restrict__ x, const float *__restrict__ w,
                                                                     int dim, float eps) {
 	__shared__ float red[33];
+	chain_wait();
+	chain_next();
 	const float *row = x + (size_t)blockIdx.x * dim;
 	const bool kept = dim <= kNormThreads * 4 * kNormKept;
 	float4 v[kNormKept];
@@ -92,6 +95,8 @@ __global__ void __launch_bounds__(512) rope_append_rows_kernel(__half *__restric
 	const int i = blockIdx.x, pos = pos0 + i, half = head_dim / 2, at_once = blockDim.x / half, q_dim = n_heads * head_dim;
 	const int j = (threadIdx.x % half) * 2, first = threadIdx.x / half;
 	if (first >= at_once) return;
+	chain_wait();
+	chain_next();
 	const float *row = qkv + (size_t)i * (q_dim + 2 * n_kv * head_dim);
 	float fcr, fci;
 	rope_angle(fcr, fci, j, pos, theta, rotary_dim);
@@ -186,21 +191,23 @@ int Model::forward_batch(InferenceState &s, const int *tokens, int n, int pos0, 
 	int rc;
 	for (auto &bp : blocks) {
 		const Block &b = *bp;
-		rmsnorm_rows_kernel<<<n, kNormThreads, 0, st>>>(P.xb, P.x, b._rms_att_weight, dim, c.norm_eps);
+		if ((rc = launch_chained(rmsnorm_rows_kernel, dim3(n), dim3(kNormThreads), 0, st, 1, P.xb, P.x, b._rms_att_weight, dim, c.norm_eps))) return rc;
 		// q | k | v of the chunk into one (n, q_dim + 2 kv_dim) fp32 buffer
 		const int ld = q_dim + 2 * kv_dim;
 		if ((rc = gemm_qkv_f16(P.qkv, ld, P.xb, b._wq, b._wk, b._wv, n, q_dim, kv_dim, dim, st))) return rc;
-		rope_append_rows_kernel<<<n, 512, 0, st>>>(P.q16, reinterpret_cast<__half *>(b._key_cache), reinterpret_cast<__half *>(b._value_cache), P.qkv, c.n_heads,
-		                                          c.n_kv_heads, c.head_dim, c.rotary_dim, c.max_seq_len, pos0, c.rope_theta, c.qkv_clip);
+		if ((rc = launch_chained(rope_append_rows_kernel, dim3(n), dim3(512), 0, st, 1, P.q16, reinterpret_cast<__half *>(b._key_cache),
+		                         reinterpret_cast<__half *>(b._value_cache), (const float *)P.qkv, c.n_heads, c.n_kv_heads, c.head_dim, c.rotary_dim, c.max_seq_len, pos0,
+		                         c.rope_theta, c.qkv_clip)))
+			return rc;
 		if ((rc = yalm_attn_prefill(P.att, P.q16, b._key_cache, b._value_cache, n, pos0, c.n_heads, c.n_kv_heads, c.head_dim, c.max_seq_len, st)))
 			return rc;
 		if ((rc = yalm_gemm_f16(P.x, dim, P.att, b._wo, n, dim, q_dim, 1, st))) return rc; // x += Wo att
-		rmsnorm_rows_kernel<<<n, kNormThreads, 0, st>>>(P.xb, P.x, b._rms_ffn_weight, dim, c.norm_eps);
+		if ((rc = launch_chained(rmsnorm_rows_kernel, dim3(n), dim3(kNormThreads), 0, st, 1, P.xb, P.x, b._rms_ffn_weight, dim, c.norm_eps))) return rc;
 		if ((rc = yalm_gemm_glu_f16(P.hb, hid, P.xb, b._w1, b._w3, n, hid, dim, act, st))) return rc;
 		if ((rc = yalm_gemm_f16(P.x, dim, P.hb, b._w2, n, dim, hid, 1, st))) return rc; // x += W2 hb
 	}
 	if (targets) { // per-position logits -> probability of the given next token (Sampler::sample_prob per row)
-		rmsnorm_rows_kernel<<<n, kNormThreads, 0, st>>>(P.xb, P.x, rms_final_weight, dim, c.norm_eps);
+		if ((rc = launch_chained(rmsnorm_rows_kernel, dim3(n), dim3(kNormThreads), 0, st, 1, P.xb, P.x, rms_final_weight, dim, c.norm_eps))) return rc;
 		if ((rc = yalm_gemm_f16(P.logits, V, P.xb, wcls, n, V, dim, 0, st))) return rc;
 		if ((rc = yalm_token_probs(P.logits, V, n, P.targets, P.probs, st))) return rc;
 		YALM_TRY(cudaMemcpyAsync(probs_out, P.probs, sizeof(float) * n, cudaMemcpyDeviceToHost, st));

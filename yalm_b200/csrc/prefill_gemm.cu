@@ -181,6 +181,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
 	if (warp == 1) tmem_alloc<2>(tslot, 512);
 	tc_fence_before();
 	cluster_sync();
+	chain_wait();
+	chain_next();
 	tc_fence_after();
 	uint32_t tmem;
 	asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(tslot));
@@ -381,6 +383,8 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ 
 	if (warp == 1) tmem_alloc<1>(tslot, cols);
 	tc_fence_before();
 	__syncthreads();
+	chain_wait();
+	chain_next();
 	tc_fence_after();
 	uint32_t tmem;
 	asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(tslot));
@@ -546,18 +550,6 @@ static int column_tiles(const GemmArgs &g, int n) {
 	return tiles;
 }
 
-static int launch_clusters(void (*kernel)(const CUtensorMap, const WeightMaps, const GemmArgs), int ctas, int cluster, size_t smem, const CUtensorMap &ta,
-                           const WeightMaps &tb, const GemmArgs &g, cudaStream_t st) {
-	cudaLaunchConfig_t cfg = {};
-	cfg.gridDim = dim3(ctas), cfg.blockDim = dim3(kGemmThreads), cfg.dynamicSmemBytes = smem, cfg.stream = st;
-	cudaLaunchAttribute at[1];
-	at[0].id = cudaLaunchAttributeClusterDimension;
-	at[0].val.clusterDim.x = cluster, at[0].val.clusterDim.y = 1, at[0].val.clusterDim.z = 1;
-	cfg.attrs = at, cfg.numAttrs = cluster > 1;
-	YALM_TRY(cudaLaunchKernelEx(&cfg, kernel, ta, tb, g));
-	return 0;
-}
-
 static size_t pair_stage_bytes(bool glu, int n) { return (size_t)(128 + (glu ? n : n / 2)) * kRowBytes; }
 static int pair_stages(bool glu, int n) { return (int)std::min<size_t>(10, 196608 / pair_stage_bytes(glu, n)); }
 static size_t pair_smem(bool glu, int n) { return pair_stages(glu, n) * pair_stage_bytes(glu, n) + kTailBytes + 1024; }
@@ -622,7 +614,7 @@ static int launch_pair(GemmArgs &g, const void *a, int a_rows, const void *const
 	}
 	if (rc) return rc;
 	const int clusters = g.splits > 1 ? g.items : std::min(g.items, here[0]);
-	return launch_clusters(kernel, clusters * 2 * g.splits, 2 * g.splits, pair_smem(GLU, g.n_tile), ta, tb, g, st);
+	return launch_chained(kernel, dim3(clusters * 2 * g.splits), dim3(kGemmThreads), pair_smem(GLU, g.n_tile), st, 2 * g.splits, ta, tb, g);
 }
 
 // Few rows: an SM's shared memory for stages, or half of it (two CTAs at once) where there are more tiles than SMs.  K parts
@@ -664,7 +656,7 @@ static int launch_few(GemmArgs &g, const void *a, int a_rows, const void *const 
 		else tb.m[i] = tb.m[0];
 	}
 	if (rc) return rc;
-	return launch_clusters(kernel, g.items * g.splits, g.splits, smem, ta, tb, g, st);
+	return launch_chained(kernel, dim3(g.items * g.splits), dim3(kGemmThreads), smem, st, g.splits, ta, tb, g);
 }
 
 // Where the few-rows kernel ends: 128 positions are one operand of it, and up to there it is ahead of the pairs (4096 x 14336: 43 us

@@ -204,6 +204,20 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 	const int rows = a.n * a.G, pairs = (rows + 2 * kTile - 1) / (2 * kTile);
 	const int pair = pairs - 1 - (int)(blockIdx.x / parts); // the longest rows first
 	const int g = blockIdx.y, r0 = pair * 2 * kTile, nt = r0 + kTile < rows ? 2 : 1;
+	if (threadIdx.x == 0) {
+		// a value stage (odd) is free again once its products are done and, in a layered model, warps 2 and 3 have passed it
+		for (int i = 0; i < NST; ++i) mbar_init(full0 + 8 * i, 1), mbar_init(empty0 + 8 * i, LAYERED && (i & 1) ? 3 : 1);
+		for (int i = 0; i < 2; ++i) mbar_init(s_full0 + 8 * i, 1);
+		for (int i = 0; i < 4; ++i) mbar_init(p_full0 + 8 * i, 4); // [tile][half of the keys]
+		mbar_init(o_full, 1);
+		if (LAYERED)
+			for (int i = 0; i < NST; ++i) mbar_init(v_clean0 + 8 * i, 1);
+		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+	}
+	if (warp == 1) tmem_alloc<1>(tslot, 512);
+	__syncwarp();
+	chain_wait();
+	chain_next();
 	const int p0 = a.ctl ? a.ctl[CTL_POS] : a.pos0;
 	const Tiles tiles(a, p0 + r0 / a.G, p0 + min((r0 + 2 * kTile - 1) / a.G, a.n - 1));
 	const int per = (tiles.total + parts - 1) / parts, k_begin = min(part * per, tiles.total), k_end = min(k_begin + per, tiles.total), nk = k_end - k_begin;
@@ -248,21 +262,10 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 		proxy_fence();
 	};
 
-	if (threadIdx.x == 0) {
-		// a value stage (odd) is free again once its products are done and, in a layered model, warps 2 and 3 have passed it
-		for (int i = 0; i < NST; ++i) mbar_init(full0 + 8 * i, 1), mbar_init(empty0 + 8 * i, LAYERED && (i & 1) ? 3 : 1);
-		for (int i = 0; i < 2; ++i) mbar_init(s_full0 + 8 * i, 1);
-		for (int i = 0; i < 4; ++i) mbar_init(p_full0 + 8 * i, 4); // [tile][half of the keys]
-		mbar_init(o_full, 1);
-		if (LAYERED)
-			for (int i = 0; i < NST; ++i) mbar_init(v_clean0 + 8 * i, 1);
-		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-	}
 	if (warp == 0) {
 		__syncwarp();
 		for (int e = 0; e < NST && e < 2 * nk; ++e) load(e >> 1, e & 1); // the stages are free: the first tiles travel while the queries are staged
 	}
-	if (warp == 1) tmem_alloc<1>(tslot, 512);
 	if (warp > 0) { // the queries' rows (rows past the last: zero), and the first tile where it is a pooled one
 		// a thread keeps its 16-byte column and steps down the rows (the position and head of a row follow without a division); all loads of
 		// a batch are in flight together: one at a time this took as long as four key tiles
@@ -696,10 +699,7 @@ static int launch(Args &a, const void *keys, const void *values, int map_rows, i
 	const int pairs = (a.n * a.G + 2 * kTile - 1) / (2 * kTile), units = pairs * a.n_kv;
 	a.parts = 1;
 	for (int i = 1; i < 4 && (1 << i) <= DV / 8 && units <= room[i] && est_tiles >= (2 << i); ++i) a.parts = 1 << i;
-	at[0].val.clusterDim.x = a.parts, cfg.numAttrs = a.parts > 1;
-	cfg.gridDim = dim3(pairs * a.parts, a.n_kv), cfg.stream = st;
-	YALM_TRY(cudaLaunchKernelEx(&cfg, kernel, tk, tv, a));
-	return 0;
+	return launch_chained(kernel, dim3(pairs * a.parts, a.n_kv), dim3(kThreads), SH::SMEM, st, a.parts, tk, tv, a);
 }
 
 constexpr float kLog2e = 1.4426950408889634f;
