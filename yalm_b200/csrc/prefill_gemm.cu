@@ -554,9 +554,11 @@ static size_t pair_stage_bytes(bool glu, int n) { return (size_t)(128 + (glu ? n
 static int pair_stages(bool glu, int n) { return (int)std::min<size_t>(10, 196608 / pair_stage_bytes(glu, n)); }
 static size_t pair_smem(bool glu, int n) { return pair_stages(glu, n) * pair_stage_bytes(glu, n) + kTailBytes + 1024; }
 
-// Tile width and K parts of the pair kernel, by estimated cycles: waves of tiles x K blocks x the larger of the MMA's cycles (2 per
-// column and block) and the staging's (an SM receives about 48 bytes a cycle), plus pipeline fill, the last tail and, with K parts, the
-// exchange.  slots: clusters of 2, 4, 8 CTAs that run at once.  Parts of K only where all tiles run at once.
+// Tile width and K parts of the pair kernel, by estimated cycles: waves of tiles x K blocks x (190 + 2.05 per accumulator column and block, the
+// MMA and what a block costs beside it), the last tail, and with K parts the exchange.  The constants are fitted to sweeps over both at 256 .. 512
+// rows: 4096 x 4096 in one part 32.1 us at 256 columns, 21.3 at 128, in two 23.0; 2048 x 8192 44.2 (128 columns, one part) against 30.8 (two); 1024 x 4096
+// 23.4 (64, one) against 16.7 (two) and 25.7 (256, four: a cluster of 8 costs some 8 us).  slots: clusters of 2, 4, 8 CTAs that run at once.
+// Parts of K only where all tiles run at once.
 static void plan_pair(GemmArgs &g, bool glu, const int (&slots)[3]) {
 	const int nkb = (g.K + BK - 1) / BK;
 	double best = 1e30;
@@ -570,8 +572,7 @@ static void plan_pair(GemmArgs &g, bool glu, const int (&slots)[3]) {
 			const int items = g.m_tiles * column_tiles(g, n);
 			if (slots[si] < 1 || (S > 1 && items > slots[si])) continue;
 			const int waves = (items + slots[si] - 1) / slots[si], nacc = glu ? 2 * n : n;
-			const double block = std::max(2.0 * nacc, (128 + nacc / 2) * (double)kRowBytes / 48.0);
-			const double cost = waves * per * block + 2500 + 16.0 * nacc / S + (S > 1 ? 3000 + 8.0 * nacc : 0);
+			const double cost = waves * per * (190 + 2.05 * nacc) + 16.0 * nacc / S + (S > 1 ? (S == 2 ? 1000 : 15000) + 36.0 * nacc : 0);
 			if (cost < best * 0.999) best = cost, g.n_tile = n, g.splits = S, g.items = items, g.kb_per = per;
 		}
 	}
