@@ -206,7 +206,7 @@ int yalm_attn_window_pool(float *out, int ldo, const float *q, int ldq, const vo
                           const float *key_pool, const float *value_pool, float *workspace, int n, int n_heads, int n_kv, int dk, int dv,
                           int ring, int max_blocks, int window, int pool, float scale, int cache_f32, int context, int pos0, const int *ctl,
                           yalm_stream_t s);
-/* The same attention for many rows over bf16 rings on the tensor cores (mma.sync bf16, fp32 scores / softmax): head sizes
+/* The same attention for many rows over bf16 rings on the tensor cores (bf16 operands, fp32 scores / softmax): head sizes
  * dk in {64, 128}, dv in {32, 64, 128} (yalm_attn_window_pool_mma_shape), ldq % 4 == 0, ldo % 2 == 0. */
 int yalm_attn_window_pool_mma_shape(int dk, int dv);
 int yalm_attn_window_pool_mma(float *out, int ldo, const float *q, int ldq, const void *key_ring, const void *value_ring,
