@@ -1,0 +1,48 @@
+"""-m gpu: the one-row products at sizes where their rows are dealt out in larger and in smaller tasks (fewer rows than warps, a last round
+with few tasks, odd counts of rows), against 64 bits.  Bound: fp32 sums of n <= 11008 products, 1e-6 of the norm (measured 3e-7)."""
+import ctypes as C
+
+import pytest
+import torch
+
+from yalm_b200 import api
+
+pytestmark = pytest.mark.gpu
+TYPES = {"fp32": (torch.float32, api.F32), "fp16": (torch.float16, api.F16), "bf16": (torch.bfloat16, api.BF16)}
+
+
+def p(t):
+    return C.c_void_p(None if t is None else t.data_ptr())
+
+
+def rel(got, want):
+    return ((got.double() - want).norm() / want.norm()).item()
+
+
+@pytest.mark.parametrize("dtype", ["fp32", "fp16", "bf16"])
+@pytest.mark.parametrize("d,n", [(1, 64), (3, 4096), (2047, 1032), (4096, 4096), (6145, 512), (9473, 256), (14211, 264), (32001, 128)])
+def test_rows(d, n, dtype):
+    L, (td, code) = api.lib(), TYPES[dtype]
+    torch.manual_seed(d)
+    w, x, out = torch.randn((d, n), device="cuda").to(td), torch.randn(n, device="cuda"), torch.full((d + 4,), 7.0, device="cuda")
+    assert L.yalm_gemv_scaled(p(out), p(x), p(w), C.c_int(n), C.c_int(d), C.c_int(code), C.c_float(0.5), None) == 0
+    assert rel(out[:d], 0.5 * (w.double() @ x.double())) < 1e-6 and (out[d:] == 7.0).all()
+
+
+@pytest.mark.parametrize("dtype", ["fp32", "fp16"])
+@pytest.mark.parametrize("dim,hidden", [(64, 32), (1024, 2816), (1600, 5120), (2048, 2050), (4096, 11008), (1024, 14336)])
+def test_feed_forward(dim, hidden, dtype):
+    L, (td, code) = api.lib(), TYPES[dtype]
+    torch.manual_seed(dim + hidden)
+    x, norm = torch.randn(dim, device="cuda"), 1 + 0.1 * torch.randn(dim, device="cuda")
+    w1, w3 = ((torch.randn((hidden, dim), device="cuda") * dim ** -0.5).to(td) for _ in range(2))
+    hb = torch.full((hidden + 4,), 7.0, device="cuda")
+    assert L.yalm_ffn_glu(p(hb), p(x), p(norm), p(w1), p(w3), None, None, None, None, C.c_int(dim), C.c_int(hidden), C.c_int(api.ACT_SILU), C.c_float(1e-5), C.c_int(code),
+                          C.c_int(0), C.c_int(0), None, None, None, None) == 0
+    y = x.double() / torch.sqrt((x.double() ** 2).mean() + 1e-5) * norm.double()
+    want = torch.nn.functional.silu(w1.double() @ y) * (w3.double() @ y)
+    assert rel(hb[:hidden], want) < 1e-6 and (hb[hidden:] == 7.0).all()
+    if hidden % 8 == 0:
+        w2, out = (torch.randn((dim, hidden), device="cuda") * hidden ** -0.5).to(td), torch.full((dim + 4,), 7.0, device="cuda")
+        assert L.yalm_gemv_residual(p(out), p(x), p(hb), p(w2), None, C.c_int(hidden), C.c_int(dim), C.c_int(code), C.c_int(1), None, None, None) == 0
+        assert rel(out[:dim], x.double() + w2.double() @ hb[:hidden].double()) < 1e-6 and (out[dim:] == 7.0).all()
