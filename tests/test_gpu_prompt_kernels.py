@@ -127,6 +127,35 @@ def test_causal_attention_far_maxima():
     assert rel(out, attend(q, k, v, seen, hd ** -0.5)) < 5e-4
 
 
+@pytest.mark.parametrize("bf16", [0, 1])
+@pytest.mark.parametrize("n,pos0,H,G,hd", [(40, 200, 8, 2, 128), (60, 1500, 8, 8, 64), (200, 700, 32, 8, 128), (33, 4000, 4, 4, 128)])
+def test_attention_rows_of_one_late_key(n, pos0, H, G, hd, bf16):
+    """Every row is dominated by one key near its end, whose score lies 2^7.3 .. 2^7.97 above those of a key in 64 before it and far above all
+    others.  The weight of a row's largest score is 1 and takes no rounding, so with one value row for all keys the result is that row: to
+    the last bit in fp16, and in the fp32 rows over bf16 weights to what the rounding (2^-9) of the at most two weights of 2^-7.3 in its own
+    tile and of the sums adds (4e-5)."""
+    T, late = pos0 + n, pos0 - 3
+    dt = torch.bfloat16 if bf16 else torch.float16
+    grow = (1 + torch.arange(n * H, device="cuda").remainder(13) / 128.0).view(n, H)           # exact in both types, as are the keys
+    q, k = torch.zeros((n, H, hd), device="cuda"), torch.zeros((G, T, hd), device="cuda")
+    to_log2 = 1.0 if bf16 else hd ** 0.5 * 0.6931471805599453                                # score in powers of two = q . k / to_log2
+    q[:, :, 0], q[:, :, 1] = grow, 1.0
+    k[:, :, 1] = -40.0 * to_log2                                                               # all others
+    k[:, 5:late:64, 1] = 0.0
+    k[:, late, 0], k[:, late, 1] = 7.3125 * to_log2, 0.0
+    k, v = k.to(dt), normal(hd, (G, 1, hd), dtype=dt).expand(G, T, hd).contiguous()
+    want = v[:, 0].repeat_interleave(H // G, 0).float().expand(n, H, hd)
+    if bf16:
+        out = torch.empty((n, H, hd), device="cuda")
+        assert L().yalm_attn_window_pool_mma(ptr(out), C.c_int(H * hd), ptr(q), C.c_int(H * hd), ptr(k), ptr(v), None, None, *i32(n, H, G, hd, hd, T, 0, 0, 0),
+                                             C.c_float(0.6931471805599453), C.c_int(pos0), None, None) == 0
+        assert ((out - want).abs() <= 4e-5 * want.abs()).all()
+    else:
+        out = torch.empty((n, H, hd), device="cuda", dtype=dt)
+        assert L().yalm_attn_prefill(ptr(out), ptr(q.to(dt)), ptr(k), ptr(v), *i32(n, pos0, H, G, hd, T), None) == 0
+        assert torch.equal(out.float(), want)
+
+
 @pytest.mark.parametrize("dk,dv", [(128, 128), (64, 64), (64, 128), (128, 64), (64, 32), (128, 32)])
 @pytest.mark.parametrize("n,pos0,H,G,Gv,window,pool,ring", [
     (32, 0, 8, 2, 2, 128, 64, 640), (512, 3584, 16, 4, 4, 1024, 64, 1536), (100, 777, 8, 2, 1, 500, 64, 1012), (257, 5000, 8, 8, 4, 300, 1, 557),

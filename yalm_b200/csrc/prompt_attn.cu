@@ -9,17 +9,16 @@
 // 12 warps.  Warp 0 streams key and value tiles of 128 positions with cp.async.bulk.tensor.3d into a ring of stages.  One thread of
 // warp 1 issues the products: S = Q K^T into TMEM, O += P V with P out of TMEM (its fp16 / bf16 words take the place of the scores).
 // Warps 4-7 and 8-11 are the softmax of tiles A and B, a thread per row: scores from TMEM, online maximum and sum in fp32, P back to
-// TMEM.  The two tiles alternate: while one's scores go through the softmax the tensor pipe works for the other.  O stays in TMEM; it is
-// rescaled only when a row's maximum has grown by more than 2^8 since its last rescaling (the weights of the meantime are up to 256
-// times larger, in fp32 sums and 16-bit operands alike, and the final division takes it out again).  Warps 2 and 3 serve the layered
-// models: they round pooled fp32 means into stages, and clear the value rows of a ring tile that hold no position (a weight of zero
-// times whatever lies there must be zero).
+// TMEM.  The two tiles alternate: while one's scores go through the softmax the tensor pipe works for the other.  O stays in TMEM and is
+// rescaled whenever a row's maximum grows, so that the weight of a row's largest score is 1 and takes no rounding.  (A reference that follows
+// only growth beyond 2^8 saves 0.3 to 8 us of the calls below, but rounds the weight that counts most: a row that one key dominates is then off by
+// up to 2^-9 over bf16; 512 rows, window 1024, against 64 bits: 2.30e-3 for 2.24e-3.)  Warps 2 and 3 serve the layered models: they round pooled
+// fp32 means into stages, and clear the value rows of a ring tile that hold no position (a weight of zero times whatever lies there must be zero).
 //
-// Bound by the chain softmax - products of a tile pair (3000 cycles per 128 keys: 1800 from scores to weights, of which the exponentials
-// alone take 1024 at 16 a cycle and SM for each of the two tiles, and 1100 for P V and the next scores) and, for short contexts, by launch,
-// query staging and the store.  Cold L2, against 64-row tiles on mma.sync: 507 rows at 7680 positions, 32 / 8 heads of 128: 672 -> 72 us
-// (919 TFLOP/s); 512 rows at 0: 42 -> 20 us; 20 rows at 7000, 8 / 8 heads: 790 -> 25 us; bf16 window 2048 and pooled blocks, 512 rows, 32 / 8
-// heads: 136 -> 38 us.
+// Bound by the chain softmax - products of a tile pair (some 3500 cycles per 128 keys: 1800 from scores to weights, of which the exponentials
+// alone take 1024 at 16 a cycle and SM for each of the two tiles, 500 for the rescaling, and 1100 for P V and the next scores) and, for short
+// contexts, by launch, query staging and the store.  Back to back, against 64-row tiles on mma.sync: 507 rows at 7680 positions, 32 / 8 heads of 128:
+// 667 -> 80 us (825 TFLOP/s); 512 rows at 0: 32.8 -> 14.0 us; bf16 window 1024 and pooled blocks of 64, 512 rows, 16 / 4 heads: 57.3 -> 22.8 us.
 #include "common.cuh"
 #include "launch.h"
 #include "stack_rows.cuh"
@@ -441,7 +440,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 #pragma unroll
 					for (int y = 0; y < 4; ++y) mx4[y] = max3(mx4[y], __uint_as_float(s[x + 2 * y]), __uint_as_float(s[x + 2 * y + 1]));
 				const float top = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * c;
-				const bool grow = top > mref + 8.0f;
+				const bool grow = top > mref; // (not later: the largest weight of a row is then 1 and takes no rounding)
 				if (__any_sync(kFull, grow)) {
 					const float f = grow ? ex2(mref - top) : 1.0f; // mref -inf: 0
 					if (grow) mref = top;
