@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("hd", [128, 64, 32, 16])
 @pytest.mark.parametrize("G", [1, 2, 4, 8])
-@pytest.mark.parametrize("n_kv", [1, 3, 8])
+@pytest.mark.parametrize("n_kv", [1, 3, 5, 8, 25])   # (5, 25: KV heads x splits odd on 148 multiprocessors)
 def test_attn_decode_splits(hd, G, n_kv):
     L, H, ring = api.lib(), G * n_kv, 5000
     gen = torch.Generator(device="cuda")

@@ -13,6 +13,7 @@
 //
 // Arithmetic follows the CPU reference (src/infer.cpp:216-248): fp32 dot over fp16 K, score /
 // sqrtf(head_dim), exp(x - max) / sum, fp32 mix over fp16 V.
+#include "attn_workspace.h"
 #include "common.cuh"
 #include "launch.h"
 
@@ -376,10 +377,7 @@ using namespace yalm;
 
 extern "C" size_t yalm_attn_workspace_bytes(int n_heads, int n_kv_heads, int head_dim) {
 	if (n_heads <= 0 || n_kv_heads <= 0 || head_dim <= 0) return 0;
-	const int S = attn_splits(n_kv_heads);
-	const size_t g = n_heads / n_kv_heads;
-	size_t floats = (size_t)n_kv_heads * S * g * (head_dim + 2);
-	return floats * sizeof(float) + (size_t)n_kv_heads * sizeof(unsigned) + 256;
+	return attn_workspace(0, n_kv_heads, attn_splits(n_kv_heads), n_heads / n_kv_heads, head_dim).bytes;
 }
 
 extern "C" int yalm_attn_decode(float *out, const uint16_t *key_cache, const uint16_t *value_cache, const float *q,
@@ -392,10 +390,10 @@ extern "C" int yalm_attn_decode(float *out, const uint16_t *key_cache, const uin
 	const int S = attn_splits(n_kv_heads);
 	AttnArgs a;
 	a.out = out, a.kb = (const __half *)key_cache, a.vb = (const __half *)value_cache, a.q = q;
-	// counters first (256-byte slot), then ml, then acc
+	const AttnWorkspace w = attn_workspace((uintptr_t)workspace, n_kv_heads, S, g, head_dim);
 	a.counters = (unsigned *)workspace;
-	a.ws_ml = (float *)((char *)workspace + 256);
-	a.ws_acc = a.ws_ml + (size_t)n_kv_heads * S * g * 2;
+	a.ws_ml = (float *)((char *)workspace + w.ml);
+	a.ws_acc = (float *)((char *)workspace + w.acc);
 	a.n_kv_heads = n_kv_heads, a.max_seq_len = max_seq_len, a.ctl = ctl;
 	cudaStream_t st = (cudaStream_t)s;
 #define YALM_ATTN_CASE(HD, G)                                                                                 \
