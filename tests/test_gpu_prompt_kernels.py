@@ -156,6 +156,29 @@ def test_attention_rows_of_one_late_key(n, pos0, H, G, hd, bf16):
         assert torch.equal(out.float(), want)
 
 
+@pytest.mark.parametrize("bf16", [0, 1])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("n,pos0,at", [(20, 4000, 3900), (20, 4000, 5), (40, 2000, 1100), (512, 0, 300)])
+def test_attention_not_finite_in_one_part(n, pos0, at, bad, bf16):
+    """A key of one kv head that is not a number, or infinite, in any part of the keys: the rows of its query heads that see it are NaN (an
+    infinite score takes itself away), and no others."""
+    H, G, hd, T, dt = 8, 4, 128, pos0 + n, torch.bfloat16 if bf16 else torch.float16
+    q = normal(n, (n, H, hd), dtype=dt)
+    k, v = normal(1, (G, T, hd), dtype=dt), normal(2, (G, T, hd), dtype=dt)
+    q[:, :, 0], k[1, at] = 1.0, 0.0                    # (scores of the key: + infinity or NaN, not a sum of both signs)
+    k[1, at, 0] = bad
+    if bf16:
+        out = torch.empty((n, H, hd), device="cuda")
+        assert L().yalm_attn_window_pool_mma(ptr(out), C.c_int(H * hd), ptr(q.float()), C.c_int(H * hd), ptr(k), ptr(v), None, None,
+                                             *i32(n, H, G, hd, hd, T, 0, 0, 0), C.c_float(hd ** -0.5), C.c_int(pos0), None, None) == 0
+    else:
+        out = torch.empty((n, H, hd), device="cuda", dtype=dt)
+        assert L().yalm_attn_prefill(ptr(out), ptr(q), ptr(k), ptr(v), *i32(n, pos0, H, G, hd, T), None) == 0
+    hit = torch.zeros((n, H), dtype=torch.bool, device="cuda")
+    hit[max(0, at - pos0):, 2:4] = True
+    assert out[hit].isnan().all() and out[~hit].isfinite().all()
+
+
 @pytest.mark.parametrize("dk,dv", [(128, 128), (64, 64), (64, 128), (128, 64), (64, 32), (128, 32)])
 @pytest.mark.parametrize("n,pos0,H,G,Gv,window,pool,ring", [
     (32, 0, 8, 2, 2, 128, 64, 640), (512, 3584, 16, 4, 4, 1024, 64, 1536), (100, 777, 8, 2, 1, 500, 64, 1012), (257, 5000, 8, 8, 4, 300, 1, 557),

@@ -539,7 +539,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 			for (int p = 0; p < parts; ++p) {
 				float pm, pl;
 				of_part(p, pm, pl);
-				if (pl > 0.f) Lsum += pl * ex2(pm - M);
+				if (pl != 0.f) Lsum += pl * ex2(pm - M); // (a part whose rows see nothing has 0; a NaN counts)
 			}
 		}
 		const int h = g * a.G + min(row, rows - 1) % a.G;
@@ -569,7 +569,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 				for (int p = 0; p < parts; ++p) {
 					float pm, pl;
 					of_part(p, pm, pl);
-					if (!(pl > 0.f)) continue;
+					if (pl == 0.f) continue;
 					const float w = ex2(pm - M);
 					if (p == part) {
 #pragma unroll
