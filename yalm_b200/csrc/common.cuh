@@ -49,7 +49,8 @@ __device__ __forceinline__ uint4 ldg_stream(const void *p) {
 
 // Kernels that are launched with launch_chained (launch.h) may begin while the kernel before them in the stream still runs: what they
 // do before chain_wait() must not touch global memory, and returns from it with everything before them complete and visible.
-// chain_next() lets the next such kernel begin (it waits in turn).
+// chain_next() lets the next such kernel begin (it waits in turn).  A kernel with tensor memory calls it behind a barrier after its
+// allocation: the next kernel's would otherwise find the columns free, take them and wait, with them, for this one.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -214,9 +214,11 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 	}
 	if (warp == 1) tmem_alloc<1>(tslot, 512);
-	__syncwarp();
+	tc_fence_before();
+	__syncthreads(); // (tensor memory is this CTA's before the next kernel may take any)
 	chain_wait();
 	chain_next();
+	tc_fence_after();
 	const int p0 = a.ctl ? a.ctl[CTL_POS] : a.pos0;
 	const Tiles tiles(a, p0 + r0 / a.G, p0 + min((r0 + 2 * kTile - 1) / a.G, a.n - 1));
 	const int per = (tiles.total + parts - 1) / parts, k_begin = min(part * per, tiles.total), k_end = min(k_begin + per, tiles.total), nk = k_end - k_begin;
