@@ -13,7 +13,7 @@ def kernels():
     out = []
     for path in sorted(glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cuh"))):
         text = re.sub(r"//[^\n]*", "", open(path).read())
-        for m in re.finditer(r"__global__[^;{]*?(\w+)\s*\(([^{;]*)\)\s*\{", text):
+        for m in re.finditer(r"__global__\s+void\s+(?:__launch_bounds__\s*\([^()]*(?:\([^()]*\)[^()]*)*\)\s*)?(\w+)\s*\(([^{;]*)\)\s*\{", text):
             depth, at = 1, m.end()
             while depth:
                 depth += {"{": 1, "}": -1}.get(text[at], 0)
@@ -39,3 +39,10 @@ def test_tensor_memory_is_taken_before_the_next_may_begin(params, body):
     if "tmem_alloc" in body:
         between = body[body.index("tmem_alloc"): body.index("chain_next()")]
         assert "__syncthreads()" in between or "cluster_sync()" in between
+
+
+@pytest.mark.parametrize("params,body", kernels())
+def test_promises_nothing_about_its_inputs(params, body):
+    """They are still being written when the kernel begins: __restrict__ and non-coherent loads state the contrary."""
+    assert "__restrict__" not in params
+    assert not re.search(r"__ldg\(|ldg_stream\(|ld\.global\.nc", body)

@@ -47,9 +47,17 @@ __device__ __forceinline__ uint4 ldg_stream(const void *p) {
 	return r;
 }
 
+// The same for what an earlier kernel writes: a coherent load, in the order of the instructions around it.
+__device__ __forceinline__ uint4 ld_stream(const void *p) {
+	uint4 r;
+	asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p) : "memory");
+	return r;
+}
+
 // Kernels that are launched with launch_chained (launch.h) may begin while the kernel before them in the stream still runs: what they
 // do before chain_wait() must not touch global memory, and returns from it with everything before them complete and visible.
-// chain_next() lets the next such kernel begin (it waits in turn).  A kernel with tensor memory calls it behind a barrier after its
+// Their lifetime begins while their inputs are still being written, so they make no promise that data stays as it is: no __restrict__ (which would
+// let loads rise above the wait) and no non-coherent loads.  chain_next() lets the next such kernel begin (it waits in turn).  A kernel with tensor memory calls it behind a barrier after its
 // allocation: the next kernel's would otherwise find the columns free, take them and wait, with them, for this one.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -115,9 +115,9 @@ __global__ void __launch_bounds__(kAttnThreads, Split<HD, G>::CTAS) attn_decode_
 	for (int r0 = t_begin + wid * SP::RPW + rgrp; r0 - rgrp < t_end; r0 += RPC * UN) { // (warp-uniform bound: the shuffles need the whole warp)
 		uint4 kv[UN], vv[UN];
 #pragma unroll
-		for (int u = 0; u < UN; ++u) kv[u] = r0 + u * RPC < t_end ? ldg_stream(kbase + (size_t)(r0 + u * RPC) * HD) : make_uint4(0, 0, 0, 0);
+		for (int u = 0; u < UN; ++u) kv[u] = r0 + u * RPC < t_end ? ld_stream(kbase + (size_t)(r0 + u * RPC) * HD) : make_uint4(0, 0, 0, 0);
 #pragma unroll
-		for (int u = 0; u < UN; ++u) vv[u] = r0 + u * RPC < t_end ? ldg_stream(vbase + (size_t)(r0 + u * RPC) * HD) : make_uint4(0, 0, 0, 0);
+		for (int u = 0; u < UN; ++u) vv[u] = r0 + u * RPC < t_end ? ld_stream(vbase + (size_t)(r0 + u * RPC) * HD) : make_uint4(0, 0, 0, 0);
 		float s[NV];
 #pragma unroll
 		for (int u = 0; u < UN; ++u) {

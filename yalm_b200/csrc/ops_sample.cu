@@ -97,8 +97,7 @@ __global__ void __launch_bounds__(kSampleThreads) sample_kernel(const float *__r
 // logits; two passes of one load at a time by 256 threads took 84 us for 512 rows of 32000, this 20.
 // VEC: rows are 16-byte aligned.
 template <bool VEC>
-__global__ void __launch_bounds__(1024) token_probs_kernel(const float *__restrict__ logits, int vocab, const int *__restrict__ targets,
-                                                           float *__restrict__ probs) {
+__global__ void __launch_bounds__(1024) token_probs_kernel(const float *logits, int vocab, const int *targets, float *probs) {
 	__shared__ float red[33];
 	chain_wait();
 	chain_next();

@@ -45,20 +45,20 @@ __global__ void embed_rows_kernel(float *__restrict__ x, const __half *__restric
 // out16[i, :] = half(x[i, :] * (1 / sqrt(mean(x^2) + eps)) * w)   (src/infer.cpp:134-144, one CTA per row)
 // Rows of up to 8192 stay in registers between the sum and the scaling, all their loads in flight at once (512 rows of 4096: 6.7 -> 5.6 us).
 constexpr int kNormThreads = 256, kNormKept = 8;
-__global__ void __launch_bounds__(kNormThreads) rmsnorm_rows_kernel(__half *__restrict__ out, const float *__restrict__ x, const float *__restrict__ w,
-                                                                    int dim, float eps) {
+__global__ void __launch_bounds__(kNormThreads) rmsnorm_rows_kernel(__half *out, const float *x, const float *w, int dim, float eps) {
 	__shared__ float red[33];
 	chain_wait();
 	chain_next();
 	const float *row = x + (size_t)blockIdx.x * dim;
 	const bool kept = dim <= kNormThreads * 4 * kNormKept;
-	float4 v[kNormKept];
+	float4 v[kNormKept], gain[kNormKept];
 	float ss = 0.f;
 	if (kept) {
 #pragma unroll
 		for (int j = 0; j < kNormKept; ++j) {
 			const int e = (threadIdx.x + j * kNormThreads) * 4;
 			v[j] = e < dim ? *reinterpret_cast<const float4 *>(row + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+			if (e < dim) gain[j] = *reinterpret_cast<const float4 *>(w + e);
 		}
 #pragma unroll
 		for (int j = 0; j < kNormKept; ++j) ss += v[j].x * v[j].x + v[j].y * v[j].y + v[j].z * v[j].z + v[j].w * v[j].w;
@@ -70,8 +70,7 @@ __global__ void __launch_bounds__(kNormThreads) rmsnorm_rows_kernel(__half *__re
 	ss = block_sum(ss, red);
 	const float scale = 1.0f / sqrtf(ss / dim + eps);
 	__half *dst = out + (size_t)blockIdx.x * dim;
-	auto put = [&](int e, float4 t) {
-		const float4 g = *reinterpret_cast<const float4 *>(w + e);
+	auto put = [&](int e, float4 t, float4 g) {
 		*reinterpret_cast<__half2 *>(dst + e) = __floats2half2_rn(t.x * scale * g.x, t.y * scale * g.y);
 		*reinterpret_cast<__half2 *>(dst + e + 2) = __floats2half2_rn(t.z * scale * g.z, t.w * scale * g.w);
 	};
@@ -79,18 +78,17 @@ __global__ void __launch_bounds__(kNormThreads) rmsnorm_rows_kernel(__half *__re
 #pragma unroll
 		for (int j = 0; j < kNormKept; ++j) {
 			const int e = (threadIdx.x + j * kNormThreads) * 4;
-			if (e < dim) put(e, v[j]);
+			if (e < dim) put(e, v[j], gain[j]);
 		}
 	} else
-		for (int e = threadIdx.x * 4; e < dim; e += kNormThreads * 4) put(e, *reinterpret_cast<const float4 *>(row + e));
+		for (int e = threadIdx.x * 4; e < dim; e += kNormThreads * 4) put(e, *reinterpret_cast<const float4 *>(row + e), *reinterpret_cast<const float4 *>(w + e));
 }
 
 // Row i of qkv (fp32: q | k | v) = position pos0 + i: clip, interleaved-pair RoPE on q and k (src/infer.cpp:200-213,
 // 282-292), q -> fp16 (attention operand), k / v -> fp16 rows pos0 + i of the head-major KV ring (src/infer.cpp:294-301).
 // A thread takes one pair of a head's channels through every blockDim / half-th head: the angle's power, sine and cosine, most of the work, are
 // formed once per thread instead of once per pair (512 rows of 32 + 8 heads of 128: 18 -> 11 us).
-__global__ void __launch_bounds__(512) rope_append_rows_kernel(__half *__restrict__ q16, __half *__restrict__ kc, __half *__restrict__ vc,
-                                                               const float *__restrict__ qkv, int n_heads, int n_kv, int head_dim,
+__global__ void __launch_bounds__(512) rope_append_rows_kernel(__half *q16, __half *kc, __half *vc, const float *qkv, int n_heads, int n_kv, int head_dim,
                                                                int rotary_dim, int max_seq_len, int pos0, float theta, float clip) {
 	const int i = blockIdx.x, pos = pos0 + i, half = head_dim / 2, at_once = blockDim.x / half, q_dim = n_heads * head_dim;
 	const int j = (threadIdx.x % half) * 2, first = threadIdx.x / half;
@@ -100,15 +98,24 @@ __global__ void __launch_bounds__(512) rope_append_rows_kernel(__half *__restric
 	const float *row = qkv + (size_t)i * (q_dim + 2 * n_kv * head_dim);
 	float fcr, fci;
 	rope_angle(fcr, fci, j, pos, theta, rotary_dim);
-#pragma unroll 4
-	for (int h = first; h < n_heads + 2 * n_kv; h += at_once) { // q heads, k heads, v heads
-		const float2 v = *reinterpret_cast<const float2 *>(row + (size_t)h * head_dim + j);
-		float v0 = clipf(v.x, clip), v1 = clipf(v.y, clip);
-		if (h < n_heads + n_kv) rope_turn(v0, v1, fcr, fci);
-		__half *dst = h < n_heads ? q16 + (size_t)i * q_dim + h * head_dim
-		                          : (h < n_heads + n_kv ? kc + ((size_t)(h - n_heads) * max_seq_len + pos) * head_dim
-		                                                : vc + ((size_t)(h - n_heads - n_kv) * max_seq_len + pos) * head_dim);
-		*reinterpret_cast<__half2 *>(dst + j) = __floats2half2_rn(v0, v1);
+	constexpr int kBatch = 4;
+	const int heads = n_heads + 2 * n_kv; // q heads, k heads, v heads
+	for (int h0 = first; h0 < heads; h0 += kBatch * at_once) {
+		float2 v[kBatch]; // reads first, then stores
+#pragma unroll
+		for (int b = 0; b < kBatch; ++b)
+			if (h0 + b * at_once < heads) v[b] = *reinterpret_cast<const float2 *>(row + (size_t)(h0 + b * at_once) * head_dim + j);
+#pragma unroll
+		for (int b = 0; b < kBatch; ++b) {
+			const int h = h0 + b * at_once;
+			if (h >= heads) break;
+			float v0 = clipf(v[b].x, clip), v1 = clipf(v[b].y, clip);
+			if (h < n_heads + n_kv) rope_turn(v0, v1, fcr, fci);
+			__half *dst = h < n_heads ? q16 + (size_t)i * q_dim + h * head_dim
+			                          : (h < n_heads + n_kv ? kc + ((size_t)(h - n_heads) * max_seq_len + pos) * head_dim
+			                                                : vc + ((size_t)(h - n_heads - n_kv) * max_seq_len + pos) * head_dim);
+			*reinterpret_cast<__half2 *>(dst + j) = __floats2half2_rn(v0, v1);
+		}
 	}
 }
 
