@@ -45,23 +45,28 @@ inline int launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t sm
 	return (int)cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
+// Lets a kernel use that much dynamic shared memory on the current device: more than 48 KB has to be asked for, on each device.
+inline cudaError_t allow_smem(const void *kernel, size_t smem) {
+	static std::mutex mu;
+	static std::map<std::pair<int, const void *>, size_t> limits;
+	if (smem <= 48 * 1024) return cudaSuccess;
+	std::lock_guard<std::mutex> lock(mu);
+	size_t &limit = limits[{device_info().device, kernel}];
+	if (smem <= limit) return cudaSuccess;
+	const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+	if (err == cudaSuccess) limit = smem;
+	return err;
+}
+
 // Resident CTAs per SM for (kernel, block, smem); raises the kernel's dynamic-smem limit on demand.
 // Results are cached: the occupancy query is not free and this sits on the per-token path when the
 // ops are used outside a CUDA graph.
 inline int resident_ctas(const void *kernel, int block, size_t smem, cudaError_t *err) {
 	static std::mutex mu;
 	static std::map<std::pair<const void *, std::pair<int, size_t>>, int> cache;
-	static std::map<const void *, size_t> smem_limit;
 	std::lock_guard<std::mutex> lock(mu);
-	*err = cudaSuccess;
-	if (smem > 48 * 1024) {
-		size_t &lim = smem_limit[kernel];
-		if (smem > lim) {
-			*err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-			if (*err != cudaSuccess) return 0;
-			lim = smem;
-		}
-	}
+	*err = allow_smem(kernel, smem);
+	if (*err != cudaSuccess) return 0;
 	auto key = std::make_pair(kernel, std::make_pair(block, smem));
 	auto it = cache.find(key);
 	if (it != cache.end()) return it->second;

@@ -362,12 +362,8 @@ static bool attn_fast_shape(int head_dim, int g) {
 template <int HD, int G>
 static int launch_attn(AttnArgs &a, int S, cudaStream_t st) {
 	a.max_splits = std::max(1, std::min(S, Split<HD, G>::CTAS * device_info().sms / a.n_kv_heads)); // all at once
-	const size_t smem = ((size_t)S * G + (size_t)kAttnWarps * G * HD) * sizeof(float);
-	static bool configured = false;
-	if (!configured && smem > 48 * 1024) {
-		YALM_TRY(cudaFuncSetAttribute(attn_decode_kernel<HD, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-		configured = true;
-	}
+	const size_t smem = ((size_t)a.max_splits * G + (size_t)kAttnWarps * G * HD) * sizeof(float);
+	YALM_TRY(allow_smem((const void *)attn_decode_kernel<HD, G>, smem));
 	return launch_chained(attn_decode_kernel<HD, G>, dim3(a.max_splits, a.n_kv_heads), dim3(kAttnThreads), smem, st, 1, a);
 }
 

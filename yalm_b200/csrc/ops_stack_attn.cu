@@ -221,11 +221,7 @@ static int launch_mma(float *out, int ldo, const float *q, int ldq, const void *
                       int n_kv, int ring, int max_blocks, int window, int pool, float scale, int pos0, const int *ctl, const float *sink, int v_heads,
                       cudaStream_t st) {
 	const size_t smem = sizeof(__nv_bfloat16) * (3 * 64 * (DK + 8) + 2 * 64 * (DV + 8)); // Q, two key tiles, two value tiles
-	static bool configured = false;
-	if (!configured && smem > 48 * 1024) {
-		YALM_TRY(cudaFuncSetAttribute(attn_window_pool_mma_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-		configured = true;
-	}
+	YALM_TRY(allow_smem((const void *)attn_window_pool_mma_kernel<DK, DV>, smem));
 	attn_window_pool_mma_kernel<DK, DV><<<dim3((n + 63) / 64, n_heads), 128, smem, st>>>(out, ldo, q, ldq, (const __nv_bfloat16 *)kr, (const __nv_bfloat16 *)vr,
 	                                                                                   kp, vp, n, n_heads, n_kv, ring, max_blocks, window, pool, scale, pos0,
 	                                                                                   ctl, sink, v_heads);
@@ -565,11 +561,7 @@ static int launch_sigmoid_mma(float *out, int ldo, const float *q, int ldq, cons
                               int window, int keep, float scale, int context, int pos0, const int *ctl, cudaStream_t st) {
 	const int tb = std::min(4096, window > 0 ? window + 64 : std::max(64, context));
 	const size_t smem = sizeof(__nv_bfloat16) * (3 * 64 * (D + 8)) + sizeof(float) * tb;
-	static size_t configured = 0;
-	if (smem > 48 * 1024 && smem > configured) {
-		YALM_TRY(cudaFuncSetAttribute(attn_sigmoid_mma_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-		configured = smem;
-	}
+	YALM_TRY(allow_smem((const void *)attn_sigmoid_mma_kernel<D>, smem));
 	attn_sigmoid_mma_kernel<D><<<dim3((n + 63) / 64, n_heads), 128, smem, st>>>(out, ldo, q, ldq, (const __nv_bfloat16 *)ring_buf,
 	                                                                            (const __nv_bfloat16 *)first_buf, gate, ldg, rel, bucket, hb, table, ldt, n, n_heads,
 	                                                                            n_kv, ring, window, keep, scale, tb, pos0, ctl);

@@ -707,11 +707,7 @@ static int launch_scan(const ScanArgs &a, dim3 grid, cudaStream_t st) {
 #define SCAN_CASE(EPL_, LPC_)                                                                                                                \
 	{                                                                                                                                        \
 		constexpr size_t smem = sizeof(float) * 2 * ScanLayout<EPL_, LPC_>::STAGE;                                                           \
-		static bool configured = false;                                                                                                      \
-		if (smem > 48 * 1024 && !configured) {                                                                                               \
-			YALM_TRY(cudaFuncSetAttribute(state_scan_kernel<EPL_, MODE, LPC_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));     \
-			configured = true;                                                                                                               \
-		}                                                                                                                                    \
+		YALM_TRY(allow_smem((const void *)state_scan_kernel<EPL_, MODE, LPC_>, smem));                                                       \
 		state_scan_kernel<EPL_, MODE, LPC_><<<grid, kScanCols * 8, smem, st>>>(a);                                                           \
 	}
 	// lanes per column: the delta rule's chain through the shuffles is shortest with 8; without it, two columns per thread on 16 lanes read
@@ -733,11 +729,7 @@ constexpr int kChunkRows = 8;
 template <int D, bool DELTA, bool PER_CHANNEL>
 static int launch_chunks_of(const ScanArgs &a, cudaStream_t st) {
 	constexpr int smem = kChunkSlots * ChunkSlot<D>::SIZE * (int)sizeof(float);
-	static bool configured = false;
-	if (!configured) {
-		YALM_TRY(cudaFuncSetAttribute(chunk_scan_kernel<D, DELTA, PER_CHANNEL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-		configured = true;
-	}
+	YALM_TRY(allow_smem((const void *)chunk_scan_kernel<D, DELTA, PER_CHANNEL>, smem));
 	return launch_chained(chunk_scan_kernel<D, DELTA, PER_CHANNEL>, dim3((a.P + kChunkCols - 1) / kChunkCols, a.H), dim3(kChunkThreads), smem, st, 1, a);
 }
 template <bool DELTA, bool PER_CHANNEL>
