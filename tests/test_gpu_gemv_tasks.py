@@ -46,3 +46,16 @@ def test_feed_forward(dim, hidden, dtype):
         w2, out = (torch.randn((dim, hidden), device="cuda") * hidden ** -0.5).to(td), torch.full((dim + 4,), 7.0, device="cuda")
         assert L.yalm_gemv_residual(p(out), p(x), p(hb), p(w2), None, C.c_int(hidden), C.c_int(dim), C.c_int(code), C.c_int(1), None, None, None) == 0
         assert rel(out[:dim], x.double() + w2.double() @ hb[:hidden].double()) < 1e-6 and (out[dim:] == 7.0).all()
+
+
+def test_refused_length_leaves_no_error():
+    """An input that does not fit into shared memory is refused, and the next call runs."""
+    L, n = api.lib(), 65536
+    w, x, out = torch.randn((4, 64), device="cuda"), torch.randn(n, device="cuda"), torch.zeros(4, device="cuda")
+    for refused in (lambda: L.yalm_gemv_scaled(p(out), p(x), p(w), C.c_int(n), C.c_int(4), C.c_int(api.F32), C.c_float(1.0), None),
+                    lambda: L.yalm_gemv_residual(p(out), None, p(x), p(w), None, C.c_int(n), C.c_int(4), C.c_int(api.F32), C.c_int(1), None, None, None),
+                    lambda: L.yalm_ffn_glu(p(out), p(x), p(x), p(w), p(w), None, None, None, None, C.c_int(n), C.c_int(4), C.c_int(api.ACT_SILU), C.c_float(1e-5),
+                                           C.c_int(api.F32), C.c_int(0), C.c_int(0), None, None, None, None)):
+        assert refused() == -1     # YALM_EINVAL, before anything is launched
+        assert L.yalm_gemv_scaled(p(out), p(x), p(w), C.c_int(64), C.c_int(4), C.c_int(api.F32), C.c_float(1.0), None) == 0
+        assert rel(out, w.double() @ x[:64].double()) < 1e-6

@@ -393,6 +393,7 @@ static int launch_persistent(K kernel, const A &args, size_t smem, long tasks, c
 template <typename K>
 static bool finer_tasks(K kernel, size_t smem, long tasks) {
 	cudaError_t err;
+	if ((int)smem > device_info().max_smem_optin) return false; // (refused by the launch; asking for it would leave an error behind for the next one)
 	const int occ = resident_ctas((const void *)kernel, kThreads, smem, &err);
 	if (err != cudaSuccess || occ < 1) return false;
 	const long warps = (long)device_info().sms * occ * (kThreads / 32);
