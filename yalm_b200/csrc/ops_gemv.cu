@@ -389,7 +389,8 @@ static int launch_persistent(K kernel, const A &args, size_t smem, long tasks, c
 // Whether tasks of half the size end sooner: a persistent grid takes whole rounds of its warps, and a last round with few tasks leaves the
 // memory idle for as long as a full one.  (Gate and up of a token, rows one or two pairs at a time: 4096 x 11008 fp16 with the down projection
 // 67 -> 57 us, fp32 122 -> 98, 1024 x 14336 fp32 70 -> 55; rows four or two at a time: 4096 x 4096 fp16 15.7 -> 11.3 us, 2048 x 2048 8.3 -> 6; where both
-// end together, as at 4096 x 14336 or 32000 x 4096, the larger tasks stay.)
+// end together, as at 4096 x 14336 or 32000 x 4096, the larger tasks stay.)  kernel: that of the larger tasks, of the type at hand; more CTAs of the
+// other one fit on an SM, which can only bring its end forward.
 template <typename K>
 static bool finer_tasks(K kernel, size_t smem, long tasks) {
 	cudaError_t err;
@@ -450,9 +451,9 @@ extern "C" int yalm_gemv_residual_ep(float *out, const float *residual, const fl
 	a.n = n, a.d = d, a.n_active = n_active, a.active_e = active_e, a.active_w = active_w;
 	a.ep_rank = ep_rank, a.ep_size = ep_size;
 	const size_t smem = (size_t)n_active * xs_bytes(dtype, n);
-	if (finer_tasks(gemv_residual_kernel<YALM_F16, 2, 8>, smem, d / 2))
-		YALM_DISPATCH_DT(dtype, return launch_persistent(gemv_residual_kernel<DT, 1, 8>, a, smem, d, (cudaStream_t)s));
-	YALM_DISPATCH_DT(dtype, return launch_persistent(gemv_residual_kernel<DT, 2, 8>, a, smem, d / 2, (cudaStream_t)s));
+	YALM_DISPATCH_DT(dtype, return finer_tasks(gemv_residual_kernel<DT, 2, 8>, smem, d / 2)
+	                                   ? launch_persistent(gemv_residual_kernel<DT, 1, 8>, a, smem, d, (cudaStream_t)s)
+	                                   : launch_persistent(gemv_residual_kernel<DT, 2, 8>, a, smem, d / 2, (cudaStream_t)s));
 	return 0;
 }
 
@@ -483,13 +484,9 @@ extern "C" int yalm_ffn_glu_ep(float *hb, const float *x, const float *rms_weigh
 	a.ep_rank = ep_rank, a.ep_size = ep_size;
 	const size_t smem = (36 + 3 * kMaxExperts) * sizeof(float) + xs_bytes(dtype, dim);
 	const long k = a.n_active;
-	if (hidden_dim % 2 == 0 && !finer_tasks(ffn_glu_kernel<YALM_F16, 2, 4>, smem, k * hidden_dim / 2)) {
-		YALM_DISPATCH_DT(dtype, return launch_persistent(ffn_glu_kernel<DT, 2, 4>, a, smem, k * hidden_dim / 2,
-		                                                  (cudaStream_t)s));
-	} else {
-		YALM_DISPATCH_DT(dtype, return launch_persistent(ffn_glu_kernel<DT, 1, 8>, a, smem, k * hidden_dim,
-		                                                  (cudaStream_t)s));
-	}
+	YALM_DISPATCH_DT(dtype, return hidden_dim % 2 || finer_tasks(ffn_glu_kernel<DT, 2, 4>, smem, k * hidden_dim / 2)
+	                                   ? launch_persistent(ffn_glu_kernel<DT, 1, 8>, a, smem, k * hidden_dim, (cudaStream_t)s)
+	                                   : launch_persistent(ffn_glu_kernel<DT, 2, 4>, a, smem, k * hidden_dim / 2, (cudaStream_t)s));
 	return 0;
 }
 
@@ -503,9 +500,8 @@ static int rows_launch(float *out, const float *x, const float *rms_w, const voi
 	if (dtype == YALM_BF16) // bf16 weights exist for this kernel only (the layered models' one-row products)
 		return finer_tasks(gemv_rows_kernel<YALM_BF16, 4, 4>, smem, (d + 3) / 4) ? launch_persistent(gemv_rows_kernel<YALM_BF16, 2, 8>, a, smem, (d + 1) / 2, st)
 		                                                                        : launch_persistent(gemv_rows_kernel<YALM_BF16, 4, 4>, a, smem, (d + 3) / 4, st);
-	if (finer_tasks(gemv_rows_kernel<YALM_F16, 4, 4>, smem, (d + 3) / 4))
-		YALM_DISPATCH_DT(dtype, return launch_persistent(gemv_rows_kernel<DT, 2, 8>, a, smem, (d + 1) / 2, st));
-	YALM_DISPATCH_DT(dtype, return launch_persistent(gemv_rows_kernel<DT, 4, 4>, a, smem, (d + 3) / 4, st));
+	YALM_DISPATCH_DT(dtype, return finer_tasks(gemv_rows_kernel<DT, 4, 4>, smem, (d + 3) / 4) ? launch_persistent(gemv_rows_kernel<DT, 2, 8>, a, smem, (d + 1) / 2, st)
+	                                                                                          : launch_persistent(gemv_rows_kernel<DT, 4, 4>, a, smem, (d + 3) / 4, st));
 	return 0;
 }
 
