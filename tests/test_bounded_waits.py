@@ -1,0 +1,33 @@
+"""-m "not gpu": what the tensor-core kernels do when a bounded wait ran out (csrc/tcgen.cuh), read from their source - making one run out would take a
+broken kernel.  A warp that gave up states no result as complete, and what was to be stored or carried on becomes NaN."""
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "yalm_b200", "csrc")
+
+
+def source(name):
+    return open(os.path.join(CSRC, name)).read()
+
+
+@pytest.mark.parametrize("name,barrier,count", [("prefill_gemm.cu", r"umma_commit_pair\(acc_full0", 1), ("prefill_gemm.cu", r"umma_commit\(acc_bar\)", 1),
+                                                ("prompt_attn.cu", r"umma_commit\(o_full\)", 1)])
+def test_results_are_not_complete_after_giving_up(name, barrier, count):
+    lines = [line for line in source(name).split("\n") if re.search(barrier, line)]
+    assert len(lines) == count and all("!dead" in line for line in lines)
+
+
+def test_nan_goes_to_results_clusters_and_state():
+    gemm, attn, scan = source("prefill_gemm.cu"), source("prompt_attn.cu"), source("chunk_scan.cuh")
+    for send in re.finditer(r"st_cluster4\((dst|slot\(buf)", gemm):              # sums for another CTA of the cluster
+        assert "if (dead)" in gemm[send.start() - 260: send.start()]
+    assert attn.index("if (dead) l =") < attn.index("st.shared::cluster.v2.f32")   # a row's sum: in the result of every part
+    assert "if (dead)" in scan[: scan.index("store_pairs<NP>(state")].rsplit("for (int j = 0; j < 4; ++j)", 1)[1]
+
+
+def test_waits_are_used():
+    text = "".join(source(n) for n in ("prefill_gemm.cu", "prompt_attn.cu", "chunk_scan.cuh"))
+    for name in re.findall(r"void (mbar_wait\w*)\(", source("tcgen.cuh")):
+        assert re.search(r"\b%s\(" % name, text), name

@@ -307,7 +307,12 @@ __global__ void __launch_bounds__(kChunkThreads, 1) chunk_scan_kernel(const Scan
 			if (lane == 0) mbar_arrive(empty0 + 8 * slot);
 		}
 #pragma unroll
-		for (int j = 0; j < 4; ++j) store_pairs<NP>(state + (size_t)j * D, s[j]);
+		for (int j = 0; j < 4; ++j) {
+			if (dead)
+#pragma unroll
+				for (int p = 0; p < NP; ++p) s[j][p] = pk(__int_as_float(0x7fc00000), __int_as_float(0x7fc00000));
+			store_pairs<NP>(state + (size_t)j * D, s[j]);
+		}
 	}
 }
 

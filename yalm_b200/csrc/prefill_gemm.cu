@@ -236,7 +236,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
 					}
 					more = 1;
 				}
-				if (elect_one()) umma_commit_pair(acc_full0 + 8 * b, pair_mask); // the accumulator is complete
+				if (!dead && elect_one()) umma_commit_pair(acc_full0 + 8 * b, pair_mask); // the accumulator is complete
 			}
 		}
 		__syncwarp();
@@ -299,6 +299,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
 					for (int c0 = 0; c0 < share; c0 += 32) {
 						float v[32];
 						tmem_ld32(trow + m * g.n_tile + p * share + c0, v);
+						if (dead)
+							for (int i = 0; i < 32; ++i) v[i] = kNaN;
 #pragma unroll
 						for (int i = 0; i < 32; i += 4)
 							st_cluster4(dst + (uint32_t)((((m * share + c0 + i) >> 2) * 128 + row) * 16), make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]));
@@ -429,7 +431,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ 
 				}
 				more = 1;
 			}
-			if (elect_one()) umma_commit(acc_bar);
+			if (!dead && elect_one()) umma_commit(acc_bar);
 		}
 		__syncwarp();
 	}
@@ -455,6 +457,8 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ 
 				for (int m = 0; m < MATS; ++m) {
 					float v[8];
 					tmem_ld8(trow + m * np + gr * 8, v);
+					if (dead)
+						for (int i = 0; i < 8; ++i) v[i] = kNaN;
 					st_cluster4(slot(buf, part < p ? part : part - 1, gr, m, 0), make_float4(v[0], v[1], v[2], v[3]));
 					st_cluster4(slot(buf, part < p ? part : part - 1, gr, m, 1), make_float4(v[4], v[5], v[6], v[7]));
 				}

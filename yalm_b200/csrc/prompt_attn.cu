@@ -374,7 +374,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 					}
 				}
 			}
-			if (elect_one()) umma_commit(o_full);
+			if (!dead && elect_one()) umma_commit(o_full);
 		}
 		__syncwarp();
 	} else if (warp < 4) {
@@ -496,6 +496,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 	const uint32_t op = tmem + ((uint32_t)(q * 32) << 16) + 256 + t * SH::DVP;
 	// from the start of shared memory (queries and stages are done with): [other part][tile][4 columns][row][4], then (reference, sum) [part][row of 256]
 	const uint32_t ml0 = base + (uint32_t)((parts - 1) * 2 * share * kTile * 4);
+	if (dead) l = __int_as_float(0x7fc00000);
 	__syncwarp();
 	if (parts > 1) {
 		cluster_sync(); // every part is done with its shared memory
@@ -546,7 +547,6 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 		}
 		const int h = g * a.G + min(row, rows - 1) % a.G;
 		float f = LAYERED ? stack::softmax_finish(M * 0.69314718055994531f, Lsum, a.sink, h) : 1.0f / Lsum;
-		if (dead) f = __int_as_float(0x7fc00000);
 		// through a patch of shared memory per warp (after what the parts exchanged), so that neighbouring lanes store neighbouring
 		// bytes: a row per lane, every 16-byte piece went to a line of its own (5 us for 256 rows of 128)
 		const uint32_t ld = (uint32_t)share * 4 + 16, patch = ml0 + (parts > 1 ? parts * 2 * kTile * 8 : 0) + (warp - 4) * 32 * ld;

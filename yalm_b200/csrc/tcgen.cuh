@@ -25,18 +25,9 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
 	             : "memory");
 	return ok;
 }
-// Bounded: a wait that ran out (a bug) marks the thread, whose later waits return at once; the kernels then store NaN.
-static __device__ __noinline__ bool mbar_wait_long(uint32_t bar, uint32_t parity) {
-	const long long t0 = clock64();
-	while (!mbar_try(bar, parity))
-		if (clock64() - t0 > 4000000000ll) return false; // ~2 s
-	return true;
-}
-__device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, bool &dead) {
-	if (mbar_try(bar, parity)) return;
-	if (!dead) dead = !mbar_wait_long(bar, parity);
-}
-// The same for a whole warp that goes on together: all lanes give up, or none.
+// Waits of a whole warp that goes on together, bounded: one that ran out (a bug) marks the warp, all its lanes or none, and its later waits return
+// at once.  A marked warp no longer signals that its part is done, so whoever needs it runs out in turn; the warps that store results store
+// NaN then, and hand NaN to the other CTAs of their cluster.
 static __device__ __noinline__ bool mbar_wait_warp_long(uint32_t bar, uint32_t parity) {
 	const long long t0 = clock64();
 	while (!__all_sync(0xffffffffu, mbar_try(bar, parity)))
