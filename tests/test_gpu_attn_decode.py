@@ -32,3 +32,27 @@ def test_attn_decode_splits(hd, G, n_kv):
         w = torch.softmax(torch.einsum("ghd,gtd->ght", q.view(n_kv, G, hd).double(), k[:, :rows].double()) * hd ** -0.5, dim=-1)
         want = torch.einsum("ght,gtd->ghd", w, v[:, :rows].double()).reshape(H, hd)
         assert ((out.double() - want).norm() / want.norm()).item() < 1e-6, rows
+
+
+@pytest.mark.parametrize("hd,size", [(64, 8.0), (16, 4.0)])
+@pytest.mark.parametrize("rows", [40, 300, 3000])
+def test_attn_decode_large_scores(hd, size, rows):
+    """Scores of about 100 that divide exactly by sqrt(head size): their differences are exact, so what is left is the exponential's unit and the
+    sums (4e-7 of the norm); a score rounded after a scaling by log2(e) would be off by 100 * 2^-24 of its weight."""
+    L, G, n_kv = api.lib(), 4, 2
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(hd + rows)
+    step = torch.randint(0, 33, (n_kv, rows), generator=gen, device="cuda") / 8.0
+    k, v = torch.zeros((n_kv, rows, hd), device="cuda"), torch.randn((n_kv, rows, hd), generator=gen, device="cuda").half()
+    k[:, :, 0], k[:, :, 1] = 1.0, step
+    q = torch.zeros((n_kv * G, hd), device="cuda")
+    q[:, 0], q[:, 1] = 100.0 * size + torch.arange(n_kv * G, device="cuda") * size, size      # scores 100 + head + step
+    k = k.half()
+    work = torch.zeros(L.yalm_attn_workspace_bytes(n_kv * G, n_kv, hd), device="cuda", dtype=torch.uint8)
+    out = torch.empty_like(q)
+    ctl = torch.tensor([0, rows - 1, 0, rows - 1, rows, 0, 0, 0], device="cuda", dtype=torch.int32)
+    p = lambda t: C.c_void_p(t.data_ptr())
+    assert L.yalm_attn_decode(p(out), p(k), p(v), p(q), p(work), n_kv * G, n_kv, hd, rows, p(ctl), None) == 0
+    w = torch.softmax(step.double(), dim=-1)
+    want = torch.einsum("gt,gtd->gd", w, v.double()).repeat_interleave(G, 0)
+    assert ((out.double() - want).norm() / want.norm()).item() < 4e-7
