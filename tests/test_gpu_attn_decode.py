@@ -56,3 +56,46 @@ def test_attn_decode_large_scores(hd, size, rows):
     w = torch.softmax(step.double(), dim=-1)
     want = torch.einsum("gt,gtd->gd", w, v.double()).repeat_interleave(G, 0)
     assert ((out.double() - want).norm() / want.norm()).item() < 4e-7
+
+
+def test_captured_calls_replay():
+    """Kernels launched chained under stream capture, behind a memset node (the entry without a workspace), each other and a copy: a replay on
+    other inputs gives what the calls give one by one."""
+    L, H, G, hd, n, rows = api.lib(), 32, 8, 128, 40, 900
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(1)
+    rnd = lambda *s: torch.randn(s, generator=gen, device="cuda")
+    k, v = rnd(G, rows, hd).half(), rnd(G, rows, hd).half()
+    q, q16 = torch.empty((H, hd), device="cuda"), torch.empty((n, H, hd), device="cuda", dtype=torch.float16)
+    w = (rnd(512, H * hd) * 0.02).half()
+    work = torch.zeros(L.yalm_attn_workspace_bytes(H, G, hd), device="cuda", dtype=torch.uint8)
+    ctl = torch.tensor([0, rows - 1, 0, rows - 1, rows, 0, 0, 0], device="cuda", dtype=torch.int32)
+    outs = [torch.empty((H, hd), device="cuda"), torch.empty((H, hd), device="cuda"), torch.empty((n, H, hd), device="cuda", dtype=torch.float16),
+            torch.empty((n, 512), device="cuda")]
+    copy = torch.empty_like(outs[3])
+    p, i = lambda t: C.c_void_p(t.data_ptr()), lambda *a: [C.c_int(x) for x in a]
+
+    def calls():
+        s = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+        rc = [L.yalm_attn_decode_static(p(outs[0]), p(k), p(v), p(q), *i(H, G, hd, rows), p(ctl), s),
+              L.yalm_attn_decode(p(outs[1]), p(k), p(v), p(q), p(work), *i(H, G, hd, rows), p(ctl), s),
+              L.yalm_attn_prefill(p(outs[2]), p(q16), p(k), p(v), *i(n, rows - n, H, G, hd, rows), s),
+              L.yalm_gemm_f16(p(outs[3]), C.c_int(512), p(outs[2]), p(w), *i(n, 512, H * hd, 0), s)]
+        copy.copy_(outs[3])
+        rc.append(L.yalm_gemm_f16(p(outs[3]), C.c_int(512), p(outs[2]), p(w), *i(n, 512, H * hd, 1), s))
+        assert rc == [0] * 5
+
+    q.copy_(rnd(H, hd)), q16.copy_(rnd(n, H, hd))
+    calls()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, capture_error_mode="thread_local"):
+        calls()
+    for _ in range(3):
+        q.copy_(rnd(H, hd)), q16.copy_(rnd(n, H, hd))
+        for o in outs:
+            o.fill_(float("nan"))
+        graph.replay()
+        got = [o.clone() for o in outs] + [copy.clone()]
+        calls()
+        assert all(torch.equal(a, b) for a, b in zip(got, outs + [copy])) and got[3].isfinite().all()
