@@ -66,8 +66,8 @@ def peaks():
 
 def ncu_traffic():
     """dram__bytes_read.sum + dram__bytes_write.sum of ONE timed-shape launch of the whole-token kernel on the headline
-    workload — logits mode at pos ~4090, captured by tools/gpu/ncu_full_logits.sh with `ncu --set full` and summarised
-    into profiles/*logits*_full_summary.txt (tools/ncu_summary.py).  None if no such capture is committed."""
+    workload — logits mode at pos ~4090, captured with `ncu --set full` and summarised into
+    profiles/*logits*_full_summary.txt (tools/ncu_summary.py).  None if no such capture is committed."""
     import glob
     import re
     files = sorted(glob.glob(os.path.join(ROOT, "profiles", "*logits*full_summary.txt")))
@@ -271,10 +271,10 @@ def run_prefill(args, arch, dtype, context, desc, base, path):
     pk = os.path.join(ROOT, "MEASURED_PEAKS.json")
     peak = float(json.load(open(pk))["bf16_tflops_sustained"]) if os.path.exists(pk) else 1374.5
     line = dict(base, impl="ours", metric="prefill tok/s (prompt tokens hydrated per second)", value=toks / t_host, steps=K, warmup=W,
-                ms_per_step=1000 * t_host / K, clocks=clk, gpu_launches=K * (2 + 12 * a.n_layers),
+                ms_per_step=1000 * t_host / K, clocks=clk, gpu_launches=K * (2 + 8 * a.n_layers),
                 e2e={"value": toks / t_host, "unit": "tok/s", "h2d_bytes_per_step": 4 * cap, "d2h_bytes_per_step": 4 * V,
                      "note": "host-timed around Model::forward_batch calls with host token buffers; each call copies the chunk's ids in and the last logits out"},
-                roofline={"bound": "tensor", "kernel": "gemm_f16_kernel (tcgen05.mma kind::f16, TMA operands, TMEM accumulator) + attn_prefill_kernel",
+                roofline={"bound": "tensor", "kernel": "gemm_pair_kernel (tcgen05.mma cta_group::2 kind::f16, TMA operands, TMEM accumulator) + prompt_attn_kernel",
                           "achieved": flop / t_host / 1e12, "peak": peak, "unit": "TFLOP/s", "frac": flop / t_host / 1e12 / peak,
                           "traffic": None, "peak_source": "MEASURED_PEAKS.json bf16_tflops_sustained"},
                 token_loop_hydrate_tok_s=loop_tok_s, speedup_vs_token_loop=toks / t_host / loop_tok_s,
