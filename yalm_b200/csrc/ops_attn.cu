@@ -70,8 +70,8 @@ struct Split {
 // rows are reduced together by halving exchanges (UN G - 1 + .. shuffles for all of them, not log2 of them for each), which leaves about
 // one exponential per lane and row batch.  Latency is what counts at a few thousand positions: a CTA's chain is control block, one batch
 // of keys and values, one exchange of partials; short contexts use fewer splits (at least one batch per warp each), one split writes the
-// result itself.  32 / 8 heads of 128, back to back, against a block-wide softmax per 512 rows: 37 positions 16 -> 6.5 us, 4096 20 -> 12 us, 32768
-// 68 -> 33 us.
+// result itself.  32 / 8 heads of 128, back to back, against a block-wide softmax per 512 rows: 37 positions 16 -> 3.9 us, 4096 19.6 -> 10.2 us, 32768
+// 68 -> 30.5 us.
 template <int HD, int G>
 __global__ void __launch_bounds__(kAttnThreads, Split<HD, G>::CTAS) attn_decode_kernel(AttnArgs a) {
 	using SP = Split<HD, G>;

@@ -14,7 +14,8 @@
 //  * gemm_pair_kernel (many rows): a pair of CTAs (cta_group::2) owns a tile of 256 rows x n columns, each CTA staging 128 rows of A
 //    and half of the columns of W: twice the products per staged byte of one CTA per 128 x 128 tile.  Persistent over tiles, the
 //    accumulator double-buffered so that a tile's tail runs under the next tile's products.  n and the number of K parts are
-//    picked per shape (plan_pair).  Bound by the tensor pipe at the clock that the power limit leaves.
+//    picked per shape (plan_pair).  Bound by the tensor pipe (gate and up of 512 rows: active 85 % of the time, at 1510 MHz in a launch by itself and less
+//    in a loop) or by SMs that have no tile (512 x 4096 x 14336: 128 of 148 work, the pipe is active 79 % of their time).
 //    512 rows, cold L2, against one CTA per 128 x 128 tile: 4096 x 14336 88 -> 65 us (919 TFLOP/s), w1 | w3 14336 x 4096 158 -> 109 us
 //    (1108), 32000 x 4096 242 -> 117 us (1150), q | k | v 74 -> 41 us, 4096 x 4096 41 -> 35 us.
 //  * gemm_few_kernel (few rows): bound by the bytes of W.  W is the 128-row operand, the positions are the N of the

@@ -18,7 +18,7 @@
 // Bound by the chain softmax - products of a tile pair (some 3500 cycles per 128 keys: 1800 from scores to weights, of which the exponentials
 // alone take 1024 at 16 a cycle and SM for each of the two tiles, 500 for the rescaling, and 1100 for P V and the next scores) and, for short
 // contexts, by launch, query staging and the store.  Back to back, against 64-row tiles on mma.sync: 507 rows at 7680 positions, 32 / 8 heads of 128:
-// 667 -> 80 us (825 TFLOP/s); 512 rows at 0: 32.8 -> 14.0 us; bf16 window 1024 and pooled blocks of 64, 512 rows, 16 / 4 heads: 57.3 -> 22.8 us.
+// 667 -> 80 us (825 TFLOP/s); 512 rows at 0: 32.8 -> 14.1 us; bf16 window 1024 and pooled blocks of 64, 512 rows, 16 / 4 heads: 57.3 -> 22.7 us.
 #include "common.cuh"
 #include "launch.h"
 #include "stack_rows.cuh"
