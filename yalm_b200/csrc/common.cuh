@@ -55,7 +55,7 @@ __device__ __forceinline__ uint4 ld_stream(const void *p) {
 }
 
 // Kernels that are launched with launch_chained (launch.h) may begin while the kernel before them in the stream still runs: what they
-// do before chain_wait() must not touch global memory, and returns from it with everything before them complete and visible.
+// do before chain_wait() must not read or write global memory (prefetches into L2 are neither), which returns with everything before them complete and visible.
 // Their lifetime begins while their inputs are still being written, so they make no promise that data stays as it is: no __restrict__ (which would
 // let loads rise above the wait) and no non-coherent loads.  chain_next() lets the next such kernel begin (it waits in turn).  A kernel with tensor memory calls it behind a barrier after its
 // allocation: the next kernel's would otherwise find the columns free, take them and wait, with them, for this one.

@@ -30,8 +30,9 @@ inline const DeviceInfo &device_info() {
 
 // Launch whose beginning - scheduling, barriers, tensor memory - overlaps the end of the kernel before it in the stream; the kernel calls
 // chain_wait() (common.cuh) before it touches global memory.  Back to back, launch and prologue were up to half of the small kernels' time
-// (decode attention at 37 positions 6.2 -> 3.8 us, first prompt portion's attention 16.4 -> 13.7 us, four scored layers 1.36 -> 1.25 ms).  Not for the
-// persistent GEMVs: their CTAs would settle where the kernel before left room first, unevenly (feed-forward of a token 75 -> 87 us).
+// (decode attention at 37 positions 6.2 -> 3.8 us, first prompt portion's attention 16.4 -> 13.7 us, four scored layers 1.36 -> 1.25 ms).  Not for persistent
+// grids of several CTAs per SM: these would settle where the kernel before left room first, unevenly (the row kernels of ops_gemv.cu, feed-forward of a token
+// 75 -> 87 us); one CTA per SM, by its shared memory, has no choice (stream_rows.cuh).
 template <typename... P, typename... A>
 inline int launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, int cluster, A &&...args) {
 	cudaLaunchConfig_t cfg = {};

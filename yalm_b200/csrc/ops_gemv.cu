@@ -3,6 +3,7 @@
 // C ABI in include/yalm_b200.h; each launcher cites the reference kernels it replaces there.
 #include "gemv.cuh"
 #include "launch.h"
+#include "stream_rows.cuh"
 
 #include <cfloat>
 
@@ -386,11 +387,13 @@ static int launch_persistent(K kernel, const A &args, size_t smem, long tasks, c
 	return (int)cudaGetLastError();
 }
 
+// Dense products go to the stream of stream_rows.cuh; the kernels of this file serve mixtures of experts, whose rows are known on the device only, and
+// rows too long for it.
+//
 // Whether tasks of half the size end sooner: a persistent grid takes whole rounds of its warps, and a last round with few tasks leaves the
-// memory idle for as long as a full one.  (Gate and up of a token, rows one or two pairs at a time: 4096 x 11008 fp16 with the down projection
-// 67 -> 57 us, fp32 122 -> 98, 1024 x 14336 fp32 70 -> 55; rows four or two at a time: 4096 x 4096 fp16 15.7 -> 11.3 us, 2048 x 2048 8.3 -> 6; where both
-// end together, as at 4096 x 14336 or 32000 x 4096, the larger tasks stay.)  kernel: that of the larger tasks, of the type at hand; more CTAs of the
-// other one fit on an SM, which can only bring its end forward.
+// memory idle for as long as a full one.  (Measured on dense matrices: gate and up of a token, rows one or two pairs at a time, 4096 x 11008 fp16 with the
+// down projection 67 -> 57 us, fp32 122 -> 98; rows four or two at a time, 4096 x 4096 fp16 15.7 -> 11.3 us; where both end together, as at 4096 x 14336, the
+// larger tasks stay.)  kernel: that of the larger tasks, of the type at hand; more CTAs of the other one fit on an SM, which can only bring its end forward.
 template <typename K>
 static bool finer_tasks(K kernel, size_t smem, long tasks) {
 	cudaError_t err;
@@ -446,6 +449,11 @@ extern "C" int yalm_gemv_residual_ep(float *out, const float *residual, const fl
 	const int ep = ep_of(dtype);
 	if (!ep || !out || !v || !w || n <= 0 || d <= 0 || n_active < 1 || ep_size < 1 || ep_rank < 0 || ep_rank >= ep_size) return YALM_EINVAL;
 	if (n % ep || d % 2 || (n_active > 1 && (!active_e || !active_w))) return YALM_EINVAL;
+	if (n_active == 1 && !active_e && !active_w && ep_size == 1 && n <= stream::longest(16 / ep)) {
+		stream::Args t{};
+		t.out = out, t.residual = residual, t.x = v, t.w = (const char *)w, t.scale = scale, t.alpha = 1.0f, t.n = n, t.d = d;
+		YALM_DISPATCH_DT(dtype, return (stream::launch<DT, false>(t, (cudaStream_t)s)));
+	}
 	ResidArgs a;
 	a.out = out, a.residual = residual, a.v = v, a.w = (const char *)w, a.scale = scale;
 	a.n = n, a.d = d, a.n_active = n_active, a.active_e = active_e, a.active_w = active_w;
@@ -474,6 +482,12 @@ extern "C" int yalm_ffn_glu_ep(float *hb, const float *x, const float *rms_weigh
 	if (!ep || !hb || !x || !w1 || !w3 || dim % ep || dim % 4 || hidden_dim <= 0) return YALM_EINVAL;
 	if (n_experts < 0 || n_experts > kMaxExperts) return YALM_EINVAL;
 	if (n_experts > 0 && (!gate || !active_e || !active_w || n_active < 1 || n_active > n_experts)) return YALM_EINVAL;
+	if (n_experts == 0 && dim <= stream::longest(16 / ep)) {
+		stream::Args t{};
+		t.out = hb, t.x = x, t.rms_w = rms_weight, t.w = (const char *)w1, t.w3 = (const char *)w3, t.scale = s1, t.scale3 = s3;
+		t.eps = norm_eps, t.act = act, t.n = dim, t.d = hidden_dim;
+		YALM_DISPATCH_DT(dtype, return (stream::launch<DT, true>(t, (cudaStream_t)s)));
+	}
 	FfnArgs a;
 	a.hb = hb, a.x = x, a.rms_w = rms_weight;
 	a.w1 = (const char *)w1, a.w3 = (const char *)w3, a.gate = (const char *)gate;
@@ -494,6 +508,12 @@ static int rows_launch(float *out, const float *x, const float *rms_w, const voi
                        int d, float eps, int dtype, cudaStream_t st, float alpha = 1.f) {
 	const int ep = ep_of(dtype);
 	if (!ep || !out || !x || !w || n <= 0 || d <= 0 || n % ep) return YALM_EINVAL;
+	if (n <= stream::longest(16 / ep)) {
+		stream::Args t{};
+		t.out = out, t.x = x, t.rms_w = rms_w, t.w = (const char *)w, t.scale = scale, t.eps = eps, t.alpha = alpha, t.n = n, t.d = d;
+		if (dtype == YALM_BF16) return stream::launch<YALM_BF16, false>(t, st);
+		YALM_DISPATCH_DT(dtype, return (stream::launch<DT, false>(t, st)));
+	}
 	RowsArgs a;
 	a.out = out, a.x = x, a.rms_w = rms_w, a.w = (const char *)w, a.scale = scale, a.n = n, a.d = d, a.eps = eps, a.alpha = alpha;
 	const size_t smem = 36 * sizeof(float) + xs_bytes(dtype, n);
