@@ -1,0 +1,79 @@
+"""-m gpu: the whole-token kernel of dense models on one GPU (csrc/decode_token.cuh) at the edges of its geometry - rows of one 512-byte chunk to four
+pieces, ragged last chunks, several rows a stage, stages that q, k and v share, fewer rows than CTAs, contexts shorter and longer than the CTAs of a head - against the oracle's tokens and logits."""
+import numpy as np
+import pytest
+
+from conftest import LOGIT_TOL
+from yalm_b200 import api
+from yalm_b200 import yalm_file as yf
+
+pytestmark = pytest.mark.gpu
+
+
+def arch(dim, hidden, hd, heads, kv, vocab=600, layers=2, seq=256, **kw):
+    return yf.Arch(dim, hidden, hd, layers, heads, kv, vocab, seq, 10000.0, name="token", **kw)
+
+
+CASES = {
+    # dim: one chunk, 16 rows a stage that straddle q | k | v; hidden: 3 chunks, the last ragged
+    "fp16-one-chunk": (arch(256, 640, 32, 8, 4), "fp16"),
+    # dim: 5 chunks (one row each for 5 of 8 warps); hidden: 11 chunks, half of one empty; gelu, clip
+    "fp16-odd-chunks": (arch(1280, 2752, 32, 8, 2, act_type="gelu", qkv_clip=0.5), "fp16"),
+    # hidden: 3 pieces, two of 15 chunks and one of 13
+    "fp16-three-pieces": (arch(1024, 11008, 64, 8, 2), "fp16"),
+    # dim: two pieces under a norm (20 chunks), hidden: four full ones; 8 query heads a KV head
+    "fp16-two-pieces-normed": (arch(5120, 16384, 128, 40, 5, layers=1, vocab=200), "fp16"),
+    # fp32: 16 chunks of dim (two of a warp), 4 pieces of hidden
+    "fp32": (arch(2048, 8192, 128, 8, 2, vocab=100, layers=1), "fp32"),
+    # fp8: rows of 2 chunks with scales, hidden 19 chunks in two pieces
+    "fp8": (arch(1024, 9728, 64, 16, 4), "fp8"),
+    # fewer rows than CTAs in every phase
+    "fp16-few-rows": (arch(64, 96, 32, 2, 1, vocab=50), "fp16"),
+}
+
+
+@pytest.mark.parametrize("case", sorted(CASES))
+def test_tokens_and_logits(oracle, case):
+    a, dt = CASES[case]
+    img = bytes(yf.random_model(a, dt, seed=5))
+    prompt, n = [1, 5, 9, 20, 7], 24 if a.dim <= 1280 else 6
+    ref = bytes(yf.dequantized_fp32_image(img)) if dt == "fp8" else img
+    to, lo = oracle.OracleModel(ref).generate(prompt, n, keep_logits=True)
+    m = api.Model(img).cuda()
+    assert m.uses_megakernel() and m.mega_info()["stages"] == 24 and not m.mega_info()["w2_pipe"]
+    s = api.InferenceState(m)
+    tg, lg = s.generate(prompt, n, keep_logits=True)
+    assert np.abs(lg - lo).max() < LOGIT_TOL and tg == to
+    for pos, tok in enumerate(prompt[:-1]):
+        s.forward(tok, pos, api.MODE_HYDRATE)
+    assert s.generate_greedy(prompt[-1], len(prompt) - 1, n) == to  # arg-max and position on the device
+    s.close()
+    m.close()
+
+
+@pytest.mark.parametrize("context", [1, 2, 63, 64, 65, 300])
+def test_contexts_around_the_units_of_attention(oracle, context):
+    """One position; the stages' edges at 32 channels (64 positions), half of a stage empty; every CTA of a head with units of its own."""
+    a = arch(256, 512, 32, 8, 2, vocab=300, layers=1, seq=512)
+    img = bytes(yf.random_model(a, "fp16", seed=6))
+    ids = [(37 * i + 1) % 300 for i in range(context)]
+    to, lo = oracle.OracleModel(img).generate(ids, 3, keep_logits=True)
+    m = api.Model(img).cuda()
+    s = api.InferenceState(m)
+    tg, lg = s.generate(ids, 3, keep_logits=True)
+    assert np.abs(lg - lo).max() < LOGIT_TOL and tg == to
+    s.close()
+    m.close()
+
+
+def test_rows_beyond_it_stay_with_the_other_kernel(oracle):
+    """A hidden size of five pieces."""
+    a = arch(512, 20480, 64, 8, 2, layers=1, vocab=100)
+    img = bytes(yf.random_model(a, "fp16", seed=7))
+    to, lo = oracle.OracleModel(img).generate([1, 2, 3], 4, keep_logits=True)
+    m = api.Model(img).cuda()
+    s = api.InferenceState(m)
+    tg, lg = s.generate([1, 2, 3], 4, keep_logits=True)
+    assert m.uses_megakernel() and np.abs(lg - lo).max() < LOGIT_TOL and tg == to
+    s.close()
+    m.close()

@@ -1,6 +1,6 @@
 // Host side of the whole-token persistent decode kernel (planning, launch) and the streaming probe.
 // The kernel itself is in decode_mega.cuh, instantiated per weight type in decode_mega_{f32,f16,f8}.cu.
-#include "decode_mega.cuh"
+#include "decode_token.cuh"
 #include "launch.h"
 
 #include <cuda.h> // CUtensorMap + enums only: cuTensorMapEncodeTiled is resolved at run time (cudaGetDriverEntryPoint)
@@ -133,6 +133,10 @@ const void *kernel_f16_pipe(int head_dim, int g, bool tp);
 const void *kernel_f8_pipe(int head_dim, int g, bool tp);
 const void *kernel_f16_mma(int head_dim, int g, bool tp);
 
+const void *kernel_f32_token(int head_dim, int g);
+const void *kernel_f16_token(int head_dim, int g);
+const void *kernel_f8_token(int head_dim, int g);
+
 // variant: 0 default, 1 pipelined hb, 2 tensor-core GEMV (decode_mega.cuh: gemv_phase); null if not compiled
 static const void *kernel_of(int dtype, int head_dim, int g, bool tp, int variant) {
 	switch (dtype) {
@@ -159,6 +163,33 @@ static bool plan_shapes(int dtype, int dim, int q_dim, int kv_dim, int hidden, i
 	s[kQKV].G = (q_dim + 2 * kv_dim) / s[kQKV].R, s[kWO].G = dim / s[kWO].R, s[kFFN].G = n_sub * (hidden / (s[kFFN].R / 2));
 	s[kW2].G = dim / s[kW2].R, s[kLM].G = vocab / s[kLM].R;
 	for (int k = 0; k < kNumKinds; ++k) shape[k][0] = s[k].R, shape[k][1] = s[k].KT, shape[k][2] = s[k].nk, shape[k][3] = s[k].G;
+	return true;
+}
+
+// The kernel of decode_token.cuh for a dense model on one GPU, where its rows fit: pieces of 16 chunks of 512 bytes, a lane's part of a vector in
+// registers (64 floats: 16384 elements; wider rows spill there, and stay with the kernels of decode_mega.cuh), a CTA's rows of x in shared memory.
+static bool plan_token(Plan &p, int dtype, int dim, int q_dim, int hidden, int head_dim, int G, int max_smem) {
+	const int B = bytes_of(dtype), ep = ep_of(dtype), n[3] = {dim, q_dim, hidden};
+	int floats[3];
+	for (int i = 0; i < 3; ++i) {
+		const int chunks = (n[i] * B + token::kChunk - 1) / token::kChunk, np = (chunks + 15) / 16, piece = (chunks + np - 1) / np;
+		const bool sides = np == 1 && piece <= kTokenWarps;
+		p.token_geo[i][0] = np, p.token_geo[i][1] = piece, p.token_geo[i][2] = sides ? kTokenWarps / piece * 2 : 1;
+		floats[i] = sides ? ep : np * 2 * ep;
+	}
+	const int most = std::max(floats[0], std::max(floats[1], floats[2]));
+	if (most > token::kFloats || floats[0] > kTokenNormFloats || (dim + p.grid - 1) / p.grid > kTokenMaxRows) return false;
+	const void *kernel = dtype == YALM_F32   ? kernel_f32_token(head_dim, G)
+	                     : dtype == YALM_F16 ? kernel_f16_token(head_dim, G)
+	                                         : kernel_f8_token(head_dim, G);
+	const size_t smem = token::smem_bytes(head_dim, G);
+	cudaFuncAttributes at;
+	if (!kernel || smem > (size_t)max_smem) return false;
+	if (cudaFuncGetAttributes(&at, kernel) != cudaSuccess || !token::regs_suffice(at.numRegs)) { // (else the hand-over of registers would wait for ever)
+		cudaGetLastError();
+		return false;
+	}
+	p.kernel = kernel, p.smem = smem, p.stages = kTokenStages, p.threads = token::kTokenThreads, p.vec_floats = 0;
 	return true;
 }
 
@@ -213,6 +244,7 @@ Plan plan(int dtype, int dim, int q_dim, int kv_dim, int head_dim, int hidden, i
 			vf += kMmaSlots * kConsumerWarps * 16; // the tiles' per-warp partial sums live behind the input vector
 		}
 	}
+	bool token_kernel = false; // decode_token.cuh
 	// Pipelined w1/w3 -> w2 hand-over (decode_mega.cuh "pipelined hb"; dense models whose w2 is K-split): hb never sits in
 	// shared memory as a whole — kHbBufs slice buffers behind the other phases' input vector replace it, and the ring gets the
 	// difference (70B-class: 112 KB -> 64 KB, six more stages; measured +6.5 % tok/s on a 16-layer slice).  It is switched
@@ -225,22 +257,25 @@ Plan plan(int dtype, int dim, int q_dim, int kv_dim, int head_dim, int hidden, i
 		const bool can = !p.mma && !tp && n_experts == 0 && nk >= 2 && nk <= kHbMaxSlices && p.shape[kW2][0] <= 2 &&
 		                 (groups + kConsumerWarps - 1) / kConsumerWarps <= kHbMaxGroups && stages_for(vf_pipe) >= 2;
 		const bool want = e ? atoi(e) != 0 : stages_for(vf_pipe) >= stages_for(vf) + 2;
-		if (can && want) p.w2_pipe = 1, p.hb_slice = p.shape[kW2][1], p.hb_off = hb_off, vf = vf_pipe;
+		// (a setting of either choice, on or off, asks for that kernel)
+		token_kernel = !e && !getenv("YALM_MEGA_MMA") && !tp && n_experts == 0 && plan_token(p, dtype, dim, q_dim, hidden, head_dim, G, di.max_smem_optin);
+		if (can && want && !token_kernel) p.w2_pipe = 1, p.hb_slice = p.shape[kW2][1], p.hb_off = hb_off, vf = vf_pipe;
 	}
-	p.kernel = kernel_of(dtype, head_dim, G, tp, p.mma ? 2 : p.w2_pipe ? 1 : 0);
-	if (!p.kernel) return p;
-	p.vec_floats = (std::max(vf, vf_attn) + 31) / 32 * 32;
-	const size_t fixed = (size_t)p.vec_floats * 4 + kSmemHeader;
-	p.stages = stages_for(vf);
-	if (p.stages < 2) return p;
-	p.smem = (size_t)p.stages * kStageBytes + fixed;
+	if (!token_kernel) {
+		p.kernel = kernel_of(dtype, head_dim, G, tp, p.mma ? 2 : p.w2_pipe ? 1 : 0);
+		if (!p.kernel) return p;
+		p.vec_floats = (std::max(vf, vf_attn) + 31) / 32 * 32;
+		p.stages = stages_for(vf);
+		if (p.stages < 2) return p;
+		p.smem = (size_t)p.stages * kStageBytes + (size_t)p.vec_floats * 4 + kSmemHeader;
+	}
 	p.dtype = dtype;
 	if (cudaFuncSetAttribute(p.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem) != cudaSuccess) {
 		cudaGetLastError();
 		return p;
 	}
 	int occ = 0;
-	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, p.kernel, kThreads, p.smem) != cudaSuccess || occ < 1) {
+	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, p.kernel, p.threads, p.smem) != cudaSuccess || occ < 1) {
 		cudaGetLastError();
 		return p;
 	}
@@ -254,6 +289,7 @@ int launch(const Plan &p, const Args &a, cudaStream_t st) {
 	args.stages = p.stages, args.vec_floats = p.vec_floats;
 	args.w2_pipe = p.w2_pipe, args.hb_slice = p.hb_slice, args.hb_off = p.hb_off;
 	args.mma = p.mma;
+	memcpy(args.token_geo, p.token_geo, sizeof(args.token_geo));
 	memcpy(args.mma_mt, p.mma_mt, sizeof(args.mma_mt));
 	if (p.mma && !a.tmaps) return YALM_EINVAL;
 	if (p.w2_pipe && (!a.hbp || !a.hb_cnt)) return YALM_EINVAL;
@@ -275,7 +311,7 @@ int launch(const Plan &p, const Args &a, cudaStream_t st) {
 	args.l2_ahead = kn.ahead;
 	if (max_stages >= 2 && max_stages < args.stages) args.stages = max_stages;
 	void *params[] = {&args};
-	return (int)cudaLaunchCooperativeKernel(p.kernel, dim3(p.grid), dim3(kThreads), params, p.smem, st);
+	return (int)cudaLaunchCooperativeKernel(p.kernel, dim3(p.grid), dim3(p.threads), params, p.smem, st);
 }
 
 } // namespace mega

@@ -46,6 +46,9 @@ constexpr int kFlagPhaseBits = 12;  // hand-over flag = launch number << kFlagPh
 constexpr int kLLRep = YALM_MEGA_LL_REP; // copies of every flagged hand-over vector (decode_mega.cuh); 1, 2 or 4
 constexpr int kProfileSlots = 6 * 8; // per (CTA, layer): phases x slots, see decode_mega.cuh
 
+// The kernel of dense models on one GPU (decode_token.cuh): consumer warps, ring stages, rows of x that a CTA keeps, floats of a normed vector a lane holds
+constexpr int kTokenWarps = 8, kTokenStages = 24, kTokenMaxRows = 128, kTokenNormFloats = 32;
+
 // ---- tensor parallelism inside the kernel (N GPUs of one NVSwitch domain) ---------------------------------------------
 // Every rank owns one region of device memory that all peers map (CUDA IPC, tp.cpp).  The row -> CTA -> warp map of a
 // phase is the same on every rank, so the all-reduce behind wo / w2 is an exchange between the warps that own the same
@@ -132,6 +135,10 @@ struct Args {
 	// class: [0] wq [1] wk / wv [2] wo [3] w1 / w3 (rows of each) [4] w2 [5] LM head
 	const void *tmaps;
 	int mma, mma_mt[6];
+	// decode_token.cuh: rows of n = dim, q_dim and hidden columns as pieces, 512-byte chunks per piece, rows per stage; flagged words of q
+	// ([kLLRep][q_dim]) and of the appended key and value (half2 words, [2][kv_dim / 2])
+	int token_geo[3][3];
+	unsigned long long *ll_q, *ll_kv;
 	char *tp_peer[kTpMaxWorld]; // every rank's region (kTpOff*), [tp_rank] = this rank's own
 };
 
@@ -141,6 +148,8 @@ struct Plan {
 	bool tp = false;
 	int w2_pipe = 0, hb_slice = 0, hb_off = 0; // pipelined hb (Args)
 	int mma = 0, mma_mt[6] = {}; // tensor-core GEMV (Args)
+	int token_geo[3][3] = {}; // decode_token.cuh (threads: of whichever kernel)
+	int threads = kThreads;
 	size_t smem = 0;
 	const void *kernel = nullptr;
 	int shape[5][4] = {};

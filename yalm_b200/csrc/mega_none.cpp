@@ -10,5 +10,8 @@ const void *kernel_f32_pipe(int, int, bool) { return nullptr; }
 const void *kernel_f16_pipe(int, int, bool) { return nullptr; }
 const void *kernel_f8_pipe(int, int, bool) { return nullptr; }
 const void *kernel_f16_mma(int, int, bool) { return nullptr; }
+const void *kernel_f32_token(int, int) { return nullptr; }
+const void *kernel_f16_token(int, int) { return nullptr; }
+const void *kernel_f8_token(int, int) { return nullptr; }
 } // namespace mega
 } // namespace yalm

@@ -321,7 +321,8 @@ void InferenceState::cuda() {
 	    {(void **)&_mega_hbp, sizeof(float) * ((size_t)k_act * lhid + 512)}, // hb in the w2 tile loop's permuted layout (padded to a chunk)
 	    {(void **)&_mega_hb_cnt, sizeof(unsigned) * (size_t)c.n_layers * yalm::mega::kHbMaxSlices},
 	    {(void **)&_mega_ll, 8 * (yalm::mega::kLLRep * ((size_t)2 * c.dim + (size_t)k_act * lhid + (size_t)lh * c.head_dim) +
-	                              (size_t)sms * lh * c.head_dim + (size_t)sms * lh * 2)},
+	                              (size_t)sms * lh * c.head_dim + (size_t)sms * lh * 2 + yalm::mega::kLLRep * (size_t)lh * c.head_dim +
+	                              (size_t)lkv * c.head_dim)},
 	};
 	size_t total = 0;
 	for (auto &s : slots) total += align_up(s.bytes, 256);
@@ -867,6 +868,7 @@ int Model::launch_mega(InferenceState &s, int token, int pos, int mode, long lon
 	constexpr size_t rep = yalm::mega::kLLRep;
 	a.ll_x = s.mega_ll(), a.ll_hb = a.ll_x + rep * 2 * c.dim, a.ll_att = a.ll_hb + rep * (size_t)a.hb_len;
 	a.ll_acc = a.ll_att + rep * a.q_dim, a.ll_ml = a.ll_acc + (size_t)_mega->plan.grid * a.q_dim;
+	a.ll_q = a.ll_ml + (size_t)_mega->plan.grid * a.n_heads * 2, a.ll_kv = a.ll_q + rep * a.q_dim;
 	// launch number behind the hand-over flags: per state on one GPU; under tensor parallelism the peers' mailboxes belong
 	// to the process, so the counter does too (every rank issues the same launches in the same order)
 	static unsigned tp_seq = 0;

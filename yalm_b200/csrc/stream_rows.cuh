@@ -313,7 +313,7 @@ static int launch_as(const Args &a, cudaStream_t st) {
 	YALM_TRY(allow_smem((const void *)kernel, kSmem));
 	return launch_chained(kernel, dim3(std::min(device_info().sms, a.d)), dim3(kThreads), kSmem, st, 1, a);
 }
-// Longest row whose part of x fits the 112 registers that 17 warps leave a thread; longer ones take the kernels of ops_gemv.cu.
+// Longest row whose part of x fits the 96 registers that 17 warps (five on one scheduler) leave a thread; longer ones take the kernels of ops_gemv.cu.
 constexpr int longest(int bytes_per_element) { return (bytes_per_element == 1 ? 2 : 4) * 32 * 512 / bytes_per_element; }
 
 // a: all but the geometry, a.n <= longest().
