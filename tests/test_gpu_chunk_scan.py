@@ -60,3 +60,26 @@ def test_chunks_match_steps(D, P, form, portions):
     assert ((out[:, :H * P].reshape(n, H, P).double() - want).norm() / want.norm()).item() < 2e-6
     assert ((state.double() - S).norm() / S.norm()).item() < 2e-6
     assert (out[:, H * P:] == 7.0).all()
+
+
+@pytest.mark.parametrize("H,D,P", [(40, 128, 64), (40, 64, 36), (148, 64, 8), (149, 64, 8), (37, 128, 4)])
+@pytest.mark.parametrize("form", ["delta_channel", "delta_head", "linear_channel"])
+def test_columns_four_and_two_a_warp(H, D, P, form):
+    """Around the rule between the two: more and fewer column groups than SMs, the last group not full."""
+    n = 21
+    g = torch.Generator(device="cuda")
+    g.manual_seed(H + D + P)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+    k, q, v = rnd(n, H, D), rnd(n, H, D) * D ** -0.5, rnd(n, H, P)
+    k = k / k.norm(dim=-1, keepdim=True)
+    decay = torch.exp(-0.3 * torch.rand((n, H) if form == "delta_head" else (n, H, D), generator=g, device="cuda"))
+    beta = torch.sigmoid(rnd(n, H)) if form.startswith("delta") else None
+    start = rnd(H, P, D)
+    state, out = start.clone(), torch.empty((n, H, P), device="cuda")
+    p = lambda t: C.c_void_p(None if t is None else t.data_ptr())
+    i = C.c_int
+    assert api.lib().yalm_state_scan_rows(p(out), i(H * P), p(k), i(H * D), p(q), i(H * D), p(v), i(H * P), p(decay), i(decay[0].numel()), i(int(decay.dim() == 3)), None, i(0),
+                                          p(beta), i(H), None, p(state), i(n), i(H), i(1), i(D), i(P), i(5), None, None) == 0
+    want, S = step_by_step(k.double(), q.double(), v.double(), decay.double(), None if beta is None else beta.double(), None, None, start.double(), 1)
+    assert ((out.double() - want).norm() / want.norm()).item() < 2e-6
+    assert ((state.double() - S).norm() / S.norm()).item() < 2e-6

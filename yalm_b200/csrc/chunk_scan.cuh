@@ -8,14 +8,16 @@
 // (without the delta correction r = v and T = diag(vscale)).  Every decay enters as a product of decays, never as a quotient, so a
 // decay may be 0.  All of it is fp32; what differs from the position-by-position form is the order of sums.
 //
-// A CTA owns 16 columns of one head.  Six warps prepare chunks in turn - everything that the columns share: b k, b q, the update rows, T and
-// B T, and the chunk's v - into a ring of shared-memory slots; four warps own 4 columns each, a lane 4 (D = 128) or 2 (D = 64) rows of all four: a
-// vector of a chunk is read once for 4 columns (at one column per thread the shared-memory reads were the limit), the 64 partial
+// A CTA owns 16 or 8 columns of one head.  Eight warps prepare chunks in turn - everything that the columns share: b k, b q, the update rows, T and
+// B T, and the chunk's v - into a ring of shared-memory slots; four warps own NC = 4 or 2 columns each, a lane 4 (D = 128) or 2 (D = 64) rows of all of them: a
+// vector of a chunk is read once for NC columns (at one column per thread the shared-memory reads were the limit), the 8 NC partial
 // products meet over the 32 lanes by halving exchanges, which leave lane (t, c) with the sums of position t and column c.
 // The packed fp32 instructions carry two rows each.
-// Bound by the column warps, one per scheduler: of about 1550 cycles a chunk 600 go to the products with M_0 (shared-memory reads of four
-// wavefronts each), 620 to the exchanges and T, 320 to the update.  (2 columns x 8 rows a lane: fewer exchanges, more reads, the same time.)
-// 512 rows, 16 heads of 128 x 128, decay per channel, delta rule: 125 -> 60 us; without the correction 80 -> 46 us; 64 x 64: 101 -> 45 us.
+// Bound by the column warps, one per scheduler: of about 1550 cycles a chunk with 4 columns 600 go to the products with M_0 (shared-memory reads of four
+// wavefronts each), 620 to the exchanges and T, 320 to the update.  (2 columns x 8 rows a lane, or eight warps of two columns in a CTA of 16, which
+// leaves registers for four warps that prepare: no faster, 60 and 64 us for 57.)
+// 512 rows, delta rule with a decay per channel: 16 heads of 128 x 128 57 -> 55 us (eight warps that prepare instead of six); 8 heads, in CTAs of 8 columns,
+// 57 -> 44 us; 16 heads of 64 x 64 44 -> 34 us; without the correction 43 -> 42, 43 -> 35, 34 -> 28 us.
 #pragma once
 
 #include "tcgen.cuh"
@@ -23,7 +25,7 @@
 namespace yalm {
 namespace stack {
 
-constexpr int kChunk = 8, kChunkCols = 16, kChunkSlots = 8, kPrepWarps = 6, kChunkThreads = 32 * (4 + kPrepWarps);
+constexpr int kChunk = 8, kChunkCols = 16, kChunkSlots = 8, kPrepWarps = 8, kChunkThreads = 32 * (4 + kPrepWarps); // (kChunkCols: the most a CTA owns)
 
 template <int D>
 struct ChunkSlot { // float offsets
@@ -78,32 +80,36 @@ __device__ __forceinline__ void exchange_sum(float (&v)[N]) {
 		}
 }
 
-// 32 values [position][4] of which slot i holds position (i / 4) ^ (lane / 4): the lanes agree on who keeps what without a select (a lane always
-// keeps the lower slots), but for the last two exchanges, over the columns.  Afterwards v[0] is the sum of (position lane / 4, column lane % 4).
-__device__ __forceinline__ void exchange_chunk(float (&v)[32]) {
+// 8 NC values [position][NC] of which slot i holds position (i / NC) ^ (lane / 4): the lanes agree on who keeps what without a select (a lane always
+// keeps the lower slots), but for the exchanges over the columns.  Afterwards v[0] is the sum of (position lane / 4, column lane % 4 NC / 4).
+template <int NC>
+__device__ __forceinline__ void exchange_chunk(float (&v)[8 * NC]) {
 	const int lane = threadIdx.x & 31;
 #pragma unroll
-	for (int o = 16, n = 16; o >= 4; o >>= 1, n >>= 1)
+	for (int o = 16, n = 4 * NC; o >= 4; o >>= 1, n >>= 1)
 #pragma unroll
 		for (int i = 0; i < n; ++i) v[i] += __shfl_xor_sync(kFull, v[i + n], o);
 #pragma unroll
-	for (int o = 2; o > 0; o >>= 1)
+	for (int o = 2, n = NC / 2; o > 0; o >>= 1, n >>= 1) {
 #pragma unroll
-		for (int i = 0; i < o; ++i) {
-			const float give = (lane & o) ? v[i] : v[i + o], keep = (lane & o) ? v[i + o] : v[i];
+		for (int i = 0; i < n; ++i) {
+			const float give = (lane & o) ? v[i] : v[i + n], keep = (lane & o) ? v[i + n] : v[i];
 			v[i] = keep + __shfl_xor_sync(kFull, give, o);
 		}
+		if (n == 0) v[0] += __shfl_xor_sync(kFull, v[0], o); // two lanes for a column
+	}
 }
 
-template <int D, bool DELTA, bool PER_CHANNEL>
+// NC: columns of a warp
+template <int D, int NC, bool DELTA, bool PER_CHANNEL>
 __global__ void __launch_bounds__(kChunkThreads, 1) chunk_scan_kernel(const ScanArgs a) {
 	using SL = ChunkSlot<D>;
 	constexpr int NP = D / 64; // pairs of rows per lane
 	extern __shared__ __align__(16) float chunk_sm[];
 	__shared__ __align__(8) unsigned long long bars[2 * kChunkSlots];
 	const int warp = uniform_warp(), lane = threadIdx.x & 31;
-	const int h = blockIdx.y, kh = h / a.rep, c0 = blockIdx.x * kChunkCols, nchunks = (a.n + kChunk - 1) / kChunk;
-	const int col_warps = min(4, (a.P - c0) / 4); // (P is a multiple of 4)
+	const int h = blockIdx.y, kh = h / a.rep, c0 = blockIdx.x * 4 * NC, nchunks = (a.n + kChunk - 1) / kChunk;
+	const int col_warps = min(4, (a.P - c0) / NC); // (P is a multiple of 4)
 	const uint32_t full0 = s32(bars), empty0 = full0 + 8 * kChunkSlots;
 	bool dead = false;
 	if (threadIdx.x == 0)
@@ -140,7 +146,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1) chunk_scan_kernel(const Scan
 			float4 v = make_float4(0.f, 0.f, 0.f, 0.f); // position lane / 4, columns 4 (lane % 4) ..
 			{
 				const int t = t0 + (lane >> 2), c = c0 + (lane & 3) * 4;
-				if (t < a.n && c < a.P) {
+				if (t < a.n && c < a.P && (lane & 3) < NC) {
 					const float *src = a.v + (size_t)t * a.ldv + (size_t)h * a.P + c;
 					v = make_float4(src[0], src[1], src[2], src[3]);
 				}
@@ -224,14 +230,14 @@ __global__ void __launch_bounds__(kChunkThreads, 1) chunk_scan_kernel(const Scan
 			__syncwarp();
 			if (lane == 0) mbar_arrive(full0 + 8 * slot);
 		}
-	} else if (warp < col_warps) { // ---- columns c0 + 4 warp .. ; a lane's rows lane D / 32 .. ----
-		__shared__ __align__(16) float2 u_sm[4][kChunk][4]; // u, twice
-		const int e0 = lane * 2 * NP, cw = c0 + 4 * warp, t = lane >> 2, c = lane & 3;
+	} else if (warp < col_warps) { // ---- columns c0 + NC warp .. ; a lane's rows lane D / 32 .. ----
+		__shared__ __align__(16) float2 u_sm[4][kChunk][NC]; // u, twice
+		const int e0 = lane * 2 * NP, cw = c0 + NC * warp, t = lane >> 2, c = (lane & 3) * NC / 4;
 		const bool fresh = first_pos(a.ctl, a.pos0) == 0;
 		float *state = a.state + ((size_t)h * a.P + cw) * D + e0;
-		f32x2 s[4][NP];
+		f32x2 s[NC][NP];
 #pragma unroll
-		for (int j = 0; j < 4; ++j) {
+		for (int j = 0; j < NC; ++j) {
 			if (fresh) {
 #pragma unroll
 				for (int p = 0; p < NP; ++p) s[j][p] = 0;
@@ -243,64 +249,68 @@ __global__ void __launch_bounds__(kChunkThreads, 1) chunk_scan_kernel(const Scan
 			const int slot = ch % kChunkSlots;
 			mbar_wait_warp(full0 + 8 * slot, (uint32_t)(ch / kChunkSlots) & 1u, dead);
 			const float *sm = chunk_sm + slot * SL::SIZE;
-			float W[DELTA ? 32 : 1], O[32];
+			float W[DELTA ? 8 * NC : 1], O[8 * NC];
 #pragma unroll
 			for (int tt = 0; tt < kChunk; ++tt) {
 				f32x2 x[NP];
 				if constexpr (DELTA) {
 					load_pairs<NP>(x, sm + SL::K + (tt ^ t) * D + e0);
 #pragma unroll
-					for (int j = 0; j < 4; ++j) {
+					for (int j = 0; j < NC; ++j) {
 						f32x2 d = mul2(x[0], s[j][0]);
 						if (NP == 2) d = fma2(x[NP - 1], s[j][NP - 1], d);
-						W[tt * 4 + j] = sum2(d);
+						W[tt * NC + j] = sum2(d);
 					}
 				}
 				load_pairs<NP>(x, sm + SL::Q + (tt ^ t) * D + e0);
 #pragma unroll
-				for (int j = 0; j < 4; ++j) {
+				for (int j = 0; j < NC; ++j) {
 					f32x2 d = mul2(x[0], s[j][0]);
 					if (NP == 2) d = fma2(x[NP - 1], s[j][NP - 1], d);
-					O[tt * 4 + j] = sum2(d);
+					O[tt * NC + j] = sum2(d);
 				}
 			}
-			const float v = sm[SL::V + t * kChunkCols + warp * 4 + c];
+			const float v = sm[SL::V + t * kChunkCols + warp * NC + c];
 			float r = v;
 			if constexpr (DELTA) {
-				exchange_chunk(W);
+				exchange_chunk<NC>(W);
 				r = v - W[0];
 			}
-			exchange_chunk(O);
+			exchange_chunk<NC>(O);
 			float u = 0.f, y = O[0];
 			float Tr[8], Br[8];
 			*reinterpret_cast<float4 *>(Tr) = *reinterpret_cast<const float4 *>(sm + SL::T + t * 8), *reinterpret_cast<float4 *>(Tr + 4) = *reinterpret_cast<const float4 *>(sm + SL::T + t * 8 + 4);
 			*reinterpret_cast<float4 *>(Br) = *reinterpret_cast<const float4 *>(sm + SL::BT + t * 8), *reinterpret_cast<float4 *>(Br + 4) = *reinterpret_cast<const float4 *>(sm + SL::BT + t * 8 + 4);
 #pragma unroll
 			for (int i = 0; i < kChunk; ++i) { // (both matrices are lower triangular, zeros included)
-				const float ri = __shfl_sync(kFull, r, i * 4 + c);
+				const float ri = __shfl_sync(kFull, r, i * 4 + c * (4 / NC));
 				if (i <= t) u = fmaf(Tr[i], ri, u), y = fmaf(Br[i], ri, y);
 			}
-			u_sm[warp][t][c] = make_float2(u, u);
+			u_sm[warp][t][c] = make_float2(u, u); // (NC 2: two lanes, the same)
 			const int pos = ch * kChunk + t;
-			if (pos < a.n) a.out[(size_t)pos * a.ldo + (size_t)h * a.P + cw + c] = dead ? __int_as_float(0x7fc00000) : fmaf(skip, v, y);
+			if (pos < a.n && (NC == 4 || !(lane & 1))) a.out[(size_t)pos * a.ldo + (size_t)h * a.P + cw + c] = dead ? __int_as_float(0x7fc00000) : fmaf(skip, v, y);
 			__syncwarp();
 			{
 				f32x2 b[NP];
 				load_pairs<NP>(b, sm + SL::B8 + e0);
 #pragma unroll
-				for (int j = 0; j < 4; ++j)
+				for (int j = 0; j < NC; ++j)
 #pragma unroll
 					for (int p = 0; p < NP; ++p) s[j][p] = mul2(s[j][p], b[p]);
 #pragma unroll
 				for (int i = 0; i < kChunk; ++i) {
-					f32x2 x[NP], ua[2], ub[2];
+					f32x2 x[NP], u2[NC];
 					load_pairs<NP>(x, sm + SL::U + i * D + e0);
-					load_pairs<2>(ua, &u_sm[warp][i][0].x), load_pairs<2>(ub, &u_sm[warp][i][2].x);
 #pragma unroll
-					for (int p = 0; p < NP; ++p) {
-						s[0][p] = fma2(x[p], ua[0], s[0][p]), s[1][p] = fma2(x[p], ua[1], s[1][p]);
-						s[2][p] = fma2(x[p], ub[0], s[2][p]), s[3][p] = fma2(x[p], ub[1], s[3][p]);
+					for (int j = 0; j < NC; j += 2) {
+						f32x2 two[2];
+						load_pairs<2>(two, &u_sm[warp][i][j].x);
+						u2[j] = two[0], u2[j + 1] = two[1];
 					}
+#pragma unroll
+					for (int p = 0; p < NP; ++p)
+#pragma unroll
+						for (int j = 0; j < NC; ++j) s[j][p] = fma2(x[p], u2[j], s[j][p]);
 				}
 			}
 			__syncwarp();
@@ -308,10 +318,11 @@ __global__ void __launch_bounds__(kChunkThreads, 1) chunk_scan_kernel(const Scan
 		}
 #pragma unroll
 		for (int j = 0; j < 4; ++j) {
+			if (j >= NC) break;
 			if (dead)
 #pragma unroll
-				for (int p = 0; p < NP; ++p) s[j][p] = pk(__int_as_float(0x7fc00000), __int_as_float(0x7fc00000));
-			store_pairs<NP>(state + (size_t)j * D, s[j]);
+				for (int p = 0; p < NP; ++p) s[j % NC][p] = pk(__int_as_float(0x7fc00000), __int_as_float(0x7fc00000));
+			store_pairs<NP>(state + (size_t)j * D, s[j % NC]);
 		}
 	}
 }

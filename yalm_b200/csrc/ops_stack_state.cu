@@ -726,15 +726,21 @@ static int launch_scan(const ScanArgs &a, dim3 grid, cudaStream_t st) {
 // From a full chunk of 8 positions on (16 heads of 128 x 128, delta rule: 16 rows 8.4 -> 7.0 us, 64 rows 21 -> 12 us; 64 x 64 the same as step by
 // step at 16 rows, 16 -> 10 us at 64; below 8 rows most of a chunk would be padding).
 constexpr int kChunkRows = 8;
-template <int D, bool DELTA, bool PER_CHANNEL>
+template <int D, int NC, bool DELTA, bool PER_CHANNEL>
 static int launch_chunks_of(const ScanArgs &a, cudaStream_t st) {
 	constexpr int smem = kChunkSlots * ChunkSlot<D>::SIZE * (int)sizeof(float);
-	YALM_TRY(allow_smem((const void *)chunk_scan_kernel<D, DELTA, PER_CHANNEL>, smem));
-	return launch_chained(chunk_scan_kernel<D, DELTA, PER_CHANNEL>, dim3((a.P + kChunkCols - 1) / kChunkCols, a.H), dim3(kChunkThreads), smem, st, 1, a);
+	YALM_TRY(allow_smem((const void *)chunk_scan_kernel<D, NC, DELTA, PER_CHANNEL>, smem));
+	return launch_chained(chunk_scan_kernel<D, NC, DELTA, PER_CHANNEL>, dim3((a.P + 4 * NC - 1) / (4 * NC), a.H), dim3(kChunkThreads), smem, st, 1, a);
+}
+// Two columns a warp while their CTAs all run at once, one per SM (512 rows, 8 heads of 128 x 128: 44 us for 57; 16 heads of 64 x 64: 34 for
+// 44): what the columns share is then prepared twice as often, on SMs that would be idle.
+template <int D, bool DELTA, bool PER_CHANNEL>
+static int launch_chunks_sized(const ScanArgs &a, cudaStream_t st) {
+	return (a.P + 7) / 8 * a.H <= device_info().sms ? launch_chunks_of<D, 2, DELTA, PER_CHANNEL>(a, st) : launch_chunks_of<D, 4, DELTA, PER_CHANNEL>(a, st);
 }
 template <bool DELTA, bool PER_CHANNEL>
 static int launch_chunks(const ScanArgs &a, cudaStream_t st) {
-	return a.D == 64 ? launch_chunks_of<64, DELTA, PER_CHANNEL>(a, st) : launch_chunks_of<128, DELTA, PER_CHANNEL>(a, st);
+	return a.D == 64 ? launch_chunks_sized<64, DELTA, PER_CHANNEL>(a, st) : launch_chunks_sized<128, DELTA, PER_CHANNEL>(a, st);
 }
 
 
