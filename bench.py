@@ -545,7 +545,8 @@ def main():
         tok_s = K / (dev_ms * 1e-3)
         if mega:
             # one persistent kernel per token IS the step: algorithmic bytes = weights + KV rows it reads
-            kname = "decode_mega_kernel (whole token: all GEMVs + flash-decode + LM head, TMA ring)"
+            one = model.mega_info()["vec_floats"] == 0  # (its input vectors live in registers)
+            kname = f"{'decode_token_kernel' if one else 'decode_mega_kernel'} (whole token: all GEMVs + flash-decode + LM head, TMA ring)"
             ffn_bytes = (wbytes + yf.kv_bytes_per_token(arch, min(context, pos - K // 2))) / world   # this rank's shard
             if world > 1:
                 kname += f", tp{world}: all-reduce fused into the wo/w2 epilogues over NVLink peer memory"

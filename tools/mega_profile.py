@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Phase profile of the whole-token decode kernel (decode_mega.cuh): where a token's time goes per phase —
+"""Phase profile of the whole-token decode kernel (decode_token.cuh, decode_mega.cuh): where a token's time goes per phase —
 grid-barrier wait, input staging, tile loop, and how much of the tile loop the consumers spent starved for
 ring stages (= HBM-bound) — from the kernel's own clock64 stamps.  Usage:
     python tools/mega_profile.py [--workload mistral-7b-fp16-4k] [--layers N] [--pos P] [--out file]"""
@@ -55,7 +55,8 @@ def main():
         lines.append(f"{PH[ph]:12s} {bar.mean():9.2f} {stg.mean():8.2f} {til.mean():8.2f}   "
                      f"[{bar.max(0).mean():.2f} {stg.max(0).mean():.2f} {til.max(0).mean():.2f}] x{nl}")
         tot += np.array([bar.mean() * nl, stg.mean() * nl, til.mean() * nl, stv.mean() * nl])
-    q = p[:, :, 1, :]
+    q = p[:, :, 1, :].copy()
+    q[..., 6] = np.where(q[..., 6] > 0, q[..., 6], q[..., 7])  # (decode_token.cuh: the partial sums are flagged words, nothing follows their stores)
     ok = q[..., 5] > 0
     un = np.where(ok, (q[..., 5] - q[..., 2]) * us, np.nan)
     mp = np.where(ok, (q[..., 6] - q[..., 5]) * us, np.nan)
