@@ -1,5 +1,6 @@
 """-m gpu: the whole-token kernel of dense models on one GPU (csrc/decode_token.cuh) at the edges of its geometry - rows of one 512-byte chunk to four
-pieces, ragged last chunks, several rows a stage, stages that q, k and v share, fewer rows than CTAs, contexts shorter and longer than the CTAs of a head - against the oracle's tokens and logits."""
+pieces, ragged last chunks, several rows a stage, stages that q, k and v share, one row of x for most CTAs, contexts shorter and longer than the CTAs of a head - against the
+oracle's tokens and logits; and on either side of its limits, which kernel runs."""
 import numpy as np
 import pytest
 
@@ -12,6 +13,11 @@ pytestmark = pytest.mark.gpu
 
 def arch(dim, hidden, hd, heads, kv, vocab=600, layers=2, seq=256, **kw):
     return yf.Arch(dim, hidden, hd, layers, heads, kv, vocab, seq, 10000.0, name="token", **kw)
+
+
+def runs_here(m):
+    """Whether a token of this model is decode_token_kernel: it keeps no input vector in shared memory."""
+    return m.uses_megakernel() and m.mega_info()["vec_floats"] == 0
 
 
 CASES = {
@@ -27,8 +33,10 @@ CASES = {
     "fp32": (arch(2048, 8192, 128, 8, 2, vocab=100, layers=1), "fp32"),
     # fp8: rows of 2 chunks with scales, hidden 19 chunks in two pieces
     "fp8": (arch(1024, 9728, 64, 16, 4), "fp8"),
-    # fewer rows than CTAs in every phase
-    "fp16-few-rows": (arch(64, 96, 32, 2, 1, vocab=50), "fp16"),
+    # a row or two of x and none of hidden or of the vocabulary for some CTAs
+    "fp16-few-rows": (arch(160, 96, 32, 2, 1, vocab=50), "fp16"),
+    # the longest normed rows
+    "fp16-longest-normed": (arch(8192, 512, 128, 16, 2, layers=1, vocab=200), "fp16"),
 }
 
 
@@ -40,7 +48,7 @@ def test_tokens_and_logits(oracle, case):
     ref = bytes(yf.dequantized_fp32_image(img)) if dt == "fp8" else img
     to, lo = oracle.OracleModel(ref).generate(prompt, n, keep_logits=True)
     m = api.Model(img).cuda()
-    assert m.uses_megakernel() and m.mega_info()["stages"] == 24 and not m.mega_info()["w2_pipe"]
+    assert runs_here(m)
     s = api.InferenceState(m)
     tg, lg = s.generate(prompt, n, keep_logits=True)
     assert np.abs(lg - lo).max() < LOGIT_TOL and tg == to
@@ -59,6 +67,7 @@ def test_contexts_around_the_units_of_attention(oracle, context):
     ids = [(37 * i + 1) % 300 for i in range(context)]
     to, lo = oracle.OracleModel(img).generate(ids, 3, keep_logits=True)
     m = api.Model(img).cuda()
+    assert runs_here(m)
     s = api.InferenceState(m)
     tg, lg = s.generate(ids, 3, keep_logits=True)
     assert np.abs(lg - lo).max() < LOGIT_TOL and tg == to
@@ -66,14 +75,17 @@ def test_contexts_around_the_units_of_attention(oracle, context):
     m.close()
 
 
-def test_rows_beyond_it_stay_with_the_other_kernel(oracle):
-    """A hidden size of five pieces."""
-    a = arch(512, 20480, 64, 8, 2, layers=1, vocab=100)
+@pytest.mark.parametrize("dim,hidden,layers", [(512, 20480, 1), (512, 16640, 1), (8448, 512, 1), (64, 96, 2)])
+def test_rows_beyond_it_stay_with_the_other_kernel(oracle, dim, hidden, layers):
+    """A hidden size of five pieces, and the least that is one; a normed row past the longest; fewer rows of x than CTAs."""
+    heads, hd = (2, 32) if dim < 512 else (8, 64)
+    a = arch(dim, hidden, hd, heads, heads // 4 or 1, layers=layers, vocab=100)
     img = bytes(yf.random_model(a, "fp16", seed=7))
     to, lo = oracle.OracleModel(img).generate([1, 2, 3], 4, keep_logits=True)
     m = api.Model(img).cuda()
+    assert m.uses_megakernel() and not runs_here(m)
     s = api.InferenceState(m)
     tg, lg = s.generate([1, 2, 3], 4, keep_logits=True)
-    assert m.uses_megakernel() and np.abs(lg - lo).max() < LOGIT_TOL and tg == to
+    assert np.abs(lg - lo).max() < LOGIT_TOL and tg == to
     s.close()
     m.close()

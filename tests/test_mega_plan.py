@@ -148,3 +148,49 @@ def test_pipelined_hb_shares_add_up_to_the_slices(name, dt, tp):
             total = sum(api.lib().yalm_mega_hb_share(groups, rh, kt, grid, cta, rot, s) for cta in range(grid))
             assert total == kt, (rot, s, total)
     assert api.lib().yalm_mega_hb_share(groups, rh, kt, grid, grid, 0, 0) < 0
+
+
+# ---- the kernel of decode_token.cuh: reuse of the hand-over buffers -----------------------------------------------------------
+def overtaken(dim, q_dim, kv_dim, hidden, n_kv, nch, grid, layers=3):
+    """Whether a CTA may store the words of a phase while another still waits for those of the same phase a layer before.  seen[c][r]: the last
+    phase whose inputs r is known to have read when c stores its own words; c learns it from the words that it reads (attention's are left out)."""
+    def owns(items):
+        return np.array([(c + 1) * items // grid > c * items // grid for c in range(grid)])
+    split, out = [], (C.c_int * 5)()
+    for c in range(grid):
+        assert api.lib().yalm_mega_attn_split(c, grid, n_kv, nch, out) == 0
+        split.append(out[:])
+    per_head = q_dim // n_kv
+    joins = np.array([(c - c0 + 1) * per_head // nc > (c - c0) * per_head // nc for c, (_, c0, nc, _, _) in enumerate(split)])
+    partial = np.array([nu > 0 for *_, nu in split])
+    stores = [owns((q_dim + 2 * kv_dim) // 2), joins | partial, owns(dim), owns(hidden), owns(dim)]   # q k v, attention, wo, w1 / w3, w2
+    sources = [stores[4], None, joins, stores[2], stores[3]]
+    seen = -np.ones((grid, grid), int)
+    for ph in range(5 * layers):
+        k = ph % 5
+        if ph > 0 and k != 1:
+            seen = np.maximum(seen, seen[sources[k]].max(0))
+        seen[np.arange(grid), np.arange(grid)] = ph
+        if ph >= 5 and (seen[stores[k]] < ph - 4).any():     # stored in ph - 5, read in ph - 4
+            return True
+    return False
+
+
+@pytest.mark.parametrize("dim,heads,kv,hd,hidden", [(64, 2, 1, 32, 96), (152, 8, 2, 32, 640), (160, 8, 2, 32, 96), (256, 8, 2, 32, 512), (4096, 32, 8, 128, 14336)])
+def test_hand_over_words_are_read_before_they_are_stored_again(dim, heads, kv, hd, hidden):
+    grid = 148
+    taken = api.lib().yalm_mega_token_plan(api.F16, dim, heads * hd, hidden, grid, (C.c_int * 9)()) == 0
+    lost = [overtaken(dim, heads * hd, kv * hd, hidden, kv, nch, grid) for nch in (1, 40)]
+    assert lost == [dim < grid] * 2 and taken == (dim >= grid)
+
+
+def test_token_kernel_limits():
+    def plan(dtype, dim, q_dim, hidden, grid=148):
+        return api.lib().yalm_mega_token_plan(dtype, dim, q_dim, hidden, grid, (C.c_int * 9)()) == 0
+    for dtype in (api.F32, api.F16, api.F8E4M3):
+        assert plan(dtype, 512, 512, 16384) and not plan(dtype, 512, 512, 16400)                  # a lane's part of a vector
+        assert plan(dtype, 512, 16384, 512) and not plan(dtype, 512, 16400, 512)
+        assert plan(dtype, 8192, 512, 512) and not plan(dtype, 8208, 512, 512)                    # ... of a normed one
+        assert plan(dtype, 1024, 512, 512, grid=8) and not plan(dtype, 1040, 512, 512, grid=8)    # 128 rows of x per CTA
+        assert plan(dtype, 160, 512, 512) and not plan(dtype, 144, 512, 512)                      # a row of wo and w2 for every CTA
+    assert api.lib().yalm_mega_token_plan(api.F16, 4096, 4096, 14336, 148, None) != 0

@@ -166,19 +166,24 @@ static bool plan_shapes(int dtype, int dim, int q_dim, int kv_dim, int hidden, i
 	return true;
 }
 
-// The kernel of decode_token.cuh for a dense model on one GPU, where its rows fit: pieces of 16 chunks of 512 bytes, a lane's part of a vector in
-// registers (64 floats: 16384 elements; wider rows spill there, and stay with the kernels of decode_mega.cuh), a CTA's rows of x in shared memory.
-static bool plan_token(Plan &p, int dtype, int dim, int q_dim, int hidden, int head_dim, int G, int max_smem) {
+// Geometry of the kernel of decode_token.cuh, for a dense model on one GPU; false where it does not serve: rows longer than pieces of 16 chunks of 512 bytes
+// with a lane's part of a vector in registers (64 floats: 16384 elements; wider rows spill there, and stay with the kernels of decode_mega.cuh), more
+// rows of x than a CTA keeps in shared memory - or fewer rows than CTAs: every CTA has to own a row of wo and of w2, because nobody would
+// wait for one that does not, and its inputs could be overwritten before it has read them.
+static bool token_geometry(int dtype, int dim, int q_dim, int hidden, int grid, int (*geo)[3]) {
 	const int B = bytes_of(dtype), ep = ep_of(dtype), n[3] = {dim, q_dim, hidden};
 	int floats[3];
 	for (int i = 0; i < 3; ++i) {
 		const int chunks = (n[i] * B + token::kChunk - 1) / token::kChunk, np = (chunks + 15) / 16, piece = (chunks + np - 1) / np;
 		const bool sides = np == 1 && piece <= kTokenWarps;
-		p.token_geo[i][0] = np, p.token_geo[i][1] = piece, p.token_geo[i][2] = sides ? kTokenWarps / piece * 2 : 1;
+		geo[i][0] = np, geo[i][1] = piece, geo[i][2] = sides ? kTokenWarps / piece * 2 : 1;
 		floats[i] = sides ? ep : np * 2 * ep;
 	}
 	const int most = std::max(floats[0], std::max(floats[1], floats[2]));
-	if (most > token::kFloats || floats[0] > kTokenNormFloats || (dim + p.grid - 1) / p.grid > kTokenMaxRows) return false;
+	return most <= token::kFloats && floats[0] <= kTokenNormFloats && (dim + grid - 1) / grid <= kTokenMaxRows && dim >= grid;
+}
+static bool plan_token(Plan &p, int dtype, int dim, int q_dim, int hidden, int head_dim, int G, int max_smem) {
+	if (!token_geometry(dtype, dim, q_dim, hidden, p.grid, p.token_geo)) return false;
 	const void *kernel = dtype == YALM_F32   ? kernel_f32_token(head_dim, G)
 	                     : dtype == YALM_F16 ? kernel_f16_token(head_dim, G)
 	                                         : kernel_f8_token(head_dim, G);
@@ -325,6 +330,10 @@ extern "C" int yalm_mega_tile_plan(int dtype, int dim, int q_dim, int kv_dim, in
 	for (int k = 0; k < 5; ++k)
 		for (int j = 0; j < 4; ++j) out20[4 * k + j] = shape[k][j];
 	return 0;
+}
+extern "C" int yalm_mega_token_plan(int dtype, int dim, int q_dim, int hidden, int grid, int *out9) {
+	if (!out9 || dim < 1 || q_dim < 1 || hidden < 1 || grid < 1 || !yalm::mega::ep_of(dtype)) return YALM_EINVAL;
+	return yalm::mega::token_geometry(dtype, dim, q_dim, hidden, grid, reinterpret_cast<int (*)[3]>(out9)) ? 0 : YALM_EINVAL;
 }
 extern "C" int yalm_mega_mma_plan(int rows, int unit, int cap, int grid, int cta, int *out4) {
 	if (!out4 || rows < 1 || unit < 1 || cap < unit || rows % unit || grid < 1 || cta < 0 || cta >= grid) return YALM_EINVAL;

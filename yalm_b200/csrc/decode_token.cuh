@@ -12,8 +12,9 @@
 //   * Attention.  A task is up to four query heads of one KV head over half a stage (8 positions of 128 channels).  q and the appended key and value
 //     travel as flagged words too, so no grid barrier stands before it (but for a ring that has wrapped, whose sink keys are rotated in place).  The CTAs'
 //     partial sums are flagged words; every CTA of the head joins its slice of the outputs.
-// Each phase's input needs every CTA's output of the phase before (attention: of its head, and wo then of all heads), so no CTA is ever two phases
-// ahead of another, which is what makes the reuse of the hand-over buffers safe.
+// The hand-over buffers are used again a layer later.  That is safe because every CTA owns a row of wo and of w2 (token_geometry() sees to it) and
+// stores it when all its warps have read that phase's input, and those of the phases before; the next phase's input needs every such row.  So whoever stores into a buffer a second
+// time has waited for every CTA's row of a product that comes after its reading of the first.
 //
 // Bound by HBM inside the phases (w1 / w3 235 MB in 35 us) and by the hand-overs between them.  A layer of 4096 / 14336 at 4096 positions, us, here and with
 // decode_mega.cuh: q k v 9.7 / 11, attention 8.7 / 13, wo 6.4 / 9, w1 w3 37.9 / 37, w2 21.7 / 24: 85 / 94; four layers and the head, a call on the host 461 -> 436;
