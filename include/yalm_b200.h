@@ -569,8 +569,9 @@ int yalm_mega_tile_plan(int dtype, int dim, int q_dim, int kv_dim, int hidden, i
 int yalm_mega_mma_plan(int rows, int unit, int cap, int grid, int cta, int *out4);
 int yalm_mega_hb_share(int groups, int rows_per_group, int slice_elems, int grid, int cta, int rotation, int slice);
 /* Geometry of the whole-token kernel of dense models on one GPU (decode_token.cuh): out9 = {pieces of a row, 512-byte chunks of a
- * piece, rows of a stage} of rows of dim, q_dim and hidden columns; YALM_EINVAL where that kernel does not serve on `grid` CTAs. */
-int yalm_mega_token_plan(int dtype, int dim, int q_dim, int hidden, int grid, int *out9);
+ * piece, rows of a stage} of rows of dim, q_dim and hidden columns; YALM_EINVAL where that kernel does not serve on `grid` CTAs
+ * or decode_mega.cuh is faster. */
+int yalm_mega_token_plan(int dtype, int dim, int q_dim, int hidden, int head_dim, int grid, int *out9);
 int yalm_mega_attn_split(int cta, int ncta, int n_kv_heads, int n_chunks, int *out5);
 
 /* The CLI's tokenizer (greedy longest-prefix match + byte fallback, src/tokenizer.cpp:57-94; decode_one :44-55) over an

@@ -176,21 +176,26 @@ def overtaken(dim, q_dim, kv_dim, hidden, n_kv, nch, grid, layers=3):
     return False
 
 
-@pytest.mark.parametrize("dim,heads,kv,hd,hidden", [(64, 2, 1, 32, 96), (152, 8, 2, 32, 640), (160, 8, 2, 32, 96), (256, 8, 2, 32, 512), (4096, 32, 8, 128, 14336)])
+@pytest.mark.parametrize("dim,heads,kv,hd,hidden", [(64, 2, 1, 64, 96), (152, 4, 1, 64, 640), (160, 4, 1, 64, 96), (512, 8, 2, 32, 512), (4096, 32, 8, 128, 14336)])
 def test_hand_over_words_are_read_before_they_are_stored_again(dim, heads, kv, hd, hidden):
     grid = 148
-    taken = api.lib().yalm_mega_token_plan(api.F16, dim, heads * hd, hidden, grid, (C.c_int * 9)()) == 0
+    taken = api.lib().yalm_mega_token_plan(api.F16, dim, heads * hd, hidden, hd, grid, (C.c_int * 9)()) == 0
     lost = [overtaken(dim, heads * hd, kv * hd, hidden, kv, nch, grid) for nch in (1, 40)]
     assert lost == [dim < grid] * 2 and taken == (dim >= grid)
 
 
 def test_token_kernel_limits():
-    def plan(dtype, dim, q_dim, hidden, grid=148):
-        return api.lib().yalm_mega_token_plan(dtype, dim, q_dim, hidden, grid, (C.c_int * 9)()) == 0
-    for dtype in (api.F32, api.F16, api.F8E4M3):
-        assert plan(dtype, 512, 512, 16384) and not plan(dtype, 512, 512, 16400)                  # a lane's part of a vector
-        assert plan(dtype, 512, 16384, 512) and not plan(dtype, 512, 16400, 512)
-        assert plan(dtype, 8192, 512, 512) and not plan(dtype, 8208, 512, 512)                    # ... of a normed one
+    def plan(dtype, dim, q_dim, hidden, head_dim=128, grid=148):
+        return api.lib().yalm_mega_token_plan(dtype, dim, q_dim, hidden, head_dim, grid, (C.c_int * 9)()) == 0
+    for dtype, piece in [(api.F32, 2048), (api.F16, 4096), (api.F8E4M3, 8192)]:
+        assert plan(dtype, 1024, 1024, 16384) and not plan(dtype, 1024, 1024, 16400)              # a lane's part of a vector
+        assert plan(dtype, 1024, piece, 512) and not plan(dtype, 1024, piece + 16, 512)           # rows of one piece
         assert plan(dtype, 1024, 512, 512, grid=8) and not plan(dtype, 1040, 512, 512, grid=8)    # 128 rows of x per CTA
-        assert plan(dtype, 160, 512, 512) and not plan(dtype, 144, 512, 512)                      # a row of wo and w2 for every CTA
-    assert api.lib().yalm_mega_token_plan(api.F16, 4096, 4096, 14336, 148, None) != 0
+    assert plan(api.F32, 2048, 512, 512) and not plan(api.F32, 2064, 512, 512)
+    assert plan(api.F16, 4096, 512, 512) and not plan(api.F16, 4112, 512, 512)
+    assert plan(api.F8E4M3, 4096, 512, 512) and not plan(api.F8E4M3, 4112, 512, 512)              # fp8: 2 (heads of 128) or 3 to 8 chunks
+    assert plan(api.F8E4M3, 528, 512, 512) and not plan(api.F8E4M3, 512, 512, 512)
+    assert plan(api.F8E4M3, 1040, 512, 512, 64) and not plan(api.F8E4M3, 1024, 512, 512, 64)
+    assert plan(api.F16, 256, 512, 512, 64) and plan(api.F16, 264, 512, 512, 32) and not plan(api.F16, 256, 512, 512, 32)
+    assert plan(api.F32, 160, 512, 512, 32) and not plan(api.F32, 144, 512, 512, 32)              # a row of wo and w2 for every CTA
+    assert api.lib().yalm_mega_token_plan(api.F16, 4096, 4096, 14336, 128, 148, None) != 0

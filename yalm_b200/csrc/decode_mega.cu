@@ -166,24 +166,30 @@ static bool plan_shapes(int dtype, int dim, int q_dim, int kv_dim, int hidden, i
 	return true;
 }
 
-// Geometry of the kernel of decode_token.cuh, for a dense model on one GPU; false where it does not serve: rows longer than pieces of 16 chunks of 512 bytes
-// with a lane's part of a vector in registers (64 floats: 16384 elements; wider rows spill there, and stay with the kernels of decode_mega.cuh), more
-// rows of x than a CTA keeps in shared memory - or fewer rows than CTAs: every CTA has to own a row of wo and of w2, because nobody would
-// wait for one that does not, and its inputs could be overwritten before it has read them.
-static bool token_geometry(int dtype, int dim, int q_dim, int hidden, int grid, int (*geo)[3]) {
+// Geometry of the kernel of decode_token.cuh, for a dense model on one GPU; false where it cannot serve: a lane's part of a vector in
+// registers (64 floats: 16384 elements; wider rows spill there), the rows of x that a CTA keeps in shared memory - or fewer rows than CTAs: every CTA has
+// to own a row of wo and of w2, because nobody would wait for one that does not, and its inputs could be overwritten before it has read them.
+// And false where the kernels of decode_mega.cuh are faster (a token of 3 layers, this kernel / that one, us, 600 positions):
+//   rows of dim or q_dim of more than one piece (16 chunks of 512 bytes) are multiplied a row at a time: fp16 5120 / 10240 598 / 366, 8192 / 16384 900 / 655; fp32
+//     4096 / 14336 611 / 510, 2560 / 5120 313 / 237; where they are one piece fp16 4096 / 14336 266 / 302 and fp32 2048 / 7168 150 / 196;
+//   fp8, two instructions an element: rows of 9 to 16 chunks, of which a warp has one or two, 5120 / 10240 314 / 272, against 4096 / 14336 224 / 232;
+//     rows so short that the sums of 16 or 8 of them a stage take the time, 512 / 1024 127 / 95, 768 / 1536 98 / 95, against 1536 / 3072 96 / 101 and, as
+//     the attention over heads of 128 gains on its own, 1024 / 3584 105 / 119;
+//   fp16 rows of one chunk with heads of 32: 256 / 512 87 / 78 (heads of 64: 91 / 99).
+static bool token_geometry(int dtype, int dim, int q_dim, int hidden, int head_dim, int grid, int (*geo)[3]) {
 	const int B = bytes_of(dtype), ep = ep_of(dtype), n[3] = {dim, q_dim, hidden};
-	int floats[3];
 	for (int i = 0; i < 3; ++i) {
 		const int chunks = (n[i] * B + token::kChunk - 1) / token::kChunk, np = (chunks + 15) / 16, piece = (chunks + np - 1) / np;
-		const bool sides = np == 1 && piece <= kTokenWarps;
-		geo[i][0] = np, geo[i][1] = piece, geo[i][2] = sides ? kTokenWarps / piece * 2 : 1;
-		floats[i] = sides ? ep : np * 2 * ep;
+		geo[i][0] = np, geo[i][1] = piece, geo[i][2] = np == 1 && piece <= kTokenWarps ? kTokenWarps / piece * 2 : 1;
 	}
-	const int most = std::max(floats[0], std::max(floats[1], floats[2]));
-	return most <= token::kFloats && floats[0] <= kTokenNormFloats && (dim + grid - 1) / grid <= kTokenMaxRows && dim >= grid;
+	if (geo[2][0] * 2 * ep > token::kFloats || (dim + grid - 1) / grid > kTokenMaxRows || dim < grid) return false;
+	if (geo[0][0] > 1 || geo[1][0] > 1) return false;
+	const int chunks = geo[0][1];
+	if (dtype == YALM_F8E4M3) return chunks <= kTokenWarps && chunks >= (head_dim >= 128 ? 2 : 3);
+	return dtype == YALM_F32 || chunks > 1 || head_dim >= 64;
 }
 static bool plan_token(Plan &p, int dtype, int dim, int q_dim, int hidden, int head_dim, int G, int max_smem) {
-	if (!token_geometry(dtype, dim, q_dim, hidden, p.grid, p.token_geo)) return false;
+	if (!token_geometry(dtype, dim, q_dim, hidden, head_dim, p.grid, p.token_geo)) return false;
 	const void *kernel = dtype == YALM_F32   ? kernel_f32_token(head_dim, G)
 	                     : dtype == YALM_F16 ? kernel_f16_token(head_dim, G)
 	                                         : kernel_f8_token(head_dim, G);
@@ -331,9 +337,9 @@ extern "C" int yalm_mega_tile_plan(int dtype, int dim, int q_dim, int kv_dim, in
 		for (int j = 0; j < 4; ++j) out20[4 * k + j] = shape[k][j];
 	return 0;
 }
-extern "C" int yalm_mega_token_plan(int dtype, int dim, int q_dim, int hidden, int grid, int *out9) {
-	if (!out9 || dim < 1 || q_dim < 1 || hidden < 1 || grid < 1 || !yalm::mega::ep_of(dtype)) return YALM_EINVAL;
-	return yalm::mega::token_geometry(dtype, dim, q_dim, hidden, grid, reinterpret_cast<int (*)[3]>(out9)) ? 0 : YALM_EINVAL;
+extern "C" int yalm_mega_token_plan(int dtype, int dim, int q_dim, int hidden, int head_dim, int grid, int *out9) {
+	if (!out9 || dim < 1 || q_dim < 1 || hidden < 1 || head_dim < 1 || grid < 1 || !yalm::mega::ep_of(dtype)) return YALM_EINVAL;
+	return yalm::mega::token_geometry(dtype, dim, q_dim, hidden, head_dim, grid, reinterpret_cast<int (*)[3]>(out9)) ? 0 : YALM_EINVAL;
 }
 extern "C" int yalm_mega_mma_plan(int rows, int unit, int cap, int grid, int cta, int *out4) {
 	if (!out4 || rows < 1 || unit < 1 || cap < unit || rows % unit || grid < 1 || cta < 0 || cta >= grid) return YALM_EINVAL;

@@ -568,7 +568,6 @@ __global__ void __launch_bounds__(kTokenThreads, 1) decode_token_kernel(const __
 		// ---- a product: the warp's part of the input vector ----
 		const Geo ge = geo_of(k == 2 ? 1 : k == 4 ? 2 : 0);
 		const int n_in = k == 2 ? a.q_dim : k == 4 ? a.hidden : a.dim;
-		const bool norm = k == 0 || k == 3 || k == 5;
 		int lo, n; // this CTA's rows (pairs of rows of w1 and w3)
 		if (k == 0) share((a.q_dim + 2 * a.kv_dim) / 2, lo, n), lo *= 2, n *= 2;
 		else share(k == 3 ? a.hidden : k == 5 ? a.vocab : a.dim, lo, n);
@@ -576,6 +575,7 @@ __global__ void __launch_bounds__(kTokenThreads, 1) decode_token_kernel(const __
 		auto product = [&](auto sides, auto slots) {
 		constexpr bool SIDES = decltype(sides)::value;
 		constexpr int SL = decltype(slots)::value;
+		const bool norm = SL <= 2 && (k == 0 || k == 3 || k == 5); // (normed rows are one piece: plan_token())
 		const int CW = SIDES ? ge.piece : kW, RG = SIDES ? ge.RS / 2 : 1; // warps that share a row; rows side by side
 		const int c = SIDES ? warp % ge.piece : warp, rg = SIDES ? warp / ge.piece : 0;
 		auto at_of = [&](int q) { return ((q >> 1) * ge.piece + (q & 1) * kW + c) * CH + lane * EP; }; // first element of this lane in slot q
@@ -585,7 +585,6 @@ __global__ void __launch_bounds__(kTokenThreads, 1) decode_token_kernel(const __
 			if (rg < RG && (SIDES || ((q >> 1) < ge.np && (q & 1) * kW + c < ge.piece)) && at_of(q) < n_in) have |= 1u << q;
 		float4 x[SL][Q];
 		{
-			constexpr int NV = SL < kTokenNormFloats / EP ? SL : kTokenNormFloats / EP; // slots of a normed vector (plan() sees to it)
 #pragma unroll
 			for (int p = 0; p < SL; ++p)
 #pragma unroll
@@ -627,7 +626,7 @@ __global__ void __launch_bounds__(kTokenThreads, 1) decode_token_kernel(const __
 			if (norm) { // o = x * (1 / sqrt(mean + eps)) * w (src/infer.cpp:134-144): the scale waits for the sums, the weights come ahead of the rows
 				float ss = 0.f;
 #pragma unroll
-				for (int p = 0; p < NV; ++p)
+				for (int p = 0; p < SL; ++p)
 #pragma unroll
 					for (int j = 0; j < Q; ++j) ss += x[p][j].x * x[p][j].x + x[p][j].y * x[p][j].y + x[p][j].z * x[p][j].z + x[p][j].w * x[p][j].w;
 				ss = warp_sum(rg == 0 ? ss : 0.f);
@@ -635,7 +634,7 @@ __global__ void __launch_bounds__(kTokenThreads, 1) decode_token_kernel(const __
 				for (int t = 0; t * kStageBytes < n_in * 4; ++t) {
 					landed(1);
 #pragma unroll
-					for (int p = 0; p < NV; ++p) {
+					for (int p = 0; p < SL; ++p) {
 						const int at = at_of(p) * 4 - t * kStageBytes;
 						if ((have >> p & 1u) && at >= 0 && at < kStageBytes)
 #pragma unroll
@@ -806,7 +805,7 @@ __global__ void __launch_bounds__(kTokenThreads, 1) decode_token_kernel(const __
 		};
 		if (ge.RS > 1) product(std::true_type(), std::integral_constant<int, 1>());
 		else if (ge.np == 1) product(std::false_type(), std::integral_constant<int, 2>());
-		else product(std::false_type(), std::integral_constant<int, kFloats / EP>());
+		else product(std::false_type(), std::integral_constant<int, kFloats / EP>()); // w2 only
 	}
 
 	if (a.mode == kGreedy) { // greedy arg-max, first maximum wins (src/sampler.cpp:27-38): lanes -> warps -> CTA -> grid

@@ -46,8 +46,8 @@ constexpr int kFlagPhaseBits = 12;  // hand-over flag = launch number << kFlagPh
 constexpr int kLLRep = YALM_MEGA_LL_REP; // copies of every flagged hand-over vector (decode_mega.cuh); 1, 2 or 4
 constexpr int kProfileSlots = 6 * 8; // per (CTA, layer): phases x slots, see decode_mega.cuh
 
-// The kernel of dense models on one GPU (decode_token.cuh): consumer warps, ring stages, rows of x that a CTA keeps, floats of a normed vector a lane holds
-constexpr int kTokenWarps = 8, kTokenStages = 24, kTokenMaxRows = 128, kTokenNormFloats = 32;
+// The kernel of dense models on one GPU (decode_token.cuh): consumer warps, ring stages, rows of x that a CTA keeps
+constexpr int kTokenWarps = 8, kTokenStages = 24, kTokenMaxRows = 128;
 
 // ---- tensor parallelism inside the kernel (N GPUs of one NVSwitch domain) ---------------------------------------------
 // Every rank owns one region of device memory that all peers map (CUDA IPC, tp.cpp).  The row -> CTA -> warp map of a
