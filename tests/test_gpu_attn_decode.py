@@ -99,3 +99,21 @@ def test_captured_calls_replay():
         got = [o.clone() for o in outs] + [copy.clone()]
         calls()
         assert all(torch.equal(a, b) for a, b in zip(got, outs + [copy])) and got[3].isfinite().all()
+
+
+@pytest.mark.parametrize("heads,kv_heads,hd", [(5, 5, 7), (3, 1, 20), (6, 2, 48), (9, 3, 64), (9, 3, 72), (12, 4, 128), (3, 1, 136)])
+def test_generic_shapes(heads, kv_heads, hd):
+    """Pieces of 64 values of a key and 16 rows of values, their remainders, and rows that are not 16-byte aligned.  fp32 sums of hd and kv_len terms of about 1,
+    exponentials of scores of about 1: 2e-6 of the norm (measured 3e-7)."""
+    L, T = api.lib(), 304
+    for kv_len in (1, 15, 16, 17, 256, 257, 300):
+        for off in (0, 1):
+            torch.manual_seed(kv_len + hd)
+            kb, vb = (torch.randn(kv_heads * T * hd + 1, device="cuda").half()[off:off + kv_heads * T * hd] for _ in range(2))
+            q, out, att = torch.randn(heads * hd, device="cuda"), torch.zeros(heads * hd, device="cuda"), torch.zeros((heads, T), device="cuda")
+            ptr = [C.c_void_p(t.data_ptr()) for t in (out, att, kb, vb, q)]
+            assert L.yalm_attn_generic(*ptr, heads, kv_heads, hd, T, kv_len, None, None) == 0
+            k, v = (t.double().view(kv_heads, T, hd)[:, :kv_len].repeat_interleave(heads // kv_heads, 0) for t in (kb, vb))
+            w = torch.softmax(torch.einsum("hd,htd->ht", q.double().view(heads, hd), k) / hd ** 0.5, 1)
+            want = torch.einsum("ht,htd->hd", w, v).flatten()
+            assert (out.double() - want).norm() < 2e-6 * want.norm() and (att[:, :kv_len].double() - w).norm() < 2e-6 * w.norm()

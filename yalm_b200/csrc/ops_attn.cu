@@ -316,6 +316,8 @@ __global__ void __launch_bounds__(kAttnThreads, Split<HD, G>::CTAS) attn_decode_
 // Generic path: any head_dim / group size, one CTA per q head, materialises the normalised attention
 // row in `att` exactly like the reference (src/infer.cu:338-384) — used for shapes the fast path does
 // not cover and by the mha test entry, which must return `att` (src/test.cpp:171-188).
+// Bound by latency: a lane reads a row of keys, then a column of values, and adds in their order.  So it has 64 values of a key and 16 rows of values in
+// flight: one by one, a layer whose weights had run through L2 since the last token paid the way to memory for each.  NOTE
 __global__ void __launch_bounds__(256) attn_generic_kernel(float *out, float *att, const __half *kb, const __half *vb,
                                                            const float *q, int head_dim, int n_heads, int n_kv_heads,
                                                            int max_seq_len, int kv_len_arg, const int *ctl) {
@@ -325,11 +327,20 @@ __global__ void __launch_bounds__(256) attn_generic_kernel(float *out, float *at
 	const __half *kh = kb + (size_t)kvh * max_seq_len * head_dim, *vh = vb + (size_t)kvh * max_seq_len * head_dim;
 	const float *qh = q + (size_t)h * head_dim;
 	float *atth = att + (size_t)h * max_seq_len;
+	const bool wide = head_dim % 8 == 0 && ((uintptr_t)kb & 15) == 0;
 	float mx = -INFINITY;
 	for (int t = threadIdx.x; t < kv_len; t += blockDim.x) {
 		const __half *k = kh + (size_t)t * head_dim;
 		float s = 0.f;
-		for (int i = 0; i < head_dim; ++i) s += qh[i] * __half2float(k[i]);
+		int i = 0;
+		for (; wide && i + 64 <= head_dim; i += 64) {
+			uint4 r[8];
+#pragma unroll
+			for (int u = 0; u < 8; ++u) r[u] = *reinterpret_cast<const uint4 *>(k + i + 8 * u);
+#pragma unroll
+			for (int e = 0; e < 64; ++e) s += qh[i + e] * __half2float(reinterpret_cast<const __half *>(r)[e]);
+		}
+		for (; i < head_dim; ++i) s += qh[i] * __half2float(k[i]);
 		s /= sqrtf((float)head_dim);
 		atth[t] = s;
 		mx = fmaxf(mx, s);
@@ -346,7 +357,16 @@ __global__ void __launch_bounds__(256) attn_generic_kernel(float *out, float *at
 	__syncthreads();
 	for (int i = threadIdx.x; i < head_dim; i += blockDim.x) {
 		float v = 0.f;
-		for (int t = 0; t < kv_len; ++t) v += atth[t] * __half2float(vh[(size_t)t * head_dim + i]);
+		int t = 0;
+		for (; t + 16 <= kv_len; t += 16) {
+			float p[16];
+			__half x[16];
+#pragma unroll
+			for (int u = 0; u < 16; ++u) p[u] = atth[t + u], x[u] = vh[(size_t)(t + u) * head_dim + i];
+#pragma unroll
+			for (int u = 0; u < 16; ++u) v += p[u] * __half2float(x[u]);
+		}
+		for (; t < kv_len; ++t) v += atth[t] * __half2float(vh[(size_t)t * head_dim + i]);
 		out[(size_t)h * head_dim + i] = v;
 	}
 }
