@@ -158,6 +158,10 @@ int yalm_token_probs(const float *logits, int vocab, int n_rows, const int *targ
 int yalm_gemv(float *xout, const float *x, const void *w, const float *scale, int n, int d, int dtype,
               yalm_stream_t s);
 
+/* Whether a dense one-row product of d rows of n columns runs as the stream of stream_rows.cuh (1) or on the row kernels (0); no device needed.
+ * product: 0 yalm_gemv, yalm_lm_head; 1 yalm_gemv_residual; 2 yalm_ffn_glu; 3 yalm_gemv_scaled. */
+int yalm_gemv_streamed(int product, int dtype, int n, int d);
+
 /* xout = alpha * W x; also takes YALM_BF16 weights (n % 8 == 0, 16-byte aligned rows). */
 int yalm_gemv_scaled(float *xout, const float *x, const void *w, int n, int d, int dtype, float alpha, yalm_stream_t s);
 

@@ -38,7 +38,7 @@ def matrix(d, n, dtype):
 def test_rows_of_every_length(row_bytes, dtype):
     L, (_, code, size) = api.lib(), TYPES[dtype]
     n = row_bytes // size
-    for d in (1, 37, 150, 617):
+    for d in (1, 37, 150, 617, (2 << 20) // row_bytes // 2 * 2 + 38):  # (short rows are streamed from some thousands on)
         torch.manual_seed(row_bytes + d)
         (w, s, plain), x = matrix(d, n, dtype), torch.randn(n, device="cuda")
         out = torch.full((d + 4,), 7.0, device="cuda")

@@ -38,7 +38,7 @@ SYMBOLS = [
     "yalm_norm_residual_rows", "yalm_norm_gather_rows", "yalm_glu_act_rows", "yalm_router_topk_rows", "yalm_moe_glu_slots", "yalm_moe_down_slots", "yalm_moe_gather_rows16", "yalm_moe_scatter_rows",
     "yalm_model_open_dir", "yalm_model_is_stack", "yalm_forward_rows", "yalm_sequence_end", "yalm_stack_read", "yalm_stack_ring_slots", "yalm_stack_tap",
     "yalm_norm_shift_rows", "yalm_conv_act_rows", "yalm_state_scan_rows", "yalm_ssm_prep_rows", "yalm_delta_prep_rows", "yalm_gated_group_norm_rows",
-    "yalm_head_norm_gate_rows", "yalm_qk_bias_append_rows", "yalm_attn_sigmoid_rows", "yalm_attn_sigmoid_workspace", "yalm_gemv_norm_shift", "yalm_gemv_residual_sum", "yalm_attn_sigmoid_mma", "yalm_attn_sigmoid_mma_shape", "yalm_residual_sum_rows", "yalm_softcap_rows", "yalm_attn_window_pool_host", "yalm_gemv_scaled", "yalm_gemv_norm_residual", "yalm_gemv_qkv_post", "yalm_attn_window_pool_mma", "yalm_attn_window_pool_mma_shape", "yalm_attn_window_pool_workspace",
+    "yalm_head_norm_gate_rows", "yalm_qk_bias_append_rows", "yalm_attn_sigmoid_rows", "yalm_attn_sigmoid_workspace", "yalm_gemv_norm_shift", "yalm_gemv_residual_sum", "yalm_attn_sigmoid_mma", "yalm_attn_sigmoid_mma_shape", "yalm_residual_sum_rows", "yalm_softcap_rows", "yalm_attn_window_pool_host", "yalm_gemv_scaled", "yalm_gemv_streamed", "yalm_gemv_norm_residual", "yalm_gemv_qkv_post", "yalm_attn_window_pool_mma", "yalm_attn_window_pool_mma_shape", "yalm_attn_window_pool_workspace",
     "yalm_norm_conv_rows", "yalm_latent_post_rows", "yalm_latent_query_rows", "yalm_head_linear_gate_rows", "yalm_gla_prep_rows", "yalm_depth_average_rows",
     "yalm_layer_norm_gather_rows", "yalm_head_norm_act_rows", "yalm_attn_window_pool_strided", "yalm_router_bias_topk_rows", "yalm_moe_glu_slots_real",
     "yalm_moe_down_slots_real", "yalm_attn_latent_rows", "yalm_attn_latent_rows_shape", "yalm_add_norm_conv_rows", "yalm_moe_identity_slots", "yalm_latent_gather_rows16", "yalm_latent_pack_rings", "yalm_rotate_heads_rows", "yalm_sigmoid_gate_rows",

@@ -387,13 +387,34 @@ static int launch_persistent(K kernel, const A &args, size_t smem, long tasks, c
 	return (int)cudaGetLastError();
 }
 
-// Dense products go to the stream of stream_rows.cuh; the kernels of this file serve mixtures of experts, whose rows are known on the device only, and
-// rows too long for it.
-//
+// Which products go to the stream of stream_rows.cuh; the others - and mixtures of experts, whose rows are known on the device only - stay on the kernels of
+// this file.  The stream has a larger fixed part (230 KB of shared memory an SM, its barriers, the first bytes), so it wants bytes of W, and fp8, two
+// instructions an element, wants them in long rows.  us, stream / row kernels, calls back to back and, in brackets, each behind an ordinary small kernel:
+//   residual, gate and up (bytes of one matrix).  fp8 512 x 256 3.7 / 2.4 (5.4 / 3.6), 1024 x 512 3.7 / 2.5 (5.4 / 3.7), 2048 x 1024 3.7 / 3.5 (5.4 / 4.7); fp16 128 x 128 2.8 / 2.3
+//     (4.5 / 3.5), 512 x 512 2.9 / 2.7 (4.4 / 3.8), 4096 x 14336 19.2 / 26.6 (23.4 / 27.8); fp32 64 x 64 1.9 / 2.3 (4.2 / 3.6), 128 x 1024 2.4 / 3.0 (4.0 / 4.1).  Between them
+//     the chain decides, a token of 3 layers on the per-op kernels with all its products on the stream / on these: 512 / 1024 fp16 66 / 75, fp8 73 / 67; 256 / 512
+//     fp16 61 / 64, fp8 72 / 62; 1024 / 2816 fp8 77 / 88; 4096 / 14336 fp16 288 / 335.
+//   bare rows.  fp16 512 x 512 2.9 / 2.3 (4.4 / 3.5), 2048 x 512 2.9 / 3.2 (4.4 / 4.4), 1024 x 1024 2.8 / 4.6 (4.4 / 5.8), 4096 x 4096 8.5 / 9.8 (12.1 / 11.0), 4096 x 14336 19.2 / 26.0
+//     (23.3 / 27.3); fp8 4096 x 1024 3.9 / 3.7 (5.7 / 4.9), 2048 x 2048 3.9 / 5.3 (5.6 / 6.4), 4096 x 14336 14.0 / 17.8 (17.3 / 19.0); fp8 rows of up to 6 KB in 32 to 250 MB take
+//     1.0 to 1.2 times as long.
+//   scaled rows (the layered models').  Between many small kernels, some of them on streams of their own, a kernel that takes every SM's shared memory costs
+//     them their overlap, whatever its own time.  Tokens a second: Retezen 2048 wide 2940 / 3030, Fapudra 3500 / 3940, Kiduvik 2440 / 2690, Desalorn 3900 / 4310, Fegizen 2970 / 3250.
+enum Product { kBare, kResidual, kGlu, kScaled };
+static bool streamed(Product what, int dtype, int n, int d) {
+	const int size = 16 / ep_of(dtype);
+	if (what == kScaled || n > stream::longest(size)) return false;
+	const int row = n * size;
+	const long bytes = (long)row * d;
+	if (what == kBare) return row >= 2048 ? dtype != YALM_F8E4M3 || row >= 8192 || bytes <= 16 << 20 : dtype != YALM_F8E4M3 && bytes >= 2 << 20;
+	const bool few = dtype == YALM_F8E4M3 ? row < 2048 && bytes < 1 << 20 : row < (dtype == YALM_F32 ? 512 : 1536) && bytes < 512 << 10;
+	return !few;
+}
+
 // Whether tasks of half the size end sooner: a persistent grid takes whole rounds of its warps, and a last round with few tasks leaves the
-// memory idle for as long as a full one.  (Measured on dense matrices: gate and up of a token, rows one or two pairs at a time, 4096 x 11008 fp16 with the
-// down projection 67 -> 57 us, fp32 122 -> 98; rows four or two at a time, 4096 x 4096 fp16 15.7 -> 11.3 us; where both end together, as at 4096 x 14336, the
-// larger tasks stay.)  kernel: that of the larger tasks, of the type at hand; more CTAs of the other one fit on an SM, which can only bring its end forward.
+// memory idle for as long as a full one.  (Measured on dense matrices, before the longer ones went to the stream: gate and up of a token, rows one or two pairs at a
+// time, 4096 x 11008 fp16 with the down projection 67 -> 57 us, fp32 122 -> 98; rows four or two at a time, 4096 x 4096 fp16 15.7 -> 11.3 us; where both
+// end together, as at 4096 x 14336, the larger tasks stay.)  kernel: that of the larger tasks, of the type at hand; more CTAs of the other one fit on an SM,
+// which can only bring its end forward.
 template <typename K>
 static bool finer_tasks(K kernel, size_t smem, long tasks) {
 	cudaError_t err;
@@ -449,7 +470,7 @@ extern "C" int yalm_gemv_residual_ep(float *out, const float *residual, const fl
 	const int ep = ep_of(dtype);
 	if (!ep || !out || !v || !w || n <= 0 || d <= 0 || n_active < 1 || ep_size < 1 || ep_rank < 0 || ep_rank >= ep_size) return YALM_EINVAL;
 	if (n % ep || d % 2 || (n_active > 1 && (!active_e || !active_w))) return YALM_EINVAL;
-	if (n_active == 1 && !active_e && !active_w && ep_size == 1 && n <= stream::longest(16 / ep)) {
+	if (n_active == 1 && !active_e && !active_w && ep_size == 1 && streamed(kResidual, dtype, n, d)) {
 		stream::Args t{};
 		t.out = out, t.residual = residual, t.x = v, t.w = (const char *)w, t.scale = scale, t.alpha = 1.0f, t.n = n, t.d = d;
 		YALM_DISPATCH_DT(dtype, return (stream::launch<DT, false>(t, (cudaStream_t)s)));
@@ -482,7 +503,7 @@ extern "C" int yalm_ffn_glu_ep(float *hb, const float *x, const float *rms_weigh
 	if (!ep || !hb || !x || !w1 || !w3 || dim % ep || dim % 4 || hidden_dim <= 0) return YALM_EINVAL;
 	if (n_experts < 0 || n_experts > kMaxExperts) return YALM_EINVAL;
 	if (n_experts > 0 && (!gate || !active_e || !active_w || n_active < 1 || n_active > n_experts)) return YALM_EINVAL;
-	if (n_experts == 0 && dim <= stream::longest(16 / ep)) {
+	if (n_experts == 0 && streamed(kGlu, dtype, dim, hidden_dim)) {
 		stream::Args t{};
 		t.out = hb, t.x = x, t.rms_w = rms_weight, t.w = (const char *)w1, t.w3 = (const char *)w3, t.scale = s1, t.scale3 = s3;
 		t.eps = norm_eps, t.act = act, t.n = dim, t.d = hidden_dim;
@@ -505,10 +526,10 @@ extern "C" int yalm_ffn_glu_ep(float *hb, const float *x, const float *rms_weigh
 }
 
 static int rows_launch(float *out, const float *x, const float *rms_w, const void *w, const float *scale, int n,
-                       int d, float eps, int dtype, cudaStream_t st, float alpha = 1.f) {
+                       int d, float eps, int dtype, cudaStream_t st, Product what = kBare, float alpha = 1.f) {
 	const int ep = ep_of(dtype);
 	if (!ep || !out || !x || !w || n <= 0 || d <= 0 || n % ep) return YALM_EINVAL;
-	if (n <= stream::longest(16 / ep)) {
+	if (streamed(what, dtype, n, d)) {
 		stream::Args t{};
 		t.out = out, t.x = x, t.rms_w = rms_w, t.w = (const char *)w, t.scale = scale, t.eps = eps, t.alpha = alpha, t.n = n, t.d = d;
 		if (dtype == YALM_BF16) return stream::launch<YALM_BF16, false>(t, st);
@@ -527,7 +548,7 @@ static int rows_launch(float *out, const float *x, const float *rms_w, const voi
 
 // xout = alpha * W x, weights fp32 / fp16 / bf16 / fp8: the bare GEMV with a scale (the layered models' one-row products)
 extern "C" int yalm_gemv_scaled(float *xout, const float *x, const void *w, int n, int d, int dtype, float alpha, yalm_stream_t s) {
-	return rows_launch(xout, x, nullptr, w, nullptr, n, d, 0.f, dtype, (cudaStream_t)s, alpha);
+	return rows_launch(xout, x, nullptr, w, nullptr, n, d, 0.f, dtype, (cudaStream_t)s, kScaled, alpha);
 }
 
 extern "C" int yalm_lm_head(float *logits, const float *x, const float *rms_weight, const void *wcls,
@@ -539,6 +560,11 @@ extern "C" int yalm_lm_head(float *logits, const float *x, const float *rms_weig
 extern "C" int yalm_gemv(float *xout, const float *x, const void *w, const float *scale, int n, int d, int dtype,
                          yalm_stream_t s) {
 	return rows_launch(xout, x, nullptr, w, scale, n, d, 0.f, dtype, (cudaStream_t)s);
+}
+
+extern "C" int yalm_gemv_streamed(int product, int dtype, int n, int d) {
+	if (product < kBare || product > kScaled || !ep_of(dtype) || n <= 0 || d <= 0) return YALM_EINVAL;
+	return streamed((Product)product, dtype, n, d) ? 1 : 0;
 }
 
 extern "C" int yalm_argmax_advance(const float *logits, int vocab, int *ctl, int max_seq_len, int *tokens_out,
