@@ -558,6 +558,9 @@ void yalm_tp_finalize(void);
  * (the reference is single-GPU). */
 int yalm_tp_shard_plan(const int *dims, int tensor, int rank, int size, long long *out);
 
+/* Tests only: the record of a wait that ran out in a whole-token kernel (8 words, the first 0 while there is none; null without a GPU).  Calls that
+ * find one behind their synchronisation report it and abort. */
+unsigned *yalm_mega_fault_record(void);
 /* Planning arithmetic of the whole-token kernel, callable without a device (tests).  It replaces the launch geometry
  * the reference hard-codes per kernel (src/infer.cu:745-880: one warp per output row, grids of d / 32 CTAs).
  * yalm_mega_tile_plan: out20 = 5 GEMV kinds (qkv, wo, w1/w3, w2, lm head) x {rows per tile, columns per tile, K splits,

@@ -1,6 +1,10 @@
 """-m gpu: the whole-token kernel of dense models on one GPU (csrc/decode_token.cuh) at the edges of its geometry - rows of one 512-byte chunk to four
 pieces, ragged last chunks, several rows a stage, stages that q, k and v share, one row of x for most CTAs, contexts shorter and longer than the CTAs of a head - against the
 oracle's tokens and logits; and on either side of its limits, which kernel runs."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -9,6 +13,7 @@ from yalm_b200 import api
 from yalm_b200 import yalm_file as yf
 
 pytestmark = pytest.mark.gpu
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def arch(dim, hidden, hd, heads, kv, vocab=600, layers=2, seq=256, **kw):
@@ -96,3 +101,31 @@ def test_rows_beyond_it_stay_with_the_other_kernel(oracle, dim, hidden, layers):
     assert np.abs(lg - lo).max() < LOGIT_TOL and tg == to
     s.close()
     m.close()
+
+
+RECORD = """
+import ctypes as C, sys
+from yalm_b200 import api
+from yalm_b200 import yalm_file as yf
+m = api.Model(bytes(yf.random_model(yf.Arch(512, 512, 64, 1, 8, 2, 100, 64, 10000.0, name="token"), "fp16", seed=3))).cuda()
+assert m.uses_megakernel() and m.mega_info()["vec_floats"] == 0
+s = api.InferenceState(m)
+s.forward(1, 0)
+f = api.lib().yalm_mega_fault_record
+f.restype = C.POINTER(C.c_uint)
+record = f()
+assert record[0] == 0
+s.forward(2, 1, api.MODE_HYDRATE)
+record[0], record[1], record[2] = 11, 7, 32     # as the kernel leaves it
+print("before", flush=True)
+s.forward(3, 2) if sys.argv[1] == "forward" else s.generate_greedy(3, 2, 4) if sys.argv[1] == "greedy" else s.mega_profile(3, 2) if sys.argv[1] == "profile" else s.forward_batch([3, 4, 5], 2)
+print("after", flush=True)
+"""
+
+
+@pytest.mark.parametrize("call", ["forward", "greedy", "profile", "portion"])
+def test_a_recorded_timeout_fails_the_call(call):
+    """The record is written by the host, no kernel waits: the call that synchronises next reports it and ends the process, as a CUDA error does."""
+    r = subprocess.run([sys.executable, "-c", RECORD, call], capture_output=True, text=True, timeout=300, cwd=ROOT)
+    assert "before" in r.stdout and "after" not in r.stdout and r.returncode != 0
+    assert "decode_token_kernel timed out" in r.stderr and "CTA 7 thread 32" in r.stderr

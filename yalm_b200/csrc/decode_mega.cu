@@ -79,10 +79,16 @@ const char *describe_fault() {
 	if (!r || !r[0]) return "";
 	static const char *names[] = {"?", "ring stage (mbarrier)", "producer: stage release counter", "consumer: stage release counter",
 	                              "flagged hand-over poll", "grid barrier", "cross-GPU barrier", "tensor-parallel mailbox", "MoE router record",
-	                              "hand-over sample", "hb slice counter"};
-	snprintf(buf, sizeof(buf), "decode_mega_kernel timed out in: %s (code %u) CTA %u thread %u values 0x%x %u", names[r[0] < 11 ? r[0] : 0], r[0],
-	         r[1], r[2], r[3], r[4]);
+	                              "hand-over sample", "hb slice counter", "ring stage, flagged hand-over poll or grid barrier"};
+	snprintf(buf, sizeof(buf), "%s timed out in: %s (code %u) CTA %u thread %u values 0x%x %u", r[0] == kFaultToken ? "decode_token_kernel" : "decode_mega_kernel",
+	         names[r[0] < 12 ? r[0] : 0], r[0], r[1], r[2], r[3], r[4]);
 	return buf;
+}
+void check_fault() {
+	const char *fault = describe_fault();
+	if (!fault[0]) return;
+	fprintf(stderr, "yalm_b200: %s\n", fault);
+	abort();
 }
 
 // ---- host side --------------------------------------------------------------------------------------------
@@ -195,7 +201,7 @@ static bool plan_token(Plan &p, int dtype, int dim, int q_dim, int hidden, int h
 	                                         : kernel_f8_token(head_dim, G);
 	const size_t smem = token::smem_bytes(head_dim, G);
 	cudaFuncAttributes at;
-	if (!kernel || smem > (size_t)max_smem) return false;
+	if (!kernel || smem > (size_t)max_smem || !fault_record()) return false; // (without a record a wait that ran out would go unseen)
 	if (cudaFuncGetAttributes(&at, kernel) != cudaSuccess || !token::regs_suffice(at.numRegs)) { // (else the hand-over of registers would wait for ever)
 		cudaGetLastError();
 		return false;
@@ -341,6 +347,7 @@ extern "C" int yalm_mega_token_plan(int dtype, int dim, int q_dim, int hidden, i
 	if (!out9 || dim < 1 || q_dim < 1 || hidden < 1 || head_dim < 1 || grid < 1 || !yalm::mega::ep_of(dtype)) return YALM_EINVAL;
 	return yalm::mega::token_geometry(dtype, dim, q_dim, hidden, head_dim, grid, reinterpret_cast<int (*)[3]>(out9)) ? 0 : YALM_EINVAL;
 }
+extern "C" unsigned *yalm_mega_fault_record(void) { return yalm::mega::fault_record(); }
 extern "C" int yalm_mega_mma_plan(int rows, int unit, int cap, int grid, int cta, int *out4) {
 	if (!out4 || rows < 1 || unit < 1 || cap < unit || rows % unit || grid < 1 || cta < 0 || cta >= grid) return YALM_EINVAL;
 	int row0, nrows;

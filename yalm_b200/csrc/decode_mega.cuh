@@ -46,7 +46,7 @@ constexpr long long kTimeoutCycles = 120000000000ll;
 static __device__ unsigned *g_fault_rec = nullptr;
 static __device__ long long g_timeout_cycles = kTimeoutCycles; // YALM_MEGA_TIMEOUT_S shortens it (debugging)
 enum { kFaultRing = 1, kFaultProducerRel = 2, kFaultConsumerRel = 3, kFaultPoll = 4, kFaultGridBarrier = 5, kFaultTpBarrier = 6,
-       kFaultTpMailbox = 7, kFaultRouter = 8, kFaultSample = 9, kFaultHb = 10 };
+       kFaultTpMailbox = 7, kFaultRouter = 8, kFaultSample = 9, kFaultHb = 10, kFaultToken = 11 };
 static __device__ __noinline__ void die(unsigned code, unsigned x, unsigned y) {
 	unsigned *r = g_fault_rec;
 	if (r && atomicCAS(r, 0u, code) == 0u) {

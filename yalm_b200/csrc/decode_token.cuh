@@ -25,7 +25,8 @@
 //     branches for each stage in turn, w1 / w3 took 60 us.
 //   * Stages freed four at a time: eight at a time is 20 % less work and still slower under load, the ring being that much shorter.
 //
-// A wait that runs out (a bug) turns what the warp computes into NaN, its later waits return at once, and the kernel leaves a record (mega.h: fault_record).
+// A wait that runs out (a bug) turns what the warp computes into NaN, its later waits return at once, and the kernel leaves a record, which the host reads behind
+// the launch and fails on (mega.h: fault_record, check_fault).
 #pragma once
 
 #include "decode_mega.cuh"
@@ -59,12 +60,16 @@ constexpr bool regs_suffice(int at_launch) { return (at_launch + 7) / 8 * 8 * kT
 __device__ __forceinline__ void tbar() { asm volatile("bar.sync 1, %0;" ::"n"(kCT2) : "memory"); }
 
 // Bounded waits.  Nobody traps: whoever gave up goes on with NaN.  (No calls in them: what lives across a call is spilled.)
-constexpr long long kPatience = 8000000000ll; // cycles, some 4 s
+constexpr long long kPatience = 8000000000ll; // cycles, some 4 s, unless YALM_MEGA_TIMEOUT_S says otherwise (g_timeout_cycles, looked up when a wait is long)
+__device__ __forceinline__ bool out_of_patience(long long t0) {
+	const long long waited = clock64() - t0;
+	return waited > 1000000 && waited > *(volatile long long *)&g_timeout_cycles;
+}
 __device__ __forceinline__ void wait_stage(uint32_t bar, uint32_t parity, bool &dead) { // whole warp
 	if (__all_sync(kFull, mbar_try_wait(bar, parity))) return;
 	dead = __any_sync(kFull, dead);
 	const long long t0 = clock64();
-	while (!dead && !__all_sync(kFull, mbar_try_wait(bar, parity))) dead = __any_sync(kFull, clock64() - t0 > kPatience);
+	while (!dead && !__all_sync(kFull, mbar_try_wait(bar, parity))) dead = __any_sync(kFull, out_of_patience(t0));
 }
 
 __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) { // does not wait
@@ -90,11 +95,10 @@ struct Backoff {
 	int round = 0;
 	long long t0 = 0;
 	__device__ __forceinline__ bool over() { // sleeps; true once patience is at its end
-		const long long now = clock64();
-		if (round == 0) t0 = now;
+		if (round == 0) t0 = clock64();
 		__nanosleep((unsigned)YALM_MEGA_LL_NS << min(round, 4));
 		++round;
-		return now - t0 > kPatience;
+		return out_of_patience(t0);
 	}
 };
 // DT: weight type, HD: head size, G: query heads per KV head
@@ -272,7 +276,7 @@ __global__ void __launch_bounds__(kTokenThreads, 1) decode_token_kernel(const __
 			while (!dead) {
 				ok = (lane & 7) >= m || mbar_try_wait(full0 + 8 * st, par);
 				if (__all_sync(kFull, ok)) break;
-				dead = __any_sync(kFull, clock64() - t0 > kPatience);
+				dead = __any_sync(kFull, out_of_patience(t0));
 			}
 		}
 		__syncwarp();
@@ -305,7 +309,7 @@ __global__ void __launch_bounds__(kTokenThreads, 1) decode_token_kernel(const __
 			const long long t0 = clock64();
 			do {
 				asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.sync) : "memory");
-				if (v < target && clock64() - t0 > kPatience) dead = true;
+				if (v < target && out_of_patience(t0)) dead = true;
 			} while (v < target && !dead);
 			asm volatile("fence.acq_rel.gpu;" ::: "memory");
 		}
@@ -853,7 +857,7 @@ __global__ void __launch_bounds__(kTokenThreads, 1) decode_token_kernel(const __
 	}
 	if (dead && lane == 0) { // which warp gave up, for the host
 		unsigned *r = g_fault_rec;
-		if (r && atomicCAS(r, 0u, (unsigned)kFaultPoll) == 0u) {
+		if (r && atomicCAS(r, 0u, (unsigned)kFaultToken) == 0u) {
 			r[1] = cta, r[2] = tid, r[3] = 0, r[4] = 0;
 			__threadfence_system();
 		}

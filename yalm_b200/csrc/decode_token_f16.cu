@@ -4,7 +4,7 @@
 namespace yalm {
 namespace mega {
 const void *kernel_f16_token(int head_dim, int g) {
-	set_fault_pointers(fault_record(), fault_timeout_cycles());
+	set_fault_pointers(fault_record(), fault_timeout_cycles() > 0 ? fault_timeout_cycles() : token::kPatience);
 	return token::token_kernel_for<YALM_F16>(head_dim, g);
 }
 } // namespace mega

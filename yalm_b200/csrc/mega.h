@@ -166,11 +166,13 @@ int launch(const Plan &p, const Args &a, cudaStream_t st);
 // Tensor-core GEMV: tensor map (128 bytes at `map128`) of a (rows, K) row-major fp16 matrix on the device for boxes of
 // 64 columns x box_rows rows x 4 column blocks, 128-byte swizzle, zero fill past the last row.  Returns 0 or YALM_EINVAL.
 int make_weight_map(void *map128, const void *dev_ptr, int rows, int K, int box_rows);
-// Failure record of the kernel's timeouts (decode_mega.cuh: die): 8 words of pinned, device-mapped host memory, all zero
-// while nothing has gone wrong.  describe_fault() formats it ("" if clean); fault_timeout_cycles(): YALM_MEGA_TIMEOUT_S.
+// Failure record of the kernels' timeouts (decode_mega.cuh: die; decode_token.cuh): 8 words of pinned, device-mapped host memory, all zero
+// while nothing has gone wrong.  describe_fault() formats it ("" if clean); fault_timeout_cycles(): YALM_MEGA_TIMEOUT_S.  check_fault(), behind a
+// synchronisation: reports the record and aborts, as a failed CUDA call does - decode_token_kernel ends without an error, with NaN for results.
 unsigned *fault_record();
 long long fault_timeout_cycles();
 const char *describe_fault();
+void check_fault();
 
 } // namespace mega
 } // namespace yalm

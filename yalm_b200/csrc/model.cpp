@@ -825,6 +825,7 @@ int Model::mega_profile(InferenceState &s, int token, int pos, long long *out, s
 	int rc = launch_mega(s, token, pos, yalm::mega::kLogits, dev);
 	_mega_trace = nullptr;
 	if (rc == 0) rc = (int)cudaStreamSynchronize(s.stream());
+	if (rc == 0) yalm::mega::check_fault();
 	if (rc == 0) rc = (int)cudaMemcpy(out, dev, need * sizeof(long long), cudaMemcpyDeviceToHost);
 	if (rc == 0 && tdev) {
 		std::vector<long long> h(tn);
@@ -974,6 +975,7 @@ void Model::forward(InferenceState &s, int token, int pos, InferenceMode mode) {
 				CUDA_CHECK(cudaMemcpyAsync(s.logits(), s.logits_dev(), sizeof(float) * c.vocab_size, cudaMemcpyDeviceToHost,
 				                           s.stream()));
 			CUDA_CHECK(cudaStreamSynchronize(s.stream()));
+			yalm::mega::check_fault();
 		}
 		CUDA_CHECK(cudaGetLastError());
 		return;
@@ -1039,6 +1041,7 @@ int Model::generate(InferenceState &s, int token, int pos, int n_gen, float temp
 		CUDA_CHECK(cudaEventRecord(e1, st));
 		CUDA_CHECK(cudaMemcpyAsync(tokens_out, s.tokens_dev(), sizeof(int) * n_gen, cudaMemcpyDeviceToHost, st));
 		CUDA_CHECK(cudaStreamSynchronize(st));
+		yalm::mega::check_fault();
 		if (device_ms) {
 			CUDA_CHECK(cudaEventElapsedTime(device_ms, e0, e1));
 			if (done && n_gen > done) *device_ms = *device_ms * n_gen / (n_gen - done); // scale to n_gen steps when step 0 ran eagerly

@@ -9,6 +9,7 @@
 
 #include "gemv.cuh"
 #include "launch.h"
+#include "mega.h"
 
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -226,5 +227,6 @@ int Model::forward_batch(InferenceState &s, const int *tokens, int n, int pos0, 
 	if (s.host_logits())
 		YALM_TRY(cudaMemcpyAsync(s.logits(), s.logits_dev(), sizeof(float) * V, cudaMemcpyDeviceToHost, st));
 	YALM_TRY(cudaStreamSynchronize(st));
+	yalm::mega::check_fault(); // (of tokens before this portion, whose keys and values it has read)
 	return (int)cudaGetLastError();
 }
