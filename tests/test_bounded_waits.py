@@ -31,3 +31,11 @@ def test_waits_are_used():
     text = "".join(source(n) for n in ("prefill_gemm.cu", "prompt_attn.cu", "chunk_scan.cuh"))
     for name in re.findall(r"void (mbar_wait\w*)\(", source("tcgen.cuh")):
         assert re.search(r"\b%s\(" % name, text), name
+
+
+def test_joins_of_the_token_kernels_attention():
+    """A sum that gave up is NaN in the join; and the weights of the joins (not of the positions) are expf, as in the kernel of decode_mega.cuh."""
+    text = source("decode_token.cuh")
+    assert "if (dead) lsum = NaN;" in text and "= dead ? NaN : ls" in text
+    joins = text[text.index("the warps' records in order"): text.index("// ---- a product")]
+    assert joins.count("expf(") == 2 and "__expf" not in joins

@@ -502,7 +502,7 @@ __global__ void __launch_bounds__(kTokenThreads, 1) decode_token_kernel(const __
 					for (int u = 0; u < UL; ++u) mm[u] = r[u * HG * kHeads * (HD + 2) + HD], M = fmaxf(M, mm[u]);
 #pragma unroll
 					for (int u = 0; u < UL; ++u) {
-						const float w = mm[u] == -INFINITY ? 0.f : __expf(mm[u] - M);
+						const float w = mm[u] == -INFINITY ? 0.f : expf(mm[u] - M);
 						v = fmaf(w, r[u * HG * kHeads * (HD + 2) + d], v), ls = fmaf(w, r[u * HG * kHeads * (HD + 2) + HD + 1], ls); // (an empty record is zero)
 					}
 					ll_store(a.ll_acc + (((size_t)sp.kvh * ncta + cta) * G + h) * HD + d, v, wflag);
@@ -515,19 +515,18 @@ __global__ void __launch_bounds__(kTokenThreads, 1) decode_token_kernel(const __
 			float *join = reinterpret_cast<float *>(sm + kOffRec); // [maximum, sum, value][warp][lane]
 			for (int ob = o_lo; ob < o_hi; ob += 32) {
 				const int o = min(ob + lane, o_hi - 1), h = o / HD;
-				float M = -INFINITY, ls = 0.f, v = 0.f;
 				constexpr int AT = 3; // partners in flight
-				for (int p0 = warp; p0 < sp.nc; p0 += kW * AT) {
+				ulonglong2 w[AT];
+				unsigned long long x[AT];
+				bool there[AT];
+				auto partners = [&](int p0) {
 					const unsigned long long *ml[AT], *ac[AT];
-					bool there[AT];
 #pragma unroll
 					for (int i = 0; i < AT; ++i) {
 						const int p = p0 + i * kW;
 						there[i] = p < sp.nc && attn_has_unit(p, sp.nc, nch);
 						ml[i] = a.ll_ml + (((size_t)sp.kvh * ncta + sp.c0 + p) * G + h) * 2, ac[i] = a.ll_acc + ((size_t)sp.kvh * ncta + sp.c0 + p) * G * HD + o;
 					}
-					ulonglong2 w[AT];
-					unsigned long long x[AT];
 					Backoff wait;
 					for (;;) {
 						bool good = true;
@@ -540,25 +539,34 @@ __global__ void __launch_bounds__(kTokenThreads, 1) decode_token_kernel(const __
 						if (good || dead) break;
 						dead = wait.over();
 					}
+				};
+				float M = -INFINITY, ls = 0.f, v = 0.f;
+				for (int p0 = warp; p0 < sp.nc; p0 += kW * AT) {
+					partners(p0);
+#pragma unroll
+					for (int i = 0; i < AT; ++i)
+						if (there[i]) M = fmaxf(M, ll_val(w[i].x));
+				}
+				tbar(); // (the records, and the join before, have been read)
+				join[warp * 32 + lane] = M;
+				tbar();
+#pragma unroll
+				for (int u = 0; u < kW; ++u) M = fmaxf(M, join[u * 32 + lane]); // of the head, before any weight
+				for (int p0 = warp; p0 < sp.nc; p0 += kW * AT) {
+					if (sp.nc > kW * AT) partners(p0); // (else they are still here)
 #pragma unroll
 					for (int i = 0; i < AT; ++i)
 						if (there[i]) {
-							const float pm = ll_val(w[i].x), Mn = fmaxf(M, pm), old = M == -INFINITY ? 0.f : __expf(M - Mn), now = pm == -INFINITY ? 0.f : __expf(pm - Mn);
-							ls = ls * old + now * ll_val(w[i].y), v = v * old + now * ll_val(x[i]), M = Mn;
+							const float pm = ll_val(w[i].x), f = pm == -INFINITY ? 0.f : expf(pm - M);
+							ls = fmaf(f, ll_val(w[i].y), ls), v = fmaf(f, ll_val(x[i]), v);
 						}
 				}
-				tbar(); // (the records, and the join before, have been read)
-				join[(0 * kW + warp) * 32 + lane] = M, join[(1 * kW + warp) * 32 + lane] = dead ? NaN : ls, join[(2 * kW + warp) * 32 + lane] = v;
+				join[(kW + warp) * 32 + lane] = dead ? NaN : ls, join[(2 * kW + warp) * 32 + lane] = v;
 				tbar();
 				if (warp == (l & (kW - 1)) && ob + lane < o_hi) {
-					float m2 = -INFINITY, l2 = 0.f, v2 = 0.f;
+					float l2 = 0.f, v2 = 0.f;
 #pragma unroll
-					for (int w = 0; w < kW; ++w) m2 = fmaxf(m2, join[w * 32 + lane]);
-#pragma unroll
-					for (int w = 0; w < kW; ++w) {
-						const float pm = join[w * 32 + lane], f = pm == -INFINITY ? 0.f : __expf(pm - m2);
-						l2 = fmaf(f, join[(kW + w) * 32 + lane], l2), v2 = fmaf(f, join[(2 * kW + w) * 32 + lane], v2);
-					}
+					for (int u = 0; u < kW; ++u) l2 += join[(kW + u) * 32 + lane], v2 += join[(2 * kW + u) * 32 + lane];
 					const float out = v2 / l2;
 #pragma unroll
 					for (int rp = 0; rp < kLLRep; ++rp) ll_store(a.ll_att + (size_t)rp * a.q_dim + (size_t)sp.kvh * G * HD + o, out, wflag);
