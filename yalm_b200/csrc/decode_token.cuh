@@ -25,8 +25,9 @@
 //     branches for each stage in turn, w1 / w3 took 60 us.
 //   * Stages freed four at a time: eight at a time is 20 % less work and still slower under load, the ring being that much shorter.
 //
-// A wait that runs out (a bug) turns what the warp computes into NaN, its later waits return at once, and the kernel leaves a record, which the host reads behind
-// the launch and fails on (mega.h: fault_record, check_fault).
+// A wait that runs out (a bug) turns what the warp computes into NaN, its later ones of the kind return at once, and the kernel leaves a record, which the host
+// reads behind the launch and fails on (mega.h: fault_record, check_fault).  Stages are waited for and given back in order all the same, so the stream
+// ends; if a stage itself does not land, none is given back any more, the stream gives up in turn, and waits for its copies, again with a limit, before it leaves.
 #pragma once
 
 #include "decode_mega.cuh"
@@ -150,10 +151,11 @@ __global__ void __launch_bounds__(kTokenThreads, 1) decode_token_kernel(const __
 			turn = turn + 1 == kIssuers ? 0 : turn + 1;
 			if (!yes) return false;
 			wait_stage(empty0 + 8 * s, phase, dead);
+			if (dead) return false;
 			dst = ring0 + s * kStageBytes, bar = full0 + 8 * s;
 			s += kIssuers;
 			if (s >= kTokenStages) s -= kTokenStages, phase ^= 1;
-			return !dead;
+			return true;
 		};
 		for (int ph = 0; ph < n_phases && !dead; ++ph) {
 			const int l = min(ph / 5, a.n_layers - 1), k = ph < a.n_layers * 5 ? ph % 5 : 5;
@@ -227,6 +229,13 @@ __global__ void __launch_bounds__(kTokenThreads, 1) decode_token_kernel(const __
 				}
 			}
 		}
+		// its own copies have landed before it leaves (the parity that a stage's last one completes is that of the round in which it would be free)
+		bool late = false;
+		for (int i = 0; i < kTokenStages / kIssuers; ++i) {
+			wait_stage(full0 + 8 * s, phase, late);
+			s += kIssuers;
+			if (s >= kTokenStages) s -= kTokenStages, phase ^= 1;
+		}
 		return;
 	}
 
@@ -261,6 +270,7 @@ __global__ void __launch_bounds__(kTokenThreads, 1) decode_token_kernel(const __
 	tbar();
 
 	uint32_t s = 0, sphase = 0; // this warp's place in the ring
+	bool lost = false; // a stage never landed: no more stages are given back, so none is filled again under a copy that may still be on its way
 	// Up to eight stages at once: lane l looks after stage l % 8, so that waits and releases cost a warp one instruction and not four in a row.
 	auto stage_of_lane = [&](uint32_t &st, uint32_t &par) {
 		st = s + (lane & 7), par = sphase;
@@ -271,13 +281,13 @@ __global__ void __launch_bounds__(kTokenThreads, 1) decode_token_kernel(const __
 		stage_of_lane(st, par);
 		bool ok = (lane & 7) >= m || mbar_try_wait(full0 + 8 * st, par);
 		if (!__all_sync(kFull, ok)) {
-			dead = __any_sync(kFull, dead);
 			const long long t0 = clock64();
-			while (!dead) {
+			while (!lost) {
 				ok = (lane & 7) >= m || mbar_try_wait(full0 + 8 * st, par);
 				if (__all_sync(kFull, ok)) break;
-				dead = __any_sync(kFull, out_of_patience(t0));
+				lost = __any_sync(kFull, out_of_patience(t0));
 			}
+			dead = dead || lost;
 		}
 		__syncwarp();
 	};
@@ -290,7 +300,7 @@ __global__ void __launch_bounds__(kTokenThreads, 1) decode_token_kernel(const __
 		uint32_t st, par;
 		stage_of_lane(st, par);
 		__syncwarp();
-		if (lane < m) mbar_arrive(empty0 + 8 * st);
+		if (lane < m && !lost) mbar_arrive(empty0 + 8 * st);
 		s += m;
 		if (s >= kTokenStages) s -= kTokenStages, sphase ^= 1;
 	};

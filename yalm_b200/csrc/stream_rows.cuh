@@ -175,6 +175,9 @@ __global__ void __launch_bounds__(kThreads, 1) stream_rows_kernel(const __grid_c
 			}
 			__syncwarp();
 		}
+		// its own copies have landed before it leaves (the parity that a stage's last one completes is that of the round in which it would be free)
+		bool late = false;
+		for (int i = 0; i < a.stages; ++i, ring.next(a.stages)) mbar_wait_warp(full0 + 8 * ring.s, ring.phase, late);
 		return;
 	}
 
@@ -236,7 +239,7 @@ __global__ void __launch_bounds__(kThreads, 1) stream_rows_kernel(const __grid_c
 				asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(w[j].x), "=r"(w[j].y), "=r"(w[j].z), "=r"(w[j].w) : "r"(at + j * (PAIR ? a.RG * a.row_bytes : a.C * 512)) : "memory");
 		}
 		__syncwarp();
-		if (lane == 0) mbar_arrive(empty0 + 8 * ring.s);
+		if (lane == 0 && !dead) mbar_arrive(empty0 + 8 * ring.s); // (else it could be filled again under a copy that may still be on its way)
 		ring.next(a.stages);
 	};
 	const int per = kCap / rows_block; // blocks whose partial sums fit
