@@ -103,6 +103,17 @@ def test_rows_beyond_it_stay_with_the_other_kernel(oracle, dim, hidden, layers):
     m.close()
 
 
+@pytest.mark.parametrize("name", ["W2_PIPE", "MMA", "STAGES", "DEBUG", "L2_AHEAD", "TUNE", "TRACE"])
+def test_settings_of_the_other_kernel_select_it(name, monkeypatch):
+    img = bytes(yf.random_model(arch(512, 512, 64, 8, 2, vocab=100, layers=1), "fp16", seed=8))
+    for value, here in ((None, True), ("0", False)):
+        if value is not None:
+            monkeypatch.setenv("YALM_MEGA_" + name, value)
+        m = api.Model(img).cuda()
+        assert m.uses_megakernel() and runs_here(m) == here
+        m.close()
+
+
 RECORD = """
 import ctypes as C, sys
 from yalm_b200 import api

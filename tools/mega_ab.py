@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""A/B of plan-time settings of the whole-token kernel on one model image (the model is re-created per setting, the
+"""A/B of plan-time settings of decode_mega_kernel (which they select; a dense model on one GPU otherwise runs on decode_token_kernel) on one model image (the model is re-created per setting, the
 environment is read when the plan is made): tok/s of the on-device greedy loop at ~4k context and token identity.
     python tools/mega_ab.py [--workload NAME] [--pos P] "YALM_MEGA_W2_PIPE=0" "YALM_MEGA_STAGES=20" ..."""
 import argparse

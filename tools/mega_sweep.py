@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Sweep of the megakernel's run-time knobs on one loaded model (with YALM_MEGA_TUNE=1 the knobs are read from the
+"""Sweep of decode_mega_kernel's run-time knobs (they select it) on one loaded model (with YALM_MEGA_TUNE=1 the knobs are read from the
 environment at every launch): tok/s of the on-device greedy loop at 4k context per setting.
     python tools/mega_sweep.py "YALM_MEGA_L2_AHEAD=-16" "YALM_MEGA_L2_AHEAD=-16 YALM_MEGA_DEBUG=16" ..."""
 import os

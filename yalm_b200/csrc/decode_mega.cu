@@ -274,8 +274,11 @@ Plan plan(int dtype, int dim, int q_dim, int kv_dim, int head_dim, int hidden, i
 		const bool can = !p.mma && !tp && n_experts == 0 && nk >= 2 && nk <= kHbMaxSlices && p.shape[kW2][0] <= 2 &&
 		                 (groups + kConsumerWarps - 1) / kConsumerWarps <= kHbMaxGroups && stages_for(vf_pipe) >= 2;
 		const bool want = e ? atoi(e) != 0 : stages_for(vf_pipe) >= stages_for(vf) + 2;
-		// (a setting of either choice, on or off, asks for that kernel)
-		token_kernel = !e && !getenv("YALM_MEGA_MMA") && !tp && n_experts == 0 && plan_token(p, dtype, dim, q_dim, hidden, head_dim, G, di.max_smem_optin);
+		// (a setting of a choice or an experiment that only that kernel has, on or off, asks for it)
+		bool mega_setting = false;
+		for (const char *name : {"YALM_MEGA_W2_PIPE", "YALM_MEGA_MMA", "YALM_MEGA_STAGES", "YALM_MEGA_DEBUG", "YALM_MEGA_L2_AHEAD", "YALM_MEGA_TUNE", "YALM_MEGA_TRACE"})
+			mega_setting = mega_setting || getenv(name);
+		token_kernel = !mega_setting && !tp && n_experts == 0 && plan_token(p, dtype, dim, q_dim, hidden, head_dim, G, di.max_smem_optin);
 		if (can && want && !token_kernel) p.w2_pipe = 1, p.hb_slice = p.shape[kW2][1], p.hb_off = hb_off, vf = vf_pipe;
 	}
 	if (!token_kernel) {
