@@ -1,4 +1,4 @@
-"""-m gpu: the whole-token persistent kernel (decode_mega.cuh) — one cooperative launch per token with the
+"""-m gpu: the whole-token persistent kernels (decode_token.cuh, or decode_mega.cuh: each shape below also by request) — one cooperative launch per token with the
 weight / KV tiles streamed through a shared-memory TMA ring — against the oracle and against the per-op kernel
 path (YALM_B200_MEGA=0) on the same models: tile shapes with and without K splits, every compiled
 (head_dim, group) pair, sliding window + sinks, on-device greedy loop."""
@@ -93,10 +93,11 @@ def test_mega_shapes_vs_oracle(oracle, case):
     ref_img = bytes(yf.dequantized_fp32_image(img)) if dt == "fp8" else img
     prompt = [1, 5, 9, 200, 77]
     to, lo = oracle.OracleModel(ref_img).generate(prompt, 40, keep_logits=True)
-    tg, lg, used = run(img, prompt, 40)
-    assert used
-    assert np.abs(lg - lo).max() < LOGIT_TOL
-    assert tg == to
+    for pipe in (None, False):      # the planner's kernel; decode_mega_kernel's plain variant
+        tg, lg, used = run(img, prompt, 40, pipe=pipe)
+        assert used
+        assert np.abs(lg - lo).max() < LOGIT_TOL
+        assert tg == to
 
 
 def test_mega_sliding_window_and_sinks(oracle):
@@ -105,10 +106,11 @@ def test_mega_sliding_window_and_sinks(oracle):
     arch = yf.Arch(256, 512, 32, 2, 8, 2, 512, 64, 10000.0, name="tiny-win")
     img = bytes(yf.random_model(arch, "fp16", seed=21))
     to, lo = oracle.OracleModel(img, context=24).generate([1, 2, 3], 90, keep_logits=True)
-    tg, lg, used = run(img, [1, 2, 3], 90, context=24)
-    assert used
-    assert np.abs(lg - lo).max() < LOGIT_TOL
-    assert tg == to
+    for pipe in (None, False):
+        tg, lg, used = run(img, [1, 2, 3], 90, context=24, pipe=pipe)
+        assert used
+        assert np.abs(lg - lo).max() < LOGIT_TOL
+        assert tg == to
 
 
 def test_mega_long_context_many_tiles(oracle):
@@ -117,10 +119,11 @@ def test_mega_long_context_many_tiles(oracle):
     img = bytes(yf.random_model(arch, "fp16", seed=8))
     prompt = [(i * 37 + 1) % 512 for i in range(690)]
     to, lo = oracle.OracleModel(img).generate(prompt, 10, keep_logits=True)
-    tg, lg, used = run(img, prompt, 10)
-    assert used
-    assert np.abs(lg - lo).max() < LOGIT_TOL
-    assert tg == to
+    for pipe in (None, False):
+        tg, lg, used = run(img, prompt, 10, pipe=pipe)
+        assert used
+        assert np.abs(lg - lo).max() < LOGIT_TOL
+        assert tg == to
 
 
 def test_mega_attention_at_depth_head_dim_128(oracle):
@@ -131,10 +134,11 @@ def test_mega_attention_at_depth_head_dim_128(oracle):
     img = bytes(yf.random_model(arch, "fp16", seed=5))
     prompt = [(i * 131 + 7) % 509 + 3 for i in range(3050)]
     to, lo = oracle.OracleModel(img).generate(prompt, 12, keep_logits=True)
-    tg, lg, used = run(img, prompt, 12)
-    assert used
-    assert np.abs(lg - lo).max() < LOGIT_TOL
-    assert tg == to
+    for pipe in (None, False):
+        tg, lg, used = run(img, prompt, 12, pipe=pipe)
+        assert used
+        assert np.abs(lg - lo).max() < LOGIT_TOL
+        assert tg == to
 
 
 def test_mega_fp8_window_1024_two_wraps(oracle):
@@ -145,10 +149,11 @@ def test_mega_fp8_window_1024_two_wraps(oracle):
     ref_img = bytes(yf.dequantized_fp32_image(img))
     prompt = [(i * 57 + 5) % 509 + 3 for i in range(2290)]
     to, lo = oracle.OracleModel(ref_img, context=1024).generate(prompt, 10, keep_logits=True)
-    tg, lg, used = run(img, prompt, 10, context=1024)
-    assert used
-    assert np.abs(lg - lo).max() < LOGIT_TOL
-    assert tg == to
+    for pipe in (None, False):
+        tg, lg, used = run(img, prompt, 10, context=1024, pipe=pipe)
+        assert used
+        assert np.abs(lg - lo).max() < LOGIT_TOL
+        assert tg == to
 
 
 def test_mega_mistral_geometry_8_layers(oracle):

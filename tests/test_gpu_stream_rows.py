@@ -98,3 +98,19 @@ def test_weights_written_just_before():
         w.fill_(float(i + 1))
         L.yalm_gemv(p(out), p(x), p(w), None, C.c_int(n), C.c_int(d), C.c_int(api.F16), None)
         assert rel(out, (i + 1) * x.double().sum() * torch.ones(d, device="cuda", dtype=torch.float64)) < 1e-4  # one sum of 4096 values that cancel
+
+
+def test_weights_written_by_the_kernel_that_lets_it_begin():
+    """The matrix of the second product is the first one's result, in fp32: that kernel lets the next begin, which fetches the matrix's first bytes, before it stores it.
+    Every round stores other values over the last one's."""
+    L, n, d = api.lib(), 2048, 512                     # 4 MB, two rounds of a CTA's first stages
+    f32 = C.c_int(api.F32)
+    v, x = torch.randn((9, 64), device="cuda"), torch.randn(n, device="cuda")
+    first = torch.randn((n * d, 64), device="cuda")    # 268 MB: its last rows are stored long after the next kernel began
+    matrix, out = torch.zeros((d, n), device="cuda"), torch.zeros((9, d), device="cuda")
+    assert L.yalm_gemv_streamed(0, api.F32, 64, n * d) == 1 and L.yalm_gemv_streamed(0, api.F32, n, d) == 1
+    for i in range(9):
+        assert L.yalm_gemv(p(matrix), p(v[i]), p(first), None, C.c_int(64), C.c_int(n * d), f32, None) == 0
+        assert L.yalm_gemv(p(out[i]), p(x), p(matrix), None, C.c_int(n), C.c_int(d), f32, None) == 0
+    for i in range(9):                                 # fp32 sums of 64, then of 2048 terms
+        assert rel(out[i], (first.double() @ v[i].double()).view(d, n) @ x.double()) < 2e-6
