@@ -1,5 +1,5 @@
 // Whole-token persistent decode kernel for dense models on one GPU: the phases, hand-over words and arithmetic of decode_mega.cuh (which serves mixtures
-// of experts, several GPUs and wider rows) with another division of the work inside a CTA.
+// of experts, several GPUs and what it is faster at: token_geometry(), decode_mega.cu) with another division of the work inside a CTA.
 //
 // 12 warps, one CTA per SM, cooperative launch.  Two warps stream the CTA's rows of every matrix, the norms' weights and its pieces of the KV ring, phase after
 // phase, through a ring of 24 stages of 8 KB (cp.async.bulk, mbarriers): they wait for free stages and for nothing else.  The other eight:
@@ -17,17 +17,17 @@
 // time has waited for every CTA's row of a product that comes after its reading of the first.
 //
 // Bound by HBM inside the phases (w1 / w3 235 MB in 35 us) and by the hand-overs between them.  A layer of 4096 / 14336 at 4096 positions, us, here and with
-// decode_mega.cuh: q k v 9.7 / 11, attention 8.7 / 13, wo 6.4 / 9, w1 w3 37.9 / 37, w2 21.7 / 24: 85 / 94; four layers and the head, a call on the host 461 -> 436;
-// 2048 / 8192 176 -> 158 (200 positions), 1024 / 2816 135 -> 99.  Without any copies a layer takes 75, with no arithmetic on rows and keys 75.  What shaped it:
+// decode_mega.cuh: q k v 9.7 / 11, attention 8.7 / 13, wo 6.4 / 9, w1 w3 37.9 / 37, w2 21.7 / 24: 85 / 94; four layers and the head, a call on the host 461 -> 437;
+// three layers at 600 positions on the device, 2048 / 7168 149 -> 123, 1024 / 3584 112 -> 77.  Without any copies a layer takes 75, with no arithmetic on rows and keys 75.  What shaped it:
 //   * Registers.  Any spill in the row loops is a round trip to an L2 that is busy with the weights: 100 bytes of them cost 10 us a layer.  Hence eight warps
 //     with 224 registers (setmaxnreg) instead of 16 with 112, q in shared memory, vectors polled for 32 words at a time.
 //   * One instruction for the barriers of four stages (lane l asks for stage l % 8) and no branches around the loads: with a wait, a release and two
 //     branches for each stage in turn, w1 / w3 took 60 us.
 //   * Stages freed four at a time: eight at a time is 20 % less work and still slower under load, the ring being that much shorter.
 //
-// A wait that runs out (a bug) turns what the warp computes into NaN, its later ones of the kind return at once, and the kernel leaves a record, which the host
-// reads behind the launch and fails on (mega.h: fault_record, check_fault).  Stages are waited for and given back in order all the same, so the stream
-// ends; if a stage itself does not land, none is given back any more, the stream gives up in turn, and waits for its copies, again with a limit, before it leaves.
+// A wait that runs out (a bug) turns what the warp computes into NaN, its later waits return at once, and the kernel leaves a record, which the host reads behind
+// the launch and fails on (mega.h: fault_record, check_fault).  Such a warp gives no stage back, so the stream gives up in turn and waits for its own copies, again with a
+// limit, before it leaves.
 #pragma once
 
 #include "decode_mega.cuh"
@@ -151,11 +151,10 @@ __global__ void __launch_bounds__(kTokenThreads, 1) decode_token_kernel(const __
 			turn = turn + 1 == kIssuers ? 0 : turn + 1;
 			if (!yes) return false;
 			wait_stage(empty0 + 8 * s, phase, dead);
-			if (dead) return false;
 			dst = ring0 + s * kStageBytes, bar = full0 + 8 * s;
 			s += kIssuers;
 			if (s >= kTokenStages) s -= kTokenStages, phase ^= 1;
-			return true;
+			return !dead; // (left earlier, where it gave up, it took 12 us a layer: place and address were no longer the same for the whole warp)
 		};
 		for (int ph = 0; ph < n_phases && !dead; ++ph) {
 			const int l = min(ph / 5, a.n_layers - 1), k = ph < a.n_layers * 5 ? ph % 5 : 5;
@@ -229,7 +228,8 @@ __global__ void __launch_bounds__(kTokenThreads, 1) decode_token_kernel(const __
 				}
 			}
 		}
-		// its own copies have landed before it leaves (the parity that a stage's last one completes is that of the round in which it would be free)
+		// its own copies have landed before it leaves (the parity that a stage's last one completes is that of the round in which it would be free; the stage that
+		// it gave up on, if it did, was not filled and runs out)
 		bool late = false;
 		for (int i = 0; i < kTokenStages / kIssuers; ++i) {
 			wait_stage(full0 + 8 * s, phase, late);
@@ -270,7 +270,6 @@ __global__ void __launch_bounds__(kTokenThreads, 1) decode_token_kernel(const __
 	tbar();
 
 	uint32_t s = 0, sphase = 0; // this warp's place in the ring
-	bool lost = false; // a stage never landed: no more stages are given back, so none is filled again under a copy that may still be on its way
 	// Up to eight stages at once: lane l looks after stage l % 8, so that waits and releases cost a warp one instruction and not four in a row.
 	auto stage_of_lane = [&](uint32_t &st, uint32_t &par) {
 		st = s + (lane & 7), par = sphase;
@@ -281,13 +280,13 @@ __global__ void __launch_bounds__(kTokenThreads, 1) decode_token_kernel(const __
 		stage_of_lane(st, par);
 		bool ok = (lane & 7) >= m || mbar_try_wait(full0 + 8 * st, par);
 		if (!__all_sync(kFull, ok)) {
+			dead = __any_sync(kFull, dead);
 			const long long t0 = clock64();
-			while (!lost) {
+			while (!dead) {
 				ok = (lane & 7) >= m || mbar_try_wait(full0 + 8 * st, par);
 				if (__all_sync(kFull, ok)) break;
-				lost = __any_sync(kFull, out_of_patience(t0));
+				dead = __any_sync(kFull, out_of_patience(t0));
 			}
-			dead = dead || lost;
 		}
 		__syncwarp();
 	};
@@ -300,7 +299,7 @@ __global__ void __launch_bounds__(kTokenThreads, 1) decode_token_kernel(const __
 		uint32_t st, par;
 		stage_of_lane(st, par);
 		__syncwarp();
-		if (lane < m && !lost) mbar_arrive(empty0 + 8 * st);
+		if (lane < m && !dead) mbar_arrive(empty0 + 8 * st); // (who gave up gives nothing back: it could be filled again under a copy on its way)
 		s += m;
 		if (s >= kTokenStages) s -= kTokenStages, sphase ^= 1;
 	};
