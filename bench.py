@@ -64,16 +64,18 @@ def peaks():
     return 6650.0, "fallback (B200_PROFILING.md)"
 
 
-def ncu_traffic():
-    """dram__bytes_read.sum + dram__bytes_write.sum of ONE timed-shape launch of the whole-token kernel on the headline
+def ncu_traffic(kernel):
+    """dram__bytes_read.sum + dram__bytes_write.sum of ONE timed-shape launch of the whole-token kernel named on the headline
     workload — logits mode at pos ~4090, captured with `ncu --set full` and summarised into
-    profiles/*logits*_full_summary.txt (tools/ncu_summary.py).  None if no such capture is committed."""
+    profiles/*logits*_full_summary.txt (tools/ncu_summary.py).  None if no capture of that kernel is committed."""
     import glob
     import re
     files = sorted(glob.glob(os.path.join(ROOT, "profiles", "*logits*full_summary.txt")))
     if not files:
         return None, None
     txt = open(files[-1]).read()
+    if not re.search(rf"\b{kernel}<", txt):
+        return None, None
     unit = {"byte": 1.0, "Kbyte": 1e3, "Mbyte": 1e6, "Gbyte": 1e9, "Tbyte": 1e12}
     tot = 0.0
     for key in ("dram__bytes_read.sum", "dram__bytes_write.sum"):
@@ -555,7 +557,7 @@ def main():
             kname = "ffn_glu_kernel (rmsnorm + w1/w3 GEMV + GLU)"
         achieved = ffn_bytes / (ffn_us * 1e-6) / 1e9
         # DRAM bytes of one launch from the committed ncu capture: only for the workload it was taken on
-        traffic, traffic_src = ncu_traffic() if (mega and world == 1 and args.workload == HEADLINE and not args.layers) else (None, None)
+        traffic, traffic_src = ncu_traffic(kname.split()[0]) if (mega and world == 1 and args.workload == HEADLINE and not args.layers) else (None, None)
         line = dict(base, impl="ours", value=tok_s, ms_per_step=dev_ms / K, clocks=clk,
                     e2e={"value": K / e2e_s, "unit": "tok/s", "h2d_bytes_per_step": 8, "d2h_bytes_per_step": 4 * V},
                     gpu_launches=(model.launches(api.MODE_LOGITS) + (0 if mega else 1)) * K,

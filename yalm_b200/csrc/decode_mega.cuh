@@ -1,5 +1,5 @@
-// Whole-token persistent decode kernel for sm_100a (see mega.h for the idea): mixtures of experts, tensor parallelism, rows of more than 16384 elements,
-// and the variants below.  Other dense models on one GPU run on the kernel of decode_token.cuh (chosen in plan(), decode_mega.cu).
+// Whole-token persistent decode kernel for sm_100a (see mega.h for the idea): mixtures of experts, tensor parallelism, dense models that it is faster at
+// (wide rows above all), and the variants below.  Other dense models on one GPU run on the kernel of decode_token.cuh (chosen in plan(), decode_mega.cu).
 //
 // Roles inside a CTA (one CTA per SM, cooperative launch so grid barriers and flag polling are safe):
 //   last warp   producer (all 32 lanes, one tile per lane and batch): walks this CTA's tile list for the WHOLE forward pass and

@@ -8,9 +8,9 @@
 // one's first stages are pulled into L2 (a prefetch only: whoever writes W before this kernel is seen).
 //
 // Feed-forward of a token (gate and up, then down), back to back, against a persistent grid of warps that load rows into registers and start
-// after x is staged: 4096 x 14336 fp16 74.3 -> 56.7 us (6.2 TB/s), fp8 47.9 -> 39.5, fp32 132.8 -> 104.4; 2752 x 7040 fp16 33.2 -> 25.3, 1024 x 2816 fp16
-// 16.5 -> 9.8.  What is left over the bytes at 6.9 TB/s is some 3 us a launch (barriers, x and its norm, the first bytes' latency, the last sums), and in
-// fp8 the conversions, two instructions an element.
+// after x is staged: 4096 x 14336 fp16 73.7 -> 55.6 us (6.3 TB/s), fp8 48.5 -> 38.7, fp32 133.2 -> 104.6; 2752 x 7040 fp16 33.1 -> 23.7, 1024 x 2816 fp16
+// 15.1 -> 8.3.  What is left over the bytes at 6.9 TB/s is some 3 us a launch (barriers, x and its norm, the first bytes' latency, the last sums), and in
+// fp8 the conversions, two instructions an element.  Which products come here: streamed(), ops_gemv.cu.
 #pragma once
 
 #include "gemv.cuh"
@@ -21,7 +21,7 @@ namespace yalm {
 namespace stream {
 
 constexpr int kWarps = 16, kThreads = 32 * (kWarps + 1), kConsumers = 32 * kWarps;
-constexpr int kStageMax = 16384, kRing = 212992, kMaxStages = 32, kCap = 256; // rows whose partial sums are held at once
+constexpr int kRing = 212992, kMaxStages = 32, kCap = 256;                    // rows whose partial sums are held at once
 constexpr int kHead = 1024;                                                   // barriers, the norm's sums
 constexpr int kSmem = kHead + kRing + kWarps * kCap * 4;
 
@@ -31,7 +31,7 @@ struct Args {
 	float *out;
 	float eps, alpha;
 	int act, n, d;                      // columns, rows (of each matrix)
-	int row_bytes, chunks, piece;       // 512-byte chunks of a row (the last may be ragged), of a piece (a row is NP pieces)
+	int row_bytes, piece;               // 512-byte chunks of a piece (a row is NP pieces, the last may be ragged)
 	int C, RG, units, stage_bytes, stages; // warps per row, rows side by side per matrix slot, rows (or row pairs) per block
 };
 
@@ -331,9 +331,9 @@ constexpr int longest(int bytes_per_element) { return (bytes_per_element == 1 ? 
 // a: all but the geometry, a.n <= longest().
 template <int DT, bool GLU>
 static int launch(Args &a, cudaStream_t st) {
-	a.row_bytes = a.n * WTraits<DT>::BYTES, a.chunks = (a.row_bytes + 511) / 512;
-	const int pieces = (a.chunks + 31) / 32, NP = pieces <= 2 ? pieces : 4;
-	a.piece = (a.chunks + NP - 1) / NP;
+	a.row_bytes = a.n * WTraits<DT>::BYTES;
+	const int chunks = (a.row_bytes + 511) / 512, pieces = (chunks + 31) / 32, NP = pieces <= 2 ? pieces : 4;
+	a.piece = (chunks + NP - 1) / NP;
 	const int JJ = a.piece > 16 || NP > 1 ? 2 : 1;
 	a.C = (a.piece + JJ - 1) / JJ;
 	a.RG = NP == 1 && JJ == 1 ? kWarps / a.C : 1, a.units = GLU ? a.RG : 2 * a.RG;

@@ -180,7 +180,7 @@ private:
 	float *_mega_tmp = nullptr; // x + first column half of w2 (YALM_MEGA_W2_SPLIT)
 	float *_mega_hbp = nullptr;        // pipelined hb (mega.h: Args::hbp, hb_cnt)
 	unsigned *_mega_hb_cnt = nullptr;
-	unsigned long long *_mega_ll = nullptr; // flagged hand-over buffers: x[2][dim] | hb | att | acc | ml (mega.h: Args::ll_*)
+	unsigned long long *_mega_ll = nullptr; // flagged hand-over buffers: x[2][dim] | hb | att | acc | ml | q | kv (mega.h: Args::ll_*)
 	unsigned _mega_seq = 0;
 	void *_arena = nullptr; // one device allocation behind all of the above
 };
