@@ -3,12 +3,12 @@
 //
 // Rows.  The G query heads that share a kv head are stacked, row r = (position r / G, head r % G), so a tile of 128 rows covers
 // 128 / G positions: a few positions already fill it, a causal edge wastes little, and every key tile is read once for all G heads.
-// A CTA owns two such tiles (A, B) of one kv head; a cluster of CTAs shares their keys where that fills the GPU, and joins
-// (sum, maximum, accumulator) through distributed shared memory in a fixed order.
+// A CTA owns two such tiles (A, B) of one kv head, or (SPLIT) one tile, for which A and B are its even and its odd key tiles, joined from TMEM at the
+// end; then a cluster of CTAs may share the keys too, and joins (sum, maximum, accumulator) through distributed shared memory in a fixed order.
 //
 // 12 warps.  Warp 0 streams key and value tiles of 128 positions with cp.async.bulk.tensor.3d into a ring of stages.  One thread of
 // warp 1 issues the products: S = Q K^T into TMEM, O += P V with P out of TMEM (its fp16 / bf16 words take the place of the scores).
-// Warps 4-7 and 8-11 are the softmax of tiles A and B, a thread per row: scores from TMEM, online maximum and sum in fp32, P back to
+// Warps 4-7 and 8-11 are the softmax of A and B, a thread per row: scores from TMEM, online maximum and sum in fp32, P back to
 // TMEM.  The two tiles alternate: while one's scores go through the softmax the tensor pipe works for the other.  O stays in TMEM and is
 // rescaled whenever a row's maximum grows, so that the weight of a row's largest score is 1 and takes no rounding.  (A reference that follows
 // only growth beyond 2^8 saves 0.3 to 8 us of the calls below, but rounds the weight that counts most: a row that one key dominates is then off by
@@ -18,7 +18,9 @@
 // Bound by the chain softmax - products of a tile pair (some 3500 cycles per 128 keys: 1800 from scores to weights, of which the exponentials
 // alone take 1024 at 16 a cycle and SM for each of the two tiles, 500 for the rescaling, and 1100 for P V and the next scores) and, for short
 // contexts, by launch, query staging and the store.  Back to back, against 64-row tiles on mma.sync: 507 rows at 7680 positions, 32 / 8 heads of 128:
-// 667 -> 80 us (825 TFLOP/s); 512 rows at 0: 32.8 -> 14.1 us; bf16 window 1024 and pooled blocks of 64, 512 rows, 16 / 4 heads: 57.3 -> 22.7 us.
+// 667 -> 67 us (980 TFLOP/s); 512 rows at 0: 32.8 -> 9.7 us; bf16 window 1024 and pooled blocks of 64, 512 rows, 16 / 4 heads: 57.3 -> 15.5 us.
+// Of these SPLIT, with the queries of fp16 calls as boxes of a tensor map, made 70.2 to 67.3, 14.1 to 9.7 and 22.7 to 15.5: in pairs of tiles whose keys two CTAs
+// share, staging took 2 us, and sending half of the accumulators (64 KB, some 20 bytes a cycle), both cluster barriers and the join 4 us.
 #include "common.cuh"
 #include "launch.h"
 #include "stack_rows.cuh"
@@ -45,7 +47,8 @@ struct Args {
 	const int *ctl;
 	float q_sign, c; // score (in powers of two) = c (q q_sign) . k
 	int parts;
-	int wide; // output rows are 16-byte aligned
+	int wide;  // output rows are 16-byte aligned
+	int q_map; // the queries come as boxes of the tensor map tq
 };
 
 // Key tiles of a CTA's rows: pooled blocks in tiles of 128 first, then the positions lo .. last in runs of slots that end at the ring's end.
@@ -87,6 +90,12 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map
 	             "r"(c0), "r"(c1), "r"(c2), "r"(bar)
 	             : "memory");
 }
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map, int c0, int c1, int c2, int c3, uint32_t bar) {
+	asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst), "l"(map),
+	             "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
+	             : "memory");
+}
+__device__ __forceinline__ void prefetch_map(const CUtensorMap *map) { asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory"); }
 // D[tmem] (+)= A[tmem] * B[smem]^T
 __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
 	asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d), "r"(tmem_a),
@@ -185,45 +194,49 @@ struct Shape {
 	static constexpr int DKP = DK < 64 ? 64 : DK, DVP = DV < 64 ? 64 : DV; // channels a row takes in shared memory
 	static constexpr int Q_BYTES = kTile * DKP * 2, K_BYTES = Q_BYTES, V_BYTES = kTile * DVP * 2, STAGE = K_BYTES > V_BYTES ? K_BYTES : V_BYTES;
 	static constexpr int STAGES = STAGE == 32768 ? 4 : 8;
-	static constexpr int SMEM = 2 * Q_BYTES + STAGES * STAGE + 512 + 1024;
+	static constexpr int smem(bool split) { return (split ? 1 : 2) * Q_BYTES + STAGES * STAGE + 512 + (split ? 2 * kTile * 8 : 0) + 1024; }
 };
 
 // T: operand type.  LAYERED: fp32 rows in and out, pooled blocks, ring tiles with rows that hold no position, sinks.
-template <typename T, int DK, int DV, bool LAYERED>
+// SPLIT: the CTA has one tile of rows, and A and B are its even and its odd key tiles.
+template <typename T, int DK, int DV, bool LAYERED, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 1)
-prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv, const __grid_constant__ Args a) {
+prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv,
+                   const __grid_constant__ Args a) {
 	using SH = Shape<DK, DV>;
-	constexpr int NST = SH::STAGES;
+	constexpr int NST = SH::STAGES, ROWS = SPLIT ? kTile : 2 * kTile; // rows of the CTA
 	extern __shared__ uint8_t smem_raw[];
-	const uint32_t base = (s32(smem_raw) + 1023u) & ~1023u, q0 = base, kv0 = q0 + 2 * SH::Q_BYTES, bars = kv0 + NST * SH::STAGE;
+	const uint32_t base = (s32(smem_raw) + 1023u) & ~1023u, q0 = base, kv0 = q0 + (ROWS / kTile) * SH::Q_BYTES, bars = kv0 + NST * SH::STAGE;
 	const uint32_t full0 = bars, empty0 = full0 + 8 * NST, s_full0 = empty0 + 8 * NST, p_full0 = s_full0 + 16, o_full = p_full0 + 32, v_clean0 = o_full + 8,
-	               tslot = v_clean0 + 8 * NST;
+	               q_full = v_clean0 + 8 * NST, tslot = q_full + 8;
 	const int warp = uniform_warp(), lane = threadIdx.x & 31;
-	const int parts = a.parts, part = parts > 1 ? (int)cluster_rank() : 0;
-	const int rows = a.n * a.G, pairs = (rows + 2 * kTile - 1) / (2 * kTile);
-	const int pair = pairs - 1 - (int)(blockIdx.x / parts); // the longest rows first
-	const int g = blockIdx.y, r0 = pair * 2 * kTile, nt = r0 + kTile < rows ? 2 : 1;
+	const int parts = SPLIT ? a.parts : 1, part = parts > 1 ? (int)cluster_rank() : 0;
+	const int rows = a.n * a.G, units = (rows + ROWS - 1) / ROWS;
+	const int unit = units - 1 - (int)(blockIdx.x / parts); // the longest rows first
+	const int g = blockIdx.y, r0 = unit * ROWS, nt = SPLIT || r0 + kTile < rows ? 2 : 1;
 	if (threadIdx.x == 0) {
 		// a value stage (odd) is free again once its products are done and, in a layered model, warps 2 and 3 have passed it
 		for (int i = 0; i < NST; ++i) mbar_init(full0 + 8 * i, 1), mbar_init(empty0 + 8 * i, LAYERED && (i & 1) ? 3 : 1);
 		for (int i = 0; i < 2; ++i) mbar_init(s_full0 + 8 * i, 1);
 		for (int i = 0; i < 4; ++i) mbar_init(p_full0 + 8 * i, 4); // [tile][half of the keys]
-		mbar_init(o_full, 1);
+		mbar_init(o_full, 1), mbar_init(q_full, 1);
 		if (LAYERED)
 			for (int i = 0; i < NST; ++i) mbar_init(v_clean0 + 8 * i, 1);
 		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 	}
+	if (warp == 0 && elect_one()) prefetch_map(&tk), prefetch_map(&tv), prefetch_map(&tq);
 	if (warp == 1) tmem_alloc<1>(tslot, 512);
 	tc_fence_before();
 	__syncthreads(); // (tensor memory is this CTA's before the next kernel may take any)
-	chain_wait();
-	chain_next();
-	tc_fence_after();
+	if (a.ctl) chain_wait(); // else the tiles' divisions run under the kernel before this one
 	const int p0 = a.ctl ? a.ctl[CTL_POS] : a.pos0;
-	const Tiles tiles(a, p0 + r0 / a.G, p0 + min((r0 + 2 * kTile - 1) / a.G, a.n - 1));
+	const Tiles tiles(a, p0 + r0 / a.G, p0 + min((r0 + ROWS - 1) / a.G, a.n - 1));
 	const int per = (tiles.total + parts - 1) / parts, k_begin = min(part * per, tiles.total), k_end = min(k_begin + per, tiles.total), nk = k_end - k_begin;
 	const bool first_pooled = LAYERED && nk > 0 && k_begin < tiles.pooled;
 	bool dead = false;
+	chain_wait();
+	chain_next();
+	tc_fence_after();
 
 	// Key / value tile i of this part (0, 1, ..) takes ring entries 2 i (keys) and 2 i + 1 (values).  Every round of a stage is waited
 	// for, also where the entry is not a copy: a parity tells neighbouring rounds apart and no more.
@@ -265,12 +278,19 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 
 	if (warp == 0) {
 		__syncwarp();
+		if (!LAYERED && a.q_map && elect_one()) { // a box is the 128 / G positions of a tile, all G heads of each; positions past the last are zero
+			mbar_expect_tx(q_full, (ROWS / kTile == 2 && nt == 2 ? 2 : 1) * SH::Q_BYTES);
+			for (int t = 0; t < (SPLIT ? 1 : nt); ++t)
+				for (int c = 0; c < SH::DKP; c += 64)
+					tma_load_4d(q0 + t * SH::Q_BYTES + (c / 64) * (kTile * 128), &tq, c, 0, g, (r0 + t * kTile) / a.G, q_full);
+		}
+		__syncwarp();
 		for (int e = 0; e < NST && e < 2 * nk; ++e) load(e >> 1, e & 1); // the stages are free: the first tiles travel while the queries are staged
 	}
-	if (warp > 0) { // the queries' rows (rows past the last: zero), and the first tile where it is a pooled one
+	if (warp > 0 && (LAYERED || !a.q_map)) { // the queries' rows (rows past the last: zero), and the first tile where it is a pooled one
 		// a thread keeps its 16-byte column and steps down the rows (the position and head of a row follow without a division); all loads of
 		// a batch are in flight together: one at a time this took as long as four key tiles
-		constexpr int PIECES = DK / 8, DOWN = (kThreads - 32) / PIECES, STEPS = (2 * kTile + DOWN - 1) / DOWN, BATCH = LAYERED ? (STEPS + 1) / 2 : STEPS;
+		constexpr int PIECES = DK / 8, DOWN = (kThreads - 32) / PIECES, STEPS = (ROWS + DOWN - 1) / DOWN, BATCH = LAYERED && !SPLIT ? (STEPS + 1) / 2 : STEPS;
 		const int c = (threadIdx.x - 32) % PIECES, di = DOWN / a.G, dh = DOWN % a.G;
 		int r = (threadIdx.x - 32) / PIECES, i = (r0 + r) / a.G, hh = (r0 + r) % a.G;
 		for (int s0 = 0; s0 < STEPS; s0 += BATCH) {
@@ -280,7 +300,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 			for (int b = 0; b < BATCH; ++b) {
 				lo[b] = make_float4(0.f, 0.f, 0.f, 0.f);
 				if constexpr (LAYERED) hi[b] = lo[b];
-				if (r < 2 * kTile && r0 + r < rows) {
+				if (r < ROWS && r0 + r < rows) {
 					if constexpr (LAYERED) {
 						const float *src = static_cast<const float *>(a.q) + (size_t)i * a.ldq + (size_t)(g * a.G + hh) * DK + c * 8;
 						lo[b] = *reinterpret_cast<const float4 *>(src), hi[b] = *reinterpret_cast<const float4 *>(src + 4);
@@ -293,7 +313,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 #pragma unroll
 			for (int b = 0; b < BATCH; ++b) {
 				const int rr = first + b * DOWN;
-				if (rr >= 2 * kTile) break;
+				if (rr >= ROWS) break;
 				float4 v = lo[b];
 				if constexpr (LAYERED) {
 					const float f = a.q_sign;
@@ -328,7 +348,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 				tc_fence_after();
 			};
 			auto scores = [&](int t, int e) {
-				const uint64_t qa = smem_desc_sw128(q0 + t * SH::Q_BYTES), ka = smem_desc_sw128(kv0 + (e % NST) * SH::STAGE);
+				const uint64_t qa = smem_desc_sw128(q0 + (SPLIT ? 0 : t) * SH::Q_BYTES), ka = smem_desc_sw128(kv0 + (e % NST) * SH::STAGE);
 				if (elect_one()) {
 #pragma unroll
 					for (int k = 0; k < DK / 16; ++k) {
@@ -339,11 +359,8 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 				}
 			};
 			uint32_t cleaned = 0; // a bit per stage: parity of its rounds of clearing
-			wait_full(0);
-			for (int t = 0; t < nt; ++t) scores(t, 0);
-			if (elect_one()) umma_commit(empty0);
-			for (int i = 0; i < nk && !dead; ++i) {
-				const int ev = 2 * i + 1, ek = 2 * i + 2;
+			auto wait_values = [&](int i) {
+				const int ev = 2 * i + 1;
 				wait_full(ev);
 				if constexpr (LAYERED) {
 					int slot, pos, valid;
@@ -354,23 +371,50 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 						tc_fence_after();
 					}
 				}
+			};
+			auto products = [&](int t, int i, int round, bool last) { // weights of round `round` of t times the values of tile i
+				const int ev = 2 * i + 1;
 				const uint64_t vdesc = desc_mn(kv0 + (ev % NST) * SH::STAGE);
-				for (int t = 0; t < nt; ++t) {
 #pragma unroll
-					for (int half = 0; half < 2; ++half) {
-						mbar_wait_warp(p_full0 + 16 * t + 8 * half, (uint32_t)i & 1u, dead);
-						tc_fence_after();
-						if (elect_one()) {
+				for (int half = 0; half < 2; ++half) {
+					mbar_wait_warp(p_full0 + 16 * t + 8 * half, (uint32_t)round & 1u, dead);
+					tc_fence_after();
+					if (elect_one()) {
 #pragma unroll
-							for (int k = 4 * half; k < 4 * half + 4; ++k) // 16 positions = 2048 bytes further in every sub-tile, 8 columns of P
-								umma_ts(tmem + 256 + t * SH::DVP, tmem + t * kTile + 8 * k, vdesc + (2048 >> 4) * k, pv_desc, (i | k) != 0);
-							if (half && t == nt - 1) umma_commit(empty0 + 8 * (ev % NST));
-						}
+						for (int k = 4 * half; k < 4 * half + 4; ++k) // 16 positions = 2048 bytes further in every sub-tile, 8 columns of P
+							umma_ts(tmem + 256 + t * SH::DVP, tmem + t * kTile + 8 * k, vdesc + (2048 >> 4) * k, pv_desc, (round | k) != 0);
+						if (half && last) umma_commit(empty0 + 8 * (ev % NST));
 					}
-					if (i + 1 < nk) {
-						if (t == 0) wait_full(ek);
-						scores(t, ek);
-						if (t == nt - 1 && elect_one()) umma_commit(empty0 + 8 * (ek % NST));
+				}
+			};
+			if (!LAYERED && a.q_map) mbar_wait_warp(q_full, 0, dead);
+			if constexpr (SPLIT) {
+				auto next_scores = [&](int i) {
+					wait_full(2 * i);
+					scores(i & 1, 2 * i);
+					if (elect_one()) umma_commit(empty0 + 8 * (2 * i % NST));
+				};
+				next_scores(0);
+				if (nk > 1) next_scores(1);
+				for (int i = 0; i < nk && !dead; ++i) {
+					wait_values(i);
+					products(i & 1, i, i >> 1, true);
+					if (i + 2 < nk) next_scores(i + 2);
+				}
+			} else {
+				wait_full(0);
+				for (int t = 0; t < nt; ++t) scores(t, 0);
+				if (elect_one()) umma_commit(empty0);
+				for (int i = 0; i < nk && !dead; ++i) {
+					const int ek = 2 * i + 2;
+					wait_values(i);
+					for (int t = 0; t < nt; ++t) {
+						products(t, i, i, t == nt - 1);
+						if (i + 1 < nk) {
+							if (t == 0) wait_full(ek);
+							scores(t, ek);
+							if (t == nt - 1 && elect_one()) umma_commit(empty0 + 8 * (ek % NST));
+						}
 					}
 				}
 			}
@@ -406,17 +450,18 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 		}
 		__syncwarp();
 	} else {
-		const int t = (warp - 4) >> 2, q = warp & 3, r = r0 + t * kTile + q * 32 + lane;
+		const int t = (warp - 4) >> 2, q = warp & 3, r = r0 + (SPLIT ? 0 : t * kTile) + q * 32 + lane;
 		if (t < nt && nk > 0) { // ---- softmax: one row per thread ----
 			const int i = p0 + min(r, rows - 1) / a.G; // rows past the last repeat it: finite values that are never stored
 			const int lo = Tiles::lo_of(a, i), nb = LAYERED ? Tiles::blocks_of(a, i) : 0;
 			const uint32_t lanes = (uint32_t)(q * 32) << 16, sp = tmem + lanes + t * kTile, op = tmem + lanes + 256 + t * SH::DVP;
 			const float c = a.c;
-			for (int k = 0; k < nk; ++k) {
+			for (int k = SPLIT ? t : 0; k < nk; k += SPLIT ? 2 : 1) {
+				const int round = SPLIT ? k >> 1 : k;
 				int slot, pos, valid;
 				const bool pooled = tiles.at(k_begin + k, slot, pos, valid);
 				const int from = pooled ? 0 : lo - pos, to = pooled ? nb - slot - 1 : min(i - pos, valid - 1); // visible: from .. to of the tile
-				mbar_wait_warp(s_full0 + 8 * t, (uint32_t)k & 1u, dead);
+				mbar_wait_warp(s_full0 + 8 * t, (uint32_t)round & 1u, dead);
 				__syncwarp();
 				tc_fence_after();
 				uint32_t s[kTile];
@@ -447,7 +492,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 					const float f = grow ? ex2(mref - top) : 1.0f; // mref -inf: 0
 					if (grow) mref = top;
 					l *= f;
-					if (k > 0) { // the products into O so far are complete: they were issued before these scores
+					if (round > 0) { // the products into O so far are complete: they were issued before these scores
 #pragma unroll 1
 						for (int x = 0; x < DV; x += 32) {
 							uint32_t o[32];
@@ -490,38 +535,67 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 		}
 	}
 
-	// ---- the rows' results: this part finishes columns part DV / parts .. of both tiles ----
+	// ---- the rows' results: this part finishes columns part DV / parts .. of its rows; in SPLIT each group of softmax warps half of these ----
 	const bool softmax_warp = warp >= 4;
-	const int t = (warp - 4) >> 2, q = warp & 3, tr = q * 32 + lane, row = r0 + t * kTile + tr, share = DV / parts;
-	const uint32_t op = tmem + ((uint32_t)(q * 32) << 16) + 256 + t * SH::DVP;
-	// from the start of shared memory (queries and stages are done with): [other part][tile][4 columns][row][4], then (reference, sum) [part][row of 256]
-	const uint32_t ml0 = base + (uint32_t)((parts - 1) * 2 * share * kTile * 4);
+	const int t = (warp - 4) >> 2, q = warp & 3, tr = q * 32 + lane, row = r0 + (SPLIT ? 0 : t * kTile) + tr, share = DV / parts;
+	const int mine = SPLIT ? share / 2 : share, first_col = SPLIT ? t * mine : 0; // columns that a thread handles of a share, from where
+	const uint32_t op = tmem + ((uint32_t)(q * 32) << 16) + 256 + (SPLIT ? 0 : t * SH::DVP);
+	// from the start of shared memory (queries and stages are done with): [other part][4 columns][row][4], then (reference, sum) [part][row]
+	const uint32_t ml0 = base + (uint32_t)((parts - 1) * share * kTile * 4);
 	if (dead) l = __int_as_float(0x7fc00000);
 	__syncwarp();
+	float w0 = 1.f, w1 = 1.f; // SPLIT: factors of the sums over the even and the odd key tiles
+	bool any0 = true, any1 = true; // whether this row sees any of them (where not, the accumulator may hold anything)
+	if constexpr (SPLIT) {
+		if (softmax_warp) {
+			const uint32_t merge = bars + 512; // (reference, sum) [even, odd][row], behind everything else
+			asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(merge + (uint32_t)((t * kTile + tr) * 8)), "f"(mref), "f"(l) : "memory");
+			asm volatile("bar.sync 2, 256;" ::: "memory");
+			float m0, l0, m1, l1;
+			asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(m0), "=f"(l0) : "r"(merge + (uint32_t)(tr * 8)) : "memory");
+			asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(m1), "=f"(l1) : "r"(merge + (uint32_t)((kTile + tr) * 8)) : "memory");
+			mref = fmaxf(m0, m1);
+			any0 = l0 != 0.f, any1 = l1 != 0.f, w0 = ex2(m0 - mref), w1 = ex2(m1 - mref);
+			l = (any0 ? w0 * l0 : 0.f) + (any1 ? w1 * l1 : 0.f);
+		}
+	}
+	// W columns from x on of this thread's row, of this part's keys
+	auto own_columns = [&](auto &v, int x) {
+		constexpr int W = sizeof(v) / 4;
+		if constexpr (SPLIT) {
+			float odd[W];
+			if constexpr (W == 32) tmem_ld32(op + x, v), tmem_ld32(op + SH::DVP + x, odd);
+			else tmem_ld8(op + x, v), tmem_ld8(op + SH::DVP + x, odd);
+#pragma unroll
+			for (int y = 0; y < W; ++y) {
+				v[y] = any0 ? w0 * v[y] : 0.f;
+				if (any1) v[y] = fmaf(w1, odd[y], v[y]);
+			}
+		} else {
+			if constexpr (W == 32) tmem_ld32(op + x, v);
+			else tmem_ld8(op + x, v);
+		}
+	};
 	if (parts > 1) {
 		cluster_sync(); // every part is done with its shared memory
-		if (softmax_warp && t < nt) {
+		if (softmax_warp) {
 			for (int p = 0; p < parts; ++p) {
 				const uint32_t there = map_rank(base, (uint32_t)p);
-				asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(there + (ml0 - base) + (uint32_t)((part * 2 * kTile + t * kTile + tr) * 8)), "f"(mref), "f"(l)
-				             : "memory");
+				if (t == 0)
+					asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(there + (ml0 - base) + (uint32_t)((part * kTile + tr) * 8)), "f"(mref), "f"(l) : "memory");
 				if (p == part || nk == 0) continue;
-				const uint32_t dst = there + (uint32_t)(((part < p ? part : part - 1) * 2 + t) * share * kTile * 4);
-				if (share % 32 == 0) {
-					for (int x = 0; x < share; x += 32) {
-						float v[32];
-						tmem_ld32(op + p * share + x, v);
+				const uint32_t dst = there + (uint32_t)((part < p ? part : part - 1) * share * kTile * 4);
+				auto send = [&](auto width, int x) {
+					constexpr int W = decltype(width)::value;
+					float v[W];
+					own_columns(v, p * share + x);
 #pragma unroll
-						for (int y = 0; y < 32; y += 4) st_cluster4(dst + (uint32_t)((((x + y) >> 2) * kTile + tr) * 16), make_float4(v[y], v[y + 1], v[y + 2], v[y + 3]));
-					}
-				} else {
-					for (int x = 0; x < share; x += 8) {
-						float v[8];
-						tmem_ld8(op + p * share + x, v);
-						st_cluster4(dst + (uint32_t)(((x >> 2) * kTile + tr) * 16), make_float4(v[0], v[1], v[2], v[3]));
-						st_cluster4(dst + (uint32_t)((((x >> 2) + 1) * kTile + tr) * 16), make_float4(v[4], v[5], v[6], v[7]));
-					}
-				}
+					for (int y = 0; y < W; y += 4) st_cluster4(dst + (uint32_t)((((x + y) >> 2) * kTile + tr) * 16), make_float4(v[y], v[y + 1], v[y + 2], v[y + 3]));
+				};
+				if (mine % 32 == 0)
+					for (int x = first_col; x < first_col + mine; x += 32) send(Width<32>(), x);
+				else
+					for (int x = first_col; x < first_col + mine; x += 8) send(Width<8>(), x);
 			}
 		}
 		__syncwarp();
@@ -530,7 +604,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 	if (softmax_warp && t < nt) {
 		float M = mref, Lsum = l;
 		auto of_part = [&](int p, float &pm, float &pl) {
-			asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(pm), "=f"(pl) : "r"(ml0 + (uint32_t)((p * 2 * kTile + t * kTile + tr) * 8)) : "memory");
+			asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(pm), "=f"(pl) : "r"(ml0 + (uint32_t)((p * kTile + tr) * 8)) : "memory");
 		};
 		if (parts > 1) {
 			M = -INFINITY, Lsum = 0.f;
@@ -549,23 +623,20 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 		float f = LAYERED ? stack::softmax_finish(M * 0.69314718055994531f, Lsum, a.sink, h) : 1.0f / Lsum;
 		// through a patch of shared memory per warp (after what the parts exchanged), so that neighbouring lanes store neighbouring
 		// bytes: a row per lane, every 16-byte piece went to a line of its own (5 us for 256 rows of 128)
-		const uint32_t ld = (uint32_t)share * 4 + 16, patch = ml0 + (parts > 1 ? parts * 2 * kTile * 8 : 0) + (warp - 4) * 32 * ld;
+		const uint32_t ld = (uint32_t)mine * 4 + 16, patch = ml0 + (parts > 1 ? parts * kTile * 8 : 0) + (warp - 4) * 32 * ld;
 		auto put = [&](int x, float4 v) { st_shared4(patch + lane * ld + x * 4, make_float4(v.x * f, v.y * f, v.z * f, v.w * f)); };
-		if (parts == 1) {
+		auto join = [&](auto width, int x) { // columns x .. x + width - 1 of this thread's, the parts of the keys in order
+			constexpr int W = decltype(width)::value;
+			float own[W];
+			__syncwarp();
+			own_columns(own, part * share + first_col + x);
+			if (parts == 1) {
 #pragma unroll
-			for (int x = 0; x < DV; x += 32) {
-				float v[32];
-				tmem_ld32(op + x, v);
-#pragma unroll
-				for (int y = 0; y < 32; y += 4) put(x + y, make_float4(v[y], v[y + 1], v[y + 2], v[y + 3]));
+				for (int y = 0; y < W; y += 4) put(x + y, make_float4(own[y], own[y + 1], own[y + 2], own[y + 3]));
+				return;
 			}
-		} else {
-			auto join = [&](auto width, int x) { // columns x .. x + width - 1 of the share, the parts of the keys in order
-				constexpr int W = decltype(width)::value;
-				float v[W], own[W];
-				__syncwarp();
-				if constexpr (W == 32) tmem_ld32(op + part * share + x, own);
-				else tmem_ld8(op + part * share + x, own);
+			if constexpr (SPLIT) {
+				float v[W];
 #pragma unroll
 				for (int y = 0; y < W; ++y) v[y] = 0.f;
 				for (int p = 0; p < parts; ++p) {
@@ -577,27 +648,28 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 #pragma unroll
 						for (int y = 0; y < W; ++y) v[y] += w * own[y];
 					} else {
-						const uint32_t src = base + (uint32_t)(((p < part ? p : p - 1) * 2 + t) * share * kTile * 4);
+						const uint32_t src = base + (uint32_t)((p < part ? p : p - 1) * share * kTile * 4);
 #pragma unroll
 						for (int y = 0; y < W; y += 4) {
-							const float4 o = ld_shared4(src + (uint32_t)((((x + y) >> 2) * kTile + tr) * 16));
+							const float4 o = ld_shared4(src + (uint32_t)((((first_col + x + y) >> 2) * kTile + tr) * 16));
 							v[y] += w * o.x, v[y + 1] += w * o.y, v[y + 2] += w * o.z, v[y + 3] += w * o.w;
 						}
 					}
 				}
 #pragma unroll
 				for (int y = 0; y < W; y += 4) put(x + y, make_float4(v[y], v[y + 1], v[y + 2], v[y + 3]));
-			};
-			if (share % 32 == 0)
-				for (int x = 0; x < share; x += 32) join(Width<32>(), x);
-			else
-				for (int x = 0; x < share; x += 8) join(Width<8>(), x);
-		}
+			}
+		};
+		if (mine % 32 == 0)
+			for (int x = 0; x < mine; x += 32) join(Width<32>(), x);
+		else
+			for (int x = 0; x < mine; x += 8) join(Width<8>(), x);
 		__syncwarp();
-		const int pieces = LAYERED ? share / 4 : share / 8, lg = 31 - __clz(pieces); // 16-byte pieces of a row's share: a power of two up to 32
+		const int pieces = LAYERED ? mine / 4 : mine / 8, lg = 31 - __clz(pieces); // 16-byte pieces of a row: a power of two up to 32
 		const int down = 32 >> lg, cc = lane & (pieces - 1), di = down / a.G, dh = down % a.G;
-		int rr = lane >> lg, to = r0 + t * kTile + q * 32 + rr, i = to / a.G, hh = to % a.G;
-		for (; rr < 32 && r0 + t * kTile + q * 32 + rr - (lane >> lg) < rows;) { // (ends after the warp's last valid row)
+		const int row0 = row - lane;
+		int rr = lane >> lg, to = row0 + rr, i = to / a.G, hh = to % a.G;
+		for (; rr < 32 && row0 + rr - (lane >> lg) < rows;) { // (ends after the warp's last valid row)
 			constexpr int BATCH = 8; // reads first, then stores
 			float4 lo[BATCH], hi[LAYERED ? 1 : BATCH];
 #pragma unroll
@@ -609,7 +681,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 #pragma unroll
 			for (int x = 0; x < BATCH; ++x) {
 				if (rr < 32 && to < rows) {
-					const int col = (g * a.G + hh) * DV + part * share;
+					const int col = (g * a.G + hh) * DV + part * share + first_col;
 					if constexpr (LAYERED) {
 						float *dst = static_cast<float *>(a.out) + (size_t)i * a.ldo + col + cc * 4;
 						if (a.wide) *reinterpret_cast<float4 *>(dst) = lo[x];
@@ -666,26 +738,38 @@ static int make_map(CUtensorMap *map, const void *ptr, int d, int rows, int ring
 	return r == CUDA_SUCCESS ? 0 : YALM_EINVAL;
 }
 
-// Parts of the keys: as many as still run all at once and leave every part at least 2 key tiles (the exchange costs about one and a
-// half: 512 rows at position 0, 32 heads, 4 tiles: 18.7 us in one part, 16.7 in two).  est_tiles: key tiles of the longest rows.
-template <typename T, int DK, int DV, bool LAYERED>
-static int launch(Args &a, const void *keys, const void *values, int map_rows, int est_tiles, cudaStream_t st) {
+// (n, kv heads, G, d) queries -> boxes of 64 channels x the G heads of one kv head x 128 / G positions: the rows of a tile, in their order
+static int make_query_map(CUtensorMap *map, const void *ptr, int d, int G, int n_kv, int n) {
+	EncodeTiledFn fn = encode_fn();
+	if (!fn) return YALM_EINVAL;
+	const cuuint64_t dims[4] = {(cuuint64_t)d, (cuuint64_t)G, (cuuint64_t)n_kv, (cuuint64_t)n};
+	const cuuint64_t strides[3] = {(cuuint64_t)d * 2, (cuuint64_t)G * d * 2, (cuuint64_t)n_kv * G * d * 2};
+	const cuuint32_t box[4] = {64, (cuuint32_t)G, 1, (cuuint32_t)(kTile / G)}, estr[4] = {1, 1, 1, 1};
+	const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<void *>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+	                      CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+	return r == CUDA_SUCCESS ? 0 : YALM_EINVAL;
+}
+
+// est_tiles: key tiles of the longest rows.
+template <typename T, int DK, int DV, bool LAYERED, bool SPLIT>
+static int launch_of(Args &a, const void *keys, const void *values, int map_rows, int est_tiles, cudaStream_t st) {
 	using SH = Shape<DK, DV>;
 	static int at_once[kMaxDevices][4]; // clusters of 1, 2, 4, 8 CTAs; 0: not asked yet
 	static std::mutex mu;
-	auto kernel = prompt_attn_kernel<T, DK, DV, LAYERED>;
+	constexpr int ROWS = SPLIT ? kTile : 2 * kTile, SMEM = SH::smem(SPLIT);
+	auto kernel = prompt_attn_kernel<T, DK, DV, LAYERED, SPLIT>;
 	const DeviceInfo &dev = device_info();
 	if (dev.device < 0 || dev.device >= kMaxDevices) return YALM_EINVAL;
 	cudaLaunchConfig_t cfg = {};
 	cudaLaunchAttribute at[1];
 	at[0].id = cudaLaunchAttributeClusterDimension;
 	at[0].val.clusterDim.x = 1, at[0].val.clusterDim.y = 1, at[0].val.clusterDim.z = 1;
-	cfg.blockDim = dim3(kThreads), cfg.dynamicSmemBytes = SH::SMEM, cfg.attrs = at, cfg.numAttrs = 1;
+	cfg.blockDim = dim3(kThreads), cfg.dynamicSmemBytes = SMEM, cfg.attrs = at, cfg.numAttrs = 1;
 	int room[4];
 	{
 		std::lock_guard<std::mutex> lock(mu);
 		if (!at_once[dev.device][0]) {
-			YALM_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SH::SMEM));
+			YALM_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
 			for (int i = 3; i >= 0; --i) {
 				at[0].val.clusterDim.x = 1 << i, cfg.gridDim = dim3(1 << i);
 				YALM_TRY(cudaOccupancyMaxActiveClusters(&at_once[dev.device][i], kernel, &cfg));
@@ -693,14 +777,28 @@ static int launch(Args &a, const void *keys, const void *values, int map_rows, i
 		}
 		for (int i = 0; i < 4; ++i) room[i] = at_once[dev.device][i];
 	}
-	CUtensorMap tk, tv;
+	CUtensorMap tq, tk, tv;
 	int rc = make_map(&tk, keys, DK, map_rows, a.ring, a.n_kv, LAYERED);
 	if (!rc) rc = make_map(&tv, values, DV, map_rows, a.ring, a.v_heads, LAYERED);
+	a.q_map = !LAYERED && kTile % a.G == 0;
+	if (!rc && a.q_map) rc = make_query_map(&tq, a.q, DK, a.G, a.n_kv, a.n);
+	else tq = tk;
 	if (rc) return rc;
-	const int pairs = (a.n * a.G + 2 * kTile - 1) / (2 * kTile), units = pairs * a.n_kv;
+	const int row_units = (a.n * a.G + ROWS - 1) / ROWS, units = row_units * a.n_kv;
 	a.parts = 1;
-	for (int i = 1; i < 4 && (1 << i) <= DV / 8 && units <= room[i] && est_tiles >= (2 << i); ++i) a.parts = 1 << i;
-	return launch_chained(kernel, dim3(pairs * a.parts, a.n_kv), dim3(kThreads), SH::SMEM, st, a.parts, tk, tv, a);
+	if (SPLIT && est_tiles >= 4)
+		for (int i = 1; i < 4 && (1 << i) <= DV / 16 && units <= room[i] && est_tiles > (1 << i); ++i) a.parts = 1 << i;
+	return launch_chained(kernel, dim3(row_units * a.parts, a.n_kv), dim3(kThreads), SMEM, st, a.parts, tq, tk, tv, a);
+}
+// One tile of rows a CTA while these run all at once, one per SM, and two beyond, which read a key tile once for both (64 / 8 heads of 128, 512 rows: at 0
+// 17.3 us in single tiles, 14.5 in pairs, at 7680 132 and 128).  Where tiles of rows leave SMs idle, a cluster shares the keys: as many parts as still run all at
+// once, at least four key tiles in all and more tiles than parts (17 rows, 32 / 8 heads of 128: three key tiles in one part 7.8 us, in two 8.4; five in two 9.7, in
+// four 9.2; nine, 128 rows of 8 / 2 heads, in four 10.9, in eight 9.9).
+template <typename T, int DK, int DV, bool LAYERED>
+static int launch(Args &a, const void *keys, const void *values, int map_rows, int est_tiles, cudaStream_t st) {
+	const long tiles = (long)((a.n * (long)a.G + kTile - 1) / kTile) * a.n_kv;
+	return tiles <= device_info().sms ? launch_of<T, DK, DV, LAYERED, true>(a, keys, values, map_rows, est_tiles, st)
+	                                  : launch_of<T, DK, DV, LAYERED, false>(a, keys, values, map_rows, est_tiles, st);
 }
 
 constexpr float kLog2e = 1.4426950408889634f;
