@@ -18,8 +18,8 @@
 // Bound by the chain softmax - products of a tile pair (some 3500 cycles per 128 keys: 1800 from scores to weights, of which the exponentials
 // alone take 1024 at 16 a cycle and SM for each of the two tiles, 500 for the rescaling, and 1100 for P V and the next scores) and, for short
 // contexts, by launch, query staging and the store.  Back to back, against 64-row tiles on mma.sync: 507 rows at 7680 positions, 32 / 8 heads of 128:
-// 667 -> 67 us (980 TFLOP/s); 512 rows at 0: 32.8 -> 9.7 us; bf16 window 1024 and pooled blocks of 64, 512 rows, 16 / 4 heads: 57.3 -> 15.5 us.
-// Of these SPLIT, with the queries of fp16 calls as boxes of a tensor map, made 70.2 to 67.3, 14.1 to 9.7 and 22.7 to 15.5: in pairs of tiles whose keys two CTAs
+// 667 -> 67 us (980 TFLOP/s); 512 rows at 0: 32.8 -> 9.3 us; bf16 window 1024 and pooled blocks of 64, 512 rows, 16 / 4 heads: 57.3 -> 15.5 us.
+// Of these SPLIT, with the queries of fp16 calls as boxes of a tensor map, made 70.2 to 67.3, 14.1 to 9.3 and 22.7 to 15.5: in pairs of tiles whose keys two CTAs
 // share, staging took 2 us, and sending half of the accumulators (64 KB, some 20 bytes a cycle), both cluster barriers and the join 4 us.
 #include "common.cuh"
 #include "launch.h"
@@ -93,6 +93,10 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map
 __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map, int c0, int c1, int c2, int c3, uint32_t bar) {
 	asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst), "l"(map),
 	             "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
+	             : "memory");
+}
+__device__ __forceinline__ void tma_store_4d(const CUtensorMap *map, int c0, int c1, int c2, int c3, uint32_t src) {
+	asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%1, %2, %3, %4}], [%5];" ::"l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(src)
 	             : "memory");
 }
 __device__ __forceinline__ void prefetch_map(const CUtensorMap *map) { asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory"); }
@@ -199,10 +203,11 @@ struct Shape {
 
 // T: operand type.  LAYERED: fp32 rows in and out, pooled blocks, ring tiles with rows that hold no position, sinks.
 // SPLIT: the CTA has one tile of rows, and A and B are its even and its odd key tiles.
-template <typename T, int DK, int DV, bool LAYERED, bool SPLIT>
+// BOXES (the keys in one part): the results leave as boxes of the tensor map to.
+template <typename T, int DK, int DV, bool LAYERED, bool SPLIT, bool BOXES>
 __global__ void __launch_bounds__(kThreads, 1)
 prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv,
-                   const __grid_constant__ Args a) {
+                   const __grid_constant__ CUtensorMap to, const __grid_constant__ Args a) {
 	using SH = Shape<DK, DV>;
 	constexpr int NST = SH::STAGES, ROWS = SPLIT ? kTile : 2 * kTile; // rows of the CTA
 	extern __shared__ uint8_t smem_raw[];
@@ -210,7 +215,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 	const uint32_t full0 = bars, empty0 = full0 + 8 * NST, s_full0 = empty0 + 8 * NST, p_full0 = s_full0 + 16, o_full = p_full0 + 32, v_clean0 = o_full + 8,
 	               q_full = v_clean0 + 8 * NST, tslot = q_full + 8;
 	const int warp = uniform_warp(), lane = threadIdx.x & 31;
-	const int parts = SPLIT ? a.parts : 1, part = parts > 1 ? (int)cluster_rank() : 0;
+	const int parts = SPLIT && !BOXES ? a.parts : 1, part = parts > 1 ? (int)cluster_rank() : 0;
 	const int rows = a.n * a.G, units = (rows + ROWS - 1) / ROWS;
 	const int unit = units - 1 - (int)(blockIdx.x / parts); // the longest rows first
 	const int g = blockIdx.y, r0 = unit * ROWS, nt = SPLIT || r0 + kTile < rows ? 2 : 1;
@@ -224,7 +229,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 			for (int i = 0; i < NST; ++i) mbar_init(v_clean0 + 8 * i, 1);
 		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 	}
-	if (warp == 0 && elect_one()) prefetch_map(&tk), prefetch_map(&tv), prefetch_map(&tq);
+	if (warp == 0 && elect_one()) prefetch_map(&tk), prefetch_map(&tv), prefetch_map(&tq), prefetch_map(&to);
 	if (warp == 1) tmem_alloc<1>(tslot, 512);
 	tc_fence_before();
 	__syncthreads(); // (tensor memory is this CTA's before the next kernel may take any)
@@ -624,7 +629,16 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 		// through a patch of shared memory per warp (after what the parts exchanged), so that neighbouring lanes store neighbouring
 		// bytes: a row per lane, every 16-byte piece went to a line of its own (5 us for 256 rows of 128)
 		const uint32_t ld = (uint32_t)mine * 4 + 16, patch = ml0 + (parts > 1 ? parts * kTile * 8 : 0) + (warp - 4) * 32 * ld;
-		auto put = [&](int x, float4 v) { st_shared4(patch + lane * ld + x * 4, make_float4(v.x * f, v.y * f, v.z * f, v.w * f)); };
+		// or all rows of a tile as fp16 in the layout of an operand tile, which the copy engine stores: no reads back, no addresses, rows past the last left out
+		const uint32_t tile = base + (SPLIT ? 0 : t * SH::Q_BYTES);
+		auto put = [&](int x, float4 v, float4 w) { // 8 columns
+			v = make_float4(v.x * f, v.y * f, v.z * f, v.w * f), w = make_float4(w.x * f, w.y * f, w.z * f, w.w * f);
+			if constexpr (BOXES) {
+				st_shared4(tile + tile_at(tr, (first_col + x) / 8), make_float4(__uint_as_float(pack2<T>(v.x, v.y)), __uint_as_float(pack2<T>(v.z, v.w)),
+				                                                                __uint_as_float(pack2<T>(w.x, w.y)), __uint_as_float(pack2<T>(w.z, w.w))));
+			} else
+				st_shared4(patch + lane * ld + x * 4, v), st_shared4(patch + lane * ld + x * 4 + 16, w);
+		};
 		auto join = [&](auto width, int x) { // columns x .. x + width - 1 of this thread's, the parts of the keys in order
 			constexpr int W = decltype(width)::value;
 			float own[W];
@@ -632,10 +646,11 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 			own_columns(own, part * share + first_col + x);
 			if (parts == 1) {
 #pragma unroll
-				for (int y = 0; y < W; y += 4) put(x + y, make_float4(own[y], own[y + 1], own[y + 2], own[y + 3]));
+				for (int y = 0; y < W; y += 8)
+					put(x + y, make_float4(own[y], own[y + 1], own[y + 2], own[y + 3]), make_float4(own[y + 4], own[y + 5], own[y + 6], own[y + 7]));
 				return;
 			}
-			if constexpr (SPLIT) {
+			if constexpr (SPLIT && !BOXES) {
 				float v[W];
 #pragma unroll
 				for (int y = 0; y < W; ++y) v[y] = 0.f;
@@ -657,7 +672,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 					}
 				}
 #pragma unroll
-				for (int y = 0; y < W; y += 4) put(x + y, make_float4(v[y], v[y + 1], v[y + 2], v[y + 3]));
+				for (int y = 0; y < W; y += 8) put(x + y, make_float4(v[y], v[y + 1], v[y + 2], v[y + 3]), make_float4(v[y + 4], v[y + 5], v[y + 6], v[y + 7]));
 			}
 		};
 		if (mine % 32 == 0)
@@ -665,40 +680,52 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 		else
 			for (int x = 0; x < mine; x += 8) join(Width<8>(), x);
 		__syncwarp();
-		const int pieces = LAYERED ? mine / 4 : mine / 8, lg = 31 - __clz(pieces); // 16-byte pieces of a row: a power of two up to 32
-		const int down = 32 >> lg, cc = lane & (pieces - 1), di = down / a.G, dh = down % a.G;
-		const int row0 = row - lane;
-		int rr = lane >> lg, to = row0 + rr, i = to / a.G, hh = to % a.G;
-		for (; rr < 32 && row0 + rr - (lane >> lg) < rows;) { // (ends after the warp's last valid row)
-			constexpr int BATCH = 8; // reads first, then stores
-			float4 lo[BATCH], hi[LAYERED ? 1 : BATCH];
-#pragma unroll
-			for (int x = 0; x < BATCH; ++x) {
-				const int at = min(rr + x * down, 31);
-				lo[x] = ld_shared4(patch + at * ld + cc * (LAYERED ? 16 : 32));
-				if constexpr (!LAYERED) hi[x] = ld_shared4(patch + at * ld + cc * 32 + 16);
+		if constexpr (BOXES) { // a sub-tile of 64 channels is one group's or (SPLIT, 64 channels in all) half by each
+			constexpr bool shared = SPLIT && DV == 64;
+			proxy_fence();
+			if (shared) asm volatile("bar.sync 2, 256;" ::: "memory");
+			else asm volatile("bar.sync %0, 128;" ::"r"(3 + t) : "memory");
+			if (q == 0 && (!shared || t == 0) && elect_one()) {
+				for (int c = first_col; c < (shared ? 64 : first_col + mine); c += 64) tma_store_4d(&to, c, 0, g, (row - tr) / a.G, tile + (c / 64) * (kTile * 128));
+				asm volatile("cp.async.bulk.commit_group;\n\tcp.async.bulk.wait_group.read 0;" ::: "memory");
 			}
+			__syncwarp();
+		} else {
+			const int pieces = LAYERED ? mine / 4 : mine / 8, lg = 31 - __clz(pieces); // 16-byte pieces of a row: a power of two up to 32
+			const int down = 32 >> lg, cc = lane & (pieces - 1), di = down / a.G, dh = down % a.G;
+			const int row0 = row - lane;
+			int rr = lane >> lg, to = row0 + rr, i = to / a.G, hh = to % a.G;
+			for (; rr < 32 && row0 + rr - (lane >> lg) < rows;) { // (ends after the warp's last valid row)
+				constexpr int BATCH = 8; // reads first, then stores
+				float4 lo[BATCH], hi[LAYERED ? 1 : BATCH];
 #pragma unroll
-			for (int x = 0; x < BATCH; ++x) {
-				if (rr < 32 && to < rows) {
-					const int col = (g * a.G + hh) * DV + part * share + first_col;
-					if constexpr (LAYERED) {
-						float *dst = static_cast<float *>(a.out) + (size_t)i * a.ldo + col + cc * 4;
-						if (a.wide) *reinterpret_cast<float4 *>(dst) = lo[x];
-						else *reinterpret_cast<float2 *>(dst) = make_float2(lo[x].x, lo[x].y), *reinterpret_cast<float2 *>(dst + 2) = make_float2(lo[x].z, lo[x].w);
-					} else {
-						const uint4 pk = make_uint4(pack2<T>(lo[x].x, lo[x].y), pack2<T>(lo[x].z, lo[x].w), pack2<T>(hi[x].x, hi[x].y), pack2<T>(hi[x].z, hi[x].w));
-						T *dst = static_cast<T *>(a.out) + (size_t)i * a.n_kv * a.G * DV + col + cc * 8;
-						if (a.wide) {
-							*reinterpret_cast<uint4 *>(dst) = pk;
+				for (int x = 0; x < BATCH; ++x) {
+					const int at = min(rr + x * down, 31);
+					lo[x] = ld_shared4(patch + at * ld + cc * (LAYERED ? 16 : 32));
+					if constexpr (!LAYERED) hi[x] = ld_shared4(patch + at * ld + cc * 32 + 16);
+				}
+#pragma unroll
+				for (int x = 0; x < BATCH; ++x) {
+					if (rr < 32 && to < rows) {
+						const int col = (g * a.G + hh) * DV + part * share + first_col;
+						if constexpr (LAYERED) {
+							float *dst = static_cast<float *>(a.out) + (size_t)i * a.ldo + col + cc * 4;
+							if (a.wide) *reinterpret_cast<float4 *>(dst) = lo[x];
+							else *reinterpret_cast<float2 *>(dst) = make_float2(lo[x].x, lo[x].y), *reinterpret_cast<float2 *>(dst + 2) = make_float2(lo[x].z, lo[x].w);
 						} else {
-							uint32_t *d32 = reinterpret_cast<uint32_t *>(dst);
-							d32[0] = pk.x, d32[1] = pk.y, d32[2] = pk.z, d32[3] = pk.w;
+							const uint4 pk = make_uint4(pack2<T>(lo[x].x, lo[x].y), pack2<T>(lo[x].z, lo[x].w), pack2<T>(hi[x].x, hi[x].y), pack2<T>(hi[x].z, hi[x].w));
+							T *dst = static_cast<T *>(a.out) + (size_t)i * a.n_kv * a.G * DV + col + cc * 8;
+							if (a.wide) {
+								*reinterpret_cast<uint4 *>(dst) = pk;
+							} else {
+								uint32_t *d32 = reinterpret_cast<uint32_t *>(dst);
+								d32[0] = pk.x, d32[1] = pk.y, d32[2] = pk.z, d32[3] = pk.w;
+							}
 						}
 					}
+					rr += down, to += down, i += di, hh += dh;
+					if (hh >= a.G) hh -= a.G, ++i;
 				}
-				rr += down, to += down, i += di, hh += dh;
-				if (hh >= a.G) hh -= a.G, ++i;
 			}
 		}
 	}
@@ -738,7 +765,7 @@ static int make_map(CUtensorMap *map, const void *ptr, int d, int rows, int ring
 	return r == CUDA_SUCCESS ? 0 : YALM_EINVAL;
 }
 
-// (n, kv heads, G, d) queries -> boxes of 64 channels x the G heads of one kv head x 128 / G positions: the rows of a tile, in their order
+// (n, kv heads, G, d) queries or results -> boxes of 64 channels x the G heads of one kv head x 128 / G positions: the rows of a tile, in their order
 static int make_query_map(CUtensorMap *map, const void *ptr, int d, int G, int n_kv, int n) {
 	EncodeTiledFn fn = encode_fn();
 	if (!fn) return YALM_EINVAL;
@@ -751,13 +778,13 @@ static int make_query_map(CUtensorMap *map, const void *ptr, int d, int G, int n
 }
 
 // est_tiles: key tiles of the longest rows.
-template <typename T, int DK, int DV, bool LAYERED, bool SPLIT>
+template <typename T, int DK, int DV, bool LAYERED, bool SPLIT, bool BOXES>
 static int launch_of(Args &a, const void *keys, const void *values, int map_rows, int est_tiles, cudaStream_t st) {
 	using SH = Shape<DK, DV>;
 	static int at_once[kMaxDevices][4]; // clusters of 1, 2, 4, 8 CTAs; 0: not asked yet
 	static std::mutex mu;
 	constexpr int ROWS = SPLIT ? kTile : 2 * kTile, SMEM = SH::smem(SPLIT);
-	auto kernel = prompt_attn_kernel<T, DK, DV, LAYERED, SPLIT>;
+	auto kernel = prompt_attn_kernel<T, DK, DV, LAYERED, SPLIT, BOXES>;
 	const DeviceInfo &dev = device_info();
 	if (dev.device < 0 || dev.device >= kMaxDevices) return YALM_EINVAL;
 	cudaLaunchConfig_t cfg = {};
@@ -777,28 +804,38 @@ static int launch_of(Args &a, const void *keys, const void *values, int map_rows
 		}
 		for (int i = 0; i < 4; ++i) room[i] = at_once[dev.device][i];
 	}
-	CUtensorMap tq, tk, tv;
+	CUtensorMap tq, tk, tv, to;
 	int rc = make_map(&tk, keys, DK, map_rows, a.ring, a.n_kv, LAYERED);
 	if (!rc) rc = make_map(&tv, values, DV, map_rows, a.ring, a.v_heads, LAYERED);
-	a.q_map = !LAYERED && kTile % a.G == 0;
-	if (!rc && a.q_map) rc = make_query_map(&tq, a.q, DK, a.G, a.n_kv, a.n);
-	else tq = tk;
 	if (rc) return rc;
 	const int row_units = (a.n * a.G + ROWS - 1) / ROWS, units = row_units * a.n_kv;
 	a.parts = 1;
-	if (SPLIT && est_tiles >= 4)
+	if (SPLIT && !BOXES && est_tiles >= 4)
 		for (int i = 1; i < 4 && (1 << i) <= DV / 16 && units <= room[i] && est_tiles > (1 << i); ++i) a.parts = 1 << i;
-	return launch_chained(kernel, dim3(row_units * a.parts, a.n_kv), dim3(kThreads), SMEM, st, a.parts, tq, tk, tv, a);
+	a.q_map = !LAYERED && kTile % a.G == 0;
+	tq = to = tk;
+	if (a.q_map) rc = make_query_map(&tq, a.q, DK, a.G, a.n_kv, a.n);
+	if (!rc && BOXES) rc = make_query_map(&to, a.out, DV, a.G, a.n_kv, a.n);
+	if (rc) return rc;
+	return launch_chained(kernel, dim3(row_units * a.parts, a.n_kv), dim3(kThreads), SMEM, st, a.parts, tq, tk, tv, to, a);
 }
 // One tile of rows a CTA while these run all at once, one per SM, and two beyond, which read a key tile once for both (64 / 8 heads of 128, 512 rows: at 0
 // 17.3 us in single tiles, 14.5 in pairs, at 7680 132 and 128).  Where tiles of rows leave SMs idle, a cluster shares the keys: as many parts as still run all at
 // once, at least four key tiles in all and more tiles than parts (17 rows, 32 / 8 heads of 128: three key tiles in one part 7.8 us, in two 8.4; five in two 9.7, in
 // four 9.2; nine, 128 rows of 8 / 2 heads, in four 10.9, in eight 9.9).
+// fp16 results of more tiles than leave two parts a place leave through the copy engine (512 rows at 0, 32 / 8 heads of 128: 9.7 -> 9.4 us; 64 / 8: 14.5 -> 13.9);
+// a store of few CTAs is there as soon from their threads.
 template <typename T, int DK, int DV, bool LAYERED>
 static int launch(Args &a, const void *keys, const void *values, int map_rows, int est_tiles, cudaStream_t st) {
 	const long tiles = (long)((a.n * (long)a.G + kTile - 1) / kTile) * a.n_kv;
-	return tiles <= device_info().sms ? launch_of<T, DK, DV, LAYERED, true>(a, keys, values, map_rows, est_tiles, st)
-	                                  : launch_of<T, DK, DV, LAYERED, false>(a, keys, values, map_rows, est_tiles, st);
+	const int sms = device_info().sms;
+	const bool split = tiles <= sms;
+	if constexpr (!LAYERED && DV % 64 == 0)
+		if (kTile % a.G == 0 && a.wide && tiles > sms / 2 + 1)
+			return split ? launch_of<T, DK, DV, LAYERED, true, true>(a, keys, values, map_rows, est_tiles, st)
+			             : launch_of<T, DK, DV, LAYERED, false, true>(a, keys, values, map_rows, est_tiles, st);
+	return split ? launch_of<T, DK, DV, LAYERED, true, false>(a, keys, values, map_rows, est_tiles, st)
+	             : launch_of<T, DK, DV, LAYERED, false, false>(a, keys, values, map_rows, est_tiles, st);
 }
 
 constexpr float kLog2e = 1.4426950408889634f;
