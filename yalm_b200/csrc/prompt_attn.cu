@@ -203,8 +203,9 @@ struct Shape {
 
 // T: operand type.  LAYERED: fp32 rows in and out, pooled blocks, ring tiles with rows that hold no position, sinks.
 // SPLIT: the CTA has one tile of rows, and A and B are its even and its odd key tiles.
-// BOXES (the keys in one part): the results leave as boxes of the tensor map to.
-template <typename T, int DK, int DV, bool LAYERED, bool SPLIT, bool BOXES>
+// SHARED: a cluster shares the keys (a kernel of its own: with the join in it, calls without one took 0.3 us longer).  BOXES: the results leave as boxes of the
+// tensor map to.
+template <typename T, int DK, int DV, bool LAYERED, bool SPLIT, bool SHARED, bool BOXES>
 __global__ void __launch_bounds__(kThreads, 1)
 prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv,
                    const __grid_constant__ CUtensorMap to, const __grid_constant__ Args a) {
@@ -215,7 +216,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 	const uint32_t full0 = bars, empty0 = full0 + 8 * NST, s_full0 = empty0 + 8 * NST, p_full0 = s_full0 + 16, o_full = p_full0 + 32, v_clean0 = o_full + 8,
 	               q_full = v_clean0 + 8 * NST, tslot = q_full + 8;
 	const int warp = uniform_warp(), lane = threadIdx.x & 31;
-	const int parts = SPLIT && !BOXES ? a.parts : 1, part = parts > 1 ? (int)cluster_rank() : 0;
+	const int parts = SHARED ? a.parts : 1, part = parts > 1 ? (int)cluster_rank() : 0;
 	const int rows = a.n * a.G, units = (rows + ROWS - 1) / ROWS;
 	const int unit = units - 1 - (int)(blockIdx.x / parts); // the longest rows first
 	const int g = blockIdx.y, r0 = unit * ROWS, nt = SPLIT || r0 + kTile < rows ? 2 : 1;
@@ -650,7 +651,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 					put(x + y, make_float4(own[y], own[y + 1], own[y + 2], own[y + 3]), make_float4(own[y + 4], own[y + 5], own[y + 6], own[y + 7]));
 				return;
 			}
-			if constexpr (SPLIT && !BOXES) {
+			if constexpr (SHARED) {
 				float v[W];
 #pragma unroll
 				for (int y = 0; y < W; ++y) v[y] = 0.f;
@@ -777,65 +778,72 @@ static int make_query_map(CUtensorMap *map, const void *ptr, int d, int G, int n
 	return r == CUDA_SUCCESS ? 0 : YALM_EINVAL;
 }
 
-// est_tiles: key tiles of the longest rows.
-template <typename T, int DK, int DV, bool LAYERED, bool SPLIT, bool BOXES>
-static int launch_of(Args &a, const void *keys, const void *values, int map_rows, int est_tiles, cudaStream_t st) {
+template <typename T, int DK, int DV, bool LAYERED, bool SPLIT, bool SHARED, bool BOXES>
+static int launch_of(Args &a, const void *keys, const void *values, int map_rows, cudaStream_t st) {
 	using SH = Shape<DK, DV>;
-	static int at_once[kMaxDevices][4]; // clusters of 1, 2, 4, 8 CTAs; 0: not asked yet
-	static std::mutex mu;
-	constexpr int ROWS = SPLIT ? kTile : 2 * kTile, SMEM = SH::smem(SPLIT);
-	auto kernel = prompt_attn_kernel<T, DK, DV, LAYERED, SPLIT, BOXES>;
-	const DeviceInfo &dev = device_info();
-	if (dev.device < 0 || dev.device >= kMaxDevices) return YALM_EINVAL;
-	cudaLaunchConfig_t cfg = {};
-	cudaLaunchAttribute at[1];
-	at[0].id = cudaLaunchAttributeClusterDimension;
-	at[0].val.clusterDim.x = 1, at[0].val.clusterDim.y = 1, at[0].val.clusterDim.z = 1;
-	cfg.blockDim = dim3(kThreads), cfg.dynamicSmemBytes = SMEM, cfg.attrs = at, cfg.numAttrs = 1;
-	int room[4];
-	{
-		std::lock_guard<std::mutex> lock(mu);
-		if (!at_once[dev.device][0]) {
-			YALM_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
-			for (int i = 3; i >= 0; --i) {
-				at[0].val.clusterDim.x = 1 << i, cfg.gridDim = dim3(1 << i);
-				YALM_TRY(cudaOccupancyMaxActiveClusters(&at_once[dev.device][i], kernel, &cfg));
-			}
-		}
-		for (int i = 0; i < 4; ++i) room[i] = at_once[dev.device][i];
-	}
+	auto kernel = prompt_attn_kernel<T, DK, DV, LAYERED, SPLIT, SHARED, BOXES>;
+	YALM_TRY(allow_smem((const void *)kernel, SH::smem(SPLIT)));
 	CUtensorMap tq, tk, tv, to;
 	int rc = make_map(&tk, keys, DK, map_rows, a.ring, a.n_kv, LAYERED);
 	if (!rc) rc = make_map(&tv, values, DV, map_rows, a.ring, a.v_heads, LAYERED);
 	if (rc) return rc;
-	const int row_units = (a.n * a.G + ROWS - 1) / ROWS, units = row_units * a.n_kv;
-	a.parts = 1;
-	if (SPLIT && !BOXES && est_tiles >= 4)
-		for (int i = 1; i < 4 && (1 << i) <= DV / 16 && units <= room[i] && est_tiles > (1 << i); ++i) a.parts = 1 << i;
 	a.q_map = !LAYERED && kTile % a.G == 0;
 	tq = to = tk;
 	if (a.q_map) rc = make_query_map(&tq, a.q, DK, a.G, a.n_kv, a.n);
 	if (!rc && BOXES) rc = make_query_map(&to, a.out, DV, a.G, a.n_kv, a.n);
 	if (rc) return rc;
-	return launch_chained(kernel, dim3(row_units * a.parts, a.n_kv), dim3(kThreads), SMEM, st, a.parts, tq, tk, tv, to, a);
+	constexpr int ROWS = SPLIT ? kTile : 2 * kTile;
+	return launch_chained(kernel, dim3((a.n * a.G + ROWS - 1) / ROWS * a.parts, a.n_kv), dim3(kThreads), SH::smem(SPLIT), st, a.parts, tq, tk, tv, to, a);
+}
+// Clusters of 2, 4, 8 CTAs that share keys and run at once, of the current device
+template <typename T, int DK, int DV, bool LAYERED>
+static int clusters_at_once(int (&room)[4]) {
+	using SH = Shape<DK, DV>;
+	static int at_once[kMaxDevices][4]; // 0: not asked yet
+	static std::mutex mu;
+	auto kernel = prompt_attn_kernel<T, DK, DV, LAYERED, true, true, false>;
+	const DeviceInfo &dev = device_info();
+	if (dev.device < 0 || dev.device >= kMaxDevices) return YALM_EINVAL;
+	std::lock_guard<std::mutex> lock(mu);
+	if (!at_once[dev.device][1]) {
+		YALM_TRY(allow_smem((const void *)kernel, SH::smem(true)));
+		for (int i = 3; i >= 1; --i) {
+			cudaLaunchConfig_t cfg = {};
+			cudaLaunchAttribute at[1];
+			at[0].id = cudaLaunchAttributeClusterDimension;
+			at[0].val.clusterDim.x = 1 << i, at[0].val.clusterDim.y = 1, at[0].val.clusterDim.z = 1;
+			cfg.gridDim = dim3(1 << i), cfg.blockDim = dim3(kThreads), cfg.dynamicSmemBytes = SH::smem(true), cfg.attrs = at, cfg.numAttrs = 1;
+			YALM_TRY(cudaOccupancyMaxActiveClusters(&at_once[dev.device][i], kernel, &cfg));
+		}
+	}
+	for (int i = 1; i < 4; ++i) room[i] = at_once[dev.device][i];
+	return 0;
 }
 // One tile of rows a CTA while these run all at once, one per SM, and two beyond, which read a key tile once for both (64 / 8 heads of 128, 512 rows: at 0
 // 17.3 us in single tiles, 14.5 in pairs, at 7680 132 and 128).  Where tiles of rows leave SMs idle, a cluster shares the keys: as many parts as still run all at
 // once, at least four key tiles in all and more tiles than parts (17 rows, 32 / 8 heads of 128: three key tiles in one part 7.8 us, in two 8.4; five in two 9.7, in
-// four 9.2; nine, 128 rows of 8 / 2 heads, in four 10.9, in eight 9.9).
-// fp16 results of more tiles than leave two parts a place leave through the copy engine (512 rows at 0, 32 / 8 heads of 128: 9.7 -> 9.4 us; 64 / 8: 14.5 -> 13.9);
+// four 9.2; nine, 128 rows of 8 / 2 heads, in four 10.9, in eight 9.9).  est_tiles: key tiles of the longest rows.
+// fp16 results of more tiles than leave two parts a place leave through the copy engine (512 rows at 0, 32 / 8 heads of 128: 9.7 -> 8.9 us; 64 / 8: 14.5 -> 13.8);
 // a store of few CTAs is there as soon from their threads.
 template <typename T, int DK, int DV, bool LAYERED>
 static int launch(Args &a, const void *keys, const void *values, int map_rows, int est_tiles, cudaStream_t st) {
 	const long tiles = (long)((a.n * (long)a.G + kTile - 1) / kTile) * a.n_kv;
 	const int sms = device_info().sms;
-	const bool split = tiles <= sms;
-	if constexpr (!LAYERED && DV % 64 == 0)
-		if (kTile % a.G == 0 && a.wide && tiles > sms / 2 + 1)
-			return split ? launch_of<T, DK, DV, LAYERED, true, true>(a, keys, values, map_rows, est_tiles, st)
-			             : launch_of<T, DK, DV, LAYERED, false, true>(a, keys, values, map_rows, est_tiles, st);
-	return split ? launch_of<T, DK, DV, LAYERED, true, false>(a, keys, values, map_rows, est_tiles, st)
-	             : launch_of<T, DK, DV, LAYERED, false, false>(a, keys, values, map_rows, est_tiles, st);
+	a.parts = 1;
+	if (tiles > sms / 2 + 1) {
+		const bool split = tiles <= sms;
+		if constexpr (!LAYERED && DV % 64 == 0)
+			if (kTile % a.G == 0 && a.wide)
+				return split ? launch_of<T, DK, DV, LAYERED, true, false, true>(a, keys, values, map_rows, st)
+				             : launch_of<T, DK, DV, LAYERED, false, false, true>(a, keys, values, map_rows, st);
+		if (!split) return launch_of<T, DK, DV, LAYERED, false, false, false>(a, keys, values, map_rows, st);
+	} else if (est_tiles >= 4) {
+		int room[4];
+		if (int rc = clusters_at_once<T, DK, DV, LAYERED>(room)) return rc;
+		for (int i = 1; i < 4 && (1 << i) <= DV / 16 && tiles <= room[i] && est_tiles > (1 << i); ++i) a.parts = 1 << i;
+		if (a.parts > 1) return launch_of<T, DK, DV, LAYERED, true, true, false>(a, keys, values, map_rows, st);
+	}
+	return launch_of<T, DK, DV, LAYERED, true, false, false>(a, keys, values, map_rows, st);
 }
 
 constexpr float kLog2e = 1.4426950408889634f;
