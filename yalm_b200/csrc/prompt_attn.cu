@@ -18,8 +18,8 @@
 // Bound by the chain softmax - products of a tile pair (some 3500 cycles per 128 keys: 1800 from scores to weights, of which the exponentials
 // alone take 1024 at 16 a cycle and SM for each of the two tiles, 500 for the rescaling, and 1100 for P V and the next scores) and, for short
 // contexts, by launch, query staging and the store.  Back to back, against 64-row tiles on mma.sync: 507 rows at 7680 positions, 32 / 8 heads of 128:
-// 667 -> 67 us (980 TFLOP/s); 512 rows at 0: 32.8 -> 9.3 us; bf16 window 1024 and pooled blocks of 64, 512 rows, 16 / 4 heads: 57.3 -> 15.5 us.
-// Of these SPLIT, with the queries of fp16 calls as boxes of a tensor map, made 70.2 to 67.3, 14.1 to 9.3 and 22.7 to 15.5: in pairs of tiles whose keys two CTAs
+// 667 -> 67 us (980 TFLOP/s); 512 rows at 0: 32.8 -> 8.9 us; bf16 window 1024 and pooled blocks of 64, 512 rows, 16 / 4 heads: 57.3 -> 14.5 us.
+// Of these SPLIT, with the queries of fp16 calls as boxes of a tensor map, made 70.2 to 67.3, 14.1 to 8.9 and 22.7 to 14.5: in pairs of tiles whose keys two CTAs
 // share, staging took 2 us, and sending half of the accumulators (64 KB, some 20 bytes a cycle), both cluster barriers and the join 4 us.
 #include "common.cuh"
 #include "launch.h"
@@ -198,7 +198,12 @@ struct Shape {
 	static constexpr int DKP = DK < 64 ? 64 : DK, DVP = DV < 64 ? 64 : DV; // channels a row takes in shared memory
 	static constexpr int Q_BYTES = kTile * DKP * 2, K_BYTES = Q_BYTES, V_BYTES = kTile * DVP * 2, STAGE = K_BYTES > V_BYTES ? K_BYTES : V_BYTES;
 	static constexpr int STAGES = STAGE == 32768 ? 4 : 8;
-	static constexpr int smem(bool split) { return (split ? 1 : 2) * Q_BYTES + STAGES * STAGE + 512 + (split ? 2 * kTile * 8 : 0) + 1024; }
+	// the parts of shared keys exchange through space of their own (no CTA waits for the others' products before it sends): (parts - 1) shares of the columns, (reference, sum) of every part
+	static constexpr int smem(bool split, int parts) {
+		return (split ? 1 : 2) * Q_BYTES + STAGES * STAGE + 512 + 1024 + (parts > 1 ? (parts - 1) * (DV / parts) * kTile * 4 + parts * kTile * 8 : 0);
+	}
+	static constexpr int MERGE = 72 * 1024; // where the even and the odd key tiles' (reference, sum) meet: over stages that are done with, behind the patches
+	static_assert(MERGE + 2 * kTile * 8 <= Q_BYTES + STAGES * STAGE, "");
 };
 
 // T: operand type.  LAYERED: fp32 rows in and out, pooled blocks, ring tiles with rows that hold no position, sinks.
@@ -230,6 +235,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 			for (int i = 0; i < NST; ++i) mbar_init(v_clean0 + 8 * i, 1);
 		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 	}
+	if (SHARED) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); // waited for before this CTA writes into the others
 	if (warp == 0 && elect_one()) prefetch_map(&tk), prefetch_map(&tv), prefetch_map(&tq), prefetch_map(&to);
 	if (warp == 1) tmem_alloc<1>(tslot, 512);
 	tc_fence_before();
@@ -262,29 +268,26 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 	auto fill_pooled = [&](int i, int tid, int nthreads) {
 		int slot, pos, valid;
 		tiles.at(k_begin + i, slot, pos, valid);
-#pragma unroll
-		for (int is_v = 0; is_v < 2; ++is_v) {
-			const int D = is_v ? DV : DK, pieces = (is_v ? SH::DVP : SH::DKP) / 8, head = is_v ? g % a.v_heads : g;
-			const float *src = (is_v ? a.value_pool : a.key_pool) + ((size_t)head * a.max_blocks + slot) * D;
-			const uint32_t dst = kv0 + ((2 * i + is_v) % NST) * SH::STAGE;
+		constexpr int KP = SH::DKP / 8, VP = SH::DVP / 8; // 16-byte pieces of a row
+		const int v_head = g % a.v_heads;
 #pragma unroll 4
-			for (int x = tid; x < (is_v ? kTile : valid) * pieces; x += nthreads) {
-				const int r = x / pieces, c = x % pieces;
-				float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
-				if (r < valid && c * 8 < D) {
-					lo = *reinterpret_cast<const float4 *>(src + (size_t)r * D + c * 8);
-					hi = *reinterpret_cast<const float4 *>(src + (size_t)r * D + c * 8 + 4);
-				}
-				st_shared4(dst + tile_at(r, c), make_float4(__uint_as_float(pack2<T>(lo.x, lo.y)), __uint_as_float(pack2<T>(lo.z, lo.w)),
-				                                            __uint_as_float(pack2<T>(hi.x, hi.y)), __uint_as_float(pack2<T>(hi.z, hi.w))));
-			}
+		for (int x = tid; x < valid * (KP + VP); x += nthreads) { // keys and values together: their loads travel at the same time
+			const bool is_v = x >= valid * KP;
+			const int y = is_v ? x - valid * KP : x, r = is_v ? y / VP : y / KP, c = is_v ? y % VP : y % KP, D = is_v ? DV : DK, head = is_v ? v_head : g;
+			const float *src = (is_v ? a.value_pool : a.key_pool) + ((size_t)head * a.max_blocks + slot + r) * D + c * 8;
+			float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
+			if (c * 8 < D) lo = *reinterpret_cast<const float4 *>(src), hi = *reinterpret_cast<const float4 *>(src + 4);
+			st_shared4(kv0 + ((2 * i + is_v) % NST) * SH::STAGE + tile_at(r, c),
+			           make_float4(__uint_as_float(pack2<T>(lo.x, lo.y)), __uint_as_float(pack2<T>(lo.z, lo.w)), __uint_as_float(pack2<T>(hi.x, hi.y)),
+			                       __uint_as_float(pack2<T>(hi.z, hi.w))));
 		}
+		for (int x = valid * VP + tid; x < kTile * VP; x += nthreads) st_shared4(kv0 + ((2 * i + 1) % NST) * SH::STAGE + tile_at(x / VP, x % VP), make_float4(0.f, 0.f, 0.f, 0.f));
 		proxy_fence();
 	};
 
 	if (warp == 0) {
 		__syncwarp();
-		if (!LAYERED && a.q_map && elect_one()) { // a box is the 128 / G positions of a tile, all G heads of each; positions past the last are zero
+		if (!LAYERED && a.q_map && nk > 0 && elect_one()) { // a box is the 128 / G positions of a tile, all G heads of each; positions past the last are zero
 			mbar_expect_tx(q_full, (ROWS / kTile == 2 && nt == 2 ? 2 : 1) * SH::Q_BYTES);
 			for (int t = 0; t < (SPLIT ? 1 : nt); ++t)
 				for (int c = 0; c < SH::DKP; c += 64)
@@ -546,15 +549,15 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 	const int t = (warp - 4) >> 2, q = warp & 3, tr = q * 32 + lane, row = r0 + (SPLIT ? 0 : t * kTile) + tr, share = DV / parts;
 	const int mine = SPLIT ? share / 2 : share, first_col = SPLIT ? t * mine : 0; // columns that a thread handles of a share, from where
 	const uint32_t op = tmem + ((uint32_t)(q * 32) << 16) + 256 + (SPLIT ? 0 : t * SH::DVP);
-	// from the start of shared memory (queries and stages are done with): [other part][4 columns][row][4], then (reference, sum) [part][row]
-	const uint32_t ml0 = base + (uint32_t)((parts - 1) * share * kTile * 4);
+	// [other part][4 columns][row][4], then (reference, sum) [part][row]
+	const uint32_t exch = bars + 512, ml0 = exch + (uint32_t)((parts - 1) * share * kTile * 4);
 	if (dead) l = __int_as_float(0x7fc00000);
 	__syncwarp();
 	float w0 = 1.f, w1 = 1.f; // SPLIT: factors of the sums over the even and the odd key tiles
 	bool any0 = true, any1 = true; // whether this row sees any of them (where not, the accumulator may hold anything)
 	if constexpr (SPLIT) {
 		if (softmax_warp) {
-			const uint32_t merge = bars + 512; // (reference, sum) [even, odd][row], behind everything else
+			const uint32_t merge = base + SH::MERGE; // (reference, sum) [even, odd][row]
 			asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(merge + (uint32_t)((t * kTile + tr) * 8)), "f"(mref), "f"(l) : "memory");
 			asm volatile("bar.sync 2, 256;" ::: "memory");
 			float m0, l0, m1, l1;
@@ -583,12 +586,12 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 		}
 	};
 	if (parts > 1) {
-		cluster_sync(); // every part is done with its shared memory
+		asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); // the other CTAs run
 		if (softmax_warp) {
 			for (int p = 0; p < parts; ++p) {
-				const uint32_t there = map_rank(base, (uint32_t)p);
+				const uint32_t there = map_rank(exch, (uint32_t)p);
 				if (t == 0)
-					asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(there + (ml0 - base) + (uint32_t)((part * kTile + tr) * 8)), "f"(mref), "f"(l) : "memory");
+					asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(there + (ml0 - exch) + (uint32_t)((part * kTile + tr) * 8)), "f"(mref), "f"(l) : "memory");
 				if (p == part || nk == 0) continue;
 				const uint32_t dst = there + (uint32_t)((part < p ? part : part - 1) * share * kTile * 4);
 				auto send = [&](auto width, int x) {
@@ -627,9 +630,9 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 		}
 		const int h = g * a.G + min(row, rows - 1) % a.G;
 		float f = LAYERED ? stack::softmax_finish(M * 0.69314718055994531f, Lsum, a.sink, h) : 1.0f / Lsum;
-		// through a patch of shared memory per warp (after what the parts exchanged), so that neighbouring lanes store neighbouring
+		// through a patch of shared memory per warp (over queries and stages, which are done with), so that neighbouring lanes store neighbouring
 		// bytes: a row per lane, every 16-byte piece went to a line of its own (5 us for 256 rows of 128)
-		const uint32_t ld = (uint32_t)mine * 4 + 16, patch = ml0 + (parts > 1 ? parts * kTile * 8 : 0) + (warp - 4) * 32 * ld;
+		const uint32_t ld = (uint32_t)mine * 4 + 16, patch = base + (warp - 4) * 32 * ld;
 		// or all rows of a tile as fp16 in the layout of an operand tile, which the copy engine stores: no reads back, no addresses, rows past the last left out
 		const uint32_t tile = base + (SPLIT ? 0 : t * SH::Q_BYTES);
 		auto put = [&](int x, float4 v, float4 w) { // 8 columns
@@ -664,7 +667,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 #pragma unroll
 						for (int y = 0; y < W; ++y) v[y] += w * own[y];
 					} else {
-						const uint32_t src = base + (uint32_t)((p < part ? p : p - 1) * share * kTile * 4);
+						const uint32_t src = exch + (uint32_t)((p < part ? p : p - 1) * share * kTile * 4);
 #pragma unroll
 						for (int y = 0; y < W; y += 4) {
 							const float4 o = ld_shared4(src + (uint32_t)((((first_col + x + y) >> 2) * kTile + tr) * 16));
@@ -782,7 +785,8 @@ template <typename T, int DK, int DV, bool LAYERED, bool SPLIT, bool SHARED, boo
 static int launch_of(Args &a, const void *keys, const void *values, int map_rows, cudaStream_t st) {
 	using SH = Shape<DK, DV>;
 	auto kernel = prompt_attn_kernel<T, DK, DV, LAYERED, SPLIT, SHARED, BOXES>;
-	YALM_TRY(allow_smem((const void *)kernel, SH::smem(SPLIT)));
+	const int smem = SH::smem(SPLIT, a.parts);
+	YALM_TRY(allow_smem((const void *)kernel, smem));
 	CUtensorMap tq, tk, tv, to;
 	int rc = make_map(&tk, keys, DK, map_rows, a.ring, a.n_kv, LAYERED);
 	if (!rc) rc = make_map(&tv, values, DV, map_rows, a.ring, a.v_heads, LAYERED);
@@ -793,7 +797,7 @@ static int launch_of(Args &a, const void *keys, const void *values, int map_rows
 	if (!rc && BOXES) rc = make_query_map(&to, a.out, DV, a.G, a.n_kv, a.n);
 	if (rc) return rc;
 	constexpr int ROWS = SPLIT ? kTile : 2 * kTile;
-	return launch_chained(kernel, dim3((a.n * a.G + ROWS - 1) / ROWS * a.parts, a.n_kv), dim3(kThreads), SH::smem(SPLIT), st, a.parts, tq, tk, tv, to, a);
+	return launch_chained(kernel, dim3((a.n * a.G + ROWS - 1) / ROWS * a.parts, a.n_kv), dim3(kThreads), smem, st, a.parts, tq, tk, tv, to, a);
 }
 // Clusters of 2, 4, 8 CTAs that share keys and run at once, of the current device
 template <typename T, int DK, int DV, bool LAYERED>
@@ -806,13 +810,14 @@ static int clusters_at_once(int (&room)[4]) {
 	if (dev.device < 0 || dev.device >= kMaxDevices) return YALM_EINVAL;
 	std::lock_guard<std::mutex> lock(mu);
 	if (!at_once[dev.device][1]) {
-		YALM_TRY(allow_smem((const void *)kernel, SH::smem(true)));
 		for (int i = 3; i >= 1; --i) {
+			const int smem = SH::smem(true, 1 << i);
+			YALM_TRY(allow_smem((const void *)kernel, smem));
 			cudaLaunchConfig_t cfg = {};
 			cudaLaunchAttribute at[1];
 			at[0].id = cudaLaunchAttributeClusterDimension;
 			at[0].val.clusterDim.x = 1 << i, at[0].val.clusterDim.y = 1, at[0].val.clusterDim.z = 1;
-			cfg.gridDim = dim3(1 << i), cfg.blockDim = dim3(kThreads), cfg.dynamicSmemBytes = SH::smem(true), cfg.attrs = at, cfg.numAttrs = 1;
+			cfg.gridDim = dim3(1 << i), cfg.blockDim = dim3(kThreads), cfg.dynamicSmemBytes = smem, cfg.attrs = at, cfg.numAttrs = 1;
 			YALM_TRY(cudaOccupancyMaxActiveClusters(&at_once[dev.device][i], kernel, &cfg));
 		}
 	}
