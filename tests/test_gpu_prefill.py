@@ -136,3 +136,33 @@ def test_forward_batch_refuses_what_it_cannot_do():
         s.forward_batch(list(range(3, 43)), 30)
     s.close()
     m.close()
+
+
+@pytest.mark.parametrize("hd,heads,kv,dim,rotary,clip,vocab,n,pos0", [
+    (32, 8, 8, 256, 32, None, 1000, 129, 0), (64, 8, 2, 512, 32, 0.5, 516, 300, 40), (128, 8, 2, 1024, 128, None, 3000, 512, 7), (128, 4, 4, 1024, 64, 0.7, 132, 511, 1),
+    (64, 4, 1, 1024, 64, None, 20000, 260, 100)])
+def test_forward_batch_of_many_rows_matches_few(hd, heads, kv, dim, rotary, clip, vocab, n, pos0):
+    """A portion of more than 128 rows, whose products rotate, append and score in their own kernels, against the same positions in portions of 100, which
+    leave that to kernels of their own: keys and values in fp16 to a unit (2^-10) or the layer's rounding, probabilities to what a unit in 16-bit operands makes of
+    them (as against the token loop: 2e-2).  One key part and several, part of a head rotated, clipped values, ragged vocabularies and portions."""
+    arch = yf.Arch(dim, 512, hd, 2, heads, kv, vocab, 1024, 10000.0, rotary_dim=rotary, qkv_clip=clip, name="many-rows")
+    img = bytes(yf.random_model(arch, "fp16", seed=hd + n))
+    m = api.Model(img).cuda()
+    ids = [1] + [(i * 131 + 7) % (vocab - 3) + 3 for i in range(pos0 + n)]
+    outs = []
+    for most in (n, 100):
+        s = api.InferenceState(m)
+        probs, pos = [], 0
+        while pos < pos0 + n:
+            c = min(100, pos0 - pos) if pos < pos0 else min(most, pos0 + n - pos)
+            probs += s.forward_batch(ids[pos: pos + c], pos, ids[pos + 1: pos + c + 1]).tolist()
+            pos += c
+        rows = [s.read(which, (pos0 + n) * kv * hd, np.uint16, layer).view(np.float16).astype(np.float32) for layer in range(2) for which in (4, 5)]
+        outs.append((np.array(probs), rows, s.logits().copy()))
+        s.close()
+    (p0, r0, l0), (p1, r1, l1) = outs
+    np.testing.assert_allclose(p0, p1, rtol=2e-2, atol=1e-7)
+    for layer, (a, b) in enumerate(zip(r0, r1)):
+        assert np.abs(a - b).max() <= (2e-3 if layer < 2 else 6e-3) * max(1.0, np.abs(b).max())
+    assert np.abs(l0 - l1).max() < LOGIT_TOL
+    m.close()

@@ -32,6 +32,20 @@ namespace prefill {
 
 // prefill_gemm.cu: the three projections as one launch
 int gemm_qkv_f16(float *c, int ldc, const void *a, const void *wq, const void *wk, const void *wv, int M, int q_dim, int kv_dim, int K, cudaStream_t st);
+// more than 128 rows: the three projections rotated and appended
+int gemm_qkv_rotate(void *q, void *k, void *v, const void *turns, const void *a, const void *wq, const void *wk, const void *wv, int M, int q_dim, int kv_dim, int K,
+                    int head_dim, int ring, int pos0, float clip, cudaStream_t st);
+constexpr int kFewRows = 128;
+
+// (cosine, sine) of every position of the portion and pair of a head's channels: the same for all layers
+__global__ void turns_kernel(float2 *turns, int head_dim, int rotary_dim, int pos0, float theta) {
+	const int half = head_dim / 2, j = threadIdx.x % half, i = blockIdx.x * (blockDim.x / half) + threadIdx.x / half;
+	float fcr, fci;
+	rope_angle(fcr, fci, 2 * j, pos0 + i, theta, rotary_dim);
+	chain_wait();
+	chain_next();
+	turns[(size_t)i * half + j] = make_float2(fcr, fci);
+}
 
 // x[i, :] = float(E[tokens[i], :])   (src/infer.cu:632-640, for a batch of rows)
 __global__ void embed_rows_kernel(float *__restrict__ x, const __half *__restrict__ table, const int *__restrict__ tokens, int dim) {
@@ -140,6 +154,7 @@ struct Model::PrefillState {
 	char *arena = nullptr;
 	float *x = nullptr, *qkv = nullptr, *logits = nullptr, *probs = nullptr;
 	__half *xb = nullptr, *q16 = nullptr, *att = nullptr, *hb = nullptr;
+	float2 *turns = nullptr;
 	int *tokens = nullptr, *targets = nullptr;
 	~PrefillState() { cudaFree(arena); }
 };
@@ -178,7 +193,7 @@ int Model::forward_batch(InferenceState &s, const int *tokens, int n, int pos0, 
 		auto pad = [](size_t b) { return (b + 255) / 256 * 256; };
 		const size_t sz[] = {pad(4ull * cap * dim), pad(4ull * cap * (q_dim + 2 * kv_dim)), pad(4ull * cap * V), pad(4ull * cap),
 		                     pad(2ull * cap * std::max(dim, q_dim)), pad(2ull * cap * q_dim), pad(2ull * cap * q_dim), pad(2ull * cap * hid),
-		                     pad(4ull * cap), pad(4ull * cap)};
+		                     pad(4ull * cap), pad(4ull * cap), pad(4ull * cap * c.head_dim)};
 		size_t total = 0;
 		for (size_t b : sz) total += b;
 		if (cudaMalloc((void **)&ps->arena, total) != cudaSuccess) {
@@ -187,8 +202,9 @@ int Model::forward_batch(InferenceState &s, const int *tokens, int n, int pos0, 
 		}
 		char *p = ps->arena;
 		void **slots[] = {(void **)&ps->x, (void **)&ps->qkv, (void **)&ps->logits, (void **)&ps->probs, (void **)&ps->xb,
-		                  (void **)&ps->q16, (void **)&ps->att, (void **)&ps->hb, (void **)&ps->tokens, (void **)&ps->targets};
-		for (int i = 0; i < 10; ++i) *slots[i] = p, p += sz[i];
+		                  (void **)&ps->q16, (void **)&ps->att, (void **)&ps->hb, (void **)&ps->tokens, (void **)&ps->targets,
+		                  (void **)&ps->turns};
+		for (int i = 0; i < 11; ++i) *slots[i] = p, p += sz[i];
 		_prefill = ps;
 	}
 	PrefillState &P = *_prefill;
@@ -196,17 +212,27 @@ int Model::forward_batch(InferenceState &s, const int *tokens, int n, int pos0, 
 	if (targets) YALM_TRY(cudaMemcpyAsync(P.targets, targets, sizeof(int) * n, cudaMemcpyHostToDevice, st));
 	embed_rows_kernel<<<n, 256, 0, st>>>(P.x, static_cast<const __half *>(token_embedding_table), P.tokens, dim);
 	const int act = c.act == ActivationType::SILU ? YALM_ACT_SILU : YALM_ACT_GELU;
+	const bool many = n > kFewRows; // the kernels of more rows finish q, k and v themselves
 	int rc;
+	if (many) {
+		const int per = 256 / (c.head_dim / 2);
+		if ((rc = launch_chained(turns_kernel, dim3((n + per - 1) / per), dim3(256), 0, st, 1, P.turns, c.head_dim, c.rotary_dim, pos0, c.rope_theta))) return rc;
+	}
 	for (auto &bp : blocks) {
 		const Block &b = *bp;
 		if ((rc = launch_chained(rmsnorm_rows_kernel, dim3(n), dim3(kNormThreads), 0, st, 1, P.xb, P.x, b._rms_att_weight, dim, c.norm_eps))) return rc;
-		// q | k | v of the chunk into one (n, q_dim + 2 kv_dim) fp32 buffer
-		const int ld = q_dim + 2 * kv_dim;
-		if ((rc = gemm_qkv_f16(P.qkv, ld, P.xb, b._wq, b._wk, b._wv, n, q_dim, kv_dim, dim, st))) return rc;
-		if ((rc = launch_chained(rope_append_rows_kernel, dim3(n), dim3(512), 0, st, 1, P.q16, reinterpret_cast<__half *>(b._key_cache),
-		                         reinterpret_cast<__half *>(b._value_cache), (const float *)P.qkv, c.n_heads, c.n_kv_heads, c.head_dim, c.rotary_dim, c.max_seq_len, pos0,
-		                         c.rope_theta, c.qkv_clip)))
-			return rc;
+		if (many) {
+			if ((rc = gemm_qkv_rotate(P.q16, b._key_cache, b._value_cache, P.turns, P.xb, b._wq, b._wk, b._wv, n, q_dim, kv_dim, dim, c.head_dim, c.max_seq_len, pos0, c.qkv_clip, st)))
+				return rc;
+		} else {
+			// q | k | v of the chunk into one (n, q_dim + 2 kv_dim) fp32 buffer
+			const int ld = q_dim + 2 * kv_dim;
+			if ((rc = gemm_qkv_f16(P.qkv, ld, P.xb, b._wq, b._wk, b._wv, n, q_dim, kv_dim, dim, st))) return rc;
+			if ((rc = launch_chained(rope_append_rows_kernel, dim3(n), dim3(512), 0, st, 1, P.q16, reinterpret_cast<__half *>(b._key_cache),
+			                         reinterpret_cast<__half *>(b._value_cache), (const float *)P.qkv, c.n_heads, c.n_kv_heads, c.head_dim, c.rotary_dim, c.max_seq_len, pos0,
+			                         c.rope_theta, c.qkv_clip)))
+				return rc;
+		}
 		if ((rc = yalm_attn_prefill(P.att, P.q16, b._key_cache, b._value_cache, n, pos0, c.n_heads, c.n_kv_heads, c.head_dim, c.max_seq_len, st)))
 			return rc;
 		if ((rc = yalm_gemm_f16(P.x, dim, P.att, b._wo, n, dim, q_dim, 1, st))) return rc; // x += Wo att

@@ -45,6 +45,15 @@ constexpr int kGemmThreads = 192;
 constexpr int kSegments = 8;
 
 enum Tail { kStoreF32 = 0, kAddF32 = 1, kGluF16 = 2 };
+enum Kind { kPlain = 0, kGlu = 1, kRotate = 2 }; // of the pair kernel
+
+// kRotate: q | k | v columns are clipped, the pairs of q and k turned, and all stored as fp16, q as rows, k and v into the head-major ring.
+struct RotateArgs {
+	__half *q, *k, *v;
+	const float2 *turns; // (row, pair of a head): cosine, sine
+	int head_dim, ring, pos0;
+	float clip;
+};
 
 struct GemmArgs {
 	int M, N, K; // valid rows of A, rows of W (per matrix), inner dimension
@@ -60,6 +69,7 @@ struct GemmArgs {
 	int n_tile;  // columns of a tile (per matrix)
 	int m_tiles, items, splits, kb_per; // 256-row tiles, tiles in all, K parts of a tile and their length in 64-wide blocks
 	int stages;
+	RotateArgs rotate;
 };
 
 // One tensor map per weight matrix: the segments' own matrices (wq, wk, wv), or w1 and w3, or one W.
@@ -108,8 +118,8 @@ __device__ __forceinline__ uint32_t pack_half2(float a, float b) {
 	const __half2 h = __floats2half2_rn(a, b);
 	return *reinterpret_cast<const uint32_t *>(&h);
 }
-// The same for fp16 results: 4 lanes store the 64 bytes of a row.
-__device__ __forceinline__ void store_patch_f16(const GemmArgs &g, uint32_t patch, const float (&v)[32], int row0, int col, int col_end) {
+// The same for fp16 results: 4 lanes store the 64 bytes of a row; base: row 0, column 0.
+__device__ __forceinline__ void store_patch_f16(const GemmArgs &g, __half *base, size_t ld, uint32_t patch, const float (&v)[32], int row0, int col, int col_end) {
 	const int lane = threadIdx.x & 31, r0 = lane >> 2, cc = (lane & 3) * 8;
 	__syncwarp();
 #pragma unroll
@@ -122,7 +132,7 @@ __device__ __forceinline__ void store_patch_f16(const GemmArgs &g, uint32_t patc
 		const int row = row0 + r0 + 8 * t;
 		if (row >= g.M || c0 >= col_end) continue;
 		const float4 o = ld_shared4(patch + ((r0 + 8 * t) * 20 + cc / 2) * 4);
-		__half *dst = g.h + (size_t)row * g.ldc + c0;
+		__half *dst = base + row * ld + c0;
 		if (c0 + 8 <= col_end) {
 			*reinterpret_cast<float4 *>(dst) = o;
 		} else {
@@ -143,6 +153,26 @@ __device__ __forceinline__ float glu(const GemmArgs &g, float a, float u) {
 }
 constexpr float kNaN = __builtin_nanf("");
 
+// 32 columns of a segment (col: from its start), all of one head: row i at position pos0 + i (src/infer.cpp:200-213, 282-301)
+__device__ __forceinline__ void rotate_store(const GemmArgs &g, int seg, uint32_t patch, float (&v)[32], int row0, int col, int col_end) {
+	const RotateArgs &r = g.rotate;
+	const int head = col / r.head_dim, c0 = col - head * r.head_dim;
+#pragma unroll
+	for (int i = 0; i < 32; ++i) v[i] = clipf(v[i], r.clip);
+	if (seg < 2) {
+		const int row = min(row0 + (int)(threadIdx.x & 31), g.M - 1);
+		const float4 *t = reinterpret_cast<const float4 *>(r.turns + ((size_t)row * r.head_dim + c0) / 2);
+#pragma unroll
+		for (int i = 0; i < 32; i += 4) {
+			const float4 cs = t[i / 4];
+			rope_turn(v[i], v[i + 1], cs.x, cs.y);
+			rope_turn(v[i + 2], v[i + 3], cs.z, cs.w);
+		}
+	}
+	if (seg == 0) store_patch_f16(g, r.q, (size_t)g.seg_end[0], patch, v, row0, col, col_end);
+	else store_patch_f16(g, (seg == 1 ? r.k : r.v) + ((size_t)head * r.ring + r.pos0) * r.head_dim, (size_t)r.head_dim, patch, v, row0, c0, c0 + (col_end - col));
+}
+
 // Column tile t of the output: its segment, first column and the segment's end.
 __device__ __forceinline__ void tile_columns(const GemmArgs &g, int t, int &seg, int &seg0, int &n0, int &n_end) {
 	seg = 0, seg0 = 0;
@@ -158,11 +188,12 @@ __device__ __forceinline__ void tile_columns(const GemmArgs &g, int t, int &seg,
 // (pair kernel), the barriers.
 constexpr int kTailBytes = 4 * kPatch + 512;
 
-// GLU: w1 | w3 tiles side by side, the pair's first CTA staging w1's rows and the second w3's; accumulator columns n .. 2 n - 1 are w3's.
-// B_SEG: every segment has a weight matrix of its own.
-template <bool GLU, bool B_SEG>
+// kGlu: w1 | w3 tiles side by side, the pair's first CTA staging w1's rows and the second w3's; accumulator columns n .. 2 n - 1 are w3's.
+// kRotate: every segment has a weight matrix of its own.
+template <int KIND>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ WeightMaps tb, const __grid_constant__ GemmArgs g) {
+	constexpr bool GLU = KIND == kGlu, B_SEG = KIND == kRotate;
 	extern __shared__ uint8_t smem_raw[];
 	const int nacc = GLU ? 2 * g.n_tile : g.n_tile; // accumulator columns = N of the instruction; each CTA stages half of them
 	const uint32_t a_bytes = 128 * kRowBytes, b_bytes = (uint32_t)(nacc / 2) * kRowBytes, stage_bytes = a_bytes + b_bytes;
@@ -266,8 +297,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
 					}
 					if (dead)
 						for (int i = 0; i < 32; ++i) v[i] = kNaN;
-					if (GLU) store_patch_f16(g, patch, v, row0, n0 + c0, n_end);
-					else store_patch_f32(g, patch, v, row0, n0 + c0, n_end);
+					if constexpr (KIND == kRotate) {
+						rotate_store(g, seg, patch, v, row0, n0 - seg0 + c0, n_end - seg0);
+					} else if constexpr (GLU)
+						store_patch_f16(g, g.h, (size_t)g.ldc, patch, v, row0, n0 + c0, n_end);
+					else
+						store_patch_f32(g, patch, v, row0, n0 + c0, n_end);
 				}
 			}
 			tc_fence_before();
@@ -344,7 +379,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
 				if (dead)
 					for (int i = 0; i < 32; ++i) v[i] = kNaN;
 				if (n0 + c0 < n_end) {
-					if (GLU) store_patch_f16(g, patch, v, row0, n0 + c0, n_end);
+					if constexpr (KIND == kRotate) rotate_store(g, seg, patch, v, row0, n0 - seg0 + c0, n_end - seg0);
+					else if constexpr (GLU) store_patch_f16(g, g.h, (size_t)g.ldc, patch, v, row0, n0 + c0, n_end);
 					else store_patch_f32(g, patch, v, row0, n0 + c0, n_end);
 				}
 			}
@@ -584,11 +620,12 @@ static void plan_pair(GemmArgs &g, bool glu, const int (&slots)[3]) {
 	g.stages = pair_stages(glu, g.n_tile);
 }
 
-template <bool GLU, bool B_SEG>
+template <int KIND>
 static int launch_pair(GemmArgs &g, const void *a, int a_rows, const void *const (&w)[3], const int (&w_rows)[3], int nw, cudaStream_t st) {
+	constexpr bool GLU = KIND == kGlu;
 	static int slots[kMaxDevices][3]; // 0: not asked yet
 	static std::mutex mu;
-	auto kernel = gemm_pair_kernel<GLU, B_SEG>;
+	auto kernel = gemm_pair_kernel<KIND>;
 	const int dev = device_info().device;
 	if (dev < 0 || dev >= kMaxDevices) return YALM_EINVAL;
 	int here[3];
@@ -668,15 +705,28 @@ static int launch_few(GemmArgs &g, const void *a, int a_rows, const void *const 
 // Where the few-rows kernel ends: 128 positions are one operand of it, and up to there it is ahead of the pairs (4096 x 14336: 43 us
 // against 53 at 128 rows, 35 against 53 at 1 row).  With two matrices its two 128-row products read as much shared memory a cycle as
 // there is from about 80 positions on (14336 x 4096: 65.6 us against 67.6 at 64 rows, 73.8 against 68.3 at 128).
-template <bool GLU, bool B_SEG>
+constexpr int kFewRows = 128;
+template <bool GLU>
 static int launch(GemmArgs &g, const void *a, int a_rows, const void *const (&w)[3], const int (&w_rows)[3], int nw, cudaStream_t st) {
-	return g.M <= (GLU ? 64 : 128) ? launch_few<GLU, B_SEG>(g, a, a_rows, w, w_rows, nw, st) : launch_pair<GLU, B_SEG>(g, a, a_rows, w, w_rows, nw, st);
+	return g.M <= kFewRows / (GLU ? 2 : 1) ? launch_few<GLU, false>(g, a, a_rows, w, w_rows, nw, st) : launch_pair<GLU ? kGlu : kPlain>(g, a, a_rows, w, w_rows, nw, st);
 }
 
-// c (M, ldc) fp32 = a (M, K) fp16 times the rows of wq, wk and wv, side by side: the three projections of a layer as one launch.
+// c (M, ldc) fp32 = a (M, K) fp16 times the rows of wq, wk and wv, side by side: the three projections of a layer as one launch, of up to 128 rows.
 int gemm_qkv_f16(float *c, int ldc, const void *a, const void *wq, const void *wk, const void *wv, int M, int q_dim, int kv_dim, int K, cudaStream_t st) {
+	if (M > kFewRows) return YALM_EINVAL;
 	GemmArgs g{M, q_dim + 2 * kv_dim, K, kStoreF32, 0, c, nullptr, ldc, 1.0f, 0, 3, {q_dim, q_dim + kv_dim, q_dim + 2 * kv_dim}, 0};
-	return launch<false, true>(g, a, M, {wq, wk, wv}, {q_dim, kv_dim, kv_dim}, 3, st);
+	return launch_few<false, true>(g, a, M, {wq, wk, wv}, {q_dim, kv_dim, kv_dim}, 3, st);
+}
+
+// The same for more rows than the few-rows kernel takes, finished: q (M, q_dim) fp16 rotated, k and v rotated and appended at positions pos0 .. of their
+// head-major rings.  turns: (M, head_dim / 2) cosines and sines.  Saves the fp32 rows on their way to a kernel of their own and back (512 rows of 32 + 2 x 8
+// heads of 128: four layers and a head 1268 -> 1221 us).
+int gemm_qkv_rotate(void *q, void *k, void *v, const void *turns, const void *a, const void *wq, const void *wk, const void *wv, int M, int q_dim, int kv_dim, int K,
+                    int head_dim, int ring, int pos0, float clip, cudaStream_t st) {
+	if (M <= kFewRows || head_dim % 32) return YALM_EINVAL;
+	GemmArgs g{M, q_dim + 2 * kv_dim, K, kStoreF32, 0, nullptr, nullptr, 0, 1.0f, 0, 3, {q_dim, q_dim + kv_dim, q_dim + 2 * kv_dim}, 0};
+	g.rotate = {static_cast<__half *>(q), static_cast<__half *>(k), static_cast<__half *>(v), static_cast<const float2 *>(turns), head_dim, ring, pos0, clip};
+	return launch_pair<kRotate>(g, a, M, {wq, wk, wv}, {q_dim, kv_dim, kv_dim}, 3, st);
 }
 
 } // namespace prefill
@@ -690,7 +740,7 @@ extern "C" int yalm_gemm_16(float *c, int ldc, const void *a, const void *w, int
 	if (!c || !a || !w || M < 1 || N < 1 || K < 8 || K % 8 || ldc < N || ldc % 4 || ((uintptr_t)a & 15) || ((uintptr_t)w & 15) || ((uintptr_t)c & 15))
 		return YALM_EINVAL;
 	GemmArgs g{M, N, K, accumulate ? kAddF32 : kStoreF32, 0, c, nullptr, ldc, alpha, bf16 != 0, 1, {N}, 0};
-	return launch<false, false>(g, a, M, {w, nullptr, nullptr}, {N, 0, 0}, 1, (cudaStream_t)s);
+	return launch<false>(g, a, M, {w, nullptr, nullptr}, {N, 0, 0}, 1, (cudaStream_t)s);
 }
 // The same with one input per segment of output columns: columns [segment_end[i - 1], segment_end[i]) of c = a_i w^T, a_i = rows
 // i M .. i M + M - 1 of a (n_segments M, K).  Segment bounds are multiples of 4 (the last one is N).
@@ -704,7 +754,7 @@ extern "C" int yalm_gemm_16_segments(float *c, int ldc, const void *a, const voi
 		if (segment_end[i] <= at || (i + 1 < n_segments && segment_end[i] % 4)) return YALM_EINVAL;
 		g.seg_end[i] = at = segment_end[i];
 	}
-	return launch<false, false>(g, a, n_segments * M, {w, nullptr, nullptr}, {N, 0, 0}, 1, (cudaStream_t)s);
+	return launch<false>(g, a, n_segments * M, {w, nullptr, nullptr}, {N, 0, 0}, 1, (cudaStream_t)s);
 }
 extern "C" int yalm_gemm_f16(float *c, int ldc, const void *a, const void *w, int M, int N, int K, int accumulate, yalm_stream_t s) {
 	return yalm_gemm_16(c, ldc, a, w, M, N, K, accumulate, 0, 1.0f, s);
@@ -715,7 +765,7 @@ extern "C" int yalm_gemm_glu_f16(void *h, int ldh, const void *a, const void *w1
                                  yalm_stream_t s) {
 	if (!h || !a || !w1 || !w3 || M < 1 || N < 1 || K < 8 || K % 8 || ldh < N || ldh % 8) return YALM_EINVAL;
 	GemmArgs g{M, N, K, kGluF16, act, nullptr, static_cast<__half *>(h), ldh, 1.0f, 0, 1, {N}, 0};
-	return launch<true, false>(g, a, M, {w1, w3, nullptr}, {N, N, 0}, 2, (cudaStream_t)s);
+	return launch<true>(g, a, M, {w1, w3, nullptr}, {N, N, 0}, 2, (cudaStream_t)s);
 }
 
 // Host-pointer test entry: c (M, N) fp32 = a (M, K) fp16 * w (N, K)^T fp16 [+ c]; w3 != NULL: h (M, N) fp16 = GLU.
