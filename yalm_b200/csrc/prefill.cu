@@ -32,9 +32,11 @@ namespace prefill {
 
 // prefill_gemm.cu: the three projections as one launch
 int gemm_qkv_f16(float *c, int ldc, const void *a, const void *wq, const void *wk, const void *wv, int M, int q_dim, int kv_dim, int K, cudaStream_t st);
-// more than 128 rows: the three projections rotated and appended
+// more than 128 rows: the three projections rotated and appended; the probabilities of targets without the logits
 int gemm_qkv_rotate(void *q, void *k, void *v, const void *turns, const void *a, const void *wq, const void *wk, const void *wv, int M, int q_dim, int kv_dim, int K,
                     int head_dim, int ring, int pos0, float clip, cudaStream_t st);
+size_t score_bytes(int N);
+int gemm_score(float *probs, void *scratch, const int *targets, const void *a, const void *w, int M, int N, int K, cudaStream_t st);
 constexpr int kFewRows = 128;
 
 // (cosine, sine) of every position of the portion and pair of a head's channels: the same for all layers
@@ -212,7 +214,7 @@ int Model::forward_batch(InferenceState &s, const int *tokens, int n, int pos0, 
 	if (targets) YALM_TRY(cudaMemcpyAsync(P.targets, targets, sizeof(int) * n, cudaMemcpyHostToDevice, st));
 	embed_rows_kernel<<<n, 256, 0, st>>>(P.x, static_cast<const __half *>(token_embedding_table), P.tokens, dim);
 	const int act = c.act == ActivationType::SILU ? YALM_ACT_SILU : YALM_ACT_GELU;
-	const bool many = n > kFewRows; // the kernels of more rows finish q, k and v themselves
+	const bool many = n > kFewRows; // the kernels of more rows finish q, k and v, and the probabilities, themselves
 	int rc;
 	if (many) {
 		const int per = 256 / (c.head_dim / 2);
@@ -242,8 +244,12 @@ int Model::forward_batch(InferenceState &s, const int *tokens, int n, int pos0, 
 	}
 	if (targets) { // per-position logits -> probability of the given next token (Sampler::sample_prob per row)
 		if ((rc = launch_chained(rmsnorm_rows_kernel, dim3(n), dim3(kNormThreads), 0, st, 1, P.xb, P.x, rms_final_weight, dim, c.norm_eps))) return rc;
-		if ((rc = yalm_gemm_f16(P.logits, V, P.xb, wcls, n, V, dim, 0, st))) return rc;
-		if ((rc = yalm_token_probs(P.logits, V, n, P.targets, P.probs, st))) return rc;
+		if (many && score_bytes(V) <= 4ull * cap * V) {
+			if ((rc = gemm_score(P.probs, P.logits, P.targets, P.xb, wcls, n, V, dim, st))) return rc;
+		} else {
+			if ((rc = yalm_gemm_f16(P.logits, V, P.xb, wcls, n, V, dim, 0, st))) return rc;
+			if ((rc = yalm_token_probs(P.logits, V, n, P.targets, P.probs, st))) return rc;
+		}
 		YALM_TRY(cudaMemcpyAsync(probs_out, P.probs, sizeof(float) * n, cudaMemcpyDeviceToHost, st));
 	}
 	// the LAST position's logits through the decode path's final norm + LM head (fp32 activations), as after forward()

@@ -45,7 +45,7 @@ constexpr int kGemmThreads = 192;
 constexpr int kSegments = 8;
 
 enum Tail { kStoreF32 = 0, kAddF32 = 1, kGluF16 = 2 };
-enum Kind { kPlain = 0, kGlu = 1, kRotate = 2 }; // of the pair kernel
+enum Kind { kPlain = 0, kGlu = 1, kRotate = 2, kScore = 3 }; // of the pair kernel
 
 // kRotate: q | k | v columns are clipped, the pairs of q and k turned, and all stored as fp16, q as rows, k and v into the head-major ring.
 struct RotateArgs {
@@ -53,6 +53,12 @@ struct RotateArgs {
 	const float2 *turns; // (row, pair of a head): cosine, sine
 	int head_dim, ring, pos0;
 	float clip;
+};
+// kScore: of every row and column tile (maximum, sum of exponentials), and the row's value at its target column
+struct ScoreArgs {
+	float2 *parts; // (tile, row of 512)
+	float *at_target;
+	const int *targets;
 };
 
 struct GemmArgs {
@@ -70,6 +76,7 @@ struct GemmArgs {
 	int m_tiles, items, splits, kb_per; // 256-row tiles, tiles in all, K parts of a tile and their length in 64-wide blocks
 	int stages;
 	RotateArgs rotate;
+	ScoreArgs score;
 };
 
 // One tensor map per weight matrix: the segments' own matrices (wq, wk, wv), or w1 and w3, or one W.
@@ -285,6 +292,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
 			tc_fence_after();
 			const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16) + 256 * b;
 			if (row0 < g.M) {
+				float top = -INFINITY, sum = 0.f; // kScore: of this thread's row
+				int target = -1;
+				if constexpr (KIND == kScore)
+					if (row0 + lane < g.M) target = g.score.targets[row0 + lane] - n0;
 #pragma unroll 1
 				for (int c0 = 0; n0 + c0 < n_end; c0 += 32) {
 					float v[32];
@@ -297,13 +308,30 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
 					}
 					if (dead)
 						for (int i = 0; i < 32; ++i) v[i] = kNaN;
-					if constexpr (KIND == kRotate) {
+					if constexpr (KIND == kScore) {
+						float t4[4] = {top, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+						for (int i = 0; i < 32; ++i) {
+							if (n0 + c0 + i >= n_end) v[i] = -INFINITY;
+							t4[i & 3] = fmaxf(t4[i & 3], v[i]);
+							if (target == c0 + i) g.score.at_target[row0 + lane] = v[i];
+						}
+						const float m = fmaxf(fmaxf(t4[0], t4[1]), fmaxf(t4[2], t4[3]));
+						sum *= expf(top - m);
+						top = m;
+						float s4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+						for (int i = 0; i < 32; ++i) s4[i & 3] += expf(v[i] - m);
+						sum += (s4[0] + s4[1]) + (s4[2] + s4[3]);
+					} else if constexpr (KIND == kRotate) {
 						rotate_store(g, seg, patch, v, row0, n0 - seg0 + c0, n_end - seg0);
 					} else if constexpr (GLU)
 						store_patch_f16(g, g.h, (size_t)g.ldc, patch, v, row0, n0 + c0, n_end);
 					else
 						store_patch_f32(g, patch, v, row0, n0 + c0, n_end);
 				}
+				if constexpr (KIND == kScore)
+					if (row0 + lane < g.M) g.score.parts[(size_t)(item / g.m_tiles) * 512 + row0 + lane] = make_float2(top, sum);
 			}
 			tc_fence_before();
 			__syncwarp();
@@ -311,7 +339,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
 		}
 	}
 
-	if (g.splits > 1) { // one tile per cluster: the pairs' sums meet in shared memory, pair p finishes columns p n / splits ..
+	if (KIND != kScore && g.splits > 1) { // one tile per cluster: the pairs' sums meet in shared memory, pair p finishes columns p n / splits ..
 		int seg, seg0, n0, n_end;
 		tile_columns(g, cluster / g.m_tiles, seg, seg0, n0, n_end);
 		const int q = warp & 3, row = q * 32 + lane, row0 = (cluster % g.m_tiles) * 256 + half * 128 + q * 32;
@@ -647,6 +675,7 @@ static int launch_pair(GemmArgs &g, const void *a, int a_rows, const void *const
 		for (int i = 0; i < 3; ++i) here[i] = slots[dev][i];
 	}
 	if (here[0] < 1) return (int)cudaErrorLaunchOutOfResources;
+	if (KIND == kScore) here[1] = here[2] = 0; // a row's sum over a tile needs the whole products
 	plan_pair(g, GLU, here);
 	CUtensorMap ta;
 	WeightMaps tb;
@@ -727,6 +756,36 @@ int gemm_qkv_rotate(void *q, void *k, void *v, const void *turns, const void *a,
 	GemmArgs g{M, q_dim + 2 * kv_dim, K, kStoreF32, 0, nullptr, nullptr, 0, 1.0f, 0, 3, {q_dim, q_dim + kv_dim, q_dim + 2 * kv_dim}, 0};
 	g.rotate = {static_cast<__half *>(q), static_cast<__half *>(k), static_cast<__half *>(v), static_cast<const float2 *>(turns), head_dim, ring, pos0, clip};
 	return launch_pair<kRotate>(g, a, M, {wq, wk, wv}, {q_dim, kv_dim, kv_dim}, 3, st);
+}
+
+// Probability of every row's target column under the softmax of its row of a w^T (src/sampler.cpp:11-25), the products themselves not stored: (maximum, sum) of
+// every column tile, joined tile by tile (512 rows of 32000 columns were 65 MB to store and to read: four layers and a head 1221 -> 1180 us).  128 < M <= 512.  parts: room for (tiles, 512) float2 and 512 floats.
+__global__ void __launch_bounds__(256) join_scores_kernel(const float2 *parts, const float *at_target, const int *targets, float *probs, int tiles, int M, int N) {
+	chain_wait();
+	chain_next();
+	const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+	if (row >= M) return;
+	float m = -INFINITY, l = 0.f;
+	for (int i = lane; i < tiles; i += 32) {
+		const float2 p = parts[(size_t)i * 512 + row];
+		const float top = fmaxf(m, p.x);
+		l = l * expf(m - top) + p.y * expf(p.x - top);
+		m = top;
+	}
+	const float top = warp_max(m);
+	l = warp_sum(l * expf(m - top));
+	const int t = targets[row];
+	if (lane == 0) probs[row] = (t >= 0 && t < N) ? expf(at_target[row] - top) / l : 0.f;
+}
+size_t score_bytes(int N) { return ((size_t)((N + 63) / 64) * 512 * 2 + 512) * sizeof(float); } // (tiles of 64 columns at least)
+int gemm_score(float *probs, void *scratch, const int *targets, const void *a, const void *w, int M, int N, int K, cudaStream_t st) {
+	if (M <= kFewRows || M > 512 || N % 4) return YALM_EINVAL; // (N as for stored rows)
+	GemmArgs g{M, N, K, kStoreF32, 0, nullptr, nullptr, 0, 1.0f, 0, 1, {N}, 0};
+	float *at_target = static_cast<float *>(scratch);
+	g.score = {reinterpret_cast<float2 *>(at_target + 512), at_target, targets};
+	if (int rc = launch_pair<kScore>(g, a, M, {w, nullptr, nullptr}, {N, 0, 0}, 1, st)) return rc;
+	return launch_chained(join_scores_kernel, dim3((M + 7) / 8), dim3(256), 0, st, 1, (const float2 *)g.score.parts, (const float *)at_target, targets, probs,
+	                      g.items / g.m_tiles, M, N);
 }
 
 } // namespace prefill
