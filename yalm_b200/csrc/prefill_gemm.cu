@@ -432,7 +432,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ 
 	constexpr int MATS = GLU ? 2 : 1;
 	const int np = (g.M + 15) / 16 * 16; // positions, padded to the instruction's N
 	const uint32_t w_bytes = 128 * kRowBytes, a_bytes = (uint32_t)np * kRowBytes, stage_bytes = MATS * w_bytes + a_bytes;
-	const uint32_t base = (s32(smem_raw) + 1023u) & ~1023u, bars = base + g.stages * stage_bytes;
+	const uint32_t base = (s32(smem_raw) + 1023u) & ~1023u, bars = base + g.stages * stage_bytes, exch = bars + 512;
 	const uint32_t full0 = bars, empty0 = bars + 8 * g.stages, acc_bar = empty0 + 8 * g.stages, tslot = acc_bar + 8;
 	const int warp = uniform_warp(), lane = threadIdx.x & 31;
 	const int part = g.splits > 1 ? (int)cluster_rank() : 0, tile = blockIdx.x / g.splits;
@@ -447,6 +447,8 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ 
 		mbar_init(acc_bar, 1);
 		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 	}
+	if (g.splits > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); // waited for before this CTA writes into the others
+	if (warp == 0 && elect_one()) prefetch_map(&ta), prefetch_map(&tb.m[B_SEG ? seg : 0]);
 	if (warp == 1) tmem_alloc<1>(tslot, cols);
 	tc_fence_before();
 	__syncthreads();
@@ -505,19 +507,35 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ 
 	const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16);
 	// words of a group of 8 positions: [matrix][4-position half][row][4]
 	auto slot = [&](uint32_t buf, int src, int group, int m, int j) { return buf + (uint32_t)((((src * mine + group / g.splits) * MATS + m) * 2 + j) * 128 + row) * 16; };
+	// residuals of this CTA's groups, kBatch groups at a time, the first while the products run: behind them every group waited for its own (1.1 of 9.4 us at
+	// 17 x 4096 x 4096).  With the exchange's own space: 9.4 -> 8.8 us, 128 rows 15.8 -> 13.2, 100 x 6144 x 4096 20.8 -> 17.9, 17 x 1024 x 1024 4.5 -> 4.1
+	constexpr int kBatch = GLU ? 1 : 4;
+	const int col = n0 + row; // lanes are neighbouring output columns
+	const bool add = !GLU && g.tail == kAddF32 && col < n_end;
+	float x[kBatch][8];
+	auto fetch = [&](int first) {
+#pragma unroll
+		for (int b = 0; b < kBatch; ++b)
+#pragma unroll
+			for (int i = 0; i < 8; ++i) {
+				const int r = (first + b * g.splits) * 8 + i;
+				x[b][i] = add && r < g.M ? g.c[(size_t)r * g.ldc + col] : 0.f;
+			}
+	};
 	if (warp >= 2) {
+		fetch(part);
 		mbar_wait_warp(acc_bar, 0, dead);
 		__syncwarp();
 		tc_fence_after();
 	}
 	__syncwarp();
 	if (g.splits > 1) {
-		cluster_sync(); // every CTA's products are complete: the stages may be overwritten
+		asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); // the other CTAs run
 		if (warp >= 2)
 			for (int gr = 0; gr < groups; ++gr) {
 				const int p = gr % g.splits;
 				if (p == part) continue;
-				const uint32_t buf = map_rank(base, (uint32_t)p);
+				const uint32_t buf = map_rank(exch, (uint32_t)p);
 #pragma unroll
 				for (int m = 0; m < MATS; ++m) {
 					float v[8];
@@ -532,8 +550,12 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ 
 		cluster_sync(); // the other CTAs' sums of this CTA's positions are here
 	}
 	if (warp >= 2) {
-		const int col = n0 + row; // lanes are neighbouring output columns
-		for (int gr = part; gr < groups; gr += g.splits) {
+		for (int g0 = part; g0 < groups; g0 += kBatch * g.splits) {
+		if (g0 != part) fetch(g0);
+#pragma unroll
+		for (int b = 0; b < kBatch; ++b) {
+			const int gr = g0 + b * g.splits;
+			if (gr >= groups) break;
 			__syncwarp();
 			float v[MATS][8];
 #pragma unroll
@@ -548,7 +570,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ 
 						for (int i = 0; i < 8; ++i) v[m][i] += own[i];
 						continue;
 					}
-					const float4 lo = ld_shared4(slot(base, p < part ? p : p - 1, gr, m, 0)), hi = ld_shared4(slot(base, p < part ? p : p - 1, gr, m, 1));
+					const float4 lo = ld_shared4(slot(exch, p < part ? p : p - 1, gr, m, 0)), hi = ld_shared4(slot(exch, p < part ? p : p - 1, gr, m, 1));
 					v[m][0] += lo.x, v[m][1] += lo.y, v[m][2] += lo.z, v[m][3] += lo.w, v[m][4] += hi.x, v[m][5] += hi.y, v[m][6] += hi.z, v[m][7] += hi.w;
 				}
 			}
@@ -563,14 +585,12 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ 
 						if (i < rows) dst[(size_t)i * g.ldc] = __float2half_rn(v[0][i]);
 				} else {
 					float *dst = g.c + (size_t)(gr * 8) * g.ldc + col;
-					float x[8];
-#pragma unroll
-					for (int i = 0; i < 8; ++i) x[i] = (g.tail == kAddF32 && i < rows) ? dst[(size_t)i * g.ldc] : 0.f;
 #pragma unroll
 					for (int i = 0; i < 8; ++i)
-						if (i < rows) dst[(size_t)i * g.ldc] = dead ? kNaN : x[i] + g.alpha * v[0][i];
+						if (i < rows) dst[(size_t)i * g.ldc] = dead ? kNaN : x[b][i] + g.alpha * v[0][i];
 				}
 			}
+		}
 		}
 		tc_fence_before();
 	}
@@ -706,12 +726,11 @@ static int launch_few(GemmArgs &g, const void *a, int a_rows, const void *const 
 		const int per = (nkb + S - 1) / S;
 		if ((nkb + per - 1) / per == S) g.splits = S, g.kb_per = per; // (the last part must not be empty)
 	}
-	const size_t room = g.items * g.splits <= d.sms ? 212992 : 106496;
-	g.stages = std::max(2, std::min(std::min(16, g.kb_per), (int)(room / stage)));
-	// the exchange reuses the stages: (parts - 1) x groups of 8 positions per CTA x 4 KB x matrices
+	// the exchange has space of its own, so that no CTA waits for the others' products before it sends: (parts - 1) x groups of 8 positions per CTA x 4 KB x matrices
 	const size_t groups = ((g.M + 7) / 8 + g.splits - 1) / g.splits, exchange = (size_t)(g.splits - 1) * groups * mats * 4096;
-	while (g.stages * stage < exchange) ++g.stages;
-	const size_t smem = g.stages * stage + 512 + 1024;
+	const size_t room = g.items * g.splits <= d.sms ? std::min<size_t>(212992, d.max_smem_optin - 1536 - exchange) : 106496;
+	g.stages = std::max(2, std::min(std::min(16, g.kb_per), (int)(room / stage)));
+	const size_t smem = g.stages * stage + exchange + 512 + 1024;
 	if ((int)smem > d.max_smem_optin) return YALM_EINVAL;
 	{
 		std::lock_guard<std::mutex> lock(mu);

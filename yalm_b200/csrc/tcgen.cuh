@@ -80,6 +80,8 @@ __device__ __forceinline__ void st_shared4(uint32_t addr, float4 v) {
 	asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
 }
 
+// a tensor map on its way before the first copy asks for it
+__device__ __forceinline__ void prefetch_map(const CUtensorMap *map) { asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory"); }
 // Tensor copies.  CG 2: `bar` may lie in the pair's other CTA.
 template <int CG>
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int c0, int c1, uint32_t bar) {
