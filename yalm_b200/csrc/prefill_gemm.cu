@@ -45,7 +45,7 @@ constexpr int kGemmThreads = 192;
 constexpr int kSegments = 8;
 
 enum Tail { kStoreF32 = 0, kAddF32 = 1, kGluF16 = 2 };
-enum Kind { kPlain = 0, kGlu = 1, kRotate = 2, kScore = 3 }; // of the pair kernel
+enum Kind { kPlain = 0, kGlu = 1, kRotate = 2, kScore = 3, kResidual = 4 }; // of the pair kernel
 
 // kRotate: q | k | v columns are clipped, the pairs of q and k turned, and all stored as fp16, q as rows, k and v into the head-major ring.
 struct RotateArgs {
@@ -87,9 +87,19 @@ struct WeightMaps {
 // ---- tails ------------------------------------------------------------------------------------------------------------
 constexpr int kPatch = 32 * 36 * 4; // bytes of one warp's staging patch: 32 rows of 32 fp32, padded to 36
 
+// What store_patch_f32 adds to a warp's 32 rows x 32 columns, read a step ahead of it (behind the products every step waited for its own: 512 x 4096 x 14336
+// 63.5 -> 62.7 us, 4096 x 4096 21.1 -> 19.7, 8192 x 2048 23.2 -> 20.9)
+__device__ __forceinline__ void load_residual(const GemmArgs &g, float4 (&x)[8], int row0, int col, int col_end) {
+	const int lane = threadIdx.x & 31, r0 = lane >> 3, c0 = col + (lane & 7) * 4;
+	const float *base = g.c + (size_t)(row0 + r0) * g.ldc + c0;
+#pragma unroll
+	for (int t = 0; t < 8; ++t)
+		x[t] = c0 + 4 <= col_end && row0 + r0 + 4 * t < g.M ? *reinterpret_cast<const float4 *>(base + (size_t)(4 * t) * g.ldc) : make_float4(0.f, 0.f, 0.f, 0.f);
+}
 // A warp's 32 rows x 32 columns: lane = row holds v.  Through the warp's patch of shared memory, so that 8 lanes store (and for the
 // residual read) 128 consecutive bytes of a row: straight from the lanes every 16-byte piece would be half a sector of its own.
-__device__ __forceinline__ void store_patch_f32(const GemmArgs &g, uint32_t patch, const float (&v)[32], int row0, int col, int col_end) {
+template <bool ADD>
+__device__ __forceinline__ void store_patch_f32(const GemmArgs &g, uint32_t patch, const float (&v)[32], const float4 (&x)[ADD ? 8 : 1], int row0, int col, int col_end) {
 	const int lane = threadIdx.x & 31, r0 = lane >> 3, cc = (lane & 7) * 4;
 	__syncwarp();
 #pragma unroll
@@ -98,17 +108,12 @@ __device__ __forceinline__ void store_patch_f32(const GemmArgs &g, uint32_t patc
 	const int c0 = col + cc;
 	float *base = g.c + (size_t)(row0 + r0) * g.ldc + c0;
 	if (c0 + 4 <= col_end) {
-		float4 x[8];
-		if (g.tail == kAddF32) { // x += W v (src/infer.cpp:335-337), residual stream stays fp32
-#pragma unroll
-			for (int t = 0; t < 8; ++t)
-				if (row0 + r0 + 4 * t < g.M) x[t] = *reinterpret_cast<const float4 *>(base + (size_t)(4 * t) * g.ldc);
-		}
 #pragma unroll
 		for (int t = 0; t < 8; ++t) {
 			if (row0 + r0 + 4 * t >= g.M) continue;
 			float4 o = ld_shared4(patch + ((r0 + 4 * t) * 36 + cc) * 4);
-			if (g.tail == kAddF32) o.x += x[t].x, o.y += x[t].y, o.z += x[t].z, o.w += x[t].w;
+			if constexpr (ADD) // x += W v (src/infer.cpp:335-337), residual stream stays fp32
+				o.x += x[t].x, o.y += x[t].y, o.z += x[t].z, o.w += x[t].w;
 			*reinterpret_cast<float4 *>(base + (size_t)(4 * t) * g.ldc) = o;
 		}
 	} else if (c0 < col_end) {
@@ -117,7 +122,7 @@ __device__ __forceinline__ void store_patch_f32(const GemmArgs &g, uint32_t patc
 			const float4 o = ld_shared4(patch + ((r0 + 4 * t) * 36 + cc) * 4);
 			const float oo[4] = {o.x, o.y, o.z, o.w};
 			float *dst = base + (size_t)(4 * t) * g.ldc;
-			for (int j = 0; j < 4 && c0 + j < col_end; ++j) dst[j] = g.tail == kAddF32 ? dst[j] + oo[j] : oo[j];
+			for (int j = 0; j < 4 && c0 + j < col_end; ++j) dst[j] = ADD ? dst[j] + oo[j] : oo[j];
 		}
 	}
 }
@@ -200,7 +205,7 @@ constexpr int kTailBytes = 4 * kPatch + 512;
 template <int KIND>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ WeightMaps tb, const __grid_constant__ GemmArgs g) {
-	constexpr bool GLU = KIND == kGlu, B_SEG = KIND == kRotate;
+	constexpr bool GLU = KIND == kGlu, B_SEG = KIND == kRotate, ADD = KIND == kResidual;
 	extern __shared__ uint8_t smem_raw[];
 	const int nacc = GLU ? 2 * g.n_tile : g.n_tile; // accumulator columns = N of the instruction; each CTA stages half of them
 	const uint32_t a_bytes = 128 * kRowBytes, b_bytes = (uint32_t)(nacc / 2) * kRowBytes, stage_bytes = a_bytes + b_bytes;
@@ -287,6 +292,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
 			int seg, seg0, n0, n_end;
 			tile_columns(g, item / g.m_tiles, seg, seg0, n0, n_end);
 			const int b = done & 1, row0 = (item % g.m_tiles) * 256 + half * 128 + q * 32;
+			float4 next[ADD ? 8 : 1];
+			if constexpr (ADD) load_residual(g, next, row0, n0, n_end);
 			mbar_wait_warp(acc_full0 + 8 * b, (uint32_t)(done / 2) & 1u, dead);
 			__syncwarp();
 			tc_fence_after();
@@ -298,6 +305,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
 					if (row0 + lane < g.M) target = g.score.targets[row0 + lane] - n0;
 #pragma unroll 1
 				for (int c0 = 0; n0 + c0 < n_end; c0 += 32) {
+					float4 x[ADD ? 8 : 1];
+					if constexpr (ADD) {
+#pragma unroll
+						for (int i = 0; i < 8; ++i) x[i] = next[i];
+						load_residual(g, next, row0, n0 + c0 + 32, n_end);
+					}
 					float v[32];
 					tmem_ld32(trow + c0, v);
 					if (GLU) {
@@ -328,7 +341,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
 					} else if constexpr (GLU)
 						store_patch_f16(g, g.h, (size_t)g.ldc, patch, v, row0, n0 + c0, n_end);
 					else
-						store_patch_f32(g, patch, v, row0, n0 + c0, n_end);
+						store_patch_f32<ADD>(g, patch, v, x, row0, n0 + c0, n_end);
 				}
 				if constexpr (KIND == kScore)
 					if (row0 + lane < g.M) g.score.parts[(size_t)(item / g.m_tiles) * 512 + row0 + lane] = make_float2(top, sum);
@@ -346,7 +359,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
 		const int share = g.n_tile / g.splits;                    // columns (per matrix) that a pair finishes: a multiple of 32
 		const int mats = GLU ? 2 : 1, words = share * mats * 128; // floats that one pair sends another (per CTA)
 		const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16);
+		float4 next[ADD ? 8 : 1];
 		if (warp >= 2) {
+			if constexpr (ADD) load_residual(g, next, row0, n0 + part * share, n_end);
 			mbar_wait_warp(acc_full0, 0, dead);
 			__syncwarp();
 			tc_fence_after();
@@ -377,6 +392,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
 			const uint32_t patch = patch0 + q * kPatch;
 #pragma unroll 1
 			for (int c0 = part * share; c0 < (part + 1) * share; c0 += 32) {
+				float4 x[ADD ? 8 : 1];
+				if constexpr (ADD) {
+#pragma unroll
+					for (int i = 0; i < 8; ++i) x[i] = next[i];
+					if (c0 + 32 < (part + 1) * share) load_residual(g, next, row0, n0 + c0 + 32, n_end);
+				}
 				float v[32], u[GLU ? 32 : 1];
 				auto total = [&](float (&out)[32], int m) { // the parts of K in order
 					float own[32];
@@ -409,7 +430,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
 				if (n0 + c0 < n_end) {
 					if constexpr (KIND == kRotate) rotate_store(g, seg, patch, v, row0, n0 - seg0 + c0, n_end - seg0);
 					else if constexpr (GLU) store_patch_f16(g, g.h, (size_t)g.ldc, patch, v, row0, n0 + c0, n_end);
-					else store_patch_f32(g, patch, v, row0, n0 + c0, n_end);
+					else store_patch_f32<ADD>(g, patch, v, x, row0, n0 + c0, n_end);
 				}
 			}
 		}
@@ -756,7 +777,10 @@ static int launch_few(GemmArgs &g, const void *a, int a_rows, const void *const 
 constexpr int kFewRows = 128;
 template <bool GLU>
 static int launch(GemmArgs &g, const void *a, int a_rows, const void *const (&w)[3], const int (&w_rows)[3], int nw, cudaStream_t st) {
-	return g.M <= kFewRows / (GLU ? 2 : 1) ? launch_few<GLU, false>(g, a, a_rows, w, w_rows, nw, st) : launch_pair<GLU ? kGlu : kPlain>(g, a, a_rows, w, w_rows, nw, st);
+	if (g.M <= kFewRows / (GLU ? 2 : 1)) return launch_few<GLU, false>(g, a, a_rows, w, w_rows, nw, st);
+	if constexpr (!GLU)
+		if (g.tail == kAddF32) return launch_pair<kResidual>(g, a, a_rows, w, w_rows, nw, st);
+	return launch_pair<GLU ? kGlu : kPlain>(g, a, a_rows, w, w_rows, nw, st);
 }
 
 // c (M, ldc) fp32 = a (M, K) fp16 times the rows of wq, wk and wv, side by side: the three projections of a layer as one launch, of up to 128 rows.
