@@ -34,6 +34,26 @@ def test_attn_decode_splits(hd, G, n_kv):
         assert ((out.double() - want).norm() / want.norm()).item() < 1e-6, rows
 
 
+@pytest.mark.parametrize("ring", [16, 64, 65, 1100, 1200, 16384, 16400])
+def test_attn_decode_rings(ring):
+    """Four heads of 128 a kv head: rings with room for one split, a few, up to one a multiprocessor and more, and both sides of the line from which two CTAs share
+    a multiprocessor again (8 kv heads x 16384 rows); full and nearly empty.  Bound as above."""
+    L, n_kv, G, hd = api.lib(), 8, 4, 128
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(ring)
+    k, v = (torch.randn((n_kv, ring, hd), generator=gen, device="cuda").half() for _ in range(2))
+    q = torch.randn((n_kv * G, hd), generator=gen, device="cuda")
+    work = torch.zeros(L.yalm_attn_workspace_bytes(n_kv * G, n_kv, hd), device="cuda", dtype=torch.uint8)
+    out = torch.empty_like(q)
+    p = lambda t: C.c_void_p(t.data_ptr())
+    for rows in (1, ring // 2 + 1, ring):
+        ctl = torch.tensor([0, rows - 1, 0, rows - 1, rows, 0, 0, 0], device="cuda", dtype=torch.int32)
+        assert L.yalm_attn_decode(p(out), p(k), p(v), p(q), p(work), n_kv * G, n_kv, hd, ring, p(ctl), None) == 0
+        w = torch.softmax(torch.einsum("ghd,gtd->ght", q.view(n_kv, G, hd).double(), k[:, :rows].double()) * hd ** -0.5, dim=-1)
+        want = torch.einsum("ght,gtd->ghd", w, v[:, :rows].double()).reshape(n_kv * G, hd)
+        assert ((out.double() - want).norm() / want.norm()).item() < 1e-6, rows
+
+
 @pytest.mark.parametrize("hd,size", [(64, 8.0), (16, 4.0)])
 @pytest.mark.parametrize("rows", [40, 300, 3000])
 def test_attn_decode_large_scores(hd, size, rows):

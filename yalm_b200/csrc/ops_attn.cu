@@ -54,15 +54,16 @@ __device__ __forceinline__ float weight(float d, float c) { return expf(d * c); 
 
 // How a row's HD / 8 lanes share the scores of UN rows x G heads (value index u G + g): after the halving exchanges a lane holds N1
 // complete values, index (sub / DUP) N1 + j.
-template <int HD, int G>
+// ONE: one CTA per SM, whose warps fetch ahead, instead of two.
+template <int HD, int G, bool ONE>
 struct Split {
 	static constexpr int L = HD / 8;                   // lanes per K / V row (16 bytes each)
 	static constexpr int RPW = 32 / L;                 // rows per warp step
 	static constexpr int RPC = RPW * kAttnWarps;       // rows per CTA step
 	static constexpr int UN = G >= 8 ? 2 : G >= 4 ? 4 : 8; // steps in flight per thread, keys and values
-	static constexpr int CTAS = G >= 8 ? 1 : 2;         // resident per SM (8 heads' queries and sums take 128 registers of a lane)
-	static constexpr bool AHEAD = G >= 8;               // the next batch is fetched under this one's arithmetic (one CTA of 8 warps has little else in flight: 64 / 8
-	                                                   // heads of 128 at 4096 positions 15.3 -> 13.3 us, 32768 69.7 -> 49.7; with fewer heads the registers are taken by the second CTA)
+	static constexpr int CTAS = ONE ? 1 : 2;            // resident per SM (8 heads' queries and sums take 128 registers of a lane: always one)
+	static constexpr bool AHEAD = ONE;                  // the next batch is fetched under this one's arithmetic: 64 / 8 heads of 128 at 4096 positions 15.3 -> 13.3 us, 32768
+	                                                    // 69.7 -> 49.7
 	static constexpr int NV = UN * G, N1 = NV > L ? NV / L : 1, DUP = NV < L ? L / NV : 1;
 	static constexpr int NG = N1 < G ? N1 : G;         // heads that a lane's values belong to
 	static constexpr int U0 = DUP * (N1 < G ? G / N1 : 1); // lanes sub and sub ^ U0, sub ^ 2 U0, .. hold the same heads of other rows
@@ -75,9 +76,9 @@ struct Split {
 // result itself.  32 / 8 heads of 128, back to back, against a block-wide softmax per 512 rows: 37 positions 16 -> 3.9 us, 4096 19.6 -> 9.5 us, 32768
 // 68 -> 30 us.  Of 4096 positions in 37 splits the join took 5 of 10.3 us; one atomic that releases and acquires for two fences around it, and (maximum, sum) read once, made
 // that 9.5 (8 / 2 heads at 130: 5.7 -> 5.4).
-template <int HD, int G>
-__global__ void __launch_bounds__(kAttnThreads, Split<HD, G>::CTAS) attn_decode_kernel(AttnArgs a) {
-	using SP = Split<HD, G>;
+template <int HD, int G, bool ONE>
+__global__ void __launch_bounds__(kAttnThreads, Split<HD, G, ONE>::CTAS) attn_decode_kernel(AttnArgs a) {
+	using SP = Split<HD, G, ONE>;
 	constexpr int L = SP::L, RPC = SP::RPC, UN = SP::UN, NV = SP::NV, N1 = SP::N1, DUP = SP::DUP, NG = SP::NG;
 	extern __shared__ __align__(16) float smem[];
 	float *o_s = smem;                         // [kAttnWarps][G][HD]
@@ -402,15 +403,29 @@ static bool attn_fast_shape(int head_dim, int g) {
 	       (g == 1 || g == 2 || g == 4 || g == 8);
 }
 
+template <int HD, int G, bool ONE>
+static int launch_attn_of(AttnArgs &a, int splits, cudaStream_t st) {
+	a.max_splits = splits;
+	const size_t smem = ((size_t)a.max_splits * G + (size_t)kAttnWarps * G * HD) * sizeof(float);
+	YALM_TRY(allow_smem((const void *)attn_decode_kernel<HD, G, ONE>, smem));
+	return launch_chained(attn_decode_kernel<HD, G, ONE>, dim3(a.max_splits, a.n_kv_heads), dim3(kAttnThreads), smem, st, 1, a);
+}
 template <int HD, int G>
 static int launch_attn(AttnArgs &a, int S, cudaStream_t st) {
 	// all at once, and no more than a full ring has batches of rows for: the rest of a grid of 296 CTAs only begins and ends (32 / 8
 	// heads of 128, a ring of 512 and 390 positions: 6.6 us -> 5.6; of 1024: 7.0 -> 5.9)
-	constexpr int kRows = Split<HD, G>::RPC * Split<HD, G>::UN;
-	a.max_splits = std::max(1, std::min({S, Split<HD, G>::CTAS * device_info().sms / a.n_kv_heads, (a.max_seq_len + kRows - 1) / kRows}));
-	const size_t smem = ((size_t)a.max_splits * G + (size_t)kAttnWarps * G * HD) * sizeof(float);
-	YALM_TRY(allow_smem((const void *)attn_decode_kernel<HD, G>, smem));
-	return launch_chained(attn_decode_kernel<HD, G>, dim3(a.max_splits, a.n_kv_heads), dim3(kAttnThreads), smem, st, 1, a);
+	using SP = Split<HD, G, (G >= 8)>;
+	constexpr int kRows = SP::RPC * SP::UN;
+	const int sms = device_info().sms, of_ring = (a.max_seq_len + kRows - 1) / kRows;
+	const int splits = std::max(1, std::min({S, SP::CTAS * sms / a.n_kv_heads, of_ring}));
+	// Four heads of 128 a kv head, more splits than SMs: half as many, which fetch ahead, are joined sooner (32 / 8 heads at 2500 positions 9.1 -> 7.8 us, 8192 13.3 ->
+	// 13.0; 16 / 4 at 4096 9.1 -> 7.8, 18184 15.0 -> 14.0).  Rings of more rows than this want both CTAs' loads (32 / 8 at 18184 20.0 us against 20.7, 32768 30.0
+	// against 31.5).
+	constexpr long kFewer = 128 * 1024;
+	if constexpr (HD == 128 && G == 4)
+		if (splits * a.n_kv_heads > sms && (long)a.max_seq_len * a.n_kv_heads <= kFewer && sms / a.n_kv_heads > 0)
+			return launch_attn_of<HD, G, true>(a, sms / a.n_kv_heads, st);
+	return launch_attn_of<HD, G, (G >= 8)>(a, splits, st);
 }
 
 } // namespace yalm
