@@ -273,7 +273,7 @@ def run_prefill(args, arch, dtype, context, desc, base, path):
     pk = os.path.join(ROOT, "MEASURED_PEAKS.json")
     peak = float(json.load(open(pk))["bf16_tflops_sustained"]) if os.path.exists(pk) else 1374.5
     line = dict(base, impl="ours", metric="prefill tok/s (prompt tokens hydrated per second)", value=toks / t_host, steps=K, warmup=W,
-                ms_per_step=1000 * t_host / K, clocks=clk, gpu_launches=K * (2 + 8 * a.n_layers),
+                ms_per_step=1000 * t_host / K, clocks=clk, gpu_launches=K * (3 + 7 * a.n_layers),
                 e2e={"value": toks / t_host, "unit": "tok/s", "h2d_bytes_per_step": 4 * cap, "d2h_bytes_per_step": 4 * V,
                      "note": "host-timed around Model::forward_batch calls with host token buffers; each call copies the chunk's ids in and the last logits out"},
                 roofline={"bound": "tensor", "kernel": "gemm_pair_kernel (tcgen05.mma cta_group::2 kind::f16, TMA operands, TMEM accumulator) + prompt_attn_kernel",

@@ -117,12 +117,15 @@ def test_causal_attention_tiles(n, pos0, H, G, hd):
 
 @pytest.mark.parametrize("hd", [64, 128])
 @pytest.mark.parametrize("n,pos0,H,G", [(5, 100, 8, 2), (5, 128, 8, 2), (5, 381, 8, 2), (5, 400, 8, 2), (5, 515, 8, 2), (5, 1020, 8, 2), (5, 1030, 8, 2),  # 1, 2, 4, 5, 8, 9 key tiles
-                                        (512, 0, 37, 37), (512, 0, 38, 38), (511, 70, 38, 38), (505, 0, 32, 8), (100, 0, 75, 75), (509, 0, 152, 19), (16, 300, 128, 1), (3, 300, 256, 1), (40, 200, 20, 4)])
+                                        (512, 0, 37, 37), (512, 0, 38, 38), (511, 70, 38, 38), (505, 0, 32, 8), (100, 0, 75, 75), (509, 0, 152, 19), (160, 4000, 64, 8), (150, 3900, 64, 8), (300, 4200, 64, 8), (16, 300, 128, 1), (3, 300, 256, 1), (40, 200, 20, 4)])
 def test_causal_attention_single_tiles_and_pairs(n, pos0, H, G, hd):
     """Key tiles that leave the odd group of softmax warps none or one less, and both sides of the lines for cluster parts; as many row tiles as SMs
-    (148 of them: one a CTA) and more (two a CTA); groups of query heads that fill a tile, exceed it or do not divide it; ragged last tiles of results that leave as boxes.  Bound as above."""
+    (148 of them: one a CTA) and more (two a CTA); groups of query heads that fill a tile, exceed it or do not divide it; ragged last tiles of results that leave as boxes; enough key tiles for
+    warps that rescale, and one less.  Bound as above."""
     T = pos0 + n
     q, k, v = normal(n, (n, H, hd), dtype=torch.float16), normal(1, (G, T, hd), dtype=torch.float16), normal(2, (G, T, hd), dtype=torch.float16)
+    k[:, T // 2] *= 4                    # (accumulators are rescaled late, too)
+    k[:, 3 * T // 4] *= 8
     out = torch.full((n + 200, H, hd), 7.0, device="cuda", dtype=torch.float16)
     assert L().yalm_attn_prefill(ptr(out), ptr(q), ptr(k), ptr(v), *i32(n, pos0, H, G, hd, T), None) == 0
     seen = torch.arange(T, device="cuda")[None] <= torch.arange(n, device="cuda")[:, None] + pos0

@@ -10,16 +10,17 @@
 // warp 1 issues the products: S = Q K^T into TMEM, O += P V with P out of TMEM (its fp16 / bf16 words take the place of the scores).
 // Warps 4-7 and 8-11 are the softmax of A and B, a thread per row: scores from TMEM, online maximum and sum in fp32, P back to
 // TMEM.  The two tiles alternate: while one's scores go through the softmax the tensor pipe works for the other.  O stays in TMEM and is
-// rescaled whenever a row's maximum grows, so that the weight of a row's largest score is 1 and takes no rounding.  (A reference that follows
+// rescaled whenever a row's maximum grows (by the softmax warps or, in long calls, by warps of their own), so that the weight of a row's largest score is 1 and takes no rounding.  (A reference that follows
 // only growth beyond 2^8 saves 0.3 to 8 us of the calls below, but rounds the weight that counts most: a row that one key dominates is then off by
 // up to 2^-9 over bf16; 512 rows, window 1024, against 64 bits: 2.30e-3 for 2.24e-3.)  Warps 2 and 3 serve the layered models: they round pooled
 // fp32 means into stages, and clear the value rows of a ring tile that hold no position (a weight of zero times whatever lies there must be zero).
 //
 // Bound by the chain softmax - products of a tile pair (some 3500 cycles per 128 keys: 1800 from scores to weights, of which the exponentials
-// alone take 1024 at 16 a cycle and SM for each of the two tiles, 500 for the rescaling, and 1100 for P V and the next scores) and, for short
+// alone take 1024 at 16 a cycle and SM for each of the two tiles, 500 for the rescaling where the softmax warps do it, and 1100 for P V and the next scores), in a loop by
+// power (1000 W at 1640 MHz for the late portion) and, for short
 // contexts, by launch, query staging and the store.  Back to back, against 64-row tiles on mma.sync: 507 rows at 7680 positions, 32 / 8 heads of 128:
-// 667 -> 67 us (980 TFLOP/s); 512 rows at 0: 32.8 -> 8.9 us; bf16 window 1024 and pooled blocks of 64, 512 rows, 16 / 4 heads: 57.3 -> 14.5 us.
-// Of these SPLIT, with the queries of fp16 calls as boxes of a tensor map, made 70.2 to 67.3, 14.1 to 8.9 and 22.7 to 14.5: in pairs of tiles whose keys two CTAs
+// 667 -> 74 us (890 TFLOP/s; 66 in the first passes); 512 rows at 0: 32.8 -> 8.9 us; bf16 window 1024 and pooled blocks of 64, 512 rows, 16 / 4 heads: 57.3 -> 14.5 us.
+// Of these SPLIT, with the queries of fp16 calls as boxes of a tensor map, made 80.5 to 78.4, 14.1 to 8.9 and 22.7 to 14.5: in pairs of tiles whose keys two CTAs
 // share, staging took 2 us, and sending half of the accumulators (64 KB, some 20 bytes a cycle), both cluster barriers and the join 4 us.
 #include "common.cuh"
 #include "launch.h"
@@ -35,7 +36,7 @@
 namespace yalm {
 namespace prompt {
 
-constexpr int kThreads = 384, kTile = 128, kMaxDevices = 64;
+constexpr int kThreads = 384, kRescaleThreads = 512, kTile = 128, kMaxDevices = 64;
 
 struct Args {
 	void *out;          // fp16 rows (n, heads DV), or fp32 rows of stride ldo
@@ -111,6 +112,20 @@ __device__ __forceinline__ float ex2(float x) {
 	asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
 	return y;
 }
+template <int N>
+__device__ __forceinline__ void fewer_registers() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N>
+__device__ __forceinline__ void more_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+// mbar_wait_warp() without a call: the compiler finds no registers for the roles' own numbers of them in a kernel that calls functions
+__device__ __forceinline__ void wait_inline(uint32_t bar, uint32_t parity, bool &dead) {
+	if (__all_sync(kFull, mbar_try(bar, parity)) || dead) return;
+	const long long t0 = clock64();
+	while (!__all_sync(kFull, mbar_try(bar, parity)))
+		if (__any_sync(kFull, clock64() - t0 > 4000000000ll)) { // ~2 s
+			dead = true;
+			return;
+		}
+}
 __device__ __forceinline__ float max3(float a, float b, float c) {
 	float y;
 	asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
@@ -131,6 +146,11 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
 __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
 	uint64_t r;
 	asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+	return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+	uint64_t r;
+	asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
 	return r;
 }
 #define YALM_R32(r, o)                                                                                                                               \
@@ -198,19 +218,25 @@ struct Shape {
 	static constexpr int Q_BYTES = kTile * DKP * 2, K_BYTES = Q_BYTES, V_BYTES = kTile * DVP * 2, STAGE = K_BYTES > V_BYTES ? K_BYTES : V_BYTES;
 	static constexpr int STAGES = STAGE == 32768 ? 4 : 8;
 	// the parts of shared keys exchange through space of their own (no CTA waits for the others' products before it sends): (parts - 1) shares of the columns, (reference, sum) of every part
-	static constexpr int smem(bool split, int parts) {
-		return (split ? 1 : 2) * Q_BYTES + STAGES * STAGE + 512 + 1024 + (parts > 1 ? (parts - 1) * (DV / parts) * kTile * 4 + parts * kTile * 8 : 0);
+	static constexpr int smem(bool split, int parts) { // (behind the barriers also the factors of RESCALE, which has one part)
+		return (parts == 1 ? 2 * kTile * 4 : 0) + (split ? 1 : 2) * Q_BYTES + STAGES * STAGE + 512 + 1024 + (parts > 1 ? (parts - 1) * (DV / parts) * kTile * 4 + parts * kTile * 8 : 0);
 	}
 	static constexpr int MERGE = 72 * 1024; // where the even and the odd key tiles' (reference, sum) meet: over stages that are done with, behind the patches
 	static_assert(MERGE + 2 * kTile * 8 <= Q_BYTES + STAGES * STAGE, "");
 };
 
+__device__ __forceinline__ int first_position(const Args &a) {
+	if (!a.ctl) return a.pos0;
+	chain_wait();
+	return a.ctl[CTL_POS];
+}
+
 // T: operand type.  LAYERED: fp32 rows in and out, pooled blocks, ring tiles with rows that hold no position, sinks.
 // SPLIT: the CTA has one tile of rows, and A and B are its even and its odd key tiles.
 // SHARED: a cluster shares the keys (a kernel of its own: with the join in it, calls without one took 0.3 us longer).  BOXES: the results leave as boxes of the
-// tensor map to.
-template <typename T, int DK, int DV, bool LAYERED, bool SPLIT, bool SHARED, bool BOXES>
-__global__ void __launch_bounds__(kThreads, 1)
+// tensor map to.  RESCALE (with BOXES): the accumulators are rescaled by four warps of their own, 12 - 15, while the softmax warps form the weights.
+template <typename T, int DK, int DV, bool LAYERED, bool SPLIT, bool SHARED, bool BOXES, bool RESCALE>
+__global__ void __launch_bounds__(RESCALE ? kRescaleThreads : kThreads, 1)
 prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv,
                    const __grid_constant__ CUtensorMap to, const __grid_constant__ Args a) {
 	using SH = Shape<DK, DV>;
@@ -218,7 +244,8 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 	extern __shared__ uint8_t smem_raw[];
 	const uint32_t base = (s32(smem_raw) + 1023u) & ~1023u, q0 = base, kv0 = q0 + (ROWS / kTile) * SH::Q_BYTES, bars = kv0 + NST * SH::STAGE;
 	const uint32_t full0 = bars, empty0 = full0 + 8 * NST, s_full0 = empty0 + 8 * NST, p_full0 = s_full0 + 16, o_full = p_full0 + 32, v_clean0 = o_full + 8,
-	               q_full = v_clean0 + 8 * NST, tslot = q_full + 8;
+	               q_full = v_clean0 + 8 * NST, f_full0 = q_full + 8, tslot = f_full0 + 64;
+	const uint32_t factors = bars + 512; // RESCALE: [A, B][row] by what a row's accumulator is rescaled
 	const int warp = uniform_warp(), lane = threadIdx.x & 31;
 	const int parts = SHARED ? a.parts : 1, part = parts > 1 ? (int)cluster_rank() : 0;
 	const int rows = a.n * a.G, units = (rows + ROWS - 1) / ROWS;
@@ -228,8 +255,10 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 		// a value stage (odd) is free again once its products are done and, in a layered model, warps 2 and 3 have passed it
 		for (int i = 0; i < NST; ++i) mbar_init(full0 + 8 * i, 1), mbar_init(empty0 + 8 * i, LAYERED && (i & 1) ? 3 : 1);
 		for (int i = 0; i < 2; ++i) mbar_init(s_full0 + 8 * i, 1);
-		for (int i = 0; i < 4; ++i) mbar_init(p_full0 + 8 * i, 4); // [tile][half of the keys]
+		for (int i = 0; i < 4; ++i) mbar_init(p_full0 + 8 * i, RESCALE && !(i & 1) ? 8 : 4); // [tile][half of the keys]: the softmax warps; for the first half those that rescale, too
 		mbar_init(o_full, 1), mbar_init(q_full, 1);
+		if (RESCALE)
+			for (int i = 0; i < 8; ++i) mbar_init(f_full0 + 8 * i, 1); // [tile][quarter of the rows]
 		if (LAYERED)
 			for (int i = 0; i < NST; ++i) mbar_init(v_clean0 + 8 * i, 1);
 		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -239,12 +268,15 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 	if (warp == 1) tmem_alloc<1>(tslot, 512);
 	tc_fence_before();
 	__syncthreads(); // (tensor memory is this CTA's before the next kernel may take any)
-	if (a.ctl) chain_wait(); // else the tiles' divisions run under the kernel before this one
-	const int p0 = a.ctl ? a.ctl[CTL_POS] : a.pos0;
+	const int p0 = first_position(a); // (where no control block has it, the tiles' divisions run under the kernel before this one)
 	const Tiles tiles(a, p0 + r0 / a.G, p0 + min((r0 + ROWS - 1) / a.G, a.n - 1));
 	const int per = (tiles.total + parts - 1) / parts, k_begin = min(part * per, tiles.total), k_end = min(k_begin + per, tiles.total), nk = k_end - k_begin;
 	const bool first_pooled = LAYERED && nk > 0 && k_begin < tiles.pooled;
 	bool dead = false;
+	auto wait = [&](uint32_t bar, uint32_t parity) {
+		if constexpr (RESCALE) wait_inline(bar, parity, dead);
+		else mbar_wait_warp(bar, parity, dead);
+	};
 	chain_wait();
 	chain_next();
 	tc_fence_after();
@@ -253,7 +285,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 	// for, also where the entry is not a copy: a parity tells neighbouring rounds apart and no more.
 	auto load = [&](int i, int is_v) {
 		const int e = 2 * i + is_v, s = e % NST;
-		if (e >= NST) mbar_wait_warp(empty0 + 8 * s, (uint32_t)(e / NST - 1) & 1u, dead);
+		if (e >= NST) wait(empty0 + 8 * s, (uint32_t)(e / NST - 1) & 1u);
 		int slot, pos, valid;
 		if (tiles.at(k_begin + i, slot, pos, valid) || dead) return; // pooled tiles are filled by other warps
 		const uint32_t dst = kv0 + s * SH::STAGE, bar = full0 + 8 * s;
@@ -295,7 +327,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 		__syncwarp();
 		for (int e = 0; e < NST && e < 2 * nk; ++e) load(e >> 1, e & 1); // the stages are free: the first tiles travel while the queries are staged
 	}
-	if (warp > 0 && (LAYERED || !a.q_map)) { // the queries' rows (rows past the last: zero), and the first tile where it is a pooled one
+	if (!BOXES && warp > 0 && (LAYERED || !a.q_map)) { // the queries' rows (rows past the last: zero), and the first tile where it is a pooled one
 		// a thread keeps its 16-byte column and steps down the rows (the position and head of a row follow without a division); all loads of
 		// a batch are in flight together: one at a time this took as long as four key tiles
 		constexpr int PIECES = DK / 8, DOWN = (kThreads - 32) / PIECES, STEPS = (ROWS + DOWN - 1) / DOWN, BATCH = LAYERED && !SPLIT ? (STEPS + 1) / 2 : STEPS;
@@ -342,7 +374,13 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 	asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(tslot));
 
 	float mref = -INFINITY, l = 0.f; // of this thread's row: reference of the weights (in powers of two), their sum
+	auto leave = [&] { // RESCALE: every role runs to its own end.  Behind a join of the branches the compiler would have to do with the fewest registers of them
+		tc_fence_before();
+		asm volatile("bar.sync 0;" ::: "memory");
+	};
 
+	if (warp < 4) {
+	if constexpr (RESCALE) fewer_registers<56>(); // 512 threads x 128 registers, as launched, are 128 threads x (56 + 2 x 192 + 72)
 	if (warp == 0) {
 		if (first_pooled && elect_one()) mbar_arrive(full0), mbar_arrive(full0 + 8);
 		for (int e = NST; e < 2 * nk; ++e) load(e >> 1, e & 1);
@@ -352,7 +390,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 			constexpr uint32_t fmt = __is_same(T, __half) ? 0u : kInstrDescBf16;
 			const uint32_t qk_desc = instr_desc_f16(128, kTile) | fmt, pv_desc = instr_desc_f16(128, SH::DVP) | fmt | kBMajorMn;
 			auto wait_full = [&](int e) {
-				mbar_wait_warp(full0 + 8 * (e % NST), (uint32_t)(e / NST) & 1u, dead);
+				wait(full0 + 8 * (e % NST), (uint32_t)(e / NST) & 1u);
 				tc_fence_after();
 			};
 			auto scores = [&](int t, int e) {
@@ -374,7 +412,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 					int slot, pos, valid;
 					if (!tiles.at(k_begin + i, slot, pos, valid) && valid < kTile) {
 						const int sv = ev % NST;
-						mbar_wait_warp(v_clean0 + 8 * sv, (cleaned >> sv) & 1u, dead);
+						wait(v_clean0 + 8 * sv, (cleaned >> sv) & 1u);
 						cleaned ^= 1u << sv;
 						tc_fence_after();
 					}
@@ -385,7 +423,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 				const uint64_t vdesc = desc_mn(kv0 + (ev % NST) * SH::STAGE);
 #pragma unroll
 				for (int half = 0; half < 2; ++half) {
-					mbar_wait_warp(p_full0 + 16 * t + 8 * half, (uint32_t)round & 1u, dead);
+					wait(p_full0 + 16 * t + 8 * half, (uint32_t)round & 1u);
 					tc_fence_after();
 					if (elect_one()) {
 #pragma unroll
@@ -395,7 +433,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 					}
 				}
 			};
-			if (!LAYERED && a.q_map) mbar_wait_warp(q_full, 0, dead);
+			if (!LAYERED && a.q_map) wait(q_full, 0);
 			if constexpr (SPLIT) {
 				auto next_scores = [&](int i) {
 					wait_full(2 * i);
@@ -429,7 +467,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 			if (!dead && elect_one()) umma_commit(o_full);
 		}
 		__syncwarp();
-	} else if (warp < 4) {
+	} else {
 		if constexpr (LAYERED) {
 			const int tid = threadIdx.x - 64;
 			for (int i = 0; i < nk; ++i) {
@@ -437,13 +475,13 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 				const bool pooled = tiles.at(k_begin + i, slot, pos, valid);
 				const int ek = 2 * i, ev = 2 * i + 1;
 				if (pooled && i > 0) {
-					if (ek >= NST) mbar_wait_warp(empty0 + 8 * (ek % NST), (uint32_t)(ek / NST - 1) & 1u, dead);
-					if (ev >= NST) mbar_wait_warp(empty0 + 8 * (ev % NST), (uint32_t)(ev / NST - 1) & 1u, dead);
+					if (ek >= NST) wait(empty0 + 8 * (ek % NST), (uint32_t)(ek / NST - 1) & 1u);
+					if (ev >= NST) wait(empty0 + 8 * (ev % NST), (uint32_t)(ev / NST - 1) & 1u);
 					fill_pooled(i, tid, 64);
 					asm volatile("bar.sync 1, 64;" ::: "memory");
 					if (tid == 0) mbar_arrive(full0 + 8 * (ek % NST)), mbar_arrive(full0 + 8 * (ev % NST));
 				}
-				mbar_wait_warp(full0 + 8 * (ev % NST), (uint32_t)(ev / NST) & 1u, dead); // of every tile, to stay with the rounds
+				wait(full0 + 8 * (ev % NST), (uint32_t)(ev / NST) & 1u); // of every tile, to stay with the rounds
 				if (!pooled && valid < kTile) {
 					const uint32_t dst = kv0 + (ev % NST) * SH::STAGE;
 					constexpr int PIECES = SH::DVP / 8;
@@ -457,7 +495,56 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 			}
 		}
 		__syncwarp();
+	}
+	if constexpr (RESCALE) {
+		leave();
+		if (warp == 1) {
+			tc_fence_after();
+			tmem_dealloc<1>(tmem, 512);
+		}
+		return;
+	}
+	} else if (RESCALE && warp >= 12) { // ---- rescaling: rows 32 q .. of A and B in turn ----
+		fewer_registers<72>();
+		const int q = warp & 3;
+		for (int k = 0; k < nk; ++k)
+			for (int t = SPLIT ? k & 1 : 0; t < (SPLIT ? (k & 1) + 1 : nt); ++t) {
+				const int round = SPLIT ? k >> 1 : k;
+				if (round > 0) { // (before it there is nothing to rescale)
+					wait(s_full0 + 8 * t, (uint32_t)round & 1u); // the products into O so far are complete: they were issued before these scores
+					wait(f_full0 + 32 * t + 8 * q, (uint32_t)(round - 1) & 1u);
+					__syncwarp();
+					tc_fence_after();
+					float f;
+					asm volatile("ld.shared.f32 %0, [%1];" : "=f"(f) : "r"(factors + (uint32_t)((t * kTile + q * 32 + lane) * 4)) : "memory");
+					if (__any_sync(kFull, f != 1.0f)) {
+						const uint32_t op = tmem + ((uint32_t)(q * 32) << 16) + 256 + t * SH::DVP;
+						const uint64_t f2 = pack64(__float_as_uint(f), __float_as_uint(f));
+#pragma unroll 1
+						for (int x = 0; x < DV; x += 32) {
+							uint32_t o[32];
+							tmem_ld32_async<0>(op + x, o);
+							tmem_wait_ld();
+							pin(o);
+#pragma unroll
+							for (int y = 0; y < 32; y += 2) {
+								float lo, hi;
+								unpack64(mul2(pack64(o[y], o[y + 1]), f2), lo, hi);
+								o[y] = __float_as_uint(lo), o[y + 1] = __float_as_uint(hi);
+							}
+							tmem_st32<0>(op + x, o);
+						}
+						tmem_wait_st();
+					}
+					tc_fence_before();
+				}
+				__syncwarp();
+				if (!dead && lane == 0) mbar_arrive(p_full0 + 16 * t);
+			}
+		leave();
+		return;
 	} else {
+		if constexpr (RESCALE) more_registers<192>();
 		const int t = (warp - 4) >> 2, q = warp & 3, r = r0 + (SPLIT ? 0 : t * kTile) + q * 32 + lane;
 		if (t < nt && nk > 0) { // ---- softmax: one row per thread ----
 			const int i = p0 + min(r, rows - 1) / a.G; // rows past the last repeat it: finite values that are never stored
@@ -469,7 +556,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 				int slot, pos, valid;
 				const bool pooled = tiles.at(k_begin + k, slot, pos, valid);
 				const int from = pooled ? 0 : lo - pos, to = pooled ? nb - slot - 1 : min(i - pos, valid - 1); // visible: from .. to of the tile
-				mbar_wait_warp(s_full0 + 8 * t, (uint32_t)round & 1u, dead);
+				wait(s_full0 + 8 * t, (uint32_t)round & 1u);
 				__syncwarp();
 				tc_fence_after();
 				uint32_t s[kTile];
@@ -496,7 +583,16 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 					for (int y = 0; y < 4; ++y) mx4[y] = max3(mx4[y], __uint_as_float(s[x + 2 * y]), __uint_as_float(s[x + 2 * y + 1]));
 				const float top = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * c;
 				const bool grow = top > mref; // (not later: the largest weight of a row is then 1 and takes no rounding)
-				if (__any_sync(kFull, grow)) {
+				if constexpr (RESCALE) {
+					const float f = grow ? ex2(mref - top) : 1.0f; // mref -inf: 0
+					if (grow) mref = top;
+					l *= f;
+					if (round > 0) { // warp 12 + q rescales O while the weights are formed
+						asm volatile("st.shared.f32 [%0], %1;" ::"r"(factors + (uint32_t)((t * kTile + q * 32 + lane) * 4)), "f"(f) : "memory");
+						__syncwarp();
+						if (lane == 0) mbar_arrive(f_full0 + 32 * t + 8 * q);
+					}
+				} else if (__any_sync(kFull, grow)) {
 					const float f = grow ? ex2(mref - top) : 1.0f; // mref -inf: 0
 					if (grow) mref = top;
 					l *= f;
@@ -537,7 +633,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 				unpack64(add2(add2(l2[0], l2[1]), add2(l2[2], l2[3])), la, lb);
 				l += la + lb;
 			}
-			mbar_wait_warp(o_full, 0, dead);
+			wait(o_full, 0);
 			__syncwarp();
 			tc_fence_after();
 		}
@@ -732,11 +828,14 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 			}
 		}
 	}
-	tc_fence_before();
-	__syncthreads();
-	if (warp == 1) {
-		tc_fence_after();
-		tmem_dealloc<1>(tmem, 512);
+	if constexpr (RESCALE) leave();
+	else {
+		tc_fence_before();
+		__syncthreads();
+		if (warp == 1) {
+			tc_fence_after();
+			tmem_dealloc<1>(tmem, 512);
+		}
 	}
 }
 
@@ -780,10 +879,10 @@ static int make_query_map(CUtensorMap *map, const void *ptr, int d, int G, int n
 	return r == CUDA_SUCCESS ? 0 : YALM_EINVAL;
 }
 
-template <typename T, int DK, int DV, bool LAYERED, bool SPLIT, bool SHARED, bool BOXES>
+template <typename T, int DK, int DV, bool LAYERED, bool SPLIT, bool SHARED, bool BOXES, bool RESCALE>
 static int launch_of(Args &a, const void *keys, const void *values, int map_rows, cudaStream_t st) {
 	using SH = Shape<DK, DV>;
-	auto kernel = prompt_attn_kernel<T, DK, DV, LAYERED, SPLIT, SHARED, BOXES>;
+	auto kernel = prompt_attn_kernel<T, DK, DV, LAYERED, SPLIT, SHARED, BOXES, RESCALE>;
 	const int smem = SH::smem(SPLIT, a.parts);
 	YALM_TRY(allow_smem((const void *)kernel, smem));
 	CUtensorMap tq, tk, tv, to;
@@ -796,7 +895,7 @@ static int launch_of(Args &a, const void *keys, const void *values, int map_rows
 	if (!rc && BOXES) rc = make_query_map(&to, a.out, DV, a.G, a.n_kv, a.n);
 	if (rc) return rc;
 	constexpr int ROWS = SPLIT ? kTile : 2 * kTile;
-	return launch_chained(kernel, dim3((a.n * a.G + ROWS - 1) / ROWS * a.parts, a.n_kv), dim3(kThreads), smem, st, a.parts, tq, tk, tv, to, a);
+	return launch_chained(kernel, dim3((a.n * a.G + ROWS - 1) / ROWS * a.parts, a.n_kv), dim3(RESCALE ? kRescaleThreads : kThreads), smem, st, a.parts, tq, tk, tv, to, a);
 }
 // Clusters of 2, 4, 8 CTAs that share keys and run at once, of the current device
 template <typename T, int DK, int DV, bool LAYERED>
@@ -804,7 +903,7 @@ static int clusters_at_once(int (&room)[4]) {
 	using SH = Shape<DK, DV>;
 	static int at_once[kMaxDevices][4]; // 0: not asked yet
 	static std::mutex mu;
-	auto kernel = prompt_attn_kernel<T, DK, DV, LAYERED, true, true, false>;
+	auto kernel = prompt_attn_kernel<T, DK, DV, LAYERED, true, true, false, false>;
 	const DeviceInfo &dev = device_info();
 	if (dev.device < 0 || dev.device >= kMaxDevices) return YALM_EINVAL;
 	std::lock_guard<std::mutex> lock(mu);
@@ -829,6 +928,10 @@ static int clusters_at_once(int (&room)[4]) {
 // four 9.2; nine, 128 rows of 8 / 2 heads, in four 10.9, in eight 9.9).  est_tiles: key tiles of the longest rows.
 // fp16 results of more tiles than leave two parts a place leave through the copy engine (512 rows at 0, 32 / 8 heads of 128: 9.7 -> 8.9 us; 64 / 8: 14.5 -> 13.8);
 // a store of few CTAs is there as soon from their threads.
+// Those calls leave the rescaling to warps of their own: pairs of tiles always (64 / 8 heads of 128, 507 rows at 7680, in a loop: 147 -> 140 us; 512 at 0 14.5 -> 13.8),
+// single ones from kManyTiles key tiles on (32 / 8 heads at 7680: 79.7 -> 74.0 us, of 64 63.8 -> 54.6; at 2048, 20 key tiles, 26.1 on both; at 0 9.0 against 9.6 at 16 / 4
+// heads: what a round hands over costs more than it hides in few of them).
+constexpr int kManyTiles = 32;
 template <typename T, int DK, int DV, bool LAYERED>
 static int launch(Args &a, const void *keys, const void *values, int map_rows, int est_tiles, cudaStream_t st) {
 	const long tiles = (long)((a.n * (long)a.G + kTile - 1) / kTile) * a.n_kv;
@@ -837,17 +940,19 @@ static int launch(Args &a, const void *keys, const void *values, int map_rows, i
 	if (tiles > sms / 2 + 1) {
 		const bool split = tiles <= sms;
 		if constexpr (!LAYERED && DV % 64 == 0)
-			if (kTile % a.G == 0 && a.wide)
-				return split ? launch_of<T, DK, DV, LAYERED, true, false, true>(a, keys, values, map_rows, st)
-				             : launch_of<T, DK, DV, LAYERED, false, false, true>(a, keys, values, map_rows, st);
-		if (!split) return launch_of<T, DK, DV, LAYERED, false, false, false>(a, keys, values, map_rows, st);
+			if (kTile % a.G == 0 && a.wide) {
+				if (!split) return launch_of<T, DK, DV, LAYERED, false, false, true, true>(a, keys, values, map_rows, st);
+				return est_tiles >= kManyTiles ? launch_of<T, DK, DV, LAYERED, true, false, true, true>(a, keys, values, map_rows, st)
+				                               : launch_of<T, DK, DV, LAYERED, true, false, true, false>(a, keys, values, map_rows, st);
+			}
+		if (!split) return launch_of<T, DK, DV, LAYERED, false, false, false, false>(a, keys, values, map_rows, st);
 	} else if (est_tiles >= 4) {
 		int room[4];
 		if (int rc = clusters_at_once<T, DK, DV, LAYERED>(room)) return rc;
 		for (int i = 1; i < 4 && (1 << i) <= DV / 16 && tiles <= room[i] && est_tiles > (1 << i); ++i) a.parts = 1 << i;
-		if (a.parts > 1) return launch_of<T, DK, DV, LAYERED, true, true, false>(a, keys, values, map_rows, st);
+		if (a.parts > 1) return launch_of<T, DK, DV, LAYERED, true, true, false, false>(a, keys, values, map_rows, st);
 	}
-	return launch_of<T, DK, DV, LAYERED, true, false, false>(a, keys, values, map_rows, st);
+	return launch_of<T, DK, DV, LAYERED, true, false, false, false>(a, keys, values, map_rows, st);
 }
 
 constexpr float kLog2e = 1.4426950408889634f;
