@@ -8,8 +8,9 @@
 // Two kernels, 192 threads a CTA and the same roles: warp 0 brings 64-column (128-byte, SWIZZLE_128B) boxes of both operands
 // with cp.async.bulk.tensor.2d into a ring of pipeline stages (mbarrier complete_tx; rows / columns past the edge are
 // zero-filled), one thread of warp 1 issues tcgen05.mma.kind::f16 out of shared memory into a fp32 accumulator in TMEM,
-// warps 2-5 read it back (tcgen05.ld) and run the fused tail: plain fp32 store (q | k | v, logits), fp32 residual add in place
-// (wo, w2: x += ...), or act(w1 x) * (w3 x) -> fp16 (the A operand of the w2 GEMM).
+// warps 2-5 read it back (tcgen05.ld) and run the fused tail: plain fp32 store (q | k | v and logits of few rows), fp32 residual add in place
+// (wo, w2: x += ...), act(w1 x) * (w3 x) -> fp16 (the A operand of the w2 GEMM); of many rows also q, k and v rotated and appended, and what the
+// softmax of a row of logits needs of a tile.
 //
 //  * gemm_pair_kernel (many rows): a pair of CTAs (cta_group::2) owns a tile of 256 rows x n columns, each CTA staging 128 rows of A
 //    and half of the columns of W: twice the products per staged byte of one CTA per 128 x 128 tile.  Persistent over tiles, the
