@@ -573,46 +573,46 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ 
 	}
 	if (warp >= 2) {
 		for (int g0 = part; g0 < groups; g0 += kBatch * g.splits) {
-		if (g0 != part) fetch(g0);
+			if (g0 != part) fetch(g0);
 #pragma unroll
-		for (int b = 0; b < kBatch; ++b) {
-			const int gr = g0 + b * g.splits;
-			if (gr >= groups) break;
-			__syncwarp();
-			float v[MATS][8];
+			for (int b = 0; b < kBatch; ++b) {
+				const int gr = g0 + b * g.splits;
+				if (gr >= groups) break;
+				__syncwarp();
+				float v[MATS][8];
 #pragma unroll
-			for (int m = 0; m < MATS; ++m) {
-				float own[8];
-				tmem_ld8(trow + m * np + gr * 8, own);
+				for (int m = 0; m < MATS; ++m) {
+					float own[8];
+					tmem_ld8(trow + m * np + gr * 8, own);
 #pragma unroll
-				for (int i = 0; i < 8; ++i) v[m][i] = 0.f;
-				for (int p = 0; p < g.splits; ++p) { // the parts of K in order
-					if (p == part) {
+					for (int i = 0; i < 8; ++i) v[m][i] = 0.f;
+					for (int p = 0; p < g.splits; ++p) { // the parts of K in order
+						if (p == part) {
 #pragma unroll
-						for (int i = 0; i < 8; ++i) v[m][i] += own[i];
-						continue;
+							for (int i = 0; i < 8; ++i) v[m][i] += own[i];
+							continue;
+						}
+						const float4 lo = ld_shared4(slot(exch, p < part ? p : p - 1, gr, m, 0)), hi = ld_shared4(slot(exch, p < part ? p : p - 1, gr, m, 1));
+						v[m][0] += lo.x, v[m][1] += lo.y, v[m][2] += lo.z, v[m][3] += lo.w, v[m][4] += hi.x, v[m][5] += hi.y, v[m][6] += hi.z, v[m][7] += hi.w;
 					}
-					const float4 lo = ld_shared4(slot(exch, p < part ? p : p - 1, gr, m, 0)), hi = ld_shared4(slot(exch, p < part ? p : p - 1, gr, m, 1));
-					v[m][0] += lo.x, v[m][1] += lo.y, v[m][2] += lo.z, v[m][3] += lo.w, v[m][4] += hi.x, v[m][5] += hi.y, v[m][6] += hi.z, v[m][7] += hi.w;
+				}
+				if (col < n_end) {
+					const int rows = min(8, g.M - gr * 8);
+					if (GLU) {
+						__half *dst = g.h + (size_t)(gr * 8) * g.ldc + col;
+#pragma unroll
+						for (int i = 0; i < 8; ++i) v[0][i] = dead ? kNaN : glu(g, v[0][i], v[MATS - 1][i]);
+#pragma unroll
+						for (int i = 0; i < 8; ++i)
+							if (i < rows) dst[(size_t)i * g.ldc] = __float2half_rn(v[0][i]);
+					} else {
+						float *dst = g.c + (size_t)(gr * 8) * g.ldc + col;
+#pragma unroll
+						for (int i = 0; i < 8; ++i)
+							if (i < rows) dst[(size_t)i * g.ldc] = dead ? kNaN : x[b][i] + g.alpha * v[0][i];
+					}
 				}
 			}
-			if (col < n_end) {
-				const int rows = min(8, g.M - gr * 8);
-				if (GLU) {
-					__half *dst = g.h + (size_t)(gr * 8) * g.ldc + col;
-#pragma unroll
-					for (int i = 0; i < 8; ++i) v[0][i] = dead ? kNaN : glu(g, v[0][i], v[MATS - 1][i]);
-#pragma unroll
-					for (int i = 0; i < 8; ++i)
-						if (i < rows) dst[(size_t)i * g.ldc] = __float2half_rn(v[0][i]);
-				} else {
-					float *dst = g.c + (size_t)(gr * 8) * g.ldc + col;
-#pragma unroll
-					for (int i = 0; i < 8; ++i)
-						if (i < rows) dst[(size_t)i * g.ldc] = dead ? kNaN : x[b][i] + g.alpha * v[0][i];
-				}
-			}
-		}
 		}
 		tc_fence_before();
 	}
@@ -802,8 +802,9 @@ int gemm_qkv_rotate(void *q, void *k, void *v, const void *turns, const void *a,
 	return launch_pair<kRotate>(g, a, M, {wq, wk, wv}, {q_dim, kv_dim, kv_dim}, 3, st);
 }
 
-// Probability of every row's target column under the softmax of its row of a w^T (src/sampler.cpp:11-25), the products themselves not stored: (maximum, sum) of
-// every column tile, joined tile by tile (512 rows of 32000 columns were 65 MB to store and to read: four layers and a head 1221 -> 1180 us).  128 < M <= 512.  parts: room for (tiles, 512) float2 and 512 floats.
+// Probability of every row's target column under the softmax of its row of a w^T (src/sampler.cpp:11-25), the products themselves not stored: (maximum, sum)
+// of every column tile, joined tile by tile (512 rows of 32000 columns were 65 MB to store and to read: four layers and a head 1221 -> 1180 us).
+// 128 < M <= 512.  parts: room for (tiles, 512) float2 and 512 floats.
 __global__ void __launch_bounds__(256) join_scores_kernel(const float2 *parts, const float *at_target, const int *targets, float *probs, int tiles, int M, int N) {
 	chain_wait();
 	chain_next();

@@ -6,14 +6,15 @@
 // A CTA owns two such tiles (A, B) of one kv head, or (SPLIT) one tile, for which A and B are its even and its odd key tiles, joined from TMEM at the
 // end; then a cluster of CTAs may share the keys too, and joins (sum, maximum, accumulator) through distributed shared memory in a fixed order.
 //
-// 12 warps.  Warp 0 streams key and value tiles of 128 positions with cp.async.bulk.tensor.3d into a ring of stages.  One thread of
+// 12 warps, or 16.  Warp 0 streams key and value tiles of 128 positions with cp.async.bulk.tensor.3d into a ring of stages.  One thread of
 // warp 1 issues the products: S = Q K^T into TMEM, O += P V with P out of TMEM (its fp16 / bf16 words take the place of the scores).
 // Warps 4-7 and 8-11 are the softmax of A and B, a thread per row: scores from TMEM, online maximum and sum in fp32, P back to
 // TMEM.  The two tiles alternate: while one's scores go through the softmax the tensor pipe works for the other.  O stays in TMEM and is
-// rescaled whenever a row's maximum grows (by the softmax warps or, in long calls, by warps of their own), so that the weight of a row's largest score is 1 and takes no rounding.  (A reference that follows
-// only growth beyond 2^8 saves 0.3 to 8 us of the calls below, but rounds the weight that counts most: a row that one key dominates is then off by
-// up to 2^-9 over bf16; 512 rows, window 1024, against 64 bits: 2.30e-3 for 2.24e-3.)  Warps 2 and 3 serve the layered models: they round pooled
-// fp32 means into stages, and clear the value rows of a ring tile that hold no position (a weight of zero times whatever lies there must be zero).
+// rescaled whenever a row's maximum grows (by the softmax warps or, in long calls, by warps of their own), so that the weight of a row's largest
+// score is 1 and takes no rounding.  (A reference that follows only growth beyond 2^8 saves 0.3 to 8 us of the calls below, but rounds the weight that
+// counts most: a row that one key dominates is then off by up to 2^-9 over bf16; 512 rows, window 1024, against 64 bits: 2.30e-3 for 2.24e-3.)  Warps 2
+// and 3 serve the layered models: they round pooled fp32 means into stages, and clear the value rows of a ring tile that hold no position (a weight of
+// zero times whatever lies there must be zero).
 //
 // Bound by the chain softmax - products of a tile pair (some 3500 cycles per 128 keys: 1800 from scores to weights, of which the exponentials
 // alone take 1024 at 16 a cycle and SM for each of the two tiles, 500 for the rescaling where the softmax warps do it, and 1100 for P V and the next scores), in a loop by
@@ -217,7 +218,8 @@ struct Shape {
 	static constexpr int DKP = DK < 64 ? 64 : DK, DVP = DV < 64 ? 64 : DV; // channels a row takes in shared memory
 	static constexpr int Q_BYTES = kTile * DKP * 2, K_BYTES = Q_BYTES, V_BYTES = kTile * DVP * 2, STAGE = K_BYTES > V_BYTES ? K_BYTES : V_BYTES;
 	static constexpr int STAGES = STAGE == 32768 ? 4 : 8;
-	// the parts of shared keys exchange through space of their own (no CTA waits for the others' products before it sends): (parts - 1) shares of the columns, (reference, sum) of every part
+	// the parts of shared keys exchange through space of their own (no CTA waits for the others' products before it sends): (parts - 1) shares of the
+	// columns, (reference, sum) of every part
 	static constexpr int smem(bool split, int parts) { // (behind the barriers also the factors of RESCALE, which has one part)
 		return (parts == 1 ? 2 * kTile * 4 : 0) + (split ? 1 : 2) * Q_BYTES + STAGES * STAGE + 512 + 1024 + (parts > 1 ? (parts - 1) * (DV / parts) * kTile * 4 + parts * kTile * 8 : 0);
 	}
@@ -380,130 +382,130 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 	};
 
 	if (warp < 4) {
-	if constexpr (RESCALE) fewer_registers<56>(); // 512 threads x 128 registers, as launched, are 128 threads x (56 + 2 x 192 + 72)
-	if (warp == 0) {
-		if (first_pooled && elect_one()) mbar_arrive(full0), mbar_arrive(full0 + 8);
-		for (int e = NST; e < 2 * nk; ++e) load(e >> 1, e & 1);
-		__syncwarp();
-	} else if (warp == 1) {
-		if (nk > 0) { // ---- products ----
-			constexpr uint32_t fmt = __is_same(T, __half) ? 0u : kInstrDescBf16;
-			const uint32_t qk_desc = instr_desc_f16(128, kTile) | fmt, pv_desc = instr_desc_f16(128, SH::DVP) | fmt | kBMajorMn;
-			auto wait_full = [&](int e) {
-				wait(full0 + 8 * (e % NST), (uint32_t)(e / NST) & 1u);
-				tc_fence_after();
-			};
-			auto scores = [&](int t, int e) {
-				const uint64_t qa = smem_desc_sw128(q0 + (SPLIT ? 0 : t) * SH::Q_BYTES), ka = smem_desc_sw128(kv0 + (e % NST) * SH::STAGE);
-				if (elect_one()) {
-#pragma unroll
-					for (int k = 0; k < DK / 16; ++k) {
-						const uint32_t off = ((k >> 2) * (kTile * 128) + (k & 3) * 32) >> 4;
-						umma_f16<1>(tmem + t * kTile, qa + off, ka + off, qk_desc, k);
-					}
-					umma_commit(s_full0 + 8 * t);
-				}
-			};
-			uint32_t cleaned = 0; // a bit per stage: parity of its rounds of clearing
-			auto wait_values = [&](int i) {
-				const int ev = 2 * i + 1;
-				wait_full(ev);
-				if constexpr (LAYERED) {
-					int slot, pos, valid;
-					if (!tiles.at(k_begin + i, slot, pos, valid) && valid < kTile) {
-						const int sv = ev % NST;
-						wait(v_clean0 + 8 * sv, (cleaned >> sv) & 1u);
-						cleaned ^= 1u << sv;
-						tc_fence_after();
-					}
-				}
-			};
-			auto products = [&](int t, int i, int round, bool last) { // weights of round `round` of t times the values of tile i
-				const int ev = 2 * i + 1;
-				const uint64_t vdesc = desc_mn(kv0 + (ev % NST) * SH::STAGE);
-#pragma unroll
-				for (int half = 0; half < 2; ++half) {
-					wait(p_full0 + 16 * t + 8 * half, (uint32_t)round & 1u);
+		if constexpr (RESCALE) fewer_registers<56>(); // 512 threads x 128 registers, as launched, are 128 threads x (56 + 2 x 192 + 72)
+		if (warp == 0) {
+			if (first_pooled && elect_one()) mbar_arrive(full0), mbar_arrive(full0 + 8);
+			for (int e = NST; e < 2 * nk; ++e) load(e >> 1, e & 1);
+			__syncwarp();
+		} else if (warp == 1) {
+			if (nk > 0) { // ---- products ----
+				constexpr uint32_t fmt = __is_same(T, __half) ? 0u : kInstrDescBf16;
+				const uint32_t qk_desc = instr_desc_f16(128, kTile) | fmt, pv_desc = instr_desc_f16(128, SH::DVP) | fmt | kBMajorMn;
+				auto wait_full = [&](int e) {
+					wait(full0 + 8 * (e % NST), (uint32_t)(e / NST) & 1u);
 					tc_fence_after();
+				};
+				auto scores = [&](int t, int e) {
+					const uint64_t qa = smem_desc_sw128(q0 + (SPLIT ? 0 : t) * SH::Q_BYTES), ka = smem_desc_sw128(kv0 + (e % NST) * SH::STAGE);
 					if (elect_one()) {
 #pragma unroll
-						for (int k = 4 * half; k < 4 * half + 4; ++k) // 16 positions = 2048 bytes further in every sub-tile, 8 columns of P
-							umma_ts(tmem + 256 + t * SH::DVP, tmem + t * kTile + 8 * k, vdesc + (2048 >> 4) * k, pv_desc, (round | k) != 0);
-						if (half && last) umma_commit(empty0 + 8 * (ev % NST));
+						for (int k = 0; k < DK / 16; ++k) {
+							const uint32_t off = ((k >> 2) * (kTile * 128) + (k & 3) * 32) >> 4;
+							umma_f16<1>(tmem + t * kTile, qa + off, ka + off, qk_desc, k);
+						}
+						umma_commit(s_full0 + 8 * t);
 					}
-				}
-			};
-			if (!LAYERED && a.q_map) wait(q_full, 0);
-			if constexpr (SPLIT) {
-				auto next_scores = [&](int i) {
-					wait_full(2 * i);
-					scores(i & 1, 2 * i);
-					if (elect_one()) umma_commit(empty0 + 8 * (2 * i % NST));
 				};
-				next_scores(0);
-				if (nk > 1) next_scores(1);
-				for (int i = 0; i < nk && !dead; ++i) {
-					wait_values(i);
-					products(i & 1, i, i >> 1, true);
-					if (i + 2 < nk) next_scores(i + 2);
-				}
-			} else {
-				wait_full(0);
-				for (int t = 0; t < nt; ++t) scores(t, 0);
-				if (elect_one()) umma_commit(empty0);
-				for (int i = 0; i < nk && !dead; ++i) {
-					const int ek = 2 * i + 2;
-					wait_values(i);
-					for (int t = 0; t < nt; ++t) {
-						products(t, i, i, t == nt - 1);
-						if (i + 1 < nk) {
-							if (t == 0) wait_full(ek);
-							scores(t, ek);
-							if (t == nt - 1 && elect_one()) umma_commit(empty0 + 8 * (ek % NST));
+				uint32_t cleaned = 0; // a bit per stage: parity of its rounds of clearing
+				auto wait_values = [&](int i) {
+					const int ev = 2 * i + 1;
+					wait_full(ev);
+					if constexpr (LAYERED) {
+						int slot, pos, valid;
+						if (!tiles.at(k_begin + i, slot, pos, valid) && valid < kTile) {
+							const int sv = ev % NST;
+							wait(v_clean0 + 8 * sv, (cleaned >> sv) & 1u);
+							cleaned ^= 1u << sv;
+							tc_fence_after();
+						}
+					}
+				};
+				auto products = [&](int t, int i, int round, bool last) { // weights of round `round` of t times the values of tile i
+					const int ev = 2 * i + 1;
+					const uint64_t vdesc = desc_mn(kv0 + (ev % NST) * SH::STAGE);
+#pragma unroll
+					for (int half = 0; half < 2; ++half) {
+						wait(p_full0 + 16 * t + 8 * half, (uint32_t)round & 1u);
+						tc_fence_after();
+						if (elect_one()) {
+#pragma unroll
+							for (int k = 4 * half; k < 4 * half + 4; ++k) // 16 positions = 2048 bytes further in every sub-tile, 8 columns of P
+								umma_ts(tmem + 256 + t * SH::DVP, tmem + t * kTile + 8 * k, vdesc + (2048 >> 4) * k, pv_desc, (round | k) != 0);
+							if (half && last) umma_commit(empty0 + 8 * (ev % NST));
+						}
+					}
+				};
+				if (!LAYERED && a.q_map) wait(q_full, 0);
+				if constexpr (SPLIT) {
+					auto next_scores = [&](int i) {
+						wait_full(2 * i);
+						scores(i & 1, 2 * i);
+						if (elect_one()) umma_commit(empty0 + 8 * (2 * i % NST));
+					};
+					next_scores(0);
+					if (nk > 1) next_scores(1);
+					for (int i = 0; i < nk && !dead; ++i) {
+						wait_values(i);
+						products(i & 1, i, i >> 1, true);
+						if (i + 2 < nk) next_scores(i + 2);
+					}
+				} else {
+					wait_full(0);
+					for (int t = 0; t < nt; ++t) scores(t, 0);
+					if (elect_one()) umma_commit(empty0);
+					for (int i = 0; i < nk && !dead; ++i) {
+						const int ek = 2 * i + 2;
+						wait_values(i);
+						for (int t = 0; t < nt; ++t) {
+							products(t, i, i, t == nt - 1);
+							if (i + 1 < nk) {
+								if (t == 0) wait_full(ek);
+								scores(t, ek);
+								if (t == nt - 1 && elect_one()) umma_commit(empty0 + 8 * (ek % NST));
+							}
 						}
 					}
 				}
+				if (!dead && elect_one()) umma_commit(o_full);
 			}
-			if (!dead && elect_one()) umma_commit(o_full);
-		}
-		__syncwarp();
-	} else {
-		if constexpr (LAYERED) {
-			const int tid = threadIdx.x - 64;
-			for (int i = 0; i < nk; ++i) {
-				int slot, pos, valid;
-				const bool pooled = tiles.at(k_begin + i, slot, pos, valid);
-				const int ek = 2 * i, ev = 2 * i + 1;
-				if (pooled && i > 0) {
-					if (ek >= NST) wait(empty0 + 8 * (ek % NST), (uint32_t)(ek / NST - 1) & 1u);
-					if (ev >= NST) wait(empty0 + 8 * (ev % NST), (uint32_t)(ev / NST - 1) & 1u);
-					fill_pooled(i, tid, 64);
-					asm volatile("bar.sync 1, 64;" ::: "memory");
-					if (tid == 0) mbar_arrive(full0 + 8 * (ek % NST)), mbar_arrive(full0 + 8 * (ev % NST));
+			__syncwarp();
+		} else {
+			if constexpr (LAYERED) {
+				const int tid = threadIdx.x - 64;
+				for (int i = 0; i < nk; ++i) {
+					int slot, pos, valid;
+					const bool pooled = tiles.at(k_begin + i, slot, pos, valid);
+					const int ek = 2 * i, ev = 2 * i + 1;
+					if (pooled && i > 0) {
+						if (ek >= NST) wait(empty0 + 8 * (ek % NST), (uint32_t)(ek / NST - 1) & 1u);
+						if (ev >= NST) wait(empty0 + 8 * (ev % NST), (uint32_t)(ev / NST - 1) & 1u);
+						fill_pooled(i, tid, 64);
+						asm volatile("bar.sync 1, 64;" ::: "memory");
+						if (tid == 0) mbar_arrive(full0 + 8 * (ek % NST)), mbar_arrive(full0 + 8 * (ev % NST));
+					}
+					wait(full0 + 8 * (ev % NST), (uint32_t)(ev / NST) & 1u); // of every tile, to stay with the rounds
+					if (!pooled && valid < kTile) {
+						const uint32_t dst = kv0 + (ev % NST) * SH::STAGE;
+						constexpr int PIECES = SH::DVP / 8;
+						for (int x = valid * PIECES + tid; x < kTile * PIECES; x += 64) st_shared4(dst + tile_at(x / PIECES, x % PIECES), make_float4(0.f, 0.f, 0.f, 0.f));
+						proxy_fence();
+						asm volatile("bar.sync 1, 64;" ::: "memory");
+						if (tid == 0) mbar_arrive(v_clean0 + 8 * (ev % NST));
+					}
+					__syncwarp();
+					if (lane == 0) mbar_arrive(empty0 + 8 * (ev % NST));
 				}
-				wait(full0 + 8 * (ev % NST), (uint32_t)(ev / NST) & 1u); // of every tile, to stay with the rounds
-				if (!pooled && valid < kTile) {
-					const uint32_t dst = kv0 + (ev % NST) * SH::STAGE;
-					constexpr int PIECES = SH::DVP / 8;
-					for (int x = valid * PIECES + tid; x < kTile * PIECES; x += 64) st_shared4(dst + tile_at(x / PIECES, x % PIECES), make_float4(0.f, 0.f, 0.f, 0.f));
-					proxy_fence();
-					asm volatile("bar.sync 1, 64;" ::: "memory");
-					if (tid == 0) mbar_arrive(v_clean0 + 8 * (ev % NST));
-				}
-				__syncwarp();
-				if (lane == 0) mbar_arrive(empty0 + 8 * (ev % NST));
 			}
+			__syncwarp();
 		}
-		__syncwarp();
-	}
-	if constexpr (RESCALE) {
-		leave();
-		if (warp == 1) {
-			tc_fence_after();
-			tmem_dealloc<1>(tmem, 512);
+		if constexpr (RESCALE) {
+			leave();
+			if (warp == 1) {
+				tc_fence_after();
+				tmem_dealloc<1>(tmem, 512);
+			}
+			return;
 		}
-		return;
-	}
 	} else if (RESCALE && warp >= 12) { // ---- rescaling: rows 32 q .. of A and B in turn ----
 		fewer_registers<72>();
 		const int q = warp & 3;
