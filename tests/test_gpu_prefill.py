@@ -166,3 +166,43 @@ def test_forward_batch_of_many_rows_matches_few(hd, heads, kv, dim, rotary, clip
         assert np.abs(a - b).max() <= (2e-3 if layer < 2 else 6e-3) * max(1.0, np.abs(b).max())
     assert np.abs(l0 - l1).max() < LOGIT_TOL
     m.close()
+
+
+@pytest.mark.parametrize("n,vocab", [(129, 132), (256, 1000), (300, 20004), (511, 516), (512, 20000), (100, 20004)])
+@pytest.mark.parametrize("infinite", [False, True])
+def test_target_probabilities_against_64_bits(n, vocab, infinite):
+    """The probability of every row's target, of vocabularies that end anywhere in a tile of columns, with targets in the first and last columns and out of range (0).
+    A layer that adds nothing leaves the embedding, so the head's fp16 operand is known but for roundings of its last bit: some 2e-4 in a logit of size 1 each, and the
+    products' sums 3e-5: 1e-3 of a probability.  All columns count alike: without a tile of 64 of 20000 every probability is off by 3e-3.  infinite: columns of -infinity, the
+    first 40, tiles as a whole and the last 8, count as nothing."""
+    dim = 256
+    arch = yf.Arch(dim, 512, 32, 1, 8, 2, vocab, 1024, 10000.0, name="score")
+    tensors, hints = {}, {}
+    for name, arr, st in yf.random_tensors(arch, "fp16", seed=n + vocab, lm_scale=1.0):
+        if ".wo." in name or ".w2." in name:
+            arr = np.zeros_like(arr)
+        tensors[name], hints[name] = arr, st
+    embed, norm, head = (tensors["model.%s.weight" % x] for x in ("embed", "norm", "output"))
+    gone = np.zeros(vocab, bool)
+    if infinite:
+        embed[:, 0] = 1.0                                    # (times a positive weight: -infinity, not a sum of both signs or NaN)
+        norm[0] = 1.0
+        gone[512:1024] = vocab > 2000
+        gone[:40] = gone[-8:] = True
+        head[gone, 0] = -np.inf
+    m = api.Model(bytes(yf.build_image(tensors, yf.metadata_of(arch, "fp16"), hints))).cuda()
+    s = api.InferenceState(m)
+    rng = np.random.default_rng(n)
+    ids, targets = rng.integers(3, vocab, n).tolist(), rng.integers(0, vocab, n)
+    targets[:6] = [0, vocab - 1, vocab // 2, -1, vocab, vocab - 4]
+    got = np.array(s.forward_batch(ids, 0, targets.tolist()))
+    x = embed[ids].astype(np.float32)
+    a = (x / np.sqrt((x.astype(np.float64) ** 2).mean(1, keepdims=True) + arch.norm_eps) * norm).astype(np.float32).astype(np.float16)
+    logits = a.astype(np.float64) @ np.where(gone[:, None], 0, head).astype(np.float64).T
+    logits[:, gone] = -np.inf
+    e = np.exp(logits - logits.max(1, keepdims=True))
+    known = (targets >= 0) & (targets < vocab)
+    want = np.where(known, e[np.arange(n), np.where(known, targets, 0)] / e.sum(1), 0.0)
+    np.testing.assert_allclose(got, want, rtol=1e-3, atol=0)
+    s.close()
+    m.close()

@@ -31,6 +31,7 @@
 #include <cuda.h> // CUtensorMap + enums only: cuTensorMapEncodeTiled is resolved at run time (cudaGetDriverEntryPoint)
 
 #include <algorithm>
+#include <cfloat>
 #include <mutex>
 
 #include "gemv.cuh"
@@ -300,7 +301,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
 			tc_fence_after();
 			const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16) + 256 * b;
 			if (row0 < g.M) {
-				float top = -INFINITY, sum = 0.f; // kScore: of this thread's row
+				float top = -FLT_MAX, sum = 0.f; // kScore: of this thread's row (a finite start: columns of -infinity then count as 0)
 				int target = -1;
 				if constexpr (KIND == kScore)
 					if (row0 + lane < g.M) target = g.score.targets[row0 + lane] - n0;
@@ -810,7 +811,7 @@ __global__ void __launch_bounds__(256) join_scores_kernel(const float2 *parts, c
 	chain_next();
 	const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
 	if (row >= M) return;
-	float m = -INFINITY, l = 0.f;
+	float m = -FLT_MAX, l = 0.f; // (finite, as of a tile whose columns are all -infinity)
 	for (int i = lane; i < tiles; i += 32) {
 		const float2 p = parts[(size_t)i * 512 + row];
 		const float top = fmaxf(m, p.x);
