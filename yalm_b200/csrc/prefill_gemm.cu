@@ -448,7 +448,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
 
 // Few rows: 128 rows of W (of w1 and w3 each for GLU) against all M <= 128 positions.  A cluster of `splits` CTAs shares a tile's K;
 // CTA r finishes the groups of 8 positions g with g % splits == r.  TMEM lane = row of W, column = position.
-template <bool GLU, bool B_SEG>
+// ADD: the results are added to what lies in c, a kernel of its own: with the choice made at run time plain stores paid for the residuals' registers and steps
+// (100 x 6144 x 4096 16.6 us, 15.4 without; 128 x 512 x 512 9.5 and 8.1).
+template <bool GLU, bool B_SEG, bool ADD>
 __global__ void __launch_bounds__(kGemmThreads)
 gemm_few_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ WeightMaps tb, const __grid_constant__ GemmArgs g) {
 	extern __shared__ uint8_t smem_raw[];
@@ -532,18 +534,19 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ 
 	auto slot = [&](uint32_t buf, int src, int group, int m, int j) { return buf + (uint32_t)((((src * mine + group / g.splits) * MATS + m) * 2 + j) * 128 + row) * 16; };
 	// residuals of this CTA's groups, kBatch groups at a time, the first while the products run: behind them every group waited for its own (1.1 of 9.4 us at
 	// 17 x 4096 x 4096).  With the exchange's own space: 9.4 -> 8.8 us, 128 rows 15.8 -> 13.2, 100 x 6144 x 4096 20.8 -> 17.9, 17 x 1024 x 1024 4.5 -> 4.1
-	constexpr int kBatch = GLU ? 1 : 4;
+	constexpr int kBatch = ADD ? 4 : 1;
 	const int col = n0 + row; // lanes are neighbouring output columns
-	const bool add = !GLU && g.tail == kAddF32 && col < n_end;
-	float x[kBatch][8];
+	float x[kBatch][ADD ? 8 : 1];
 	auto fetch = [&](int first) {
+		if constexpr (ADD) {
 #pragma unroll
-		for (int b = 0; b < kBatch; ++b)
+			for (int b = 0; b < kBatch; ++b)
 #pragma unroll
-			for (int i = 0; i < 8; ++i) {
-				const int r = (first + b * g.splits) * 8 + i;
-				x[b][i] = add && r < g.M ? g.c[(size_t)r * g.ldc + col] : 0.f;
-			}
+				for (int i = 0; i < 8; ++i) {
+					const int r = (first + b * g.splits) * 8 + i;
+					x[b][i] = col < n_end && r < g.M ? g.c[(size_t)r * g.ldc + col] : 0.f;
+				}
+		}
 	};
 	if (warp >= 2) {
 		fetch(part);
@@ -610,7 +613,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ 
 						float *dst = g.c + (size_t)(gr * 8) * g.ldc + col;
 #pragma unroll
 						for (int i = 0; i < 8; ++i)
-							if (i < rows) dst[(size_t)i * g.ldc] = dead ? kNaN : x[b][i] + g.alpha * v[0][i];
+							if (i < rows) dst[(size_t)i * g.ldc] = dead ? kNaN : (ADD ? x[b][ADD ? i : 0] : 0.f) + g.alpha * v[0][i];
 					}
 				}
 			}
@@ -734,11 +737,11 @@ static int launch_pair(GemmArgs &g, const void *a, int a_rows, const void *const
 
 // Few rows: an SM's shared memory for stages, or half of it (two CTAs at once) where there are more tiles than SMs.  K parts
 // while every CTA still has an SM to itself: more CTAs than SMs would halve the stages of each.
-template <bool GLU, bool B_SEG>
+template <bool GLU, bool B_SEG, bool ADD>
 static int launch_few(GemmArgs &g, const void *a, int a_rows, const void *const (&w)[3], const int (&w_rows)[3], int nw, cudaStream_t st) {
 	static bool configured[kMaxDevices];
 	static std::mutex mu;
-	auto kernel = gemm_few_kernel<GLU, B_SEG>;
+	auto kernel = gemm_few_kernel<GLU, B_SEG, ADD>;
 	const DeviceInfo &d = device_info();
 	if (d.device < 0 || d.device >= kMaxDevices) return YALM_EINVAL;
 	const int np = (g.M + 15) / 16 * 16, mats = GLU ? 2 : 1, nkb = (g.K + BK - 1) / BK;
@@ -779,9 +782,10 @@ static int launch_few(GemmArgs &g, const void *a, int a_rows, const void *const 
 constexpr int kFewRows = 128;
 template <bool GLU>
 static int launch(GemmArgs &g, const void *a, int a_rows, const void *const (&w)[3], const int (&w_rows)[3], int nw, cudaStream_t st) {
-	if (g.M <= kFewRows / (GLU ? 2 : 1)) return launch_few<GLU, false>(g, a, a_rows, w, w_rows, nw, st);
+	const bool few = g.M <= kFewRows / (GLU ? 2 : 1);
 	if constexpr (!GLU)
-		if (g.tail == kAddF32) return launch_pair<kResidual>(g, a, a_rows, w, w_rows, nw, st);
+		if (g.tail == kAddF32) return few ? launch_few<false, false, true>(g, a, a_rows, w, w_rows, nw, st) : launch_pair<kResidual>(g, a, a_rows, w, w_rows, nw, st);
+	if (few) return launch_few<GLU, false, false>(g, a, a_rows, w, w_rows, nw, st);
 	return launch_pair<GLU ? kGlu : kPlain>(g, a, a_rows, w, w_rows, nw, st);
 }
 
@@ -789,7 +793,7 @@ static int launch(GemmArgs &g, const void *a, int a_rows, const void *const (&w)
 int gemm_qkv_f16(float *c, int ldc, const void *a, const void *wq, const void *wk, const void *wv, int M, int q_dim, int kv_dim, int K, cudaStream_t st) {
 	if (M > kFewRows) return YALM_EINVAL;
 	GemmArgs g{M, q_dim + 2 * kv_dim, K, kStoreF32, 0, c, nullptr, ldc, 1.0f, 0, 3, {q_dim, q_dim + kv_dim, q_dim + 2 * kv_dim}, 0};
-	return launch_few<false, true>(g, a, M, {wq, wk, wv}, {q_dim, kv_dim, kv_dim}, 3, st);
+	return launch_few<false, true, false>(g, a, M, {wq, wk, wv}, {q_dim, kv_dim, kv_dim}, 3, st);
 }
 
 // The same for more rows than the few-rows kernel takes, finished: q (M, q_dim) fp16 rotated, k and v rotated and appended at positions pos0 .. of their
