@@ -97,7 +97,7 @@ def attend(q, k, v, seen, scale, sink=None):
 
 @pytest.mark.parametrize("hd", [128, 64, 32])
 @pytest.mark.parametrize("n,pos0,H,G", [(1, 0, 4, 1), (2, 127, 8, 8), (7, 397, 32, 8), (129, 0, 8, 8), (33, 5000, 8, 8), (300, 77, 64, 8), (512, 511, 12, 2), (512, 0, 32, 8),
-                                        (260, 3000, 3, 1)])
+                                        (260, 3000, 3, 1), (33, 1100, 4, 2)])
 def test_causal_attention_tiles(n, pos0, H, G, hd):
     """Rows that fill a tile in part, both tiles, several CTAs; one key tile to many, in one part and in several; 3 query heads per
     kv head.  Slots past the portion hold NaN.  P is rounded to fp16 (2^-11) and so is the result: 5e-4 of the norm."""
@@ -200,9 +200,10 @@ def test_attention_not_finite_in_one_part(n, pos0, at, bad, bf16):
 @pytest.mark.parametrize("dk,dv", [(128, 128), (64, 64), (64, 128), (128, 64), (64, 32), (128, 32)])
 @pytest.mark.parametrize("n,pos0,H,G,Gv,window,pool,ring", [
     (32, 0, 8, 2, 2, 128, 64, 640), (512, 3584, 16, 4, 4, 1024, 64, 1536), (100, 777, 8, 2, 1, 500, 64, 1012), (257, 5000, 8, 8, 4, 300, 1, 557),
-    (300, 4000, 8, 2, 2, 128, 8, 700), (40, 9000, 16, 4, 4, 130, 16, 170), (64, 300, 6, 2, 2, 0, 0, 400), (90, 1000, 4, 4, 4, 200, 0, 289)])
+    (300, 4000, 8, 2, 2, 128, 8, 700), (40, 9000, 16, 4, 4, 130, 16, 170), (64, 300, 6, 2, 2, 0, 0, 400), (90, 1000, 4, 4, 4, 200, 0, 289),
+    (33, 2000, 8, 2, 2, 1500, 64, 2100)])
 def test_window_attention_tiles(n, pos0, H, G, Gv, window, pool, ring, dk, dv):
-    """Windows that wrap in the ring, rings that are no multiple of a tile, pooled blocks in one tile and in many (as blocks of one
+    """Windows that wrap in the ring, rings that are no multiple of a tile, keys in as many parts as there are, pooled blocks in one tile and in many (as blocks of one
     position too), value heads that several key heads share, sinks, a scale of either sign, positions from a control block.  Slots that
     hold no position are NaN.  Queries, pooled means and weights are rounded to bf16 (2^-9): 4e-3 of the norm."""
     q = normal(n, (n, H, dk))

@@ -644,7 +644,8 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 	// ---- the rows' results: this part finishes columns part DV / parts .. of its rows; in SPLIT each group of softmax warps half of these ----
 	const bool softmax_warp = warp >= 4;
 	const int t = (warp - 4) >> 2, q = warp & 3, tr = q * 32 + lane, row = r0 + (SPLIT ? 0 : t * kTile) + tr, share = DV / parts;
-	const int mine = SPLIT ? share / 2 : share, first_col = SPLIT ? t * mine : 0; // columns that a thread handles of a share, from where
+	const int mine = SPLIT ? max(share / 2, 8) : share, first_col = SPLIT ? t * mine : 0; // columns that a thread handles of a share, from where
+	const bool has_columns = !SHARED || first_col < share; // (a share of 8 is the even group's)
 	const uint32_t op = tmem + ((uint32_t)(q * 32) << 16) + 256 + (SPLIT ? 0 : t * SH::DVP);
 	// [other part][4 columns][row][4], then (reference, sum) [part][row]
 	const uint32_t exch = bars + 512, ml0 = exch + (uint32_t)((parts - 1) * share * kTile * 4);
@@ -689,7 +690,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 				const uint32_t there = map_rank(exch, (uint32_t)p);
 				if (t == 0)
 					asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(there + (ml0 - exch) + (uint32_t)((part * kTile + tr) * 8)), "f"(mref), "f"(l) : "memory");
-				if (p == part || nk == 0) continue;
+				if (p == part || nk == 0 || !has_columns) continue;
 				const uint32_t dst = there + (uint32_t)((part < p ? part : part - 1) * share * kTile * 4);
 				auto send = [&](auto width, int x) {
 					constexpr int W = decltype(width)::value;
@@ -707,7 +708,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 		__syncwarp();
 		cluster_sync(); // the other parts' share of these columns is here
 	}
-	if (softmax_warp && t < nt) {
+	if (softmax_warp && t < nt && has_columns) {
 		float M = mref, Lsum = l;
 		auto of_part = [&](int p, float &pm, float &pl) {
 			asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(pm), "=f"(pl) : "r"(ml0 + (uint32_t)((p * kTile + tr) * 8)) : "memory");
@@ -927,7 +928,8 @@ static int clusters_at_once(int (&room)[4]) {
 // One tile of rows a CTA while these run all at once, one per SM, and two beyond, which read a key tile once for both (64 / 8 heads of 128, 512 rows: at 0
 // 17.3 us in single tiles, 14.5 in pairs, at 7680 132 and 128).  Where tiles of rows leave SMs idle, a cluster shares the keys: as many parts as still run all at
 // once, at least four key tiles in all and more tiles than parts (17 rows, 32 / 8 heads of 128: three key tiles in one part 7.8 us, in two 8.4; five in two 9.7, in
-// four 9.2; nine, 128 rows of 8 / 2 heads, in four 10.9, in eight 9.9).  est_tiles: key tiles of the longest rows.
+// four 9.2; nine, 128 rows of 8 / 2 heads, in four 10.9, in eight 9.9).  Every part finishes 8 columns at least: 33 rows at 7680, 16 / 8 heads of 32: 29.2 us in two parts, 17.5 in four;
+// 12 / 4 of 64: 19.5 in four, 13.5 in eight.  est_tiles: key tiles of the longest rows.
 // fp16 results of more tiles than leave two parts a place leave through the copy engine (512 rows at 0, 32 / 8 heads of 128: 9.7 -> 8.9 us; 64 / 8: 14.5 -> 13.8);
 // a store of few CTAs is there as soon from their threads.
 // Those calls leave the rescaling to warps of their own: pairs of tiles always (64 / 8 heads of 128, 507 rows at 7680, in a loop: 147 -> 140 us; 512 at 0 14.5 -> 13.8),
@@ -951,7 +953,7 @@ static int launch(Args &a, const void *keys, const void *values, int map_rows, i
 	} else if (est_tiles >= 4) {
 		int room[4];
 		if (int rc = clusters_at_once<T, DK, DV, LAYERED>(room)) return rc;
-		for (int i = 1; i < 4 && (1 << i) <= DV / 16 && tiles <= room[i] && est_tiles > (1 << i); ++i) a.parts = 1 << i;
+		for (int i = 1; i < 4 && (1 << i) <= DV / 8 && tiles <= room[i] && est_tiles > (1 << i); ++i) a.parts = 1 << i;
 		if (a.parts > 1) return launch_of<T, DK, DV, LAYERED, true, true, false, false>(a, keys, values, map_rows, st);
 	}
 	return launch_of<T, DK, DV, LAYERED, true, false, false, false>(a, keys, values, map_rows, st);
