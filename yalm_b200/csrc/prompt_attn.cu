@@ -243,6 +243,10 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
                    const __grid_constant__ CUtensorMap to, const __grid_constant__ Args a) {
 	using SH = Shape<DK, DV>;
 	constexpr int NST = SH::STAGES, ROWS = SPLIT ? kTile : 2 * kTile; // rows of the CTA
+	// Of a tile's value rows only the groups of 16 that hold a position are cleared and multiplied (the weights of the others are 0): where values are wider than keys, a window
+	// over few keys waited for both (heads of 64 / 128 channels, 16 / 4 of them, 16 rows at 0: 5.27 us, 5.07; 32 rows 6.02, 5.83).  Else that is done under the scores and
+	// the softmax, and the conditions cost calls of many tiles 1 % (128 / 128 channels, 33 rows behind a window of 1500: 10.70 us against 10.88).
+	constexpr bool FEWER = LAYERED && !SHARED && DK < DV;
 	extern __shared__ uint8_t smem_raw[];
 	const uint32_t base = (s32(smem_raw) + 1023u) & ~1023u, q0 = base, kv0 = q0 + (ROWS / kTile) * SH::Q_BYTES, bars = kv0 + NST * SH::STAGE;
 	const uint32_t full0 = bars, empty0 = full0 + 8 * NST, s_full0 = empty0 + 8 * NST, p_full0 = s_full0 + 16, o_full = p_full0 + 32, v_clean0 = o_full + 8,
@@ -297,6 +301,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 			for (int c = 0; c < d; c += 64) tma_load_3d(dst + (c / 64) * (kTile * 128), is_v ? &tv : &tk, c, slot, head, bar);
 		}
 	};
+	auto cleared_to = [](int valid) { return FEWER ? (valid + 15) / 16 * 16 : kTile; }; // the first value row of a tile that no product reads
 	// a pooled tile's means into its two stages, rounded; value rows past the last block are zero (the scores of such keys are masked)
 	auto fill_pooled = [&](int i, int tid, int nthreads) {
 		int slot, pos, valid;
@@ -314,7 +319,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 			           make_float4(__uint_as_float(pack2<T>(lo.x, lo.y)), __uint_as_float(pack2<T>(lo.z, lo.w)), __uint_as_float(pack2<T>(hi.x, hi.y)),
 			                       __uint_as_float(pack2<T>(hi.z, hi.w))));
 		}
-		for (int x = valid * VP + tid; x < kTile * VP; x += nthreads) st_shared4(kv0 + ((2 * i + 1) % NST) * SH::STAGE + tile_at(x / VP, x % VP), make_float4(0.f, 0.f, 0.f, 0.f));
+		for (int x = valid * VP + tid; x < cleared_to(valid) * VP; x += nthreads) st_shared4(kv0 + ((2 * i + 1) % NST) * SH::STAGE + tile_at(x / VP, x % VP), make_float4(0.f, 0.f, 0.f, 0.f));
 		proxy_fence();
 	};
 
@@ -407,20 +412,22 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 					}
 				};
 				uint32_t cleaned = 0; // a bit per stage: parity of its rounds of clearing
-				auto wait_values = [&](int i) {
+				auto wait_values = [&](int i) { // returns how many groups of 16 rows count
 					const int ev = 2 * i + 1;
 					wait_full(ev);
 					if constexpr (LAYERED) {
 						int slot, pos, valid;
-						if (!tiles.at(k_begin + i, slot, pos, valid) && valid < kTile) {
+						if (!tiles.at(k_begin + i, slot, pos, valid) && valid < cleared_to(valid)) {
 							const int sv = ev % NST;
 							wait(v_clean0 + 8 * sv, (cleaned >> sv) & 1u);
 							cleaned ^= 1u << sv;
 							tc_fence_after();
 						}
-					}
+						return cleared_to(valid) / 16;
+					} else
+						return kTile / 16;
 				};
-				auto products = [&](int t, int i, int round, bool last) { // weights of round `round` of t times the values of tile i
+				auto products = [&](int t, int i, int round, bool last, int groups) { // weights of round `round` of t times the values of tile i
 					const int ev = 2 * i + 1;
 					const uint64_t vdesc = desc_mn(kv0 + (ev % NST) * SH::STAGE);
 #pragma unroll
@@ -430,7 +437,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 						if (elect_one()) {
 #pragma unroll
 							for (int k = 4 * half; k < 4 * half + 4; ++k) // 16 positions = 2048 bytes further in every sub-tile, 8 columns of P
-								umma_ts(tmem + 256 + t * SH::DVP, tmem + t * kTile + 8 * k, vdesc + (2048 >> 4) * k, pv_desc, (round | k) != 0);
+								if (!FEWER || k < groups) umma_ts(tmem + 256 + t * SH::DVP, tmem + t * kTile + 8 * k, vdesc + (2048 >> 4) * k, pv_desc, (round | k) != 0);
 							if (half && last) umma_commit(empty0 + 8 * (ev % NST));
 						}
 					}
@@ -445,8 +452,8 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 					next_scores(0);
 					if (nk > 1) next_scores(1);
 					for (int i = 0; i < nk && !dead; ++i) {
-						wait_values(i);
-						products(i & 1, i, i >> 1, true);
+						const int groups = wait_values(i);
+						products(i & 1, i, i >> 1, true, groups);
 						if (i + 2 < nk) next_scores(i + 2);
 					}
 				} else {
@@ -455,9 +462,9 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 					if (elect_one()) umma_commit(empty0);
 					for (int i = 0; i < nk && !dead; ++i) {
 						const int ek = 2 * i + 2;
-						wait_values(i);
+						const int groups = wait_values(i);
 						for (int t = 0; t < nt; ++t) {
-							products(t, i, i, t == nt - 1);
+							products(t, i, i, t == nt - 1, groups);
 							if (i + 1 < nk) {
 								if (t == 0) wait_full(ek);
 								scores(t, ek);
@@ -484,10 +491,10 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 						if (tid == 0) mbar_arrive(full0 + 8 * (ek % NST)), mbar_arrive(full0 + 8 * (ev % NST));
 					}
 					wait(full0 + 8 * (ev % NST), (uint32_t)(ev / NST) & 1u); // of every tile, to stay with the rounds
-					if (!pooled && valid < kTile) {
+					if (!pooled && valid < cleared_to(valid)) {
 						const uint32_t dst = kv0 + (ev % NST) * SH::STAGE;
 						constexpr int PIECES = SH::DVP / 8;
-						for (int x = valid * PIECES + tid; x < kTile * PIECES; x += 64) st_shared4(dst + tile_at(x / PIECES, x % PIECES), make_float4(0.f, 0.f, 0.f, 0.f));
+						for (int x = valid * PIECES + tid; x < cleared_to(valid) * PIECES; x += 64) st_shared4(dst + tile_at(x / PIECES, x % PIECES), make_float4(0.f, 0.f, 0.f, 0.f));
 						proxy_fence();
 						asm volatile("bar.sync 1, 64;" ::: "memory");
 						if (tid == 0) mbar_arrive(v_clean0 + 8 * (ev % NST));
@@ -671,8 +678,12 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 		constexpr int W = sizeof(v) / 4;
 		if constexpr (SPLIT) {
 			float odd[W];
-			if constexpr (W == 32) tmem_ld32(op + x, v), tmem_ld32(op + SH::DVP + x, odd);
-			else tmem_ld8(op + x, v), tmem_ld8(op + SH::DVP + x, odd);
+			if constexpr (W == 32) tmem_ld32(op + x, v);
+			else tmem_ld8(op + x, v);
+			if (!FEWER || nk > 1) { // (one key tile: no odd ones)
+				if constexpr (W == 32) tmem_ld32(op + SH::DVP + x, odd);
+				else tmem_ld8(op + SH::DVP + x, odd);
+			}
 #pragma unroll
 			for (int y = 0; y < W; ++y) {
 				v[y] = any0 ? w0 * v[y] : 0.f;
