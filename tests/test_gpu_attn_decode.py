@@ -34,11 +34,11 @@ def test_attn_decode_splits(hd, G, n_kv):
         assert ((out.double() - want).norm() / want.norm()).item() < 1e-6, rows
 
 
-@pytest.mark.parametrize("ring", [16, 64, 65, 1100, 1200, 16384, 16400])
-def test_attn_decode_rings(ring):
-    """Four heads of 128 a kv head: rings with room for one split, a few, up to one a multiprocessor and more, and both sides of the line from which two CTAs share
-    a multiprocessor again (8 kv heads x 16384 rows); full and nearly empty.  Bound as above."""
-    L, n_kv, G, hd = api.lib(), 8, 4, 128
+@pytest.mark.parametrize("ring,n_kv", [(16, 8), (64, 8), (65, 8), (1100, 8), (1200, 8), (16384, 8), (16400, 8), (8484, 14), (8500, 14), (900, 15)])
+def test_attn_decode_rings(ring, n_kv):
+    """Four heads of 128 a kv head: rings with room for one split, a few, up to one a multiprocessor and more, and both sides of the lines from which two CTAs share
+    a multiprocessor again (128 K rows of up to 8 kv heads, 116 K of up to 14); full and nearly empty.  Bound as above."""
+    L, G, hd = api.lib(), 4, 128
     gen = torch.Generator(device="cuda")
     gen.manual_seed(ring)
     k, v = (torch.randn((n_kv, ring, hd), generator=gen, device="cuda").half() for _ in range(2))

@@ -73,9 +73,9 @@ struct Split {
 // rows are reduced together by halving exchanges (UN G - 1 + .. shuffles for all of them, not log2 of them for each), which leaves about
 // one exponential per lane and row batch.  Latency is what counts at a few thousand positions: a CTA's chain is control block, one batch
 // of keys and values, one exchange of partials; short contexts use fewer splits (at least one batch per warp each), one split writes the
-// result itself.  32 / 8 heads of 128, back to back, against a block-wide softmax per 512 rows: 37 positions 16 -> 3.9 us, 4096 19.6 -> 9.5 us, 32768
-// 68 -> 30 us.  Of 4096 positions in 37 splits the join took 5 of 10.3 us; one atomic that releases and acquires for two fences around it, and (maximum, sum) read once, made
-// that 9.5 (8 / 2 heads at 130: 5.7 -> 5.4).
+// result itself.  32 / 8 heads of 128, back to back, against a block-wide softmax per 512 rows: 37 positions 16 -> 3.9 us, 4096 19.6 -> 9.1 us, 32768
+// 68 -> 30 us.  Of 4096 positions in 37 splits (two CTAs an SM) the join took 5 of 10.3 us; one atomic that releases and acquires for two fences around it, and
+// (maximum, sum) read once, made that 9.5 (8 / 2 heads at 130: 5.7 -> 5.4); half the splits, which fetch ahead (launch_attn()), 9.1.
 template <int HD, int G, bool ONE>
 __global__ void __launch_bounds__(kAttnThreads, Split<HD, G, ONE>::CTAS) attn_decode_kernel(AttnArgs a) {
 	using SP = Split<HD, G, ONE>;
@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(kAttnThreads, Split<HD, G, ONE>::CTAS) attn_de
 // row in `att` exactly like the reference (src/infer.cu:338-384) — used for shapes the fast path does
 // not cover and by the mha test entry, which must return `att` (src/test.cpp:171-188).
 // Bound by latency: a lane reads a row of keys, then a column of values, and adds in their order.  So it has 64 values of a key and 16 rows of values in
-// flight: one by one, a layer whose weights had run through L2 since the last token paid the way to memory for each.  NOTE
+// flight: one by one, a layer whose weights had run through L2 since the last token paid the way to memory for each.
 __global__ void __launch_bounds__(256) attn_generic_kernel(float *out, float *att, const __half *kb, const __half *vb,
                                                            const float *q, int head_dim, int n_heads, int n_kv_heads,
                                                            int max_seq_len, int kv_len_arg, const int *ctl) {
@@ -418,12 +418,16 @@ static int launch_attn(AttnArgs &a, int S, cudaStream_t st) {
 	constexpr int kRows = SP::RPC * SP::UN;
 	const int sms = device_info().sms, of_ring = (a.max_seq_len + kRows - 1) / kRows;
 	const int splits = std::max(1, std::min({S, SP::CTAS * sms / a.n_kv_heads, of_ring}));
-	// Four heads of 128 a kv head, more splits than SMs: half as many, which fetch ahead, are joined sooner (32 / 8 heads at 2500 positions 9.1 -> 7.8 us, 8192 13.3 ->
-	// 13.0; 16 / 4 at 4096 9.1 -> 7.8, 18184 15.0 -> 14.0).  Rings of more rows than this want both CTAs' loads (32 / 8 at 18184 20.0 us against 20.7, 32768 30.0
-	// against 31.5).
-	constexpr long kFewer = 128 * 1024;
+	// Four heads of 128 a kv head, more splits than SMs: half as many, one CTA an SM that fetches ahead, are joined sooner.  Keys and values out of memory, us with two CTAs an SM
+	// against one: full rings, 32 / 8 heads 2048 8.0 7.6, 4096 9.8 9.4, 8192 13.3 13.1, 14336 18.3 17.5, 15360 18.5 18.5, 16384 18.6 19.3; 16 / 4 16384 14.8 13.1, 32768 20.0
+	// 19.6; 4 / 1 32768 17.2 13.6, 131072 26.1 22.9; 56 / 14 1755 9.4 8.5, 7021 16.4 15.8, 8777 18.2 18.4, 9362 18.4 19.3; 40 / 10 11468 18.1 17.6, 12697 18.5 19.3.  With 15 kv heads
+	// and more the few splits leave SMs idle or save little of the join: 60 / 15 4369 12.7 13.1, 64 / 16 4096 12.6 12.9, 160 / 40 2048 14.1 15.2.  The context is known on the
+	// device only, so the ring decides, which is full at the end alone: of 16384 rows of 8 heads 37 positions take 3.5 3.7 (with one CTA an SM the next kernel's
+	// wait for it), 390 6.6 6.3, 1000 7.1 6.6, 2500 9.6 8.5, 4096 10.0 9.5, 8192 13.3 13.0, 12000 16.5 15.7.  So: rings of up to 128 K rows of up to 8 kv heads, 116 K of up to 14.
+	constexpr int kFewHeads = 14;
+	const long few_rows = (a.n_kv_heads <= 8 ? 128 : 116) * 1024;
 	if constexpr (HD == 128 && G == 4)
-		if (splits * a.n_kv_heads > sms && (long)a.max_seq_len * a.n_kv_heads <= kFewer && sms / a.n_kv_heads > 0)
+		if (splits * a.n_kv_heads > sms && a.n_kv_heads <= kFewHeads && (long)a.max_seq_len * a.n_kv_heads <= few_rows)
 			return launch_attn_of<HD, G, true>(a, sms / a.n_kv_heads, st);
 	return launch_attn_of<HD, G, (G >= 8)>(a, splits, st);
 }
