@@ -53,3 +53,12 @@ def test_joins_of_the_token_kernels_attention():
     assert "if (dead) lsum = NaN;" in text and "= dead ? NaN : ls" in text
     joins = text[text.index("the warps' records in order"): text.index("// ---- a product")]
     assert joins.count("expf(") == 2 and "__expf" not in joins
+
+
+def test_rescaling_warps_wait_for_every_round():
+    """A parity tells neighbouring rounds of a barrier apart and no more: a warp that leaves out round 0 of the scores would find the parity of round 1 while round 0 is
+    still open."""
+    text = source("prompt_attn.cu")
+    rescale = text[text.index("---- rescaling:"): text.index("---- softmax: one row per thread")]
+    assert rescale.count("wait(s_full0 + 8 * t, (uint32_t)round & 1u)") == 1
+    assert rescale.index("wait(s_full0") < rescale.index("if (round > 0)") < rescale.index("wait(f_full0")

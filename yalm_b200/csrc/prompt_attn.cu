@@ -519,8 +519,8 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 		for (int k = 0; k < nk; ++k)
 			for (int t = SPLIT ? k & 1 : 0; t < (SPLIT ? (k & 1) + 1 : nt); ++t) {
 				const int round = SPLIT ? k >> 1 : k;
-				if (round > 0) { // (before it there is nothing to rescale)
-					wait(s_full0 + 8 * t, (uint32_t)round & 1u); // the products into O so far are complete: they were issued before these scores
+				wait(s_full0 + 8 * t, (uint32_t)round & 1u); // (of every round: a parity tells neighbouring ones apart and no more)
+				if (round > 0) { // before it there is nothing to rescale; the products into O so far are complete: they were issued before these scores
 					wait(f_full0 + 32 * t + 8 * q, (uint32_t)(round - 1) & 1u);
 					__syncwarp();
 					tc_fence_after();
