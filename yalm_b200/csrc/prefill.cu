@@ -10,6 +10,7 @@
 #include "gemv.cuh"
 #include "launch.h"
 #include "mega.h"
+#include "prefill.h"
 
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -29,15 +30,6 @@ int causal_f16(void *out, const void *q, const void *keys, const void *values, i
 }
 
 namespace prefill {
-
-// prefill_gemm.cu: the three projections as one launch
-int gemm_qkv_f16(float *c, int ldc, const void *a, const void *wq, const void *wk, const void *wv, int M, int q_dim, int kv_dim, int K, cudaStream_t st);
-// more than 128 rows: the three projections rotated and appended; the probabilities of targets without the logits
-int gemm_qkv_rotate(void *q, void *k, void *v, const void *turns, const void *a, const void *wq, const void *wk, const void *wv, int M, int q_dim, int kv_dim, int K,
-                    int head_dim, int ring, int pos0, float clip, cudaStream_t st);
-size_t score_bytes(int N);
-int gemm_score(float *probs, void *scratch, const int *targets, const void *a, const void *w, int M, int N, int K, cudaStream_t st);
-constexpr int kFewRows = 128;
 
 // (cosine, sine) of every position of the portion and pair of a head's channels: the same for all layers
 __global__ void turns_kernel(float2 *turns, int head_dim, int rotary_dim, int pos0, float theta) {
@@ -173,7 +165,7 @@ bool Model::supports_batch() const {
 
 int Model::batch_capacity() const {
 	if (config->stack) return supports_batch() ? config->max_seq_len : 0;
-	return supports_batch() ? 512 : 0;
+	return supports_batch() ? kPortionRows : 0;
 }
 
 int Model::forward_batch(InferenceState &s, const int *tokens, int n, int pos0, const int *targets, float *probs_out) {

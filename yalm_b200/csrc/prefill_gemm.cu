@@ -36,6 +36,7 @@
 
 #include "gemv.cuh"
 #include "launch.h"
+#include "prefill.h"
 #include "tcgen.cuh"
 
 namespace yalm {
@@ -58,7 +59,7 @@ struct RotateArgs {
 };
 // kScore: of every row and column tile (maximum, sum of exponentials), and the row's value at its target column
 struct ScoreArgs {
-	float2 *parts; // (tile, row of 512)
+	float2 *parts; // (tile, row of kPortionRows)
 	float *at_target;
 	const int *targets;
 };
@@ -346,7 +347,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
 						store_patch_f32<ADD>(g, patch, v, x, row0, n0 + c0, n_end);
 				}
 				if constexpr (KIND == kScore)
-					if (row0 + lane < g.M) g.score.parts[(size_t)(item / g.m_tiles) * 512 + row0 + lane] = make_float2(top, sum);
+					if (row0 + lane < g.M) g.score.parts[(size_t)(item / g.m_tiles) * kPortionRows + row0 + lane] = make_float2(top, sum);
 			}
 			tc_fence_before();
 			__syncwarp();
@@ -779,7 +780,6 @@ static int launch_few(GemmArgs &g, const void *a, int a_rows, const void *const 
 // Where the few-rows kernel ends: 128 positions are one operand of it, and up to there it is ahead of the pairs (4096 x 14336: 43 us
 // against 53 at 128 rows, 35 against 53 at 1 row).  With two matrices its two 128-row products read as much shared memory a cycle as
 // there is from about 80 positions on (14336 x 4096: 65.6 us against 67.6 at 64 rows, 73.8 against 68.3 at 128).
-constexpr int kFewRows = 128;
 template <bool GLU>
 static int launch(GemmArgs &g, const void *a, int a_rows, const void *const (&w)[3], const int (&w_rows)[3], int nw, cudaStream_t st) {
 	const bool few = g.M <= kFewRows / (GLU ? 2 : 1);
@@ -809,7 +809,7 @@ int gemm_qkv_rotate(void *q, void *k, void *v, const void *turns, const void *a,
 
 // Probability of every row's target column under the softmax of its row of a w^T (src/sampler.cpp:11-25), the products themselves not stored: (maximum, sum)
 // of every column tile, joined tile by tile (512 rows of 32000 columns were 65 MB to store and to read: four layers and a head 1221 -> 1180 us).
-// 128 < M <= 512.  parts: room for (tiles, 512) float2 and 512 floats.
+// kFewRows < M <= kPortionRows.  scratch: a float for every row, then (tile, row) float2.
 __global__ void __launch_bounds__(256) join_scores_kernel(const float2 *parts, const float *at_target, const int *targets, float *probs, int tiles, int M, int N) {
 	chain_wait();
 	chain_next();
@@ -817,7 +817,7 @@ __global__ void __launch_bounds__(256) join_scores_kernel(const float2 *parts, c
 	if (row >= M) return;
 	float m = -FLT_MAX, l = 0.f; // (finite, as of a tile whose columns are all -infinity)
 	for (int i = lane; i < tiles; i += 32) {
-		const float2 p = parts[(size_t)i * 512 + row];
+		const float2 p = parts[(size_t)i * kPortionRows + row];
 		const float top = fmaxf(m, p.x);
 		l = l * expf(m - top) + p.y * expf(p.x - top);
 		m = top;
@@ -827,12 +827,12 @@ __global__ void __launch_bounds__(256) join_scores_kernel(const float2 *parts, c
 	const int t = targets[row];
 	if (lane == 0) probs[row] = (t >= 0 && t < N) ? expf(at_target[row] - top) / l : 0.f;
 }
-size_t score_bytes(int N) { return ((size_t)((N + 63) / 64) * 512 * 2 + 512) * sizeof(float); } // (tiles of 64 columns at least)
+size_t score_bytes(int N) { return ((size_t)((N + 63) / 64) * 2 + 1) * kPortionRows * sizeof(float); } // (tiles of 64 columns at least)
 int gemm_score(float *probs, void *scratch, const int *targets, const void *a, const void *w, int M, int N, int K, cudaStream_t st) {
-	if (M <= kFewRows || M > 512 || N % 4) return YALM_EINVAL; // (N as for stored rows)
+	if (M <= kFewRows || M > kPortionRows || N % 4) return YALM_EINVAL; // (N as for stored rows)
 	GemmArgs g{M, N, K, kStoreF32, 0, nullptr, nullptr, 0, 1.0f, 0, 1, {N}, 0};
 	float *at_target = static_cast<float *>(scratch);
-	g.score = {reinterpret_cast<float2 *>(at_target + 512), at_target, targets};
+	g.score = {reinterpret_cast<float2 *>(at_target + kPortionRows), at_target, targets};
 	if (int rc = launch_pair<kScore>(g, a, M, {w, nullptr, nullptr}, {N, 0, 0}, 1, st)) return rc;
 	return launch_chained(join_scores_kernel, dim3((M + 7) / 8), dim3(256), 0, st, 1, (const float2 *)g.score.parts, (const float *)at_target, targets, probs,
 	                      g.items / g.m_tiles, M, N);
