@@ -206,3 +206,20 @@ def test_target_probabilities_against_64_bits(n, vocab, infinite):
     np.testing.assert_allclose(got, want, rtol=1e-3, atol=0)
     s.close()
     m.close()
+
+
+def test_portion_keeps_no_space_for_what_it_does_not_store():
+    """fp32 logits are stored of up to 128 rows: 66 MB of 128256 columns, not the 263 MB of 512 rows.  Other space is under 10 MB here."""
+    import torch
+    used = []
+    for vocab in (512, 128256):                             # (the first loads the kernels)
+        arch = yf.Arch(256, 512, 32, 1, 8, 2, vocab, 1024, 10000.0, tied=True, name="space")
+        m = api.Model(bytes(yf.random_model(arch, "fp16", seed=1))).cuda()
+        s = api.InferenceState(m)
+        free = torch.cuda.mem_get_info()[0]
+        for n in (40, 130):
+            assert np.isfinite(s.forward_batch([3] * n, 0, [4] * n)).all()
+        used.append(free - torch.cuda.mem_get_info()[0])
+        s.close()
+        m.close()
+    assert used[1] < 100e6

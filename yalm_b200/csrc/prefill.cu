@@ -185,7 +185,8 @@ int Model::forward_batch(InferenceState &s, const int *tokens, int n, int pos0, 
 		auto ps = std::make_shared<PrefillState>();
 		ps->cap = cap;
 		auto pad = [](size_t b) { return (b + 255) / 256 * 256; };
-		const size_t sz[] = {pad(4ull * cap * dim), pad(4ull * cap * (q_dim + 2 * kv_dim)), pad(4ull * cap * V), pad(4ull * cap),
+		// fp32 projections and logits are stored of few rows only; of more, what the softmax of a row needs of every tile of logits
+		const size_t sz[] = {pad(4ull * cap * dim), pad(4ull * kFewRows * (q_dim + 2 * kv_dim)), pad(std::max<size_t>(4ull * kFewRows * V, score_bytes(V))), pad(4ull * cap),
 		                     pad(2ull * cap * std::max(dim, q_dim)), pad(2ull * cap * q_dim), pad(2ull * cap * q_dim), pad(2ull * cap * hid),
 		                     pad(4ull * cap), pad(4ull * cap), pad(4ull * cap * c.head_dim)};
 		size_t total = 0;
@@ -236,7 +237,7 @@ int Model::forward_batch(InferenceState &s, const int *tokens, int n, int pos0, 
 	}
 	if (targets) { // per-position logits -> probability of the given next token (Sampler::sample_prob per row)
 		if ((rc = launch_chained(rmsnorm_rows_kernel, dim3(n), dim3(kNormThreads), 0, st, 1, P.xb, P.x, rms_final_weight, dim, c.norm_eps))) return rc;
-		if (many && score_bytes(V) <= 4ull * cap * V) {
+		if (many) {
 			if ((rc = gemm_score(P.probs, P.logits, P.targets, P.xb, wcls, n, V, dim, st))) return rc;
 		} else {
 			if ((rc = yalm_gemm_f16(P.logits, V, P.xb, wcls, n, V, dim, 0, st))) return rc;
