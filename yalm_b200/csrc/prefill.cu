@@ -32,13 +32,13 @@ int causal_f16(void *out, const void *q, const void *keys, const void *values, i
 namespace prefill {
 
 // (cosine, sine) of every position of the portion and pair of a head's channels: the same for all layers
-__global__ void turns_kernel(float2 *turns, int head_dim, int rotary_dim, int pos0, float theta) {
+__global__ void turns_kernel(float2 *turns, int n, int head_dim, int rotary_dim, int pos0, float theta) {
 	const int half = head_dim / 2, j = threadIdx.x % half, i = blockIdx.x * (blockDim.x / half) + threadIdx.x / half;
 	float fcr, fci;
 	rope_angle(fcr, fci, 2 * j, pos0 + i, theta, rotary_dim);
 	chain_wait();
 	chain_next();
-	turns[(size_t)i * half + j] = make_float2(fcr, fci);
+	if (i < n) turns[(size_t)i * half + j] = make_float2(fcr, fci);
 }
 
 // x[i, :] = float(E[tokens[i], :])   (src/infer.cu:632-640, for a batch of rows)
@@ -211,7 +211,7 @@ int Model::forward_batch(InferenceState &s, const int *tokens, int n, int pos0, 
 	int rc;
 	if (many) {
 		const int per = 256 / (c.head_dim / 2);
-		if ((rc = launch_chained(turns_kernel, dim3((n + per - 1) / per), dim3(256), 0, st, 1, P.turns, c.head_dim, c.rotary_dim, pos0, c.rope_theta))) return rc;
+		if ((rc = launch_chained(turns_kernel, dim3((n + per - 1) / per), dim3(256), 0, st, 1, P.turns, n, c.head_dim, c.rotary_dim, pos0, c.rope_theta))) return rc;
 	}
 	for (auto &bp : blocks) {
 		const Block &b = *bp;
