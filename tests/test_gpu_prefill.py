@@ -140,7 +140,9 @@ def test_forward_batch_refuses_what_it_cannot_do():
 
 @pytest.mark.parametrize("hd,heads,kv,dim,rotary,clip,vocab,n,pos0", [
     (32, 8, 8, 256, 32, None, 1000, 129, 0), (64, 8, 2, 512, 32, 0.5, 516, 300, 40), (128, 8, 2, 1024, 128, None, 3000, 512, 7), (128, 4, 4, 1024, 64, 0.7, 132, 511, 1),
-    (64, 4, 1, 1024, 64, None, 20000, 260, 100)])
+    (64, 4, 1, 1024, 64, None, 20000, 260, 100),
+    # K in two parts (dim 2048 and more, few columns), a last half tile that is empty, or has some rows
+    (64, 4, 1, 2048, 64, None, 516, 260, 40), (64, 4, 1, 2048, 32, 0.5, 516, 511, 3), (128, 4, 2, 4096, 64, 0.7, 132, 300, 5), (32, 8, 8, 4096, 32, None, 516, 129, 0)])
 def test_forward_batch_of_many_rows_matches_few(hd, heads, kv, dim, rotary, clip, vocab, n, pos0):
     """A portion of more than 128 rows, whose products rotate, append and score in their own kernels, against the same positions in portions of 100, which
     leave that to kernels of their own: keys and values in fp16 to a unit (2^-10) or the layer's rounding, probabilities to what a unit in 16-bit operands makes of

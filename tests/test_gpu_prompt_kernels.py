@@ -201,7 +201,9 @@ def test_attention_not_finite_in_one_part(n, pos0, at, bad, bf16):
 @pytest.mark.parametrize("n,pos0,H,G,Gv,window,pool,ring", [
     (32, 0, 8, 2, 2, 128, 64, 640), (512, 3584, 16, 4, 4, 1024, 64, 1536), (100, 777, 8, 2, 1, 500, 64, 1012), (257, 5000, 8, 8, 4, 300, 1, 557),
     (300, 4000, 8, 2, 2, 128, 8, 700), (40, 9000, 16, 4, 4, 130, 16, 170), (64, 300, 6, 2, 2, 0, 0, 400), (90, 1000, 4, 4, 4, 200, 0, 289),
-    (33, 2000, 8, 2, 2, 1500, 64, 2100)])
+    (33, 2000, 8, 2, 2, 1500, 64, 2100),
+    # a tile a CTA while these all run at once, two a CTA beyond: 80, 148, 152 (kv heads of a tile and a half each), 200, 256 tiles of 128 rows
+    (300, 600, 32, 8, 8, 128, 64, 640), (460, 0, 37, 37, 37, 200, 0, 500), (190, 333, 76, 76, 19, 300, 64, 900), (513, 100, 40, 40, 40, 130, 16, 700), (512, 700, 64, 8, 8, 300, 64, 1000)])
 def test_window_attention_tiles(n, pos0, H, G, Gv, window, pool, ring, dk, dv):
     """Windows that wrap in the ring, rings that are no multiple of a tile, keys in as many parts as there are, pooled blocks in one tile and in many (as blocks of one
     position too), value heads that several key heads share, sinks, a scale of either sign, positions from a control block.  Slots that
