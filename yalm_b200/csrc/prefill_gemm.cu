@@ -90,8 +90,8 @@ struct WeightMaps {
 // ---- tails ------------------------------------------------------------------------------------------------------------
 constexpr int kPatch = 32 * 36 * 4; // bytes of one warp's staging patch: 32 rows of 32 fp32, padded to 36
 
-// What store_patch_f32 adds to a warp's 32 rows x 32 columns, read a step ahead of it (behind the products every step waited for its own: 512 x 4096 x 14336
-// 63.5 -> 62.7 us, 4096 x 4096 21.1 -> 19.7, 8192 x 2048 23.2 -> 20.9)
+// What store_patch_f32 adds to a warp's 32 rows x 32 columns, read a step ahead of it (behind the products every step waited for its own: 512 x 4096 x 4096
+// 19.8 -> 18.7 us, 6144 x 4096 28.7 -> 26.6, 4096 x 14336 53.6 -> 52.6, in a loop, under the power limit, within its noise)
 __device__ __forceinline__ void load_residual(const GemmArgs &g, float4 (&x)[8], int row0, int col, int col_end) {
 	const int lane = threadIdx.x & 31, r0 = lane >> 3, c0 = col + (lane & 7) * 4;
 	const float *base = g.c + (size_t)(row0 + r0) * g.ldc + c0;

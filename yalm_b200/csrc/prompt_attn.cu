@@ -17,12 +17,17 @@
 // zero times whatever lies there must be zero).
 //
 // Bound by the chain softmax - products of a tile pair (some 3500 cycles per 128 keys: 1800 from scores to weights, of which the exponentials
-// alone take 1024 at 16 a cycle and SM for each of the two tiles, 500 for the rescaling where the softmax warps do it, and 1100 for P V and the next scores), in a loop by
-// power (1000 W at 1640 MHz for the late portion) and, for short
-// contexts, by launch, query staging and the store.  Back to back, against 64-row tiles on mma.sync: 507 rows at 7680 positions, 32 / 8 heads of 128:
+// alone take 1024 at 16 a cycle and SM for each of the two tiles, 500 for the rescaling where the softmax warps do it, and 1100 for P V and the next scores: the late portion by
+// itself takes 72.0 us at 1720 MHz, the tensor pipe active 58 % and the unit of the exponentials 58 % of the time; in a loop, at 1000 W, 74.6), for short
+// contexts by launch, query staging and the store.  Back to back, against 64-row tiles on mma.sync: 507 rows at 7680 positions, 32 / 8 heads of 128:
 // 667 -> 74 us (890 TFLOP/s; 66 in the first passes); 512 rows at 0: 32.8 -> 8.9 us; bf16 window 1024 and pooled blocks of 64, 512 rows, 16 / 4 heads: 57.3 -> 14.5 us.
-// Of these SPLIT, with the queries of fp16 calls as boxes of a tensor map, made 80.5 to 78.4, 14.1 to 8.9 and 22.7 to 14.5: in pairs of tiles whose keys two CTAs
-// share, staging took 2 us, and sending half of the accumulators (64 KB, some 20 bytes a cycle), both cluster barriers and the join 4 us.
+// Of these SPLIT, with the queries of fp16 calls as boxes of a tensor map, made 80.5 to 78.4, 14.1 to 9.7 and 22.7 to 15.5: in pairs of tiles whose keys two CTAs
+// share, staging took 2 us, and sending half of the accumulators (64 KB, some 20 bytes a cycle), both cluster barriers and the join 4 us.  (The even and the odd tiles'
+// 16-bit weights are then rounded against a maximum each: results differ from those of one maximum by 3e-4, over bf16 1.3e-3, and are as far from 64 bits.)
+//
+// Weights are ex2.approx of score x c - maximum x c in one FMA, c = log2(e) scale rounded: an error that grows with the scores' size, 2^-24 of it, far below the 2^-9 or
+// 2^-11 that the weights are rounded to behind it.  Registers: 168 a thread beside 128 scores; the forms for layered models spill 16 to 56
+// bytes of them, the others 8 to 36 (with two tiles a CTA throughout it was 4 to 60), those that rescale in warps of their own none.
 #include "common.cuh"
 #include "launch.h"
 #include "stack_rows.cuh"
@@ -944,11 +949,11 @@ static int clusters_at_once(int (&room)[4]) {
 // once, at least four key tiles in all and more tiles than parts (17 rows, 32 / 8 heads of 128: three key tiles in one part 7.8 us, in two 8.4; five in two 9.7, in
 // four 9.2; nine, 128 rows of 8 / 2 heads, in four 10.9, in eight 9.9).  Every part finishes 8 columns at least: 33 rows at 7680, 16 / 8 heads of 32: 29.2 us in two parts, 17.5 in four;
 // 12 / 4 of 64: 19.5 in four, 13.5 in eight.  est_tiles: key tiles of the longest rows.
-// fp16 results of more tiles than leave two parts a place leave through the copy engine (512 rows at 0, 32 / 8 heads of 128: 9.7 -> 8.9 us; 64 / 8: 14.5 -> 13.8);
+// fp16 results of more tiles than leave two parts a place leave through the copy engine (512 rows at 0, 32 / 8 heads of 128: 9.7 -> 8.9 us; 64 / 8, in pairs: 14.2 -> 13.4);
 // a store of few CTAs is there as soon from their threads.
-// Those calls leave the rescaling to warps of their own: pairs of tiles always (64 / 8 heads of 128, 507 rows at 7680, in a loop: 147 -> 140 us; 512 at 0 14.5 -> 13.8),
-// single ones from kManyTiles key tiles on (32 / 8 heads at 7680: 79.7 -> 74.0 us, of 64 63.8 -> 54.6; at 2048, 20 key tiles, 26.1 on both; at 0 9.0 against 9.6 at 16 / 4
-// heads: what a round hands over costs more than it hides in few of them).
+// Those calls leave the rescaling to warps of their own: pairs of tiles always (64 / 8 heads of 128, 512 rows at 0 13.4 -> 12.7 us, at 1536 37.7 -> 34.4, 507 at 7680 143 -> 130; of 64
+// 11.2 -> 10.8, 33.5 -> 30.9, 120 -> 107), single ones from kManyTiles key tiles on (32 / 8 heads at 7680: 79.7 -> 74.0 us, of 64 63.8 -> 54.6; at 2048, 20 key tiles, 26.1 on
+// both; at 0 9.0 against 9.6 at 16 / 4 heads: what a round hands over costs more than it hides in few of them).
 constexpr int kManyTiles = 32;
 template <typename T, int DK, int DV, bool LAYERED>
 static int launch(Args &a, const void *keys, const void *values, int map_rows, int est_tiles, cudaStream_t st) {
