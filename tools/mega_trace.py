@@ -2,7 +2,7 @@
 """Offline analysis of decode_mega_kernel's event trace (CTA 0; library built with -DYALM_MEGA_TRACE, file written by
 tools/mega_profile.py under YALM_MEGA_TRACE=<file>): per phase of one layer, how long tiles take to arrive, how long the
 owning warp lets a landed tile wait, how long it works on it, and what the warps do between tiles.
-    python tools/mega_trace.py gpurun_out/trace.bin [--layer L] [--mhz 1965]"""
+    python tools/mega_trace.py trace.bin [--layer L] [--mhz 1965]"""
 import argparse
 import sys
 
