@@ -537,6 +537,8 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ 
 	// 17 x 4096 x 4096).  With the exchange's own space: 9.4 -> 8.8 us, 128 rows 15.8 -> 13.2, 100 x 6144 x 4096 20.8 -> 17.9, 17 x 1024 x 1024 4.5 -> 4.1
 	constexpr int kBatch = ADD ? 4 : 1;
 	const int col = n0 + row; // lanes are neighbouring output columns
+	// (ADD says as much; without the tail asked again the compiler's order of this costs 0.3 to 2 %, 1 x 1024 x 1024 3.46 -> 3.53 us)
+	const bool add = ADD && g.tail == kAddF32 && col < n_end;
 	float x[kBatch][ADD ? 8 : 1];
 	auto fetch = [&](int first) {
 		if constexpr (ADD) {
@@ -545,7 +547,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ 
 #pragma unroll
 				for (int i = 0; i < 8; ++i) {
 					const int r = (first + b * g.splits) * 8 + i;
-					x[b][i] = col < n_end && r < g.M ? g.c[(size_t)r * g.ldc + col] : 0.f;
+					x[b][i] = add && r < g.M ? g.c[(size_t)r * g.ldc + col] : 0.f;
 				}
 		}
 	};
